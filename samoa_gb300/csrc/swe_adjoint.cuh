@@ -33,15 +33,16 @@ struct Grad4 {
 // bathymetries, velocities, delphi, the Einfeldt speeds and sqrt(g h)).
 
 // d sqrt(x) / dx times b (0 where the root is 0, as the reference gradient has it)
-__device__ __forceinline__ double dsqrt(double root, double b) { return gt0(root) ? b * 0.5 / root : 0.0; }
+__device__ __forceinline__ double dsqrt(double root, double b) { return gt0(root) ? div_one(b * 0.5, root) : 0.0; }
 
 // Cotangents of riemanntype's inputs.
 struct RsCot {
     double hL, hR, uL, uR, sqL, sqR;
 };
-// a / b for cotangents: the reciprocal to about one ulp (rcp_nr) for a normal divisor, else IEEE
+// a / b for cotangents: the reciprocal to about half an ulp in recip_fix's range, else IEEE
 __device__ __forceinline__ double cdiv(double a, double b) {
-    return exp_in(b, -1000, 1000) ? a * rcp_nr(b) : a / b;
+    const u64 y = recip_fix(b);
+    return y ? a * recip_near(b, y) : a / b;
 }
 
 __device__ __forceinline__ void rs_rev(const AugRec& r, double hL, double hR, double uL, double uR, double sqL,
@@ -60,7 +61,7 @@ __device__ __forceinline__ void rs_rev(const AugRec& r, double hL, double hR, do
     if (r.rs == 1) {  // two rarefactions
         const double t = r.t_pos ? -delu + 2.0 * (sqL + sqR) : 0.0;
         const double hm = (1.0 / (16.0 * g)) * (t * t);
-        const double sqm = sqrt(g * hm);
+        const double sqm = sqrt_fix(g * hm);
         c.uL += b1;
         c.sqL += 2.0 * b1;
         c.uR += b2;
@@ -76,17 +77,17 @@ __device__ __forceinline__ void rs_rev(const AugRec& r, double hL, double hR, do
     } else if (r.rs == 2) {  // two shocks: one Newton step
         const double h0 = r.highR ? hR : hL;
         const double i0 = cdiv(1.0, h0), iL = cdiv(1.0, hL), iR = cdiv(1.0, hR);
-        const double gL = sqrt((0.5 * g) * (i0 + iL)), gR = sqrt((0.5 * g) * (i0 + iR));
+        const double gL = sqrt_fix((0.5 * g) * (i0 + iL)), gR = sqrt_fix((0.5 * g) * (i0 + iR));
         const double F0 = (delu + (h0 - hL) * gL) + (h0 - hR) * gR;
         const double kk = 4.0 * (h0 * h0);
         const double eL = cdiv((g * (h0 - hL)), (kk * gL)), eR = cdiv((g * (h0 - hR)), (kk * gR));
         const double dfdh = ((gL - eL) + gR) - eR;
-        const double sq0 = sqrt(h0);
+        const double sq0 = sqrt_fix(h0);
         const double slope = 2.0 * sq0 * dfdh;
         const double tt = sq0 - cdiv(F0, slope);
         const double hm = tt * tt, im = cdiv(1.0, hm);
-        const double cL = sqrt((0.5 * g) * (im + iL)), cR = sqrt((0.5 * g) * (im + iR));
-        const double sqm = sqrt(g * hm);
+        const double cL = sqrt_fix((0.5 * g) * (im + iL)), cR = sqrt_fix((0.5 * g) * (im + iR));
+        const double sqm = sqrt_fix(g * hm);
         // s1m = u1m - sqm, s2m = u2m + sqm
         double b_hm = dsqrt(sqm, (b2 - b1) * g);
         // u2m = uR + (hm - hR) cR, u1m = uL - (hm - hL) cL
@@ -155,12 +156,12 @@ __device__ __forceinline__ void rs_rev(const AugRec& r, double hL, double hR, do
         const double sqmn = r.lowR ? sqR : sqL, sqmx = r.highR ? sqR : sqL;
         const double F0 = delu + 2.0 * (sqmn - sqmx);
         const double P = cdiv(((0.5 * g) * (hmx + hmn)), (hmx * hmn));
-        const double W = sqrt(P);
+        const double W = sqrt_fix(P);
         const double Fmax = delu + (hmx - hmn) * W;
         const double den = hmx - hmn;
         const double slope = cdiv((Fmax - F0), den);
         const double hm = hmn - cdiv(F0, slope);
-        const double sqm = sqrt(g * hm);
+        const double sqm = sqrt_fix(g * hm);
         double b_sqm;
         if (r.lhigh) {
             const double bb = b1 + b2;
@@ -399,7 +400,7 @@ __device__ __forceinline__ void aug_rev(const AugRec& r, const double F[3][3], d
 // handling, Einfeldt speeds and net-update split of c_bind_geoclaw_solver_dp).
 template <int SOLVER>
 __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& QL, const State& QR, double dL0,
-                                            double dR0, double sqL0, double sqR0, double yL0, double yR0,
+                                            double dR0, double sqL0, double sqR0, u64 yL0, u64 yR0,
                                             double drytol, const double gL[3], const double gR[3], Grad4& outL,
                                             Grad4& outR, int axis = 0) {
     const double g = kG;
@@ -422,9 +423,9 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
         if (still && lt(drytol, dL0) && lt(drytol, dR0) && dbits((QR.b + dR0) - QL.b) == dbits(dL0) &&
             is_finite(dL0)) {
             const double ghalf = c * (dR0 + dL0);
-            const double chat = sqrt(ghalf);
+            const double chat = sqrt_fix(ghalf);
             const double sE1 = -imax(sqL0, chat), sE2 = imax(sqR0, chat);
-            const double rD = rcp_nr(sE2 - sE1);
+            const double rD = rcp_near(sE2 - sE1);
             // n . (g1, g2) of each side's cotangent: a signed component for the
             // axis-aligned normals (1, 0) and (0, 1) up to sign, whose other
             // component is a zero; the cotangents need no bit-exact rounding, so
@@ -490,16 +491,16 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
     if (!wetL && !wetR && !is_nan(hL) && !is_nan(hR)) return;  // no flux, no derivative
     double huL, huR, uL, uR, vL, vR;
     // a wet cell whose reciprocal was left for the edges that need it (f-wave, zero momenta)
-    if (SOLVER == FWAVE && wetR && dbits(yR0) == 0) yR0 = recip_rn(hR).y;
-    if (SOLVER == FWAVE && wetL && dbits(yL0) == 0) yL0 = recip_rn(hL).y;
+    if (SOLVER == FWAVE && wetR && yR0 == 0) yR0 = recip_fix(hR);
+    if (SOLVER == FWAVE && wetL && yL0 == 0) yL0 = recip_fix(hL);
     if (wetR) {
-        const Recip r{hR, yR0, recip_fast(hR)};
+        const Recip r{hR, yR0};
         huR = pR1; uR = div_rn(pR1, r); vR = div_rn(pR2, r);
     } else {
         hR = 0.0; huR = 0.0; uR = 0.0; vR = 0.0;
     }
     if (wetL) {
-        const Recip r{hL, yL0, recip_fast(hL)};
+        const Recip r{hL, yL0};
         huL = pL1; uL = div_rn(pL1, r); vL = div_rn(pL2, r);
     } else {
         hL = 0.0; huL = 0.0; uL = 0.0; vL = 0.0;
@@ -533,9 +534,9 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
     const double sqR = (wetR || wall_r) ? (wall_r ? sqL0 : sqR0) : 0.0;
     const double sL = uL - sqL, sR = uR + sqR;
     const double A = sqL * uL + sqR * uR, B = sqR + sqL;
-    const Recip rB = recip_rn(B);
-    const double uhat = div_rn(A, rB);
-    const double chat = sqrt((g * 0.5) * Hs);
+    const Recip rB = recip_of(B);
+    const double uhat = div_rn(A, rB), yB = recip_near(B, rB.y);
+    const double chat = sqrt_fix((g * 0.5) * Hs);
     const double r1 = uhat - chat, r2 = uhat + chat;
     const bool e1_is_sL = lt(sL, r1), e2_is_sR = lt(r2, sR);
     const double sE1 = e1_is_sL ? sL : r1, sE2 = e2_is_sR ? sR : r2;
@@ -543,24 +544,24 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
     const double delhu = huR - huL;
     const double K = (g * 0.5) * Hs;
     double beta1 = 0.0, beta2 = 0.0, sw[3];
-    Recip rD{1.0, 1.0, false};
+    double yD = 0.0;  // 1 / D
     AugRec rec{};
     if (SOLVER == FWAVE) {
         const double ddp = -(K * dB);
         const double dpd = delphi - ddp;
         const double D = sE2 - sE1;
-        rD = recip_rn(D);
+        const Recip rD = recip_of(D);
+        yD = recip_near(D, rD.y);
         beta1 = div_rn(sE2 * delhu - dpd, rD);
         beta2 = div_rn(dpd - sE1 * delhu, rD);
         sw[0] = sE1;
         sw[1] = 0.5 * (sE1 + sE2);
         sw[2] = sE2;
     } else {  // the same call as geoclaw_solver's, recording the branch decisions
-        const double yLf = wall_l ? yR0 : yL0, yRf = wall_r ? yL0 : yR0;
-        const bool okL = (wetL || wall_l) && recip_fast(hL), okR = (wetR || wall_r) && recip_fast(hR);
+        const u64 yLf = wall_l ? yR0 : yL0, yRf = wall_r ? yL0 : yR0;
         double fwa[3][3];
-        riemann_aug_rec<true>(hL, hR, huL, huR, bL, bR, uL, uR, vL, vR, delphi, sE1, sE2, sqL, sqR, yLf, yRf, okL,
-                              okR, drytol, sw, fwa, &rec);
+        riemann_aug_rec<true>(hL, hR, huL, huR, bL, bR, uL, uR, vL, vR, delphi, sE1, sE2, sqL, sqR, yLf, yRf,
+                              drytol, sw, fwa, &rec);
     }
     // ---------------- reverse (cotangents: products fused into FMAs where they feed a sum; they
     // need no bit-exact agreement, only the forward recompute above does)
@@ -608,8 +609,8 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
         b_vL = fma(F30, beta1, b_vL);
         b_vR = fma(F32, beta2, b_vR);
         // beta1 = (sE2 delhu - dpd) / D, beta2 = (dpd - sE1 delhu) / D, D = sE2 - sE1
-        const double N1b = b_beta1 * rD.y, N2b = b_beta2 * rD.y;
-        const double b_D = -fma(b_beta1, beta1, b_beta2 * beta2) * rD.y;
+        const double N1b = b_beta1 * yD, N2b = b_beta2 * yD;
+        const double b_D = -fma(b_beta1, beta1, b_beta2 * beta2) * yD;
         b_sE2 += fma(N1b, delhu, b_D);
         b_sE1 -= fma(N2b, delhu, b_D);
         double b_delhu = fma(N1b, sE2, -(N2b * sE1));
@@ -649,10 +650,10 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
     double b_sR = e2_is_sR ? b_sE2 : 0.0, b_r2 = e2_is_sR ? 0.0 : b_sE2;
     const double b_uhat = b_r1 + b_r2;
     const double b_chat = b_r2 - b_r1;
-    if (chat > 0.0) b_Hs = fma(b_chat * (0.5 * rcp_nr(chat)), g * 0.5, b_Hs);
+    if (chat > 0.0) b_Hs = fma(b_chat * (0.5 * rcp_near(chat)), g * 0.5, b_Hs);
     double b_uL = b_sL + k_uL, b_uR = b_sR + k_uR;
     double b_sqL = k_sqL - b_sL, b_sqR = b_sR + k_sqR;
-    const double b_A = b_uhat * rB.y, b_B = -b_uhat * uhat * rB.y;
+    const double b_A = b_uhat * yB, b_B = -b_uhat * uhat * yB;
     b_sqL += fma(b_A, uL, b_B);
     b_sqR += fma(b_A, uR, b_B);
     b_uL = fma(b_A, sqL, b_uL);
@@ -680,8 +681,8 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
         b_bR += b_dB;
         b_bL -= b_dB;
         // sqrt(g h) of the fixed-up depths
-        if (sqL > 0.0) b_hL = fma(b_sqL, 0.5 * g * rcp_nr(sqL), b_hL);
-        if (sqR > 0.0) b_hR = fma(b_sqR, 0.5 * g * rcp_nr(sqR), b_hR);
+        if (sqL > 0.0) b_hL = fma(b_sqL, 0.5 * g * rcp_near(sqL), b_hL);
+        if (sqR > 0.0) b_hR = fma(b_sqR, 0.5 * g * rcp_near(sqR), b_hR);
         // undo the wall / lowering fix-ups: map the cotangents back to the original sides
         double b_hL0 = 0.0, b_hR0 = 0.0, b_bL0 = 0.0, b_bR0 = 0.0;
         if (wall_r) {  // hR = hL, huR = -huL, bR = bL, uR = -uL, vR = vL
@@ -711,14 +712,16 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
         // wet extraction: u = hu / h, v = hv / h on wet sides; dry sides are constants
         double b_pL1 = 0.0, b_pL2 = 0.0, b_pR1 = 0.0, b_pR2 = 0.0;
         if (wetR) {
-            b_pR1 += fma(b_uR, yR0, b_huR);
-            b_pR2 = fma(b_vR, yR0, b_pR2);
-            b_hR0 = fma(-fma(b_uR, uR, b_vR * vR), yR0, b_hR);
+            const double iR = recip_near(hR, yR0);
+            b_pR1 += fma(b_uR, iR, b_huR);
+            b_pR2 = fma(b_vR, iR, b_pR2);
+            b_hR0 = fma(-fma(b_uR, uR, b_vR * vR), iR, b_hR);
         }
         if (wetL) {
-            b_pL1 += fma(b_uL, yL0, b_huL);
-            b_pL2 = fma(b_vL, yL0, b_pL2);
-            b_hL0 = fma(-fma(b_uL, uL, b_vL * vL), yL0, b_hL);
+            const double iL = recip_near(hL, yL0);
+            b_pL1 += fma(b_uL, iL, b_huL);
+            b_pL2 = fma(b_vL, iL, b_pL2);
+            b_hL0 = fma(-fma(b_uL, uL, b_vL * vL), iL, b_hL);
         }
         // depths h - b, rotations p_edge = T p
         outL.h += b_hL0;
@@ -759,7 +762,7 @@ __device__ __forceinline__ void nv_vjp(double n1, double n2, double v, double d,
 
 // d sqrt(g h) / dh times bs (0 where h = 0, as the reference gradient has it)
 __device__ __forceinline__ double sqrt_g_vjp(double h, double bs) {
-    return gt0(h) ? cdiv(bs * (0.5 * kG), sqrt(kG * h)) : 0.0;
+    return gt0(h) ? cdiv(bs * (0.5 * kG), sqrt_fix(kG * h)) : 0.0;
 }
 
 template <int SOLVER>
@@ -779,8 +782,8 @@ __device__ __forceinline__ void lf_vjp(double n1, double n2, const State& QL, co
             const double* gg = right ? gR : gL;
             const double sgw = right ? -1.0 : 1.0;  // fR: -(0.5 v p) - pr n; fL: +(0.5 v p) + pr n
             const double hw = dmx(d, 0.0);
-            const double v = normal_velocity(n1, n2, Q.p1, Q.p2, d);
-            const double sp = sqrt(g * hw) + fabs(v);
+            const double v = normal_velocity(n1, n2, Q.p1, Q.p2, recip_of(d));
+            const double sp = sqrt_fix(g * hw) + fabs(v);
             double b_v = sgw * 0.5 * fma(gg[1], Q.p1, gg[2] * Q.p2);
             const double b_pr = sgw * fma(gg[1], n1, gg[2] * n2);
             const double b_sp = 0.5 * fma(gg[1], Q.p1, gg[2] * Q.p2);
@@ -798,9 +801,9 @@ __device__ __forceinline__ void lf_vjp(double n1, double n2, const State& QL, co
             return;
         }
         const double hL = dmx(dL, 0.0), hR = dmx(dR, 0.0);
-        const double vL = normal_velocity(n1, n2, QL.p1, QL.p2, dL);
-        const double vR = normal_velocity(n1, n2, QR.p1, QR.p2, dR);
-        const double sL = sqrt(g * hL) + fabs(vL), sR = sqrt(g * hR) + fabs(vR);
+        const double vL = normal_velocity(n1, n2, QL.p1, QL.p2, recip_of(dL));
+        const double vR = normal_velocity(n1, n2, QR.p1, QR.p2, recip_of(dR));
+        const double sL = sqrt_fix(g * hL) + fabs(vL), sR = sqrt_fix(g * hR) + fabs(vR);
         const bool left_max = sL > sR;
         const double alpha = (SOLVER == LLF_BATH) ? (left_max ? sL : sR) : 100.0;
         // fL = (F_h, F_p1 + src n1, F_p2 + src n2), fR = (-F_h, -F_p1 + src n1, -F_p2 + src n2)
@@ -844,9 +847,9 @@ __device__ __forceinline__ void lf_vjp(double n1, double n2, const State& QL, co
         // no bathymetry: depth = surface
         const double dL = QL.h - 0.0, dR = QR.h - 0.0;
         const double hL = dmx(dL, 0.0), hR = dmx(dR, 0.0);
-        const double vL = normal_velocity(n1, n2, QL.p1, QL.p2, dL);
-        const double vR = normal_velocity(n1, n2, QR.p1, QR.p2, dR);
-        const double sL = sqrt(g * dL) + fabs(vL), sR = sqrt(g * dR) + fabs(vR);
+        const double vL = normal_velocity(n1, n2, QL.p1, QL.p2, recip_of(dL));
+        const double vR = normal_velocity(n1, n2, QR.p1, QR.p2, recip_of(dR));
+        const double sL = sqrt_fix(g * dL) + fabs(vL), sR = sqrt_fix(g * dR) + fabs(vR);
         const bool left_max = sL > sR;
         const double alpha = (SOLVER == LLF) ? (left_max ? sL : sR) : 100.0;
         const double bFh = gL[0] - gR[0], bF1 = gL[1] - gR[1], bF2 = gL[2] - gR[2];
@@ -942,7 +945,7 @@ __device__ __forceinline__ void cell_mu(const AdjointArgs& A, int c, double ndv,
 // The edge VJP of the step's flux for each solver.
 template <int SOLVER>
 __device__ __forceinline__ void edge_vjp(double n1, double n2, const State& QL, const State& QR, double dL,
-                                         double dR, double sqL, double sqR, double yL, double yR, double drytol,
+                                         double dR, double sqL, double sqR, u64 yL, u64 yR, double drytol,
                                          const double gL[3], const double gR[3], Grad4& oL, Grad4& oR, int axis) {
     if (SOLVER == FWAVE || SOLVER == AUG_RIEMANN)
         geoclaw_vjp<SOLVER>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, gL, gR, oL, oR, axis);
@@ -967,8 +970,8 @@ __global__ void SWE_ADJ_BOUNDS adjoint_kernel(const AdjointArgs A) {
     double* sh_hu = sh_h + T;
     double* sh_hv = sh_hu + T;
     double* sh_b = sh_hv + T;
-    double* sh_rh = sh_b + T;          // RN(1 / depth) where wet
-    double* sh_sq = sh_rh + T;
+    u64* sh_rh = reinterpret_cast<u64*>(sh_b + T);  // recip_fix(depth) where wet
+    double* sh_sq = reinterpret_cast<double*>(sh_rh + T);
     double* sh_mu = sh_sq + T;         // [3][T]
     double* slot = sh_mu + 3 * T;      // [4 quantities][3 local edges][T]
     const InstParams& P = A.P;
@@ -1009,7 +1012,7 @@ __global__ void SWE_ADJ_BOUNDS adjoint_kernel(const AdjointArgs A) {
             // sqrt(g d) from the step's memo when the depth has the same bits (a
             // pair (d, sqrt(g d)) either way, so a hit is the root's value; a miss
             // is written back by this CTA, which owns the cell). The f-wave's
-            // RN(1 / d) is left to the VJP of an edge that takes the general path
+            // reciprocal is left to the VJP of an edge that takes the general path
             // (0 here) when the cell's momenta are +-0, since its edges may all be
             // at rest; a cell with momentum has general edges and gets it here.
             const double d = h - b;
@@ -1024,11 +1027,11 @@ __global__ void SWE_ADJ_BOUNDS adjoint_kernel(const AdjointArgs A) {
                 }
             }
             if (miss) {
-                sq = sqrt(kG * d);
+                sq = sqrt_fix(kG * d);
                 if (A.memo) A.memo[cc] = make_double2(d, sq);
             }
             const bool still = ((dbits(sh_hu[i]) | dbits(sh_hv[i])) << 1) == 0;
-            sh_rh[i] = (wet && (SOLVER != FWAVE || !still)) ? recip_rn(d).y : 0.0;
+            sh_rh[i] = (wet && (SOLVER != FWAVE || !still)) ? recip_fix(d) : 0;
             sh_sq[i] = sq;
             const int dd = A.depth[cc];
             double m0, m1, m2;
@@ -1063,7 +1066,8 @@ __global__ void SWE_ADJ_BOUNDS adjoint_kernel(const AdjointArgs A) {
             const bool lin = (unsigned)sl < (unsigned)cn;
             const bool rin = !bnd && (unsigned)sr < (unsigned)cn;
             State QL, QR;
-            double dL, dR, sqL, sqR, yL, yR, mL[3], mR[3] = {0.0, 0.0, 0.0};
+            double dL, dR, sqL, sqR, mL[3], mR[3] = {0.0, 0.0, 0.0};
+            u64 yL, yR;
             int depL, depR = 0;
             if (lin) {
                 QL = State{sh_h[sl], sh_hu[sl], sh_hv[sl], sh_b[sl]};

@@ -215,15 +215,15 @@ __device__ __forceinline__ void flush_instance(const StepArgs& A, int inst, doub
 // parity, pre-update states), both sides' updates stored by cell (a, then b).
 // depth_terms for the cross-edge pass: sqrt(g d) from the memo when the depth has
 // the same bits (the pass only reads it; the step kernel's owner CTAs write it),
-// and, for the f-wave, no RN(1 / d) for a cell with both momenta +-0 (its
-// quotients are zeros with the numerator's sign for any positive reciprocal).
+// and, for the f-wave, no reciprocal for a cell with both momenta +-0 (its
+// quotients are zeros with the numerator's sign, which need none).
 template <int SOLVER>
 __device__ __forceinline__ void cross_depth_terms(const StepArgs& A, int c, const State& Q, double drytol, double& d,
-                                                  double& sq, double& y) {
+                                                  double& sq, u64& y) {
     d = Q.h - Q.b;
     const bool wet = lt(drytol, d);
     sq = 0.0;
-    y = 0.0;
+    y = 0;
     if (!wet) return;
     bool hit = false;
     if (A.memo) {
@@ -233,9 +233,9 @@ __device__ __forceinline__ void cross_depth_terms(const StepArgs& A, int c, cons
             hit = true;
         }
     }
-    if (!hit) sq = sqrt(kG * d);
+    if (!hit) sq = sqrt_fix(kG * d);
     const bool still = ((dbits(Q.p1) | dbits(Q.p2)) << 1) == 0;
-    y = (SOLVER == FWAVE && still) ? 1.0 : recip_rn(d).y;
+    y = (SOLVER == FWAVE && still) ? 0 : recip_fix(d);
 }
 
 template <int SOLVER, int FZ = 0>
@@ -267,7 +267,8 @@ __global__ void __launch_bounds__(256) cross_edges_kernel(const StepArgs A) {
     const double n1 = c_normal[pL][iL][0], n2 = c_normal[pL][iL][1];
     const State QL{hin[L], huin[L], hvin[L], A.b[L]};
     const State QR{hin[R], huin[R], hvin[R], A.b[R]};
-    double dL, dR, sqL, sqR, yL, yR;
+    double dL, dR, sqL, sqR;
+    u64 yL, yR;
     cross_depth_terms<SOLVER>(A, L, QL, drytol, dL, sqL, yL);
     cross_depth_terms<SOLVER>(A, R, QR, drytol, dR, sqR, yR);
     Update fL, fR;
@@ -327,8 +328,8 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
     // segment's bulk copies land in one buffer while the CTA works on the other
     const bool depth2 = A.stage_depth > 1;
     double* stage = reinterpret_cast<double*>(smem_raw);
-    double* sh_rh = stage + (depth2 ? 8 : 4) * T;  // RN(1 / depth) where the cell is wet
-    double* sh_sq = sh_rh + T;      // sqrt(g * depth) where the cell is wet
+    u64* sh_rh = reinterpret_cast<u64*>(stage + (depth2 ? 8 : 4) * T);  // recip_fix(depth) where the cell is wet
+    double* sh_sq = reinterpret_cast<double*>(sh_rh + T);      // sqrt(g * depth) where the cell is wet
     double* upd = sh_sq + T;        // [4 quantities][3 local edges][T cells]
     double* tab_leg = upd + 12 * T; // per depth of the current instance
     double* tab_hyp = tab_leg + A.max_ndepth;
@@ -483,7 +484,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
             // depth_terms, with the square root and reciprocal skipped by warps of dry cells.
             // The f-wave path divides only the cell's own (rotated) momenta by its depth:
             // with both momenta +-0 every such quotient is a zero with the numerator's
-            // sign for any positive reciprocal, so those cells skip RN(1 / d) (1.0 stands in)
+            // sign, so those cells skip the reciprocal
             // sqrt(g d) comes from the memo when the cell's depth has the same bits as
             // the depth it was last taken for (water at rest keeps its depth from step
             // to step); the memo holds only pairs (d, sqrt(g d)), written by the CTA
@@ -491,7 +492,8 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
             const double d = sh_h[i] - sh_b[i];
             const bool wet = lt(P.drytol, d);
             const bool need_y = wet && (SOLVER != FWAVE || ((dbits(sh_hu[i]) | dbits(sh_hv[i])) << 1) != 0);
-            double sq = 0.0, y = wet ? 1.0 : 0.0;
+            double sq = 0.0;
+            u64 y = 0;
             bool miss = wet;
             if (wet && A.memo) {
                 const double2 m = A.memo[c0 + i];
@@ -502,11 +504,11 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
             }
             if (__any_sync(__activemask(), miss)) {
                 if (miss) {
-                    sq = sqrt(kG * d);
+                    sq = sqrt_fix(kG * d);
                     if (A.memo) A.memo[c0 + i] = make_double2(d, sq);
                 }
             }
-            if (__any_sync(__activemask(), need_y)) y = need_y ? recip_rn(d).y : y;
+            if (__any_sync(__activemask(), need_y)) y = need_y ? recip_fix(d) : y;
             sh_rh[i] = y;
             sh_sq[i] = sq;
         }
@@ -562,7 +564,8 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
             const bool lin = (unsigned)sl < (unsigned)cn;
             const bool rin = !bnd && (unsigned)sr < (unsigned)cn;
             State QL, QR;
-            double dL, dR, sqL, sqR, yL, yR;
+            double dL, dR, sqL, sqR;
+            u64 yL, yR;
             if (lin) {
                 QL = State{sh_h[sl], sh_hu[sl], sh_hv[sl], sh_b[sl]};
                 dL = QL.h - QL.b;

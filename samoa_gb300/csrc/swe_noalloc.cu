@@ -126,7 +126,8 @@ __global__ void edges_kernel(Args A, unsigned char* scratch) {
         } else {
             QR = load(A, R);
         }
-        double dL, dR, sqL, sqR, yL, yR;
+        double dL, dR, sqL, sqR;
+        u64 yL, yR;
         depth_terms(QL, A.drytol, dL, sqL, yL);
         depth_terms(QR, A.drytol, dR, sqR, yR);
         Update fL, fR;

@@ -18,8 +18,11 @@ namespace swe {}
 
 #include <stdint.h>
 
+#include "swe_exact.cuh"
+
 namespace SWE_KNS {
 using namespace ::swe;
+using namespace ::swe_exact;
 
 constexpr double kG = 9.80665;  // src/SWE/SWE_data_types.f90:34
 
@@ -122,80 +125,18 @@ __device__ __forceinline__ double scale_pow2(double x, int k, double p) {
 }
 
 // ---------------------------------------------------------------------------
-// Correctly rounded division with a shared reciprocal.
 // Several quotients in the step share a divisor (a cell's depth divides its
 // edges' normal and tangential momenta; the two f-wave coefficients share
-// s2 - s1). recip_rn computes y = RN(1/b) once: two Newton-Raphson steps from
-// the hardware approximation bring y within one ulp of 1/b, and a third step
-// with an exact residual e = 1 - b y rounds it correctly unless b's significand
-// is all ones (Markstein's reciprocal theorem). div_rn then gets RN(a/b) from y:
-// q0 = RN(a y) is within 1.5 ulp of a/b, one correction q1 = RN(q0 + (a - b q0) y)
-// brings it well inside one ulp, and a second correction is Markstein's
-// division theorem: if y = RN(1/b) and q is within one ulp of a/b, then
-// r = a - b q is exact and RN(q + r y) = RN(a/b) (P. Markstein, IBM J. Res.
-// Dev. 34(1), 1990; M. Cornea-Hasegan, R. Golliver, P. Markstein, ARITH-14,
-// 1999). The exponents of a and b are kept within [-500, 500], where no
-// intermediate result under- or overflows; outside that range, for a zero
-// divisor and for the all-ones significand, plain IEEE division is used. All
-// tests are integer operations, so the FP64 pipe only sees the arithmetic.
-// swe_division_check compares the results with IEEE division on the device.
-__device__ __forceinline__ double rcp_approx(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    return y;
-}
-
+// s2 - s1): the divisor with its reciprocal (recip_fix; 0 where it is left out or
+// out of range, and div_fix then takes the IEEE division).
 struct Recip {
-    double b, y;
-    bool fast;
+    double b;
+    u64 y;
 };
-
-// 1/b to about one ulp (two Newton-Raphson steps from the hardware
-// approximation), for cotangents, which need no correct rounding; b must be
-// a normal number.
-__device__ __forceinline__ double rcp_nr(double b) {
-    double y = rcp_approx(b);
-    double e = fma(-b, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-b, y, 1.0);
-    return fma(y, e, y);
-}
-
-__device__ __forceinline__ bool exp_in(double x, int lo, int hi) {
-    const int e = (int)((dbits(x) >> 52) & 0x7ff) - 1023;
-    return e >= lo && e <= hi;
-}
-
-__device__ __forceinline__ bool recip_fast(double b) {
-    const long long bits = dbits(b);
-    return exp_in(b, -500, 500) && ((bits & 0x000fffffffffffffLL) != 0x000fffffffffffffLL);
-}
-
-__device__ __forceinline__ Recip recip_rn(double b) {
-    Recip r;
-    r.b = b;
-    r.fast = recip_fast(b);
-    double y = rcp_approx(b);
-    double e = fma(-b, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-b, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-b, y, 1.0);
-    r.y = fma(y, e, y);
-    return r;
-}
-
-__device__ __forceinline__ double div_rn(double a, const Recip& r) {
-    if (!r.fast) return a / r.b;
-    if ((dbits(a) << 1) == 0) return a * r.y;  // +-0 with the IEEE sign
-    if (!exp_in(a, -500, 500)) return a / r.b;
-    double q = prod(a, r.y);
-    double res = fma(-r.b, q, a);
-    q = fma(res, r.y, q);
-    res = fma(-r.b, q, a);
-    return fma(res, r.y, q);
-}
-
+__device__ __forceinline__ Recip recip_of(double b) { return Recip{b, recip_fix(b)}; }
+__device__ __forceinline__ double div_rn(double a, const Recip& r) { return div_fix(a, r.b, r.y); }
+// 1 / b to about half an ulp, for cotangents, which need no correct rounding
+__device__ __forceinline__ double rcp_near(double b) { return recip_near(b, recip_fix(b)); }
 
 // Non-strict comparisons on the integer pipe with IEEE semantics (false if either is NaN).
 __device__ __forceinline__ bool le(double a, double b) {  // a <= b
@@ -203,9 +144,8 @@ __device__ __forceinline__ bool le(double a, double b) {  // a <= b
 }
 __device__ __forceinline__ double iabs(double x) { return bitsd(abs_bits(x)); }  // fabs
 
-// RN(1 / h) from a precomputed reciprocal y when it is known to be correctly
-// rounded (recip_rn's fast range), else the IEEE division.
-__device__ __forceinline__ double inv_of(double h, double y, bool y_ok) { return y_ok ? y : 1.0 / h; }
+// RN(1 / h) from y = recip_fix(h) (0: the IEEE division).
+__device__ __forceinline__ double inv_of(double h, u64 y) { return div_fix(1.0, h, y); }
 
 // The branch decisions of one augmented-solver evaluation, for its reverse
 // (the discrete adjoint re-evaluates the values; the decisions fix the branch).
@@ -223,12 +163,11 @@ struct AugRec {
 
 // Riemann structure with one Newton step, src/geoclaw/riemannsolvers.f:507-618.
 // sqL / sqR are sqrt(g * hL) and sqrt(g * hR) (the caller's, the same operands
-// and so the same bits as computing them here); yL / yR are RN(1 / hL) and
-// RN(1 / hR) where yL_ok / yR_ok, else the divisions are done here.
+// and so the same bits as computing them here); yL / yR are recip_fix of hL / hR
+// (0: the IEEE division).
 template <bool REC>
 __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, double uL, double uR, double drytol,
-                                                     double sqL, double sqR, double yL, double yR, bool yL_ok,
-                                                     bool yR_ok, double& hm, double& s1m, double& s2m,
+                                                     double sqL, double sqR, u64 yL, u64 yR, double& hm, double& s1m, double& s2m,
                                                      AugRec* rec) {
     const double g = kG;
     const bool r_lower = lt(hR, hL);  // h_min = dmn(hR, hL) is hR
@@ -250,7 +189,7 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
     }
     double F_min = delu + scale_pow2(sq_min - sq_max, 1, 2.0);
     double F_max = 0.0;  // needed only when F_min <= 0
-    if (!gt0(F_min)) F_max = delu + (h_max - h_min) * sqrt(((0.5 * g) * (h_max + h_min)) / (h_max * h_min));
+    if (!gt0(F_min)) F_max = delu + (h_max - h_min) * sqrt_fix(div_one((0.5 * g) * (h_max + h_min), h_max * h_min));
     if (gt0(F_min)) {  // two rarefactions
         const double t0 = -delu + scale_pow2(sqL + sqR, 1, 2.0);
         double t = imax(0.0, t0);
@@ -259,27 +198,27 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
             rec->t_pos = !lt(t0, 0.0);
         }
         hm = (1.0 / (16.0 * g)) * (t * t);
-        const double sqm = sqrt(g * hm);
+        const double sqm = sqrt_fix(g * hm);
         s1m = (uL + scale_pow2(sqL, 1, 2.0)) - 3.0 * sqm;
         s2m = (uR - scale_pow2(sqR, 1, 2.0)) + 3.0 * sqm;
     } else if (le(F_max, 0.0)) {  // two shocks: one Newton step on sqrt(h)
         if (REC) rec->rs = 2;
         double h0 = h_max;
-        const double i0 = r_higher ? inv_of(hR, yR, yR_ok) : inv_of(hL, yL, yL_ok);
-        const double iL = inv_of(hL, yL, yL_ok), iR = inv_of(hR, yR, yR_ok);
-        double gL = sqrt((0.5 * g) * (i0 + iL));
-        double gR = sqrt((0.5 * g) * (i0 + iR));
+        const double i0 = r_higher ? inv_of(hR, yR) : inv_of(hL, yL);
+        const double iL = inv_of(hL, yL), iR = inv_of(hR, yR);
+        double gL = sqrt_fix((0.5 * g) * (i0 + iL));
+        double gR = sqrt_fix((0.5 * g) * (i0 + iR));
         double F0 = (delu + (h0 - hL) * gL) + (h0 - hR) * gR;
-        double dfdh = ((gL - (g * (h0 - hL)) / ((4.0 * (h0 * h0)) * gL)) + gR) -
-                      (g * (h0 - hR)) / ((4.0 * (h0 * h0)) * gR);
-        const double sq0 = sqrt(h0);
+        double dfdh = ((gL - div_one(g * (h0 - hL), (4.0 * (h0 * h0)) * gL)) + gR) -
+                      div_one(g * (h0 - hR), (4.0 * (h0 * h0)) * gR);
+        const double sq0 = sqrt_fix(h0);
         double slope = scale_pow2(sq0, 1, 2.0) * dfdh;
-        double t = sq0 - F0 / slope;
+        double t = sq0 - div_one(F0, slope);
         hm = t * t;
-        const double im = 1.0 / hm;
-        double u1m = uL - (hm - hL) * sqrt((0.5 * g) * (im + iL));
-        double u2m = uR + (hm - hR) * sqrt((0.5 * g) * (im + iR));
-        const double sqm = sqrt(g * hm);
+        const double im = div_one(1.0, hm);
+        double u1m = uL - (hm - hL) * sqrt_fix((0.5 * g) * (im + iL));
+        double u2m = uR + (hm - hR) * sqrt_fix((0.5 * g) * (im + iR));
+        const double sqm = sqrt_fix(g * hm);
         s1m = u1m - sqm;
         s2m = u2m + sqm;
     } else {  // one shock, one rarefaction
@@ -288,11 +227,11 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
             rec->lhigh = lt(hR, hL);
         }
         double h0 = h_min;
-        const double i0 = r_lower ? inv_of(hR, yR, yR_ok) : inv_of(hL, yL, yL_ok);
-        double F0 = (delu + scale_pow2(sq_min - sq_max, 1, 2.0)) + (h0 - h_min) * sqrt((0.5 * g) * (i0 + i0));
-        double slope = (F_max - F0) / (h_max - h_min);
-        hm = h0 - F0 / slope;
-        const double sqm = sqrt(g * hm);
+        const double i0 = r_lower ? inv_of(hR, yR) : inv_of(hL, yL);
+        double F0 = (delu + scale_pow2(sq_min - sq_max, 1, 2.0)) + (h0 - h_min) * sqrt_fix((0.5 * g) * (i0 + i0));
+        double slope = div_one(F_max - F0, h_max - h_min);
+        hm = h0 - div_one(F0, slope);
+        const double sqm = sqrt_fix(g * hm);
         if (lt(hR, hL)) {
             s1m = (uL + scale_pow2(sqL, 1, 2.0)) - 3.0 * sqm;
             s2m = (uL + scale_pow2(sqL, 1, 2.0)) - sqm;
@@ -304,17 +243,16 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
 }
 
 __device__ __forceinline__ void riemann_structure_core(double hL, double hR, double uL, double uR, double drytol,
-                                                      double sqL, double sqR, double yL, double yR, bool yL_ok,
-                                                      bool yR_ok, double& hm, double& s1m, double& s2m) {
-    riemann_structure_rec<false>(hL, hR, uL, uR, drytol, sqL, sqR, yL, yR, yL_ok, yR_ok, hm, s1m, s2m, nullptr);
+                                                      double sqL, double sqR, u64 yL, u64 yR, double& hm, double& s1m, double& s2m) {
+    riemann_structure_rec<false>(hL, hR, uL, uR, drytol, sqL, sqR, yL, yR, hm, s1m, s2m, nullptr);
 }
 
 // The same with sqrt(g * h) and the reciprocals computed here (the wet/dry
 // edges' wall test; a call, so the callers keep their registers).
 static __device__ __noinline__ void riemann_structure(double hL, double hR, double uL, double uR, double drytol,
                                                       double& hm, double& s1m, double& s2m) {
-    riemann_structure_core(hL, hR, uL, uR, drytol, sqrt(kG * hL), sqrt(kG * hR), 0.0, 0.0, false, false, hm, s1m,
-                           s2m);
+    riemann_structure_core(hL, hR, uL, uR, drytol, sqrt_fix(kG * hL), sqrt_fix(kG * hR), recip_fix(hL),
+                           recip_fix(hR), hm, s1m, s2m);
 }
 
 __device__ __forceinline__ double det3(double a00, double a01, double a02, double a10, double a11, double a12,
@@ -335,7 +273,7 @@ __device__ __forceinline__ bool moderate(double x) { return abs_bits(x) < 0x52b0
 // Augmented solver (George 2008) with maxiter = 1, src/geoclaw/riemannsolvers.f:2-258.
 // The entropy corrector is off in the source; with one iteration the star
 // states after the Cramer solve never reach the outputs.
-// sqL / sqR: sqrt(g * h) of the (fixed-up) depths; yL / yR: RN(1 / h) where yL_ok / yR_ok.
+// sqL / sqR: sqrt(g * h) of the (fixed-up) depths; yL / yR: recip_fix of them (or 0).
 //
 // The 3x3 Cramer solve has the eigenvector matrix R = [[1, 0, 1], [l0, 0, l2],
 // [l0^2, 1, l2^2]] with constant 0 and 1 entries. Evaluated in the source's
@@ -351,15 +289,15 @@ __device__ __forceinline__ bool moderate(double x) { return abs_bits(x) < 0x52b0
 template <bool REC>
 __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL, double huR, double bL, double bR,
                                                double uL, double uR, double vL, double vR, double delphi,
-                                               double sE1, double sE2, double sqL, double sqR, double yL,
-                                               double yR, bool yL_ok, bool yR_ok, double drytol, double sw[3],
+                                               double sE1, double sE2, double sqL, double sqR, u64 yL,
+                                               u64 yR, double drytol, double sw[3],
                                                double fw[3][3], AugRec* rec) {
     const double g = kG;
     double delh = hR - hL;
     double delhu = huR - huL;
     double delb = bR - bL;
     double hm, s1m, s2m;
-    riemann_structure_rec<REC>(hL, hR, uL, uR, drytol, sqL, sqR, yL, yR, yL_ok, yR_ok, hm, s1m, s2m, rec);
+    riemann_structure_rec<REC>(hL, hR, uL, uR, drytol, sqL, sqR, yL, yR, hm, s1m, s2m, rec);
     double l0 = imin(sE1, s2m);
     double l2 = imax(sE2, s1m);
     if (REC) {
@@ -373,7 +311,7 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
     // sE2 - sE1 = -(l0 - l2) exactly (round to nearest is symmetric): one
     // reciprocal serves hstarHLL's divisor and the Cramer determinant
     const double dsp = sE2 - sE1;
-    const Recip rsp = recip_rn(dsp);
+    const Recip rsp = recip_of(dsp);
     const double hq = div_rn(((huL - huR) + sE2 * hR) - sE1 * hL, rsp);
     double hstarHLL = imax(hq, 0.0);
     double l1 = scale_pow2(l0 + l2, -1, 0.5);
@@ -410,7 +348,7 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
         deldelh = flip(delb, true);
         deldelphi = flip(ghbar * delb, true);
     } else {
-        const Recip rb = recip_rn(s1s2bar);
+        const Recip rb = recip_of(s1s2bar);
         deldelh = div_rn(dgh, rb);
         deldelphi = flip(div_rn(dgh * s1s2tilde, rb), true);
     }
@@ -419,16 +357,16 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
     double lo = 0.0, hi = 0.0;  // the two bounds of the case
     if (lt(sE1, -ct) && lt(ct, sE2)) {
         dcase = 1;
-        hi = hsd / sE2;
-        lo = hsd / sE1;
+        hi = div_one(hsd, sE2);
+        lo = div_one(hsd, sE1);
     } else if (le(ct, sE1)) {
         dcase = 2;
-        hi = hsd / sE1;
+        hi = div_one(hsd, sE1);
         lo = flip(hL, true);
     } else if (le(sE2, -ct)) {
         dcase = 3;
         hi = hR;
-        lo = hsd / sE2;
+        lo = div_one(hsd, sE2);
     }
     if (dcase) {
         const double x1 = imin(deldelh, hi);
@@ -458,7 +396,7 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
     // beta1's numerator, the source's expression with the products by 1 dropped
     const double n1 = ((d1 * r22 - l2 * d2) - d0 * (l0 * r22 - l2 * r20)) + (l0 * d2 - d1 * r20);
     if (quick) {
-        const Recip rd{det, flip(rsp.y, true), rsp.fast};  // RN(1 / det) = -RN(1 / (sE2 - sE1))
+        const Recip rd{det, rsp.y};  // det = -(sE2 - sE1): the same significand
         beta0 = div_rn(d1 - d0 * l2, rd);
         beta1 = div_rn(n1, rd);
         beta2 = div_rn(d0 * l0 - d1, rd);
@@ -482,11 +420,11 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
 
 static __device__ __noinline__ void riemann_aug(double hL, double hR, double huL, double huR, double bL, double bR,
                                                 double uL, double uR, double vL, double vR, double delphi,
-                                                double sE1, double sE2, double sqL, double sqR, double yL,
-                                                double yR, bool yL_ok, bool yR_ok, double drytol, double sw[3],
+                                                double sE1, double sE2, double sqL, double sqR, u64 yL,
+                                                u64 yR, double drytol, double sw[3],
                                                 double fw[3][3]) {
-    riemann_aug_rec<false>(hL, hR, huL, huR, bL, bR, uL, uR, vL, vR, delphi, sE1, sE2, sqL, sqR, yL, yR, yL_ok,
-                           yR_ok, drytol, sw, fw, nullptr);
+    riemann_aug_rec<false>(hL, hR, huL, huR, bL, bR, uL, uR, vL, vR, delphi, sE1, sE2, sqL, sqR, yL, yR,
+                           drytol, sw, fw, nullptr);
 }
 
 // Wet/dry handling, wave speeds and net updates of c_bind_geoclaw_solver_dp
@@ -496,7 +434,8 @@ static __device__ __noinline__ void riemann_aug(double hL, double hR, double huL
 // sqL0 / sqR0 are sqrt(g * depth) of the two cells, computed once per cell by the
 // caller; they are used only where the reference evaluates sqrt(g * h) on an
 // unmodified wet depth (the same operands, so the same bits).
-// yL0 / yR0 are RN(1 / depth) of the two cells (read only for wet sides).
+// yL0 / yR0 are recip_fix of the two depths (0 for a dry side, or left out where the
+// side's momenta are zeros).
 // Branch-frozen evaluation (FZ, the f-wave only): FZ = 1 records the decisions
 // of the edge into *fz, FZ = 2 takes them from *fz instead of the comparisons
 // (a forward run whose every branch is that of a recorded run, for checking the
@@ -513,7 +452,7 @@ __device__ __forceinline__ bool fzb(uint16_t* fz, int bit, bool v) {
 template <int SOLVER, int FZ = 0>
 __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL, double huR, double hvL,
                                                double hvR, double bL, double bR, double sqL0, double sqR0,
-                                               double yL0, double yR0, double drytol, double netL[3],
+                                               u64 yL0, u64 yR0, double drytol, double netL[3],
                                                double netR[3], double& maxspeed, uint16_t* fz = nullptr) {
     const double g = kG;
     netL[0] = netL[1] = netL[2] = 0.0;
@@ -523,8 +462,8 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     const bool wetR0 = fzb<FZ>(fz, 1, lt(drytol, hR)), wetL0 = fzb<FZ>(fz, 2, lt(drytol, hL));  // h > drytol
     if (fzb<FZ>(fz, 0, !wetL0 && !wetR0 && !is_nan(hL) && !is_nan(hR) && !is_nan(drytol))) return;  // both dry
     if (FZ == 2) {  // a recorded wet side is wet here, whatever its current depth
-        if (wetL0) sqL0 = sqrt(g * hL);
-        if (wetR0) sqR0 = sqrt(g * hR);
+        if (wetL0) sqL0 = sqrt_fix(g * hL);
+        if (wetR0) sqR0 = sqrt_fix(g * hR);
     }
     double uL, uR, vL, vR;
     if (wetR0) {
@@ -532,7 +471,7 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
             uR = huR / hR;
             vR = hvR / hR;
         } else {
-            const Recip r{hR, yR0, recip_fast(hR)};
+            const Recip r{hR, yR0};
             uR = div_rn(huR, r);
             vR = div_rn(hvR, r);
         }
@@ -544,7 +483,7 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
             uL = huL / hL;
             vL = hvL / hL;
         } else {
-            const Recip r{hL, yL0, recip_fast(hL)};
+            const Recip r{hL, yL0};
             uL = div_rn(huL, r);
             vL = div_rn(hvL, r);
         }
@@ -586,27 +525,23 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     double sqR = wetR ? (wall_r ? sqL0 : sqR0) : 0.0;
     double sL = uL - sqL;
     double sR = uR + sqR;
-    // one division with its own divisor: the IEEE division (correctly rounded, as
-    // recip_rn + div_rn is) needs fewer FP64 instructions than a private reciprocal
-    double uhat = (prod(sqL, uL) + prod(sqR, uR)) / (sqR + sqL);
-    double chat = sqrt(ghalf_h);
+    double uhat = div_one(prod(sqL, uL) + prod(sqR, uR), sqR + sqL);
+    double chat = sqrt_fix(ghalf_h);
     const double r1 = uhat - chat, r2 = uhat + chat;
     double sE1 = fzb<FZ>(fz, 7, lt(sL, r1)) ? sL : r1;  // imin(sL, r1)
     double sE2 = fzb<FZ>(fz, 8, lt(r2, sR)) ? sR : r2;  // imax(sR, r2)
 
     double sw[3], fw[3][3];
     if (SOLVER == AUG_RIEMANN) {
-        // RN(1 / h) of the fixed-up depths: a wet side's own, a wall's mirrored one
-        const double yLf = wall_l ? yR0 : yL0, yRf = wall_r ? yL0 : yR0;
-        const bool okL = wetL && recip_fast(hL), okR = wetR && recip_fast(hR);
-        riemann_aug(hL, hR, huL, huR, bL, bR, uL, uR, vL, vR, delphi, sE1, sE2, sqL, sqR, yLf, yRf, okL, okR,
-                    drytol, sw, fw);
+        // the reciprocals of the fixed-up depths: a wet side's own, a wall's mirrored one
+        const u64 yLf = wall_l ? yR0 : yL0, yRf = wall_r ? yL0 : yR0;
+        riemann_aug(hL, hR, huL, huR, bL, bR, uL, uR, vL, vR, delphi, sE1, sE2, sqL, sqR, yLf, yRf, drytol, sw, fw);
     } else {
         double delhu = huR - huL;
         double delb = bR - bL;
         double deldelphi = -prod(ghalf_h, delb);
         double dpd = delphi - deldelphi;
-        const Recip rD = recip_rn(sE2 - sE1);
+        const Recip rD = recip_of(sE2 - sE1);
         double beta1 = div_rn(prod(sE2, delhu) - dpd, rD);
         double beta2 = div_rn(dpd - prod(sE1, delhu), rD);
         sw[0] = sE1; sw[1] = scale_pow2(sE1 + sE2, -1, 0.5); sw[2] = sE2;
@@ -675,7 +610,7 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
 // the bit patterns. Otherwise the general form runs.
 template <int SOLVER, int FZ = 0>
 __device__ __forceinline__ void geoclaw_flux(double n1, double n2, const State& QL, const State& QR, double dL,
-                                             double dR, double sqL, double sqR, double yL, double yR,
+                                             double dR, double sqL, double sqR, u64 yL, u64 yR,
                                              double drytol, Update& fL, Update& fR, int axis = 0,
                                              uint16_t* fz = nullptr) {
     // both sides dry: the solver returns zero net updates and speed, and their
@@ -788,23 +723,22 @@ __device__ __forceinline__ void geoclaw_flux(double n1, double n2, const State& 
     }
 }
 
-__device__ __forceinline__ double normal_velocity(double n1, double n2, double p1, double p2, double d) {
-    return z0(n1 * (p1 / d)) + n2 * (p2 / d);
-}
-// The same with the quotients from r = {d, RN(1 / d)} (div_rn: IEEE results).
+// z0(n1 (p1 / d)) + n2 (p2 / d), r = {d, recip_fix(d)}
 __device__ __forceinline__ double normal_velocity(double n1, double n2, double p1, double p2, const Recip& r) {
     return z0(n1 * div_rn(p1, r)) + n2 * div_rn(p2, r);
 }
 
 // compute_lf_flux, src/SWE/SWE_euler_timestep.f90:359-446
-// yL / yR: RN(1 / depth) of the two states where the depth is above the dry
-// tolerance (else not read).
+// sqL / sqR, yL / yR: sqrt(g * depth) and recip_fix of the two depths where they are
+// above the dry tolerance (else not read).
 template <int SOLVER>
 __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, const State& QR, double dL,
-                                        double dR, double drytol, Update& fL, Update& fR, double yL, double yR) {
+                                        double dR, double drytol, Update& fL, Update& fR, double sqL,
+                                        double sqR, u64 yL, u64 yR) {
     const double g = kG;
     if (SOLVER == LF_BATH || SOLVER == LLF_BATH) {
-        const Recip rL{dL, yL, lt(drytol, dL) && recip_fast(dL)}, rR{dR, yR, lt(drytol, dR) && recip_fast(dR)};
+        const bool aL = lt(drytol, dL), aR = lt(drytol, dR);
+        const Recip rL{dL, aL ? yL : recip_fix(dL)}, rR{dR, aR ? yR : recip_fix(dR)};
         if (dL < drytol || dR < drytol) {
             fL = Update{0.0, 0.0, 0.0, 0.0};
             fR = Update{0.0, 0.0, 0.0, 0.0};
@@ -812,14 +746,14 @@ __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, c
             } else if (dL < drytol) {
                 double hR = dmx(dR, 0.0);
                 double vR = normal_velocity(n1, n2, QR.p1, QR.p2, rR);
-                fR.s = sqrt(g * hR) + fabs(vR);
+                fR.s = (aR ? sqR : sqrt_fix(g * hR)) + fabs(vR);
                 double pr = ((0.5 * g) * hR) * hR;
                 fR.p1 = (-((0.5 * vR) * QR.p1) - pr * n1) + (0.5 * fR.s) * QR.p1;
                 fR.p2 = (-((0.5 * vR) * QR.p2) - pr * n2) + (0.5 * fR.s) * QR.p2;
             } else {
                 double hL = dmx(dL, 0.0);
                 double vL = normal_velocity(n1, n2, QL.p1, QL.p2, rL);
-                fL.s = sqrt(g * hL) + fabs(vL);
+                fL.s = (aL ? sqL : sqrt_fix(g * hL)) + fabs(vL);
                 double pr = ((0.5 * g) * hL) * hL;
                 fL.p1 = ((0.5 * vL) * QL.p1 + pr * n1) + (0.5 * fL.s) * QL.p1;
                 fL.p2 = ((0.5 * vL) * QL.p2 + pr * n2) + (0.5 * fL.s) * QL.p2;
@@ -829,8 +763,8 @@ __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, c
         double hL = dmx(dL, 0.0), hR = dmx(dR, 0.0);
         double vL = normal_velocity(n1, n2, QL.p1, QL.p2, rL);
         double vR = normal_velocity(n1, n2, QR.p1, QR.p2, rR);
-        fL.s = sqrt(g * hL) + fabs(vL);
-        fR.s = sqrt(g * hR) + fabs(vR);
+        fL.s = (aL ? sqL : sqrt_fix(g * hL)) + fabs(vL);
+        fR.s = (aR ? sqR : sqrt_fix(g * hR)) + fabs(vR);
         double alpha = (SOLVER == LLF_BATH) ? dmx(fL.s, fR.s) : 100.0;
         fL.h = 0.5 * ((hL * vL + hR * vR) + alpha * (QL.h - QR.h));
         fR.h = -fL.h;
@@ -848,10 +782,10 @@ __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, c
         dL = QL.h - 0.0;
         dR = QR.h - 0.0;
         double hL = dmx(dL, 0.0), hR = dmx(dR, 0.0);
-        double vL = normal_velocity(n1, n2, QL.p1, QL.p2, dL);
-        double vR = normal_velocity(n1, n2, QR.p1, QR.p2, dR);
-        fL.s = sqrt(g * dL) + fabs(vL);
-        fR.s = sqrt(g * dR) + fabs(vR);
+        double vL = normal_velocity(n1, n2, QL.p1, QL.p2, recip_of(dL));
+        double vR = normal_velocity(n1, n2, QR.p1, QR.p2, recip_of(dR));
+        fL.s = sqrt_fix(g * dL) + fabs(vL);
+        fR.s = sqrt_fix(g * dR) + fabs(vR);
         double alpha = (SOLVER == LLF) ? dmx(fL.s, fR.s) : 100.0;
         fL.h = 0.5 * ((vL * hL + vR * hR) + alpha * (QL.h - QR.h));
         fR.h = -fL.h;
@@ -865,29 +799,24 @@ __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, c
 }
 
 // One edge: dL/dR are the depths h - b of the two states, sqL/sqR their
-// sqrt(g * depth) and yL/yR RN(1 / depth) (only read for depths above the dry
+// sqrt(g * depth) and yL/yR recip_fix(depth) (only read for depths above the dry
 // tolerance).
 template <int SOLVER, int FZ = 0>
 __device__ __forceinline__ void edge_flux(double n1, double n2, const State& QL, const State& QR, double dL,
-                                          double dR, double sqL, double sqR, double yL, double yR, double drytol,
+                                          double dR, double sqL, double sqR, u64 yL, u64 yR, double drytol,
                                           Update& fL, Update& fR, int axis = 0, uint16_t* fz = nullptr) {
     if (SOLVER == FWAVE || SOLVER == AUG_RIEMANN)
         geoclaw_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, fz);
     else
-        lf_flux<SOLVER>(n1, n2, QL, QR, dL, dR, drytol, fL, fR, yL, yR);
+        lf_flux<SOLVER>(n1, n2, QL, QR, dL, dR, drytol, fL, fR, sqL, sqR, yL, yR);
 }
 
-// depth, sqrt(g * depth) and RN(1 / depth) of a state, as the edge code needs them
-__device__ __forceinline__ void depth_terms(const State& Q, double drytol, double& d, double& sq) {
-    d = Q.h - Q.b;
-    sq = d > drytol ? sqrt(kG * d) : 0.0;
-}
-
-__device__ __forceinline__ void depth_terms(const State& Q, double drytol, double& d, double& sq, double& y) {
+// depth, sqrt(g * depth) and recip_fix(depth) of a state, as the edge code needs them
+__device__ __forceinline__ void depth_terms(const State& Q, double drytol, double& d, double& sq, u64& y) {
     d = Q.h - Q.b;
     const bool wet = lt(drytol, d);
-    sq = wet ? sqrt(kG * d) : 0.0;
-    y = wet ? recip_rn(d).y : 0.0;
+    sq = wet ? sqrt_fix(kG * d) : 0.0;
+    y = wet ? recip_fix(d) : 0;
 }
 
 // Ghost state of bnd_skeleton_scalar_op, src/SWE/SWE_euler_timestep.f90:231-255.

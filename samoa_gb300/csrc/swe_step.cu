@@ -47,7 +47,8 @@ __global__ void riemann_batch_kernel(int64_t n, const double* nrm, const double*
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         State L{ql[4 * i], ql[4 * i + 1], ql[4 * i + 2], ql[4 * i + 3]};
         State R{qr[4 * i], qr[4 * i + 1], qr[4 * i + 2], qr[4 * i + 3]};
-        double dL, dR, sqL, sqR, yL, yR;
+        double dL, dR, sqL, sqR;
+        u64 yL, yR;
         depth_terms(L, drytol, dL, sqL, yL);
         depth_terms(R, drytol, dR, sqR, yR);
         Update fL, fR;
@@ -81,8 +82,8 @@ __device__ __forceinline__ double draw_double(unsigned long long z, int e_span) 
     return __longlong_as_double((long long)(sign | ((unsigned long long)(e + 1023) << 52) | mant));
 }
 
-// Compares div_rn(a, recip_rn(b)) and div_rn(c, recip_rn(b)) with the IEEE
-// quotients bit for bit (a NaN matches any NaN); counts mismatches.
+// Compares div_rn(a, recip_of(b)), div_rn(c, recip_of(b)) and sqrt_fix of all three
+// with the IEEE results bit for bit (a NaN matches any NaN); counts mismatches.
 __global__ void division_check_kernel(int64_t n, unsigned long long seed, int e_span,
                                       unsigned long long* mismatches) {
     unsigned long long bad = 0;
@@ -91,11 +92,14 @@ __global__ void division_check_kernel(int64_t n, unsigned long long seed, int e_
         const double b = draw_double(z, e_span);
         const double a = draw_double(z + 1, e_span);
         const double c = (i & 15) == 0 ? 0.0 : draw_double(z + 2, e_span);
-        const Recip r = recip_rn(b);
-        const double q1 = div_rn(a, r), q2 = div_rn(c, r), e1 = a / b, e2 = c / b;
-        const bool ok1 = (q1 != q1 && e1 != e1) || __double_as_longlong(q1) == __double_as_longlong(e1);
-        const bool ok2 = (q2 != q2 && e2 != e2) || __double_as_longlong(q2) == __double_as_longlong(e2);
-        bad += (ok1 ? 0 : 1) + (ok2 ? 0 : 1);
+        const Recip r = recip_of(b);
+        const double got[5] = {div_rn(a, r), div_rn(c, r), sqrt_fix(a), sqrt_fix(fabs(b)), sqrt_fix(c)};
+        const double want[5] = {a / b, c / b, sqrt(a), sqrt(fabs(b)), sqrt(c)};
+        for (int k = 0; k < 5; ++k) {
+            const bool ok = (got[k] != got[k] && want[k] != want[k]) ||
+                            __double_as_longlong(got[k]) == __double_as_longlong(want[k]);
+            bad += ok ? 0 : 1;
+        }
     }
     if (bad) atomicAdd(mismatches, bad);
 }
