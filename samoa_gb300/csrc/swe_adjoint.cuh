@@ -507,8 +507,7 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
     }
     bool wall_l = false, wall_r = false, lower_l = false, lower_r = false;
     if (!wetR) {
-        double hstar, s1m, s2m;
-        riemann_structure(hL, hL, uL, -uL, drytol, hstar, s1m, s2m);
+        const double hstar = wall_depth(hL, uL, sqL0, yL0, drytol);
         if (dmx(hL, hstar) + bL < bR) {
             wall_r = true;
             hR = hL; huR = -huL; bR = bL; uR = -uL; vR = vL;
@@ -517,8 +516,7 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
             bR = hL + bL;
         }
     } else if (!wetL) {
-        double hstar, s1m, s2m;
-        riemann_structure(hR, hR, -uR, uR, drytol, hstar, s1m, s2m);
+        const double hstar = wall_depth(hR, -uR, sqR0, yR0, drytol);
         if (dmx(hR, hstar) + bR < bL) {
             wall_l = true;
             hL = hR; huL = -huR; bL = bR; uL = -uR; vL = vR;
