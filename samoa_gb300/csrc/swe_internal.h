@@ -49,6 +49,14 @@ struct InstParams {
     int32_t min_depth, max_depth, dmin, ndepth, bc, dt_by_max;
 };
 
+// Per instance and depth (from the instance's dmin on), the values of the cell
+// update that only the parameters set: edge lengths, volume, 2^(d+1), and the
+// lengths rounded up to float. Written by the host with the parameters.
+struct alignas(8) DepthRow {
+    double leg, hyp, vol, pow;
+    float leg_up, hyp_up;
+};
+
 // Per-instance scalars on the device. The step kernel reads dt, reduces into
 // dt_acc / refine_acc, and the last CTA to finish advances time and dt, so
 // many steps run back to back without the host.
@@ -60,13 +68,14 @@ struct InstScalars {
     unsigned long long ds_acc;      // bits of the running maximum of ds * 2^(d+1) (dt_by_max)
     unsigned long long refine_acc;  // refinements issued in the running step
     unsigned long long n_refine;    // refinements issued in the last step
+    unsigned long long ds_ring[3];  // ds_acc of the multi-step kernel, by step modulo 3 (0 between launches)
 };
 
 struct GlobalScalars {
     unsigned int done;       // CTAs finished in the running step
     unsigned int error;      // nonzero: a kernel saw a bad index or a wait ran out
-    unsigned int next_seg;   // next segment to hand out in the running step
-    unsigned int pad;
+    unsigned int next_seg;   // segments handed out in the running step beyond each CTA's first
+    unsigned int arrived;    // CTAs that reached the multi-step kernel's barriers in the running launch
     long long step;          // steps since the mesh upload (parity = traversal direction)
     long long dt_seq_base;   // step at which the frozen dt sequence starts
 };

@@ -62,6 +62,7 @@ struct StepArgs {
     uint16_t* erec;            // branch-frozen runs: this step's edge decisions, per task ...
     uint16_t* xrec;            // ... and per cross-segment edge
     const InstParams* ip;
+    const DepthRow* rows;      // [instance][max_ndepth]
     InstScalars* is;
     GlobalScalars* gs;
     uint8_t* branch;           // optional per-cell output: bit 0 wetting fix, bit 1 drying clamp (adjoint)
@@ -144,70 +145,80 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
-__device__ __forceinline__ double warp_min(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = dmn(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
+// Warp-wide maximum of u64 values: of the high words, then of the low words among the lanes that hold it.
 __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w > v ? w : v;
-    }
-    return v;
+    const unsigned hi = (unsigned)(v >> 32);
+    const unsigned m = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = __reduce_max_sync(0xffffffffu, hi == m ? (unsigned)v : 0u);
+    return ((unsigned long long)m << 32) | lo;
 }
 
-__device__ __forceinline__ long long warp_sum(long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// dt of step `step` for instance `inst`: the frozen sequence if one is set,
-// else grid%r_dt clamped as in pre_traversal_grid_op (src/SWE/SWE_euler_timestep.f90:89-109)
-__device__ __forceinline__ double step_dt(const StepArgs& A, const InstParams& P, int inst, long long k) {
-    if (A.dt_seq && k >= 0 && k < A.dt_seq_len) return A.dt_seq[k * A.n_inst + inst];
-    double dt = A.is[inst].dt;
-    if (P.max_time > 0.0) dt = dmn(P.max_time, dt);
-    if (P.tout > 0.0) dt = dmn(P.tout, dt);
+// grid%r_dt clamped as in pre_traversal_grid_op (src/SWE/SWE_euler_timestep.f90:89-109)
+__device__ __forceinline__ double clamp_dt(double dt, double max_time, double tout) {
+    if (max_time > 0.0) dt = dmn(max_time, dt);
+    if (tout > 0.0) dt = dmn(tout, dt);
     return dt;
 }
 
-// Block-wide reduction of (dtmin, dskey, nref) into instance `inst`; all threads call it.
-__device__ __forceinline__ void flush_instance(const StepArgs& A, int inst, double& dtmin, unsigned long long& dskey,
-                                               long long& nref, double* red_min, unsigned long long* red_max,
-                                               long long* red_sum) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    double m = warp_min(dtmin);
-    unsigned long long x = warp_max_u64(dskey);
-    long long s = warp_sum(nref);
-    if (lane == 0) {
-        red_min[warp] = m;
-        red_max[warp] = x;
-        red_sum[warp] = s;
+// grid%r_dt_new from the reductions of a step (the smallest volume / ds, or the
+// bits x of the largest ds 2^(d+1))
+__device__ __forceinline__ double dt_new_of(const InstParams& P, double dt_acc, unsigned long long x) {
+    return x ? dmn(dt_acc, div_one(P.scaling * P.scaling, __longlong_as_double((long long)x))) : dt_acc;
+}
+
+// The scalars after a step (post_traversal_grid_op, src/SWE/SWE_euler_timestep.f90:111-131)
+__device__ __forceinline__ void advance_time(InstScalars* S, const InstParams& P, double time, double dt_acc,
+                                             unsigned long long x, unsigned long long n_refine) {
+    const double dtn = dt_new_of(P, dt_acc, x);
+    S->time = time;
+    S->dt_new = dtn;
+    S->dt = P.courant * dtn;
+    S->n_refine = n_refine;
+}
+
+// What the CTA's threads reduce over the cells of an instance: the bits of the
+// largest ds 2^(d+1) (dt_by_max) or the complement of the bits of the smallest
+// volume / ds (non-negative doubles order like their bits, and the complement
+// turns the minimum into a maximum), and the refinements.
+struct Reduced {
+    unsigned long long key;
+    int nref;
+};
+struct RedSlots {
+    unsigned long long key[8];
+    int nref[8];
+};
+__device__ __forceinline__ void warp_reduce(const Reduced& r, RedSlots& slots) {
+    const unsigned long long k = warp_max_u64(r.key);
+    const int n = __reduce_add_sync(0xffffffffu, r.nref);
+    if ((threadIdx.x & 31) == 0) {
+        slots.key[threadIdx.x >> 5] = k;
+        slots.nref[threadIdx.x >> 5] = n;
     }
+}
+__device__ __forceinline__ Reduced block_reduced(const RedSlots& slots) {  // after a barrier
+    Reduced r{0ull, 0};
+    const int nw = (blockDim.x + 31) >> 5;
+    for (int w = 0; w < nw; ++w) {
+        r.key = slots.key[w] > r.key ? slots.key[w] : r.key;
+        r.nref += slots.nref[w];
+    }
+    return r;
+}
+// The CTA's reductions into instance `inst`; all threads call it.
+__device__ __forceinline__ void flush_instance(const StepArgs& A, int inst, bool by_max, Reduced& r, RedSlots& slots) {
+    warp_reduce(r, slots);
     __syncthreads();
-    if (warp == 0) {
-        const int nw = (blockDim.x + 31) >> 5;
-        m = lane < nw ? red_min[lane] : DBL_MAX;
-        x = lane < nw ? red_max[lane] : 0ull;
-        s = lane < nw ? red_sum[lane] : 0;
-        m = warp_min(m);
-        x = warp_max_u64(x);
-        s = warp_sum(s);
-        if (lane == 0) {
-            // non-negative doubles order like their bit patterns
-            if (m != DBL_MAX) atomicMin(&A.is[inst].dt_acc, (unsigned long long)__double_as_longlong(m));
-            if (x) atomicMax(&A.is[inst].ds_acc, x);
-            if (s) atomicAdd(&A.is[inst].refine_acc, (unsigned long long)s);
+    if (threadIdx.x == 0) {
+        const Reduced b = block_reduced(slots);
+        if (by_max) {
+            if (b.key) atomicMax(&A.is[inst].ds_acc, b.key);
+        } else if (b.key) {
+            atomicMin(&A.is[inst].dt_acc, ~b.key);
         }
+        if (b.nref) atomicAdd(&A.is[inst].refine_acc, (unsigned long long)b.nref);
     }
-    __syncthreads();
-    dtmin = DBL_MAX;
-    dskey = 0;
-    nref = 0;
+    r = Reduced{0ull, 0};
 }
 
 // The edges between two segments, one thread each, before the step kernel:
@@ -320,6 +331,240 @@ __device__ __forceinline__ bool key_below(float2 up, double s0, double s1, doubl
     return bound < m;
 }
 
+// The depth-dependent values of the running instance, in shared memory.
+struct DepthTab {
+    double* leg;
+    double* hyp;
+    double* vol;
+    double* pow;  // 2^(d+1)
+    double* ndv;  // -dt / volume
+    float2* up;   // (leg, hyp) rounded up to float
+    __device__ __forceinline__ DepthTab(double* base, int n)
+        : leg(base), hyp(base + n), vol(base + 2 * n), pow(base + 3 * n), ndv(base + 4 * n),
+          up(reinterpret_cast<float2*>(base + 5 * n)) {}
+    __device__ __forceinline__ void load(const StepArgs& A, int inst, int i) const {
+        const DepthRow* row = A.rows + (size_t)inst * A.max_ndepth + i;
+        leg[i] = row->leg;
+        hyp[i] = row->hyp;
+        vol[i] = row->vol;
+        pow[i] = row->pow;
+        up[i] = make_float2(row->leg_up, row->hyp_up);
+    }
+};
+
+// A segment's working set in shared memory.
+struct SegMem {
+    int T;
+    double* h;    // staged h, hu, hv, b: [4][T]
+    u64* rh;      // recip_fix(depth) where the cell is wet
+    double* sq;   // sqrt(g * depth) where the cell is wet
+    double* upd;  // [4 quantities][3 local edges][T]
+    int8_t* dep;  // the cells' depths
+    __device__ __forceinline__ double* hu() const { return h + T; }
+    __device__ __forceinline__ double* hv() const { return h + 2 * T; }
+    __device__ __forceinline__ double* b() const { return h + 3 * T; }
+};
+
+// Edge tasks [tid, nt) in steps of the CTA (skeleton_scalar_op /
+// bnd_skeleton_scalar_op, src/SWE/SWE_euler_timestep.f90:196-255): the updates of
+// both sides into the slots of the cells in the segment. Each thread loads its
+// next task while it works on the current one. With SHARED_STATE other CTAs
+// write the neighbours' state in this launch, so it is read past the L1 cache.
+// Returns nonzero on a bad index.
+template <int SOLVER, int FZ, bool SHARED_STATE>
+__device__ __forceinline__ unsigned int edge_tasks(const StepArgs& A, const SegMem& M, const int4* tasks, int nt,
+                                                   uint16_t* erec, int c0, int cn, int odd, double drytol, int bc,
+                                                   const double* hin, const double* huin, const double* hvin) {
+    const int tid = threadIdx.x, T = M.T;
+    unsigned int bad = 0;
+    int4 tk_next = make_int4(0, 0, 0, 0);
+    if (tid < nt) tk_next = __ldg(&tasks[tid]);
+    for (int t = tid; t < nt; t += blockDim.x) {
+        const int4 tk = tk_next;
+        if (t + (int)blockDim.x < nt) tk_next = __ldg(&tasks[t + blockDim.x]);
+        const uint32_t meta = (uint32_t)tk.z;
+        const bool bnd = (meta >> 14) & 1u;
+        int L, R, iL, iR, pL;
+        if (bnd || !odd) {
+            L = tk.x; iL = meta & 3u; pL = (meta >> 4) & 31u;
+            R = tk.y; iR = (meta >> 2) & 3u;
+        } else {
+            L = tk.y; iL = (meta >> 2) & 3u; pL = (meta >> 9) & 31u;
+            R = tk.x; iR = meta & 3u;
+        }
+        if ((unsigned)L >= (unsigned)A.n_cells_total || (!bnd && (unsigned)R >= (unsigned)A.n_cells_total) ||
+            iL > 2 || iR > 2 || pL > 16) {
+            bad = 1u;
+            continue;
+        }
+        const double n1 = c_normal[pL][iL][0], n2 = c_normal[pL][iL][1];
+        const int sl = L - c0, sr = R - c0;
+        const bool lin = (unsigned)sl < (unsigned)cn;
+        const bool rin = !bnd && (unsigned)sr < (unsigned)cn;
+        State QL, QR;
+        double dL, dR, sqL, sqR;
+        u64 yL, yR;
+        auto far = [&](int c, State& Q, double& d, double& sq, u64& y) {
+            if (SHARED_STATE) Q = State{__ldcg(hin + c), __ldcg(huin + c), __ldcg(hvin + c), A.b[c]};
+            else Q = State{hin[c], huin[c], hvin[c], A.b[c]};
+            depth_terms(Q, drytol, d, sq, y);
+        };
+        auto near = [&](int i, State& Q, double& d, double& sq, u64& y) {
+            Q = State{M.h[i], M.hu()[i], M.hv()[i], M.b()[i]};
+            d = Q.h - Q.b;
+            sq = M.sq[i];
+            y = M.rh[i];
+        };
+        if (lin) near(sl, QL, dL, sqL, yL);
+        else far(L, QL, dL, sqL, yL);
+        if (bnd) {  // the ghost has the cell's h and b
+            if (bc == BC_SLIP) QR = boundary_ghost<BC_SLIP>(n1, n2, QL);
+            else if (bc == BC_NOSLIP) QR = boundary_ghost<BC_NOSLIP>(n1, n2, QL);
+            else QR = QL;
+            dR = dL;
+            sqR = sqL;
+            yR = yL;
+        } else if (rin) {
+            near(sr, QR, dR, sqR, yR);
+        } else {
+            far(R, QR, dR, sqR, yR);
+        }
+        Update fL, fR;
+        edge_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, (int)((meta >> 15) & 3u),
+                              FZ ? erec + t : nullptr);
+        if (lin) {
+            M.upd[(0 * 3 + iL) * T + sl] = fL.h;
+            M.upd[(1 * 3 + iL) * T + sl] = fL.p1;
+            M.upd[(2 * 3 + iL) * T + sl] = fL.p2;
+            M.upd[(3 * 3 + iL) * T + sl] = fL.s;
+        }
+        if (rin) {
+            M.upd[(0 * 3 + iR) * T + sr] = fR.h;
+            M.upd[(1 * 3 + iR) * T + sr] = fR.p1;
+            M.upd[(2 * 3 + iR) * T + sr] = fR.p2;
+            M.upd[(3 * 3 + iR) * T + sr] = fR.s;
+        }
+    }
+    return bad;
+}
+
+// A cell's new state, its flag and its branch bits (cell_update_op + volume_op,
+// src/SWE/SWE_euler_timestep.f90:257-355); folds its CFL term and refinement
+// into r. wkey: a lower bound of the largest CFL key the lanes of this warp have
+// taken so far (dt_by_max); a cell whose key is certainly below it cannot raise
+// the maximum. rb: the recorded fixes of a branch-frozen run (FZ = 2).
+struct CellOut {
+    double h, p1, p2;
+    int8_t flag;
+    uint8_t branch;
+};
+template <int FZ>
+__device__ __forceinline__ CellOut update_cell(const SegMem& M, const DepthTab& tab, const InstParams& P, int i,
+                                               int odd, unsigned long long wkey, uint8_t rb, Reduced& r) {
+    const int T = M.T, k0 = odd ? 2 : 0, k2 = odd ? 0 : 2;
+    const int d = M.dep[i];
+    const int di = d - P.dmin;
+    const double leg = tab.leg[di], hyp = tab.hyp[di], ndv = tab.ndv[di];
+    double u[4][3];
+    long long nz = 0, sz = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        u[q][0] = M.upd[(q * 3 + k0) * T + i];
+        u[q][1] = M.upd[(q * 3 + 1) * T + i];
+        u[q][2] = M.upd[(q * 3 + k2) * T + i];
+        (q < 3 ? nz : sz) |= (dbits(u[q][0]) | dbits(u[q][1]) | dbits(u[q][2])) << 1;
+    }
+    // quiet: every update of h, hu, hv is +-0 (dry land, water at rest). Then
+    // each sum below is +0 (positive edge lengths), RN(ndv * +0) is a zero with
+    // ndv's sign, and adding it leaves the state as add_zero says: the same
+    // bits, without the FP64 arithmetic. Water at rest still has wave speeds,
+    // so the speed sum ds has its own test below.
+    const bool quiet = nz == 0 && is_finite(ndv);
+    double dh = 0.0, dp1 = 0.0, dp2 = 0.0, ds = 0.0;
+    if (__any_sync(__activemask(), !quiet)) {
+        if (!quiet) {
+            dh = z0(prod_cell(leg, u[0][0])) + prod_cell(hyp, u[0][1]);
+            dh = dh + prod_cell(leg, u[0][2]);
+            dp1 = z0(prod_cell(leg, u[1][0])) + prod_cell(hyp, u[1][1]);
+            dp1 = dp1 + prod_cell(leg, u[1][2]);
+            dp2 = z0(prod_cell(leg, u[2][0])) + prod_cell(hyp, u[2][1]);
+            dp2 = dp2 + prod_cell(leg, u[2][2]);
+        }
+    }
+    // ds is +0 when every speed is +-0 (dry land) or when the cell's key stays
+    // below wkey (key_below), else it is summed
+    bool need_ds = sz != 0;
+    if (need_ds && wkey != 0ull) need_ds = !key_below(tab.up[di], u[3][0], u[3][1], u[3][2], d + 1, wkey);
+    if (__any_sync(__activemask(), need_ds)) {
+        if (need_ds) {
+            ds = z0(prod_cell(leg, u[3][0])) + prod_cell(hyp, u[3][1]);
+            ds = ds + prod_cell(leg, u[3][2]);
+        }
+    }
+    CellOut o;
+    o.flag = 0;
+    // |dh| > thr and |dh| < thr / 8 on the bit patterns (thresholds are positive;
+    // a NaN |dh| passes neither test, as in IEEE)
+    const long long nrm = abs_bits(dh);
+    if (d < P.max_depth && not_nan(nrm) && nrm > __double_as_longlong(P.thr_refine)) {
+        o.flag = 1;
+        ++r.nref;
+    } else if (d > P.min_depth && nrm < __double_as_longlong(P.thr_coarsen)) {
+        o.flag = -1;
+    }
+    unsigned long long key;
+    if (P.dt_by_max) {  // ds >= 0, so its bits order like its value; RN(ds * 2^(d+1))
+        key = (unsigned long long)dbits(scale_pow2(ds, d + 1, tab.pow[di]));
+    } else {  // r_dt_new = min(huge, volume / ds): a NaN quotient never wins
+        const double q = tab.vol[di] / ds;
+        key = q < DBL_MAX ? ~(unsigned long long)dbits(q) : 0ull;
+    }
+    r.key = key > r.key ? key : r.key;
+    if (quiet) {
+        dh = dp1 = dp2 = bitsd(dbits(ndv) & (long long)0x8000000000000000ULL);  // RN(ndv * +0)
+    } else {
+        dh = prod_cell(ndv, dh);
+        dp1 = prod_cell(ndv, dp1);
+        dp2 = prod_cell(ndv, dp2);
+    }
+    double h = M.h[i], p1 = M.hu()[i], p2 = M.hv()[i];
+    const double b = M.b()[i];
+    uint8_t br = 0;
+    const double bdry = b + P.drytol;
+    // flooded land starts at the dry tolerance, at rest
+    if (FZ == 2 ? (rb & 1u) != 0 : (lt(h, bdry) && gt0(dh))) {
+        h = bdry;
+        p1 = 0.0;
+        p2 = 0.0;
+        br = 1;
+    }
+    if (quiet) {
+        h = add_zero(h, dh);
+        p1 = add_zero(p1, dp1);
+        p2 = add_zero(p2, dp2);
+    } else {
+        h = h + dh;
+        p1 = p1 + dp1;
+        p2 = p2 + dp2;
+    }
+    if (FZ == 2 ? (rb & 2u) != 0 : lt(h, bdry)) {  // dried out: surface to min(b, 0), at rest
+        h = lt0(b) ? b : 0.0;
+        p1 = 0.0;
+        p2 = 0.0;
+        br |= 2;
+    }
+    o.h = h;
+    o.p1 = p1;
+    o.p2 = p2;
+    o.branch = br;
+    return o;
+}
+
+// A lower bound of the largest key in the warp: its high word.
+__device__ __forceinline__ unsigned long long warp_key_bound(unsigned long long key) {
+    return (unsigned long long)__reduce_max_sync(0xffffffffu, (unsigned)(key >> 32)) << 32;
+}
+
 template <int SOLVER, int FZ = 0>
 __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -328,24 +573,23 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
     // segment's bulk copies land in one buffer while the CTA works on the other
     const bool depth2 = A.stage_depth > 1;
     double* stage = reinterpret_cast<double*>(smem_raw);
-    u64* sh_rh = reinterpret_cast<u64*>(stage + (depth2 ? 8 : 4) * T);  // recip_fix(depth) where the cell is wet
-    double* sh_sq = reinterpret_cast<double*>(sh_rh + T);      // sqrt(g * depth) where the cell is wet
-    double* upd = sh_sq + T;        // [4 quantities][3 local edges][T cells]
-    double* tab_leg = upd + 12 * T; // per depth of the current instance
-    double* tab_hyp = tab_leg + A.max_ndepth;
-    double* tab_vol = tab_hyp + A.max_ndepth;
-    double* tab_ndv = tab_vol + A.max_ndepth;  // -dt / volume
-    double* tab_pow = tab_ndv + A.max_ndepth;  // 2^(d+1)
-    float2* tab_up = reinterpret_cast<float2*>(tab_pow + A.max_ndepth);  // (leg, hyp) rounded up to float
+    SegMem M;
+    M.T = T;
+    M.rh = reinterpret_cast<u64*>(stage + (depth2 ? 8 : 4) * T);
+    M.sq = reinterpret_cast<double*>(M.rh + T);
+    M.upd = M.sq + T;
+    const DepthTab tab(M.upd + 12 * T, A.max_ndepth);
+    M.dep = reinterpret_cast<int8_t*>(tab.up + A.max_ndepth);
     __shared__ uint64_t bar[2];
-    __shared__ double red_min[32];
-    __shared__ unsigned long long red_max[32];
-    __shared__ long long red_sum[32];
+    __shared__ RedSlots red;
+    __shared__ InstParams P;  // the running instance's
     __shared__ unsigned int s_error;
     __shared__ int s_last;
     __shared__ int s_seg;
 
     const int tid = threadIdx.x;
+    // The first segment of CTA k is the k-th to be handed out; the counter deals the rest.
+    int seg = A.seg_order ? __ldg(&A.seg_order[blockIdx.x]) : (int)blockIdx.x;
     const long long step = A.gs->step;
     const long long kseq = step - A.gs->dt_seq_base;
     const int odd = (int)(step & 1);
@@ -353,9 +597,6 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
     const double* hin = A.h[ib];
     const double* huin = A.hu[ib];
     const double* hvin = A.hv[ib];
-    double* hout = A.h[ib ^ 1];
-    double* huout = A.hu[ib ^ 1];
-    double* hvout = A.hv[ib ^ 1];
 
     if (tid == 0) {
         s_error = 0;
@@ -365,13 +606,10 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
     }
     __syncthreads();
 
-    double dtmin = DBL_MAX;  // r_dt_new = huge(1.0) (pre_traversal_op, :133-140)
-    unsigned long long dskey = 0;  // bits of max ds * 2^(d+1) (dt_by_max)
-    long long nref = 0;
+    Reduced r{0ull, 0};
     uint32_t phase = 0;    // bit k: parity of barrier k
     uint32_t pending = 0;  // bit k: bulk copies in flight into buffer k
     int cur = -1;
-    InstParams P;
 
     // Stage segment `sg` into buffer k: bulk copies of the 16-byte multiple (the
     // segment starts at an even cell) completing on barrier k, plain loads for an
@@ -435,20 +673,17 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
     // segments are handed out dynamically (CTAs that draw cheap segments, e.g.
     // dry land, take more), in the order seg_order gives: spread over the
     // domain, so that the CTAs an SM holds at one time mix wet and dry work
-    auto draw = [&]() {
-        const int k = (int)atomicAdd(&A.gs->next_seg, 1u);
-        s_seg = k < A.n_seg ? (A.seg_order ? __ldg(&A.seg_order[k]) : k) : A.n_seg;
+    auto drawn = [&](unsigned int ticket) {
+        const long long k = (long long)gridDim.x + ticket;
+        s_seg = k < A.n_seg ? (A.seg_order ? __ldg(&A.seg_order[k]) : (int)k) : A.n_seg;
     };
-    if (tid == 0) draw();
-    __syncthreads();
-    int seg = s_seg;
     int kbuf = 0;
-    if (seg < A.n_seg) issue(seg, 0);
+    issue(seg, 0);
     while (seg < A.n_seg) {
         int seg_next = A.n_seg;
         if (depth2) {  // draw and stage the next segment before working on this one
             __syncthreads();
-            if (tid == 0) draw();
+            if (tid == 0) drawn(atomicAdd(&A.gs->next_seg, 1u));
             __syncthreads();
             seg_next = s_seg;
             if (seg_next < A.n_seg) issue(seg_next, kbuf ^ 1);
@@ -456,19 +691,22 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
         const int4 si = __ldg(&A.seg_info[seg]);
         const int c0 = si.x, cn = si.y, inst = si.z;
         if (inst != cur) {  // uniform across the CTA
-            if (cur >= 0) flush_instance(A, cur, dtmin, dskey, nref, red_min, red_max, red_sum);
-            P = A.ip[inst];
-            const double dt = step_dt(A, P, inst, kseq);
-            for (int i = tid; i < P.ndepth; i += blockDim.x) {
-                const int d = P.dmin + i;
-                const double vol = (P.scaling * P.scaling) * c_vol[d];
-                const double leg = P.scaling * c_leg[d + 1], hyp = P.scaling * c_leg[d];
-                tab_leg[i] = leg;
-                tab_hyp[i] = hyp;
-                tab_up[i] = make_float2(__double2float_ru(leg), __double2float_ru(hyp));
-                tab_vol[i] = vol;
-                tab_ndv[i] = -dt / vol;
-                tab_pow[i] = ldexp(2.0, d);
+            if (cur >= 0) {
+                flush_instance(A, cur, P.dt_by_max != 0, r, red);
+                __syncthreads();  // P and the slots are read
+            }
+            // the parameters, the rows of the depths and dt come in one round of loads
+            if (tid < (int)(sizeof(InstParams) / 4))
+                reinterpret_cast<int*>(&P)[tid] = __ldg(reinterpret_cast<const int*>(A.ip + inst) + tid);
+            const int nd = __ldg(&A.ip[inst].ndepth);
+            const InstParams* Pg = A.ip + inst;
+            for (int i = tid; i < nd; i += blockDim.x) {
+                tab.load(A, inst, i);
+                double dt = A.is[inst].dt;
+                const double tm = Pg->max_time, to = Pg->tout;
+                if (A.dt_seq && kseq >= 0 && kseq < A.dt_seq_len) dt = A.dt_seq[kseq * A.n_inst + inst];
+                else dt = clamp_dt(dt, tm, to);
+                tab.ndv[i] = div_one(-dt, tab.vol[i]);
             }
             cur = inst;
         }
@@ -476,10 +714,8 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
         wait(kbuf);
         __syncthreads();
         if (s_error) break;
-        double* sh_h = stage + (size_t)kbuf * 4 * T;
-        double* sh_hu = sh_h + T;
-        double* sh_hv = sh_hu + T;
-        double* sh_b = sh_hv + T;
+        M.h = stage + (size_t)kbuf * 4 * T;
+        const double drytol = P.drytol;
         for (int i = tid; i < cn; i += blockDim.x) {
             // depth_terms, with the square root and reciprocal skipped by warps of dry cells.
             // The f-wave path divides only the cell's own (rotated) momenta by its depth:
@@ -489,9 +725,10 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
             // the depth it was last taken for (water at rest keeps its depth from step
             // to step); the memo holds only pairs (d, sqrt(g d)), written by the CTA
             // that owns the cell, so a hit is the value the square root would give
-            const double d = sh_h[i] - sh_b[i];
-            const bool wet = lt(P.drytol, d);
-            const bool need_y = wet && (SOLVER != FWAVE || ((dbits(sh_hu[i]) | dbits(sh_hv[i])) << 1) != 0);
+            M.dep[i] = A.depth[c0 + i];
+            const double d = M.h[i] - M.b()[i];
+            const bool wet = lt(drytol, d);
+            const bool need_y = wet && (SOLVER != FWAVE || ((dbits(M.hu()[i]) | dbits(M.hv()[i])) << 1) != 0);
             double sq = 0.0;
             u64 y = 0;
             bool miss = wet;
@@ -509,15 +746,17 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
                 }
             }
             if (__any_sync(__activemask(), need_y)) y = need_y ? recip_fix(d) : y;
-            sh_rh[i] = y;
-            sh_sq[i] = sq;
+            M.rh[i] = y;
+            M.sq[i] = sq;
         }
         // halo tasks: the cross-edge pass computed these edges' updates; copy
         // this segment's side into its slot
-        const long long t0 = A.seg_ptr[seg], t1 = A.seg_ptr[seg + 1];
-        const long long tm = A.halo_solve ? t1 : t1 - min((long long)max(si.w, 0), t1 - t0);
-        for (long long t = tm + tid; t < t1; t += blockDim.x) {
-            const int4 tk = __ldg(&A.tasks[t]);
+        const long long t0 = __ldg(&A.seg_ptr[seg]);
+        const int nt = (int)(__ldg(&A.seg_ptr[seg + 1]) - t0);
+        const int nm = A.halo_solve ? nt : nt - min(max(si.w, 0), nt);
+        const int4* tasks = A.tasks + t0;
+        for (int t = nm + tid; t < nt; t += blockDim.x) {
+            const int4 tk = __ldg(&tasks[t]);
             const uint32_t meta = (uint32_t)tk.z;
             const int sa = tk.x - c0;
             const bool ain = (unsigned)sa < (unsigned)cn;
@@ -530,195 +769,38 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
             }
             const double2* u = reinterpret_cast<const double2*>(A.xflux + 8 * (long long)(unsigned)tk.w + (ain ? 0 : 4));
             const double2 u0 = u[0], u1 = u[1];
-            upd[(0 * 3 + le) * T + cl] = u0.x;
-            upd[(1 * 3 + le) * T + cl] = u0.y;
-            upd[(2 * 3 + le) * T + cl] = u1.x;
-            upd[(3 * 3 + le) * T + cl] = u1.y;
+            M.upd[(0 * 3 + le) * T + cl] = u0.x;
+            M.upd[(1 * 3 + le) * T + cl] = u0.y;
+            M.upd[(2 * 3 + le) * T + cl] = u1.x;
+            M.upd[(3 * 3 + le) * T + cl] = u1.y;
         }
         __syncthreads();
 
-        // ---- 2. edge tasks (skeleton_scalar_op / bnd_skeleton_scalar_op, :196-255)
-        // each thread loads its next task while it works on the current one
-        int4 tk_next = make_int4(0, 0, 0, 0);
-        if (t0 + tid < tm) tk_next = __ldg(&A.tasks[t0 + tid]);
-        for (long long t = t0 + tid; t < tm; t += blockDim.x) {
-            const int4 tk = tk_next;
-            if (t + blockDim.x < tm) tk_next = __ldg(&A.tasks[t + blockDim.x]);
-            const uint32_t meta = (uint32_t)tk.z;
-            const bool bnd = (meta >> 14) & 1u;
-            int L, R, iL, iR, pL;
-            if (bnd || !odd) {
-                L = tk.x; iL = meta & 3u; pL = (meta >> 4) & 31u;
-                R = tk.y; iR = (meta >> 2) & 3u;
-            } else {
-                L = tk.y; iL = (meta >> 2) & 3u; pL = (meta >> 9) & 31u;
-                R = tk.x; iR = meta & 3u;
-            }
-            if ((unsigned)L >= (unsigned)A.n_cells_total || (!bnd && (unsigned)R >= (unsigned)A.n_cells_total) ||
-                iL > 2 || iR > 2 || pL > 16) {
-                atomicOr(&s_error, 1u);
-                continue;
-            }
-            const double n1 = c_normal[pL][iL][0], n2 = c_normal[pL][iL][1];
-            const int sl = L - c0, sr = R - c0;
-            const bool lin = (unsigned)sl < (unsigned)cn;
-            const bool rin = !bnd && (unsigned)sr < (unsigned)cn;
-            State QL, QR;
-            double dL, dR, sqL, sqR;
-            u64 yL, yR;
-            if (lin) {
-                QL = State{sh_h[sl], sh_hu[sl], sh_hv[sl], sh_b[sl]};
-                dL = QL.h - QL.b;
-                sqL = sh_sq[sl];
-                yL = sh_rh[sl];
-            } else {
-                QL = State{hin[L], huin[L], hvin[L], A.b[L]};
-                depth_terms(QL, P.drytol, dL, sqL, yL);
-            }
-            if (bnd) {  // the ghost has the cell's h and b
-                if (P.bc == BC_SLIP) QR = boundary_ghost<BC_SLIP>(n1, n2, QL);
-                else if (P.bc == BC_NOSLIP) QR = boundary_ghost<BC_NOSLIP>(n1, n2, QL);
-                else QR = QL;
-                dR = dL;
-                sqR = sqL;
-                yR = yL;
-            } else if (rin) {
-                QR = State{sh_h[sr], sh_hu[sr], sh_hv[sr], sh_b[sr]};
-                dR = QR.h - QR.b;
-                sqR = sh_sq[sr];
-                yR = sh_rh[sr];
-            } else {
-                QR = State{hin[R], huin[R], hvin[R], A.b[R]};
-                depth_terms(QR, P.drytol, dR, sqR, yR);
-            }
-            Update fL, fR;
-            edge_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, P.drytol, fL, fR,
-                                  (int)((meta >> 15) & 3u), FZ ? &A.erec[t] : nullptr);
-            if (lin) {
-                upd[(0 * 3 + iL) * T + sl] = fL.h;
-                upd[(1 * 3 + iL) * T + sl] = fL.p1;
-                upd[(2 * 3 + iL) * T + sl] = fL.p2;
-                upd[(3 * 3 + iL) * T + sl] = fL.s;
-            }
-            if (rin) {
-                upd[(0 * 3 + iR) * T + sr] = fR.h;
-                upd[(1 * 3 + iR) * T + sr] = fR.p1;
-                upd[(2 * 3 + iR) * T + sr] = fR.p2;
-                upd[(3 * 3 + iR) * T + sr] = fR.s;
-            }
-        }
+        // ---- 2. edge tasks
+        if (edge_tasks<SOLVER, FZ, false>(A, M, tasks, nm, FZ ? A.erec + t0 : nullptr, c0, cn, odd, drytol, P.bc, hin,
+                                          huin, hvin))
+            atomicOr(&s_error, 1u);
         __syncthreads();
 
-        // ---- 3. cell updates: cell_update_op + volume_op (src/SWE/SWE_euler_timestep.f90:257-355)
+        // ---- 3. cell updates
         // With one staging buffer, thread 0 takes the next segment's ticket now and
         // reads it after its cells, so the atomic's round trip overlaps the updates.
         unsigned int ticket = 0u;
         if (!depth2 && tid == 0) ticket = atomicAdd(&A.gs->next_seg, 1u);
-        const int k0 = odd ? 2 : 0, k2 = odd ? 0 : 2;
-        // the largest CFL key the lanes of this warp have taken so far (dt_by_max);
-        // a cell whose key is certainly below it cannot raise the maximum
-        const unsigned long long wkey = P.dt_by_max ? warp_max_u64(dskey) : 0ull;
+        const unsigned long long wkey = P.dt_by_max ? warp_key_bound(r.key) : 0ull;
+        double* hout = A.h[ib ^ 1];
+        double* huout = A.hu[ib ^ 1];
+        double* hvout = A.hv[ib ^ 1];
         for (int i = tid; i < cn; i += blockDim.x) {
             const int c = c0 + i;
-            const int d = A.depth[c];
-            const int di = d - P.dmin;
-            const double leg = tab_leg[di], hyp = tab_hyp[di], ndv = tab_ndv[di];
-            double u[4][3];
-            long long nz = 0, sz = 0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                u[q][0] = upd[(q * 3 + k0) * T + i];
-                u[q][1] = upd[(q * 3 + 1) * T + i];
-                u[q][2] = upd[(q * 3 + k2) * T + i];
-                (q < 3 ? nz : sz) |= (dbits(u[q][0]) | dbits(u[q][1]) | dbits(u[q][2])) << 1;
-            }
-            // quiet: every update of h, hu, hv is +-0 (dry land, water at rest). Then
-            // each sum below is +0 (positive edge lengths), RN(ndv * +0) is a zero with
-            // ndv's sign, and adding it leaves the state as add_zero says: the same
-            // bits, without the FP64 arithmetic. Water at rest still has wave speeds,
-            // so the speed sum ds has its own test below.
-            const bool quiet = nz == 0 && is_finite(ndv);
-            double dh = 0.0, dp1 = 0.0, dp2 = 0.0, ds = 0.0;
-            if (__any_sync(__activemask(), !quiet)) {
-                if (!quiet) {
-                    dh = z0(prod_cell(leg, u[0][0])) + prod_cell(hyp, u[0][1]);
-                    dh = dh + prod_cell(leg, u[0][2]);
-                    dp1 = z0(prod_cell(leg, u[1][0])) + prod_cell(hyp, u[1][1]);
-                    dp1 = dp1 + prod_cell(leg, u[1][2]);
-                    dp2 = z0(prod_cell(leg, u[2][0])) + prod_cell(hyp, u[2][1]);
-                    dp2 = dp2 + prod_cell(leg, u[2][2]);
-                }
-            }
-            // ds is +0 when every speed is +-0 (dry land) or when the cell's key stays
-            // below wkey (key_below), else it is summed
-            bool need_ds = sz != 0;
-            if (need_ds && wkey != 0ull) need_ds = !key_below(tab_up[di], u[3][0], u[3][1], u[3][2], d + 1, wkey);
-            if (__any_sync(__activemask(), need_ds)) {
-                if (need_ds) {
-                    ds = z0(prod_cell(leg, u[3][0])) + prod_cell(hyp, u[3][1]);
-                    ds = ds + prod_cell(leg, u[3][2]);
-                }
-            }
-            int8_t f = 0;
-            // |dh| > thr and |dh| < thr / 8 on the bit patterns (thresholds are positive;
-            // a NaN |dh| passes neither test, as in IEEE)
-            const long long nrm = abs_bits(dh);
-            if (d < P.max_depth && not_nan(nrm) && nrm > __double_as_longlong(P.thr_refine)) {
-                f = 1;
-                ++nref;
-            } else if (d > P.min_depth && nrm < __double_as_longlong(P.thr_coarsen)) {
-                f = -1;
-            }
-            if (P.dt_by_max) {  // ds >= 0, so its bits order like its value; RN(ds * 2^(d+1))
-                const unsigned long long x = (unsigned long long)dbits(scale_pow2(ds, d + 1, tab_pow[di]));
-                dskey = x > dskey ? x : dskey;
-            } else {
-                dtmin = dmn(dtmin, tab_vol[di] / ds);
-            }
-            if (quiet) {
-                dh = dp1 = dp2 = bitsd(dbits(ndv) & (long long)0x8000000000000000ULL);  // RN(ndv * +0)
-            } else {
-                dh = prod_cell(ndv, dh);
-                dp1 = prod_cell(ndv, dp1);
-                dp2 = prod_cell(ndv, dp2);
-            }
-            double h = sh_h[i], p1 = sh_hu[i], p2 = sh_hv[i];
-            const double b = sh_b[i];
-            uint8_t br = 0;
-            const double bdry = b + P.drytol;
-            const uint8_t rb = FZ == 2 ? A.branch[c] : 0;  // a branch-frozen run takes the recorded fixes
-            // flooded land starts at the dry tolerance, at rest
-            if (FZ == 2 ? (rb & 1u) != 0 : (lt(h, bdry) && gt0(dh))) {
-                h = bdry;
-                p1 = 0.0;
-                p2 = 0.0;
-                br = 1;
-            }
-            if (quiet) {
-                h = add_zero(h, dh);
-                p1 = add_zero(p1, dp1);
-                p2 = add_zero(p2, dp2);
-            } else {
-                h = h + dh;
-                p1 = p1 + dp1;
-                p2 = p2 + dp2;
-            }
-            if (FZ == 2 ? (rb & 2u) != 0 : lt(h, bdry)) {  // dried out: surface to min(b, 0), at rest
-                h = lt0(b) ? b : 0.0;
-                p1 = 0.0;
-                p2 = 0.0;
-                br |= 2;
-            }
-            if (FZ != 2 && A.branch) A.branch[c] = br;
-            hout[c] = h;
-            huout[c] = p1;
-            hvout[c] = p2;
-            A.flags[c] = f;
+            const CellOut o = update_cell<FZ>(M, tab, P, i, odd, wkey, FZ == 2 ? A.branch[c] : (uint8_t)0, r);
+            if (FZ != 2 && A.branch) A.branch[c] = o.branch;
+            hout[c] = o.h;
+            huout[c] = o.p1;
+            hvout[c] = o.p2;
+            A.flags[c] = o.flag;
         }
-        if (!depth2 && tid == 0) {
-            const int k = (int)ticket;
-            s_seg = k < A.n_seg ? (A.seg_order ? __ldg(&A.seg_order[k]) : k) : A.n_seg;
-        }
+        if (!depth2 && tid == 0) drawn(ticket);
         __syncthreads();
         if (!depth2) {  // stage the next segment now
             seg_next = s_seg;
@@ -734,7 +816,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
     }
 
     // ---- 4. reductions and the last-CTA finalisation (post_traversal_grid_op, :111-131)
-    if (cur >= 0) flush_instance(A, cur, dtmin, dskey, nref, red_min, red_max, red_sum);
+    flush_instance(A, cur, P.dt_by_max != 0, r, red);
     if (tid == 0) {
         if (s_error) atomicOr(&A.gs->error, s_error);
         __threadfence();
@@ -744,25 +826,23 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
     if (s_last) {
         __threadfence();
         for (int i = tid; i < A.n_inst; i += blockDim.x) {
-            const InstParams Q = A.ip[i];
-            const double dt = step_dt(A, Q, i, kseq);
+            // past the L1 cache: the other CTAs' atomics wrote the accumulators
             InstScalars* S = &A.is[i];
-            double dtn = __longlong_as_double((long long)atomicAdd(&S->dt_acc, 0ull));
-            const unsigned long long x = atomicAdd(&S->ds_acc, 0ull);
-            if (x) dtn = dmn(dtn, (Q.scaling * Q.scaling) / __longlong_as_double((long long)x));
-            S->time = S->time + dt;
-            S->dt_new = dtn;
-            S->dt = Q.courant * dtn;
-            S->n_refine = atomicExch(&S->refine_acc, 0ull);
+            const InstParams* Q = A.ip + i;
+            const double time = S->time, dt0 = S->dt;
+            const double dt_acc = __longlong_as_double((long long)__ldcg(&S->dt_acc));
+            const unsigned long long x = __ldcg(&S->ds_acc), n = __ldcg(&S->refine_acc);
+            const double dt = A.dt_seq && kseq >= 0 && kseq < A.dt_seq_len ? A.dt_seq[kseq * A.n_inst + i]
+                                                                           : clamp_dt(dt0, Q->max_time, Q->tout);
+            advance_time(S, *Q, time + dt, dt_acc, x, n);
             S->dt_acc = (unsigned long long)__double_as_longlong(DBL_MAX);
             S->ds_acc = 0;
+            S->refine_acc = 0;
         }
-        __syncthreads();
         if (tid == 0) {
             A.gs->done = 0;
             A.gs->next_seg = 0;
             A.gs->step = step + 1;
-            __threadfence();
         }
     }
 }

@@ -111,6 +111,7 @@ __global__ void set_times_kernel(InstScalars* S, const double* t, const double* 
         S[i].dt_acc = (unsigned long long)__double_as_longlong(DBL_MAX);
         S[i].ds_acc = 0;
         S[i].refine_acc = 0;
+        for (int k = 0; k < 3; ++k) S[i].ds_ring[k] = 0;
     }
 }
 
@@ -123,11 +124,13 @@ __global__ void reset_scalars_kernel(InstScalars* S, GlobalScalars* G, int n) {
         S[i].ds_acc = 0;
         S[i].refine_acc = 0;
         S[i].n_refine = 0;
+        for (int k = 0; k < 3; ++k) S[i].ds_ring[k] = 0;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         G->done = 0;
         G->error = 0;
         G->next_seg = 0;
+        G->arrived = 0;
         G->step = 0;
         G->dt_seq_base = 0;
     }
@@ -279,6 +282,8 @@ struct swe_ctx {
     SegInfo* seg_info = nullptr;
     int32_t* seg_order = nullptr;   // hand-out order of the segments (spread over each instance's domain)
     InstParams* ip = nullptr;
+    DepthRow* rows = nullptr;       // [instance][max_ndepth]
+    size_t cap_rows = 0;
     InstScalars* is = nullptr;
     GlobalScalars* gs = nullptr;
     double* dt_seq = nullptr;
@@ -334,6 +339,9 @@ void free_mesh_buffers(swe_ctx* c, bool release = true) {
     cudaFree(c->b); cudaFree(c->depth); cudaFree(c->flags); cudaFree(c->tasks); cudaFree(c->seg_ptr);
     cudaFree(c->seg_info); cudaFree(c->seg_order); cudaFree(c->ip); cudaFree(c->is); cudaFree(c->xtasks); cudaFree(c->xflux);
     cudaFree(c->memo);
+    cudaFree(c->rows);
+    c->rows = nullptr;
+    c->cap_rows = 0;
     c->memo = nullptr;
     c->b = nullptr; c->depth = nullptr; c->flags = nullptr; c->tasks = nullptr; c->seg_ptr = nullptr;
     c->seg_info = nullptr; c->seg_order = nullptr; c->ip = nullptr; c->is = nullptr; c->xtasks = nullptr; c->xflux = nullptr;
@@ -352,8 +360,10 @@ int device_alloc(void** p, size_t bytes) {
 }
 
 size_t smem_bytes_for(int64_t seg_cells, int stage_depth, int max_ndepth) {
-    // staging [depth][4][T], RN(1/depth) and sqrt(g depth) [2][T], edge slots [12][T], depth tables [6][nd]
-    return (size_t)(14 + 4 * stage_depth) * (size_t)seg_cells * sizeof(double) + (size_t)6 * max_ndepth * sizeof(double);
+    // staging [depth][4][T], recip_fix(depth) and sqrt(g depth) [2][T], edge slots [12][T], depth tables [6][nd],
+    // the cells' depths [T] bytes
+    return (size_t)(14 + 4 * stage_depth) * (size_t)seg_cells * sizeof(double) + (size_t)6 * max_ndepth * sizeof(double) +
+           (((size_t)seg_cells + 15) & ~(size_t)15);
 }
 
 size_t smem_bytes(const swe_ctx* c) { return smem_bytes_for(c->seg_cells, c->stage_depth, c->max_ndepth); }
@@ -368,6 +378,12 @@ int check_params(const swe_params* p) {
     if (p->min_depth < 0 || p->max_depth > kMaxDepth || p->min_depth > p->max_depth)
         return set_error(SWE_E_INVALID, "depth limits %d..%d invalid", p->min_depth, p->max_depth);
     return SWE_OK;
+}
+
+// The smallest float that is not below x.
+float float_not_below(double x) {
+    const float f = (float)x;
+    return (double)f < x ? std::nextafterf(f, INFINITY) : f;
 }
 
 int upload_inst_params(swe_ctx* c) {
@@ -394,6 +410,27 @@ int upload_inst_params(swe_ctx* c) {
         const int dmax = c->mesh[(size_t)i].max_depth;
         q.dt_by_max = (std::isfinite(v0) && v0 > 0.0 && std::ldexp(v0, -(dmax + 1)) >= DBL_MIN) ? 1 : 0;
     }
+    std::vector<DepthRow> rows((size_t)n * (size_t)c->max_ndepth);
+    for (int i = 0; i < n; ++i)
+        for (int k = 0; k < v[(size_t)i].ndepth; ++k) {
+            const InstParams& q = v[(size_t)i];
+            const int d = q.dmin + k;
+            DepthRow& row = rows[(size_t)i * (size_t)c->max_ndepth + (size_t)k];
+            row.leg = q.scaling * c->leg[d + 1];
+            row.hyp = q.scaling * c->leg[d];
+            row.vol = (q.scaling * q.scaling) * c->vol[d];
+            row.pow = std::ldexp(2.0, d);
+            row.leg_up = float_not_below(row.leg);
+            row.hyp_up = float_not_below(row.hyp);
+        }
+    if (rows.size() > c->cap_rows) {
+        cudaFree(c->rows);
+        c->rows = nullptr;
+        c->cap_rows = 0;
+        if (int rc = device_alloc((void**)&c->rows, sizeof(DepthRow) * rows.size())) return rc;
+        c->cap_rows = rows.size();
+    }
+    CUDA_TRY(cudaMemcpyAsync(c->rows, rows.data(), sizeof(DepthRow) * rows.size(), cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(cudaMemcpyAsync(c->ip, v.data(), sizeof(InstParams) * v.size(), cudaMemcpyHostToDevice, c->stream));
     c->ip_host = v;
     CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -687,6 +724,7 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     A.xflux = c->xflux;
     A.n_xtasks = c->n_xtasks;
     A.ip = c->ip;
+    A.rows = c->rows;
     A.is = c->is;
     A.gs = c->gs;
     A.dt_seq = c->dt_seq;
