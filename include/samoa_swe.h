@@ -117,7 +117,8 @@ int swe_state_device(swe_ctx* ctx, double** h, double** hu, double** hv, const d
 int swe_set_time(swe_ctx* ctx, double time, double dt);
 int swe_get_time(swe_ctx* ctx, double* time, double* dt, double* dt_new);
 
-/* Run n_steps time steps, asynchronously on the context's stream.
+/* Run n_steps time steps, asynchronously on the context's stream (on small
+ * meshes up to 4096 of them per kernel launch).
  * Replaces n_steps calls of swe%euler%traverse(grid) (src/SWE/SWE.f90:393). */
 int swe_traverse(swe_ctx* ctx, int64_t n_steps);
 
@@ -141,8 +142,9 @@ int swe_last_error(char* buf, size_t n);
  * per block (multiple of 32, 64..256); 0 keeps
  * the current value. A mesh upload or
  * this call rebuilds the segment task lists. Until a segment length is set
- * here, each mesh upload picks it by size: 384 cells from 2^20 cells on, 256
- * below (more segments than resident CTAs on small meshes). */
+ * here, each mesh upload picks it by size: 384 cells on large meshes, 256 on
+ * middling ones, and on meshes that fit the GPU at once two segments per SM (at
+ * least 64 cells); it then picks the threads too, unless they were set. */
 int swe_set_tiling(swe_ctx* ctx, int32_t segment_cells, int32_t block_threads);
 
 /* Staging depth of the step kernel: 1 = a CTA stages a segment's state into
@@ -167,9 +169,11 @@ int swe_get_tiling(swe_ctx* ctx, int32_t* segment_cells, int32_t* block_threads)
 /* How the edges between two segments are solved. PASS: once per step by a
  * kernel before the step kernel, which copies the updates. INKERNEL: by both
  * segments' CTAs, each keeping its side (no extra launch). AUTO (the default):
- * PASS for steps on device-resident state (swe_traverse and the calls built on
- * it), INKERNEL for swe_step_host, whose state is in host memory. The results
- * are bit identical. No reference counterpart. */
+ * PASS for steps on device-resident state of 2^20 cells and more, INKERNEL for
+ * smaller meshes and for swe_step_host, whose state is in host memory; and many
+ * steps of one call on a mesh whose segments all fit the GPU at once run in one
+ * launch that keeps each segment's state on its SM. The results are bit
+ * identical. No reference counterpart. */
 #define SWE_CROSS_AUTO 0
 #define SWE_CROSS_PASS 1
 #define SWE_CROSS_INKERNEL 2
@@ -188,8 +192,8 @@ int swe_set_segment_order(swe_ctx* ctx, int32_t mode);
 
 /* Sizes of the uploaded mesh's work lists: segments, edge tasks in the segment
  * lists (an edge between two segments counted once per segment), edges between
- * two segments (computed once per step by a pass before the step kernel) and
- * kernel launches per device-resident step (1, or 2 with that pass). Any pointer may be null.
+ * two segments (computed once per step where a pass runs before the step kernel)
+ * and kernel launches of a device-resident step (1, or 2 with that pass). Any pointer may be null.
  * No reference counterpart (the reference's sections, src/SFC_edge_traversal.f90). */
 int swe_get_task_counts(swe_ctx* ctx, int64_t* n_segments, int64_t* n_tasks, int64_t* n_cross_edges,
                         int32_t* launches_per_step);

@@ -47,6 +47,7 @@ inline uint32_t pack_meta(int la, int lb, int pa, int pb, bool bnd, int axis = 0
 struct InstParams {
     double drytol, courant, scaling, thr_refine, thr_coarsen, max_time, tout;
     int32_t min_depth, max_depth, dmin, ndepth, bc, dt_by_max;
+    int32_t n_segs, first_seg;  // the instance's segments [first_seg, first_seg + n_segs)
 };
 
 // Per instance and depth (from the instance's dmin on), the values of the cell
@@ -68,14 +69,17 @@ struct InstScalars {
     unsigned long long ds_acc;      // bits of the running maximum of ds * 2^(d+1) (dt_by_max)
     unsigned long long refine_acc;  // refinements issued in the running step
     unsigned long long n_refine;    // refinements issued in the last step
-    unsigned long long ds_ring[3];  // ds_acc of the multi-step kernel, by step modulo 3 (0 between launches)
+    // the multi-step kernel's (0 between launches): ds_acc by step modulo 3, and the
+    // CTAs that have finished a step, counted over the launch's steps
+    unsigned long long ds_ring[3];
+    unsigned int arrived, pad;
 };
 
 struct GlobalScalars {
     unsigned int done;       // CTAs finished in the running step
     unsigned int error;      // nonzero: a kernel saw a bad index or a wait ran out
     unsigned int next_seg;   // segments handed out in the running step beyond each CTA's first
-    unsigned int arrived;    // CTAs that reached the multi-step kernel's barriers in the running launch
+    unsigned int pad;
     long long step;          // steps since the mesh upload (parity = traversal direction)
     long long dt_seq_base;   // step at which the frozen dt sequence starts
 };

@@ -365,87 +365,76 @@ struct SegMem {
     __device__ __forceinline__ double* b() const { return h + 3 * T; }
 };
 
-// Edge tasks [tid, nt) in steps of the CTA (skeleton_scalar_op /
-// bnd_skeleton_scalar_op, src/SWE/SWE_euler_timestep.f90:196-255): the updates of
-// both sides into the slots of the cells in the segment. Each thread loads its
-// next task while it works on the current one. With SHARED_STATE other CTAs
-// write the neighbours' state in this launch, so it is read past the L1 cache.
-// Returns nonzero on a bad index.
+// One edge task (skeleton_scalar_op / bnd_skeleton_scalar_op,
+// src/SWE/SWE_euler_timestep.f90:196-255): the updates of both sides into the
+// slots of the cells in the segment. With SHARED_STATE other CTAs write the
+// neighbours' state in this launch, so it is read past the L1 cache. Returns
+// nonzero on a bad index.
 template <int SOLVER, int FZ, bool SHARED_STATE>
-__device__ __forceinline__ unsigned int edge_tasks(const StepArgs& A, const SegMem& M, const int4* tasks, int nt,
-                                                   uint16_t* erec, int c0, int cn, int odd, double drytol, int bc,
-                                                   const double* hin, const double* huin, const double* hvin) {
-    const int tid = threadIdx.x, T = M.T;
-    unsigned int bad = 0;
-    int4 tk_next = make_int4(0, 0, 0, 0);
-    if (tid < nt) tk_next = __ldg(&tasks[tid]);
-    for (int t = tid; t < nt; t += blockDim.x) {
-        const int4 tk = tk_next;
-        if (t + (int)blockDim.x < nt) tk_next = __ldg(&tasks[t + blockDim.x]);
-        const uint32_t meta = (uint32_t)tk.z;
-        const bool bnd = (meta >> 14) & 1u;
-        int L, R, iL, iR, pL;
-        if (bnd || !odd) {
-            L = tk.x; iL = meta & 3u; pL = (meta >> 4) & 31u;
-            R = tk.y; iR = (meta >> 2) & 3u;
-        } else {
-            L = tk.y; iL = (meta >> 2) & 3u; pL = (meta >> 9) & 31u;
-            R = tk.x; iR = meta & 3u;
-        }
-        if ((unsigned)L >= (unsigned)A.n_cells_total || (!bnd && (unsigned)R >= (unsigned)A.n_cells_total) ||
-            iL > 2 || iR > 2 || pL > 16) {
-            bad = 1u;
-            continue;
-        }
-        const double n1 = c_normal[pL][iL][0], n2 = c_normal[pL][iL][1];
-        const int sl = L - c0, sr = R - c0;
-        const bool lin = (unsigned)sl < (unsigned)cn;
-        const bool rin = !bnd && (unsigned)sr < (unsigned)cn;
-        State QL, QR;
-        double dL, dR, sqL, sqR;
-        u64 yL, yR;
-        auto far = [&](int c, State& Q, double& d, double& sq, u64& y) {
-            if (SHARED_STATE) Q = State{__ldcg(hin + c), __ldcg(huin + c), __ldcg(hvin + c), A.b[c]};
-            else Q = State{hin[c], huin[c], hvin[c], A.b[c]};
-            depth_terms(Q, drytol, d, sq, y);
-        };
-        auto near = [&](int i, State& Q, double& d, double& sq, u64& y) {
-            Q = State{M.h[i], M.hu()[i], M.hv()[i], M.b()[i]};
-            d = Q.h - Q.b;
-            sq = M.sq[i];
-            y = M.rh[i];
-        };
-        if (lin) near(sl, QL, dL, sqL, yL);
-        else far(L, QL, dL, sqL, yL);
-        if (bnd) {  // the ghost has the cell's h and b
-            if (bc == BC_SLIP) QR = boundary_ghost<BC_SLIP>(n1, n2, QL);
-            else if (bc == BC_NOSLIP) QR = boundary_ghost<BC_NOSLIP>(n1, n2, QL);
-            else QR = QL;
-            dR = dL;
-            sqR = sqL;
-            yR = yL;
-        } else if (rin) {
-            near(sr, QR, dR, sqR, yR);
-        } else {
-            far(R, QR, dR, sqR, yR);
-        }
-        Update fL, fR;
-        edge_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, (int)((meta >> 15) & 3u),
-                              FZ ? erec + t : nullptr);
-        if (lin) {
-            M.upd[(0 * 3 + iL) * T + sl] = fL.h;
-            M.upd[(1 * 3 + iL) * T + sl] = fL.p1;
-            M.upd[(2 * 3 + iL) * T + sl] = fL.p2;
-            M.upd[(3 * 3 + iL) * T + sl] = fL.s;
-        }
-        if (rin) {
-            M.upd[(0 * 3 + iR) * T + sr] = fR.h;
-            M.upd[(1 * 3 + iR) * T + sr] = fR.p1;
-            M.upd[(2 * 3 + iR) * T + sr] = fR.p2;
-            M.upd[(3 * 3 + iR) * T + sr] = fR.s;
-        }
+__device__ __forceinline__ unsigned int edge_task(const StepArgs& A, const SegMem& M, const int4 tk, uint16_t* erec,
+                                                  int c0, int cn, int odd, double drytol, int bc, const double* hin,
+                                                  const double* huin, const double* hvin) {
+    const int T = M.T;
+    const uint32_t meta = (uint32_t)tk.z;
+    const bool bnd = (meta >> 14) & 1u;
+    int L, R, iL, iR, pL;
+    if (bnd || !odd) {
+        L = tk.x; iL = meta & 3u; pL = (meta >> 4) & 31u;
+        R = tk.y; iR = (meta >> 2) & 3u;
+    } else {
+        L = tk.y; iL = (meta >> 2) & 3u; pL = (meta >> 9) & 31u;
+        R = tk.x; iR = meta & 3u;
     }
-    return bad;
+    if ((unsigned)L >= (unsigned)A.n_cells_total || (!bnd && (unsigned)R >= (unsigned)A.n_cells_total) || iL > 2 ||
+        iR > 2 || pL > 16)
+        return 1u;
+    const double n1 = c_normal[pL][iL][0], n2 = c_normal[pL][iL][1];
+    const int sl = L - c0, sr = R - c0;
+    const bool lin = (unsigned)sl < (unsigned)cn;
+    const bool rin = !bnd && (unsigned)sr < (unsigned)cn;
+    State QL, QR;
+    double dL, dR, sqL, sqR;
+    u64 yL, yR;
+    auto far = [&](int c, State& Q, double& d, double& sq, u64& y) {
+        if (SHARED_STATE) Q = State{__ldcg(hin + c), __ldcg(huin + c), __ldcg(hvin + c), A.b[c]};
+        else Q = State{hin[c], huin[c], hvin[c], A.b[c]};
+        depth_terms(Q, drytol, d, sq, y);
+    };
+    auto near = [&](int i, State& Q, double& d, double& sq, u64& y) {
+        Q = State{M.h[i], M.hu()[i], M.hv()[i], M.b()[i]};
+        d = Q.h - Q.b;
+        sq = M.sq[i];
+        y = M.rh[i];
+    };
+    if (lin) near(sl, QL, dL, sqL, yL);
+    else far(L, QL, dL, sqL, yL);
+    if (bnd) {  // the ghost has the cell's h and b
+        if (bc == BC_SLIP) QR = boundary_ghost<BC_SLIP>(n1, n2, QL);
+        else if (bc == BC_NOSLIP) QR = boundary_ghost<BC_NOSLIP>(n1, n2, QL);
+        else QR = QL;
+        dR = dL;
+        sqR = sqL;
+        yR = yL;
+    } else if (rin) {
+        near(sr, QR, dR, sqR, yR);
+    } else {
+        far(R, QR, dR, sqR, yR);
+    }
+    Update fL, fR;
+    edge_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, (int)((meta >> 15) & 3u), erec);
+    if (lin) {
+        M.upd[(0 * 3 + iL) * T + sl] = fL.h;
+        M.upd[(1 * 3 + iL) * T + sl] = fL.p1;
+        M.upd[(2 * 3 + iL) * T + sl] = fL.p2;
+        M.upd[(3 * 3 + iL) * T + sl] = fL.s;
+    }
+    if (rin) {
+        M.upd[(0 * 3 + iR) * T + sr] = fR.h;
+        M.upd[(1 * 3 + iR) * T + sr] = fR.p1;
+        M.upd[(2 * 3 + iR) * T + sr] = fR.p2;
+        M.upd[(3 * 3 + iR) * T + sr] = fR.s;
+    }
+    return 0u;
 }
 
 // A cell's new state, its flag and its branch bits (cell_update_op + volume_op,
@@ -776,10 +765,18 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
         }
         __syncthreads();
 
-        // ---- 2. edge tasks
-        if (edge_tasks<SOLVER, FZ, false>(A, M, tasks, nm, FZ ? A.erec + t0 : nullptr, c0, cn, odd, drytol, P.bc, hin,
-                                          huin, hvin))
-            atomicOr(&s_error, 1u);
+        // ---- 2. edge tasks; each thread loads its next task while it works on the current one
+        {
+            int4 next = make_int4(0, 0, 0, 0);
+            if (tid < nm) next = __ldg(&tasks[tid]);
+            for (int t = tid; t < nm; t += blockDim.x) {
+                const int4 tk = next;
+                if (t + (int)blockDim.x < nm) next = __ldg(&tasks[t + blockDim.x]);
+                if (edge_task<SOLVER, FZ, false>(A, M, tk, FZ ? A.erec + t0 + t : nullptr, c0, cn, odd, drytol, P.bc,
+                                                 hin, huin, hvin))
+                    atomicOr(&s_error, 1u);
+            }
+        }
         __syncthreads();
 
         // ---- 3. cell updates
@@ -843,6 +840,192 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
             A.gs->done = 0;
             A.gs->next_seg = 0;
             A.gs->step = step + 1;
+        }
+    }
+}
+
+// Wait (one thread, bounded like the staging wait) until *count reaches target;
+// other CTAs' writes before their arrivals are visible afterwards.
+__device__ __forceinline__ bool wait_count(const unsigned int* count, unsigned int target, unsigned long long wait_ns) {
+    unsigned int polls = 0, v;
+    unsigned long long t0 = 0;
+    while (true) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+        if ((int)(v - target) >= 0) return true;
+        ++polls;
+        if ((polls & 63u) == 1u) {
+            const unsigned long long now = global_ns();
+            if (polls == 1u) t0 = now;
+            else if (now - t0 > wait_ns) return false;
+        }
+        if (polls >= kPollLimit) return false;
+    }
+}
+
+// Many steps of a mesh whose segments all fit the GPU at once, one CTA each, in
+// one cooperative launch: a segment's state stays in its CTA's shared memory from
+// step to step. On such a mesh a step launched by itself is mostly fixed cost (at
+// 2^12 cells 20 us, of which the launch, the staging and the end of the step take
+// about half) and the serial chain of one edge and one cell.
+// The CTAs of an instance meet once per step, and the meeting is split: a CTA
+// writes its new state to global memory, folds its largest CFL key into the
+// instance's and counts itself as arrived; then it solves the edges inside its
+// segment, which need neither neighbours nor the new dt; the warps with halo
+// tasks (solved here by both segments' CTAs) and the warp that prepares dt wait
+// for the count. No CTA passes a count before every CTA of its instance has
+// finished reading the buffer that the next cell updates overwrite, and the ring
+// slot of the key cleared after step k was last read in step k (its next use is
+// in step k + 2, past another meeting).
+// For instances with dt_by_max and a dt from the CFL condition.
+template <int SOLVER>
+__global__ void __launch_bounds__(256) multi_step_kernel(const StepArgs A, const int n_steps) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int T = A.seg_cells, tid = threadIdx.x, bd = blockDim.x;
+    SegMem M;
+    M.T = T;
+    M.h = reinterpret_cast<double*>(smem_raw);
+    M.rh = reinterpret_cast<u64*>(M.h + 4 * T);
+    M.sq = reinterpret_cast<double*>(M.rh + T);
+    M.upd = M.sq + T;
+    const DepthTab tab(M.upd + 12 * T, A.max_ndepth);
+    M.dep = reinterpret_cast<int8_t*>(tab.up + A.max_ndepth);
+    __shared__ RedSlots red;
+    __shared__ InstParams P;
+    __shared__ unsigned int s_error;
+
+    const int seg = (int)blockIdx.x;
+    const int4 si = __ldg(&A.seg_info[seg]);
+    const int c0 = si.x, cn = si.y, inst = si.z;
+    const long long t0 = __ldg(&A.seg_ptr[seg]);
+    const int nt = (int)(__ldg(&A.seg_ptr[seg + 1]) - t0);
+    const int halo = min(max(si.w, 0), nt), nm = nt - halo;
+    const int4* tasks = A.tasks + t0;
+    const long long step0 = A.gs->step;
+    InstScalars* S = &A.is[inst];
+    const int nd = __ldg(&A.ip[inst].ndepth);
+    if (tid < (int)(sizeof(InstParams) / 4))
+        reinterpret_cast<int*>(&P)[tid] = __ldg(reinterpret_cast<const int*>(A.ip + inst) + tid);
+    for (int i = tid; i < nd; i += bd) tab.load(A, inst, i);
+    if (tid == 0) s_error = 0;
+    {
+        const int ib = (int)(step0 & 1);
+        const double *hin = A.h[ib] + c0, *huin = A.hu[ib] + c0, *hvin = A.hv[ib] + c0;
+        for (int i = tid; i < cn; i += bd) {
+            M.h[i] = hin[i];
+            M.hu()[i] = huin[i];
+            M.hv()[i] = hvin[i];
+            M.b()[i] = A.b[c0 + i];
+            M.dep[i] = A.depth[c0 + i];
+        }
+    }
+    // sqrt(g d) and the reciprocal of a cell, as in the step kernel's staging loop; a
+    // cell whose depth kept its bits keeps them (a reciprocal left out while the
+    // cell was at rest is taken when it moves)
+    auto terms = [&](int i, double drytol, bool same_depth) {
+        const double d = M.h[i] - M.b()[i];
+        const bool wet = lt(drytol, d);
+        const bool need_y = wet && (SOLVER != FWAVE || ((dbits(M.hu()[i]) | dbits(M.hv()[i])) << 1) != 0);
+        if (!same_depth) M.sq[i] = wet ? sqrt_fix(kG * d) : 0.0;
+        if (!same_depth || (need_y && M.rh[i] == 0)) M.rh[i] = need_y ? recip_fix(d) : 0;
+    };
+    __syncthreads();
+    const double drytol = P.drytol;
+    for (int i = tid; i < cn; i += bd) terms(i, drytol, false);
+    // the last warp prepares dt; in the instance's first CTA its first lane keeps the time
+    const bool dt_warp = tid >= bd - 32, keeper = tid == bd - 32 && seg == P.first_seg;
+    double time = S->time, dt = S->dt;
+    const unsigned int n_cta = (unsigned int)P.n_segs;
+    __syncthreads();
+
+    int k = 0;
+    for (; k < n_steps; ++k) {
+        const int odd = (int)((step0 + k) & 1);
+        // ---- edges: tid, tid + bd, ... of those inside the segment, then the halo tasks
+        // from the last warp down; dt before a warp's edges if it has none inside
+        const double *hin = A.h[odd], *huin = A.hu[odd], *hvin = A.hv[odd];
+        unsigned int bad = 0;
+        bool met = k == 0;
+        auto meet = [&]() {
+            if (!met && !wait_count(&S->arrived, (unsigned int)k * n_cta, A.wait_ns)) bad = 4u;
+            met = true;
+        };
+        auto prepare_dt = [&]() {
+            meet();
+            if (k > 0) {
+                dt = P.courant * dt_new_of(P, DBL_MAX, __ldcg(&S->ds_ring[(k - 1) % 3]));
+                if (keeper) S->ds_ring[(k + 1) % 3] = 0;
+            }
+            const double c = clamp_dt(dt, P.max_time, P.tout);
+            time = time + c;
+            for (int i = tid - (bd - 32); i < nd; i += 32) tab.ndv[i] = div_one(-c, tab.vol[i]);
+        };
+        if (dt_warp && bd - 32 >= nm) prepare_dt();
+        auto after = [&](int t) {  // the thread's task after t (a task inside the segment)
+            return t + bd < nm ? t + bd : nm + bd - 1 - tid;
+        };
+        int t = tid < nm ? tid : nm + bd - 1 - tid;
+        int4 next = t < nt ? __ldg(&tasks[t]) : make_int4(0, 0, 0, 0);
+        while (t < nt) {
+            if (t >= nm) meet();
+            if (bad) break;
+            const int4 tk = next;
+            t = t < nm ? after(t) : t + bd;
+            if (t < nt) next = __ldg(&tasks[t]);
+            bad = edge_task<SOLVER, 0, true>(A, M, tk, nullptr, c0, cn, odd, drytol, P.bc, hin, huin, hvin);
+        }
+        if (dt_warp && bd - 32 < nm) prepare_dt();
+        if (bad) atomicOr(&s_error, bad);
+        __syncthreads();
+        if (s_error) break;
+
+        // ---- cells
+        Reduced r{0ull, 0};
+        const bool last = k == n_steps - 1;
+        double *hout = A.h[odd ^ 1], *huout = A.hu[odd ^ 1], *hvout = A.hv[odd ^ 1];
+        for (int i = tid; i < cn; i += bd) {
+            const CellOut o = update_cell<0>(M, tab, P, i, odd, 0ull, 0, r);
+            const bool same = dbits(o.h) == dbits(M.h[i]);
+            M.h[i] = o.h;
+            M.hu()[i] = o.p1;
+            M.hv()[i] = o.p2;
+            const int c = c0 + i;
+            hout[c] = o.h;
+            huout[c] = o.p1;
+            hvout[c] = o.p2;
+            if (last) A.flags[c] = o.flag;
+            else terms(i, drytol, same);
+        }
+        warp_reduce(r, red);
+        __syncthreads();
+        if (tid == bd - 32) {  // the last warp has the fewest edges inside the segment
+            const Reduced b = block_reduced(red);
+            if (b.key) atomicMax(&S->ds_ring[k % 3], b.key);
+            if (last && b.nref) atomicAdd(&S->refine_acc, (unsigned long long)b.nref);
+            __threadfence();
+            atomicAdd(&S->arrived, 1u);
+        }
+    }
+    // ---- the instance's scalars, and the counters for the next launch
+    if (keeper && k == n_steps) {
+        if (wait_count(&S->arrived, (unsigned int)n_steps * n_cta, A.wait_ns)) {
+            advance_time(S, P, time, DBL_MAX, __ldcg(&S->ds_ring[(n_steps - 1) % 3]), __ldcg(&S->refine_acc));
+            S->refine_acc = 0;
+        } else {
+            atomicOr(&s_error, 4u);
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        if (s_error) atomicOr(&A.gs->error, s_error);
+        __threadfence();
+        if (atomicAdd(&A.gs->done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            for (int i = 0; i < A.n_inst; ++i) {
+                A.is[i].arrived = 0;
+                for (int q = 0; q < 3; ++q) A.is[i].ds_ring[q] = 0;
+            }
+            A.gs->done = 0;
+            A.gs->step = step0 + n_steps;
         }
     }
 }

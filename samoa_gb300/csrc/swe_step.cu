@@ -112,6 +112,7 @@ __global__ void set_times_kernel(InstScalars* S, const double* t, const double* 
         S[i].ds_acc = 0;
         S[i].refine_acc = 0;
         for (int k = 0; k < 3; ++k) S[i].ds_ring[k] = 0;
+        S[i].arrived = 0;
     }
 }
 
@@ -125,12 +126,12 @@ __global__ void reset_scalars_kernel(InstScalars* S, GlobalScalars* G, int n) {
         S[i].refine_acc = 0;
         S[i].n_refine = 0;
         for (int k = 0; k < 3; ++k) S[i].ds_ring[k] = 0;
+        S[i].arrived = 0;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         G->done = 0;
         G->error = 0;
         G->next_seg = 0;
-        G->arrived = 0;
         G->step = 0;
         G->dt_seq_base = 0;
     }
@@ -218,8 +219,21 @@ static void* cross_kernel_for(int solver) {
     }
 }
 
+static void* multi_kernel_for(int solver) {
+    switch (solver) {
+        case FWAVE: return (void*)multi_step_kernel<FWAVE>;
+        case AUG_RIEMANN: return (void*)multi_step_kernel<AUG_RIEMANN>;
+        case LF: return (void*)multi_step_kernel<LF>;
+        case LF_BATH: return (void*)multi_step_kernel<LF_BATH>;
+        case LLF: return (void*)multi_step_kernel<LLF>;
+        case LLF_BATH: return (void*)multi_step_kernel<LLF_BATH>;
+        default: return nullptr;
+    }
+}
+
 void* fma_step_kernel(int solver);
 void* fma_cross_kernel(int solver);
+void* fma_multi_kernel(int solver);
 cudaError_t fma_upload_tables();
 
 static int upload_tables() {
@@ -250,15 +264,9 @@ struct swe_ctx {
     int64_t cells_packed = 0;      // sum of the instances' cells (host layout)
     bool has_mesh = false, has_state = false;
     // tiling
-    // 384 x 128 until the caller sets a tiling: the best on GB300 where most water
-    // is at rest (2^26 basin 1.16e10 against 1.07e10 at 512; 2^22 adjoint step
-    // 1.15 against 1.17 ms), within 2 % of 512 where it moves (2^22 bowls).
-    // Meshes below 2^20 cells get 256-cell segments: with more cells per segment a
-    // 2^18-cell mesh has too few segments for the ~600 resident CTAs, and a step
-    // takes two segment-times (measured at 2^18: forward step 0.170 -> 0.145 ms,
-    // adjoint step 0.242 -> 0.222 ms against 512).
+    // until the caller sets a tiling, auto_tiling picks both
     int32_t seg_cells = 384, block_threads = 128;
-    bool tiling_set = false;
+    bool tiling_set = false, threads_set = false;
     int32_t stage_depth = 1;                        // segments staged ahead per CTA (1 or 2)
     int32_t arith = SWE_ARITH_STRICT;
     int32_t cross_mode = SWE_CROSS_AUTO;
@@ -267,6 +275,8 @@ struct swe_ctx {
     int64_t n_seg = 0, n_tasks = 0;
     int grid = 0, max_ndepth = 1;
     size_t smem = 0;
+    std::vector<int32_t> first_seg; // of each instance, and n_seg
+    bool multi_fits = false;        // every segment has a CTA of the multi-step kernel on the GPU at once
     // device memory
     double* h[2] = {nullptr, nullptr};
     double* hu[2] = {nullptr, nullptr};
@@ -408,6 +418,8 @@ int upload_inst_params(swe_ctx* c) {
         // RN(scaling^2) * 2^-(d+1) must stay a normal number for the deepest cell
         const double v0 = p.scaling * p.scaling;
         const int dmax = c->mesh[(size_t)i].max_depth;
+        q.first_seg = c->first_seg[(size_t)i];
+        q.n_segs = c->first_seg[(size_t)i + 1] - q.first_seg;
         q.dt_by_max = (std::isfinite(v0) && v0 > 0.0 && std::ldexp(v0, -(dmax + 1)) >= DBL_MIN) ? 1 : 0;
     }
     std::vector<DepthRow> rows((size_t)n * (size_t)c->max_ndepth);
@@ -471,6 +483,12 @@ int configure_launch(swe_ctx* c) {
                          c->block_threads);
     int64_t g = (int64_t)per_sm * c->num_sms;
     c->grid = (int)std::max<int64_t>(1, std::min<int64_t>(g, c->n_seg));
+    c->multi_fits = true;
+    for (void* m : {multi_kernel_for(c->params[0].solver), fma_multi_kernel(c->params[0].solver)}) {
+        if ((rc = raise_smem_limit(m, c->smem))) return rc;
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, m, c->block_threads, c->smem));
+        c->multi_fits = c->multi_fits && c->n_seg <= (int64_t)per_sm * c->num_sms;
+    }
     drop_graphs(c);
     return SWE_OK;
 }
@@ -506,10 +524,12 @@ int rebuild_tasks(swe_ctx* c) {
     std::vector<int64_t> seg_ptr;
     std::vector<SegInfo> seg_info;
     hvec<Task> tasks, xtasks;
+    c->first_seg.assign(1, 0);
     for (int i = 0; i < n_inst(c); ++i) {
         int rc = build_tasks(c->mesh[(size_t)i], c->offset[(size_t)i], i, c->seg_cells, seg_ptr, seg_info, tasks,
                              xtasks);
         if (rc) return rc;
+        c->first_seg.push_back((int32_t)std::min<size_t>(seg_info.size(), INT32_MAX));
     }
     c->n_xtasks = (int64_t)xtasks.size();
     c->n_seg = (int64_t)seg_info.size();
@@ -562,7 +582,7 @@ int rebuild_tasks(swe_ctx* c) {
     if (order.size() != seg_info.size()) return set_error(SWE_E_INVALID, "segment order is not a permutation");
     CUDA_TRY(cudaMemcpyAsync(c->seg_order, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice,
                              c->stream));
-    CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if ((rc = upload_inst_params(c))) return rc;  // they carry the instances' segments
     return configure_launch(c);
 }
 
@@ -576,7 +596,9 @@ int check_device_error(swe_ctx* c) {
         CUDA_TRY(cudaMemsetAsync(&c->gs->error, 0, sizeof(err), c->stream));
         CUDA_TRY(cudaStreamSynchronize(c->stream));
         return set_error(SWE_E_DEVICE, "step kernel reported error 0x%x (%s)", err,
-                         (err & 2u) ? "TMA wait ran out" : "edge task index out of range");
+                         (err & 2u)   ? "TMA wait ran out"
+                         : (err & 4u) ? "wait for the instance's other CTAs ran out"
+                                      : "edge task index out of range");
     }
     return SWE_OK;
 }
@@ -584,6 +606,40 @@ int check_device_error(swe_ctx* c) {
 int current_index(swe_ctx* c, int* idx) {
     *idx = (int)(c->step_mirror & 1);
     return SWE_OK;
+}
+
+// Segment length and block size until the caller sets them, by the cells of all
+// instances (measured on wet/dry bowls and water moving everywhere).
+// Up to 1500 cells per SM a mesh is resident (multi_step_kernel): two CTAs of
+// 256 threads per SM, in segments that give every SM two (2^16 cells, us per step:
+// 216 x 256 27.0, 108 x 128 31.2, 256 x 256 29.7; 2^17: 432 x 256 41, 216 x 128
+// 49), but not below 64 cells, whose edges give one warp to each of an SM's four
+// schedulers (2^12 cells: 64 x 128 12.2, 32 x 64 14.5). Larger meshes take the
+// step kernel: 256 x 256 below 2^19 cells (2^18: 97 against 102 at 128 threads),
+// then 384 x 128 (an ensemble of 5e5 cells: 159 against 169 at 256 x 256; 2^22: 346 against 443 at 256 threads where the water rests, 768
+// against 830 where it moves).
+void auto_tiling(swe_ctx* c) {
+    const int64_t n = c->cells_total, resident = (int64_t)2 * c->num_sms;
+    int32_t seg = 384, threads = 128;
+    if (n <= resident * 750) {
+        seg = (int32_t)std::max<int64_t>(64, ((n + resident - 1) / resident + 1) & ~(int64_t)1);
+        threads = seg > 64 ? 256 : 128;
+    } else if (n < ((int64_t)1 << 19)) {
+        seg = 256;
+        threads = 256;
+    }
+    if (!c->tiling_set) c->seg_cells = seg;
+    if (!c->threads_set && !c->tiling_set) c->block_threads = threads;
+}
+
+// Whether the edges between two segments get a pass of their own before the
+// step kernel (AUTO: for device-resident steps from 2^20 cells on). Below, the
+// pass's launch and its serial chain cost more than solving those edges in both
+// segments' CTAs (us per step: 2^16 cells 49 against 38, 2^18 110 against 97, 2^20
+// 252 against 255); with the state in host memory its scattered reads do.
+bool cross_pass(const swe_ctx* c, bool host_io) {
+    if (c->n_xtasks == 0 || c->cross_mode == SWE_CROSS_INKERNEL) return false;
+    return c->cross_mode == SWE_CROSS_PASS || (!host_io && c->cells_total >= ((int64_t)1 << 20));
 }
 
 // Ingest and upload the instances' meshes (arrays concatenated, indices local to each instance).
@@ -622,7 +678,7 @@ int upload_meshes(swe_ctx* c, int64_t ni, const int64_t* n_cells, const int64_t*
     c->offset.swap(offset);
     c->cells_total = off;
     c->cells_packed = pc;
-    if (!c->tiling_set) c->seg_cells = off < ((int64_t)1 << 20) ? 256 : 384;
+    auto_tiling(c);
     c->max_ndepth = max_nd;
     swe_params p0 = c->params.empty() ? swe_params{} : c->params[0];
     c->params.assign((size_t)ni, p0);
@@ -660,7 +716,7 @@ int upload_meshes(swe_ctx* c, int64_t ni, const int64_t* n_cells, const int64_t*
         CUDA_TRY(cudaMemcpyAsync(c->depth + c->offset[(size_t)i], c->mesh[(size_t)i].depth.data(),
                                  (size_t)c->mesh[(size_t)i].n_cells, cudaMemcpyHostToDevice, c->stream));
     c->has_mesh = true;
-    if ((rc = upload_inst_params(c)) || (rc = rebuild_tasks(c))) {
+    if ((rc = rebuild_tasks(c))) {
         free_mesh_buffers(c);
         return rc;
     }
@@ -743,10 +799,7 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     A.memo = c->memo;
     A.extra_tx = c->inject == SWE_INJECT_STAGING_TX ? 16u : 0u;
     A.wait_ns = c->inject == SWE_INJECT_STAGING_TX ? 20000000ull : kWaitNs;
-    // edges between two segments: a pass before the step kernel for device-resident
-    // steps; solved by both segments' CTAs when the state is in host memory (the
-    // pass's scattered reads of host memory cost more than the duplicated solves)
-    const bool pass = c->n_xtasks > 0 && (c->cross_mode == SWE_CROSS_PASS || (c->cross_mode == SWE_CROSS_AUTO && !io));
+    const bool pass = cross_pass(c, io != nullptr);
     A.halo_solve = pass ? 0 : 1;
     if (io) {
         A.h[0] = io[0]; A.hu[0] = io[1]; A.hv[0] = io[2];
@@ -772,6 +825,31 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     // the cross-edge pass waits mostly on its scattered cell reads: 128-thread CTAs
     // (90 registers) fit 5 per SM, 20 warps, against 2 CTAs of 256 threads
     constexpr int kCrossThreads = 128;
+    // many plain steps of a mesh that fits the GPU at once: the multi-step kernel
+    bool multi = n_steps > 1 && c->multi_fits && !io && !branch && !fz && c->dt_seq_len == 0 && c->stage_depth == 1 &&
+                 c->cross_mode == SWE_CROSS_AUTO && c->inject == SWE_INJECT_NONE;
+    for (const InstParams& q : c->ip_host) multi = multi && q.dt_by_max;
+    if (multi) {
+        constexpr int64_t kMaxSteps = 4096;  // of one launch
+        void* km = fma ? fma_multi_kernel(c->params[0].solver) : multi_kernel_for(c->params[0].solver);
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)c->n_seg);
+        cfg.blockDim = dim3((unsigned)c->block_threads);
+        cfg.dynamicSmemBytes = c->smem;
+        cfg.stream = c->stream;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        for (int64_t s = 0; s < n_steps; s += kMaxSteps) {
+            int ns = (int)std::min<int64_t>(kMaxSteps, n_steps - s);
+            void* margs[] = {&A, &ns};
+            CUDA_TRY(cudaLaunchKernelExC(&cfg, km, margs));
+            if (!c->capturing) c->step_mirror += ns;
+        }
+        return SWE_OK;
+    }
     const unsigned xblocks = pass ? (unsigned)((c->n_xtasks + kCrossThreads - 1) / kCrossThreads) : 0u;
     void* args[] = {&A};
     for (int64_t s = 0; s < n_steps; ++s) {
@@ -911,7 +989,10 @@ int swe_set_tiling(swe_ctx* c, int32_t seg_cells, int32_t block_threads) {
         c->seg_cells = seg_cells;
         c->tiling_set = true;
     }
-    if (block_threads) c->block_threads = block_threads;
+    if (block_threads) {
+        c->block_threads = block_threads;
+        c->threads_set = true;
+    }
     if (!c->has_mesh) return SWE_OK;
     cudaSetDevice(c->device);
     return rebuild_tasks(c);
@@ -969,7 +1050,7 @@ int swe_get_task_counts(swe_ctx* c, int64_t* n_segments, int64_t* n_tasks, int64
     if (n_tasks) *n_tasks = c->n_tasks;
     if (n_cross_edges) *n_cross_edges = c->n_xtasks;
     if (launches_per_step)
-        *launches_per_step = (c->n_xtasks > 0 && c->cross_mode != SWE_CROSS_INKERNEL) ? 2 : 1;
+        *launches_per_step = cross_pass(c, false) ? 2 : 1;
     return SWE_OK;
 }
 
