@@ -558,8 +558,9 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
     } else {  // the same call as geoclaw_solver's, recording the branch decisions
         const u64 yLf = wall_l ? yR0 : yL0, yRf = wall_r ? yL0 : yR0;
         double fwa[3][3];
+        SafeOps so;
         riemann_aug_rec<true>(hL, hR, huL, huR, bL, bR, uL, uR, vL, vR, delphi, sE1, sE2, sqL, sqR, yLf, yRf,
-                              drytol, sw, fwa, &rec);
+                              drytol, sw, fwa, &rec, so);
     }
     // ---------------- reverse (cotangents: products fused into FMAs where they feed a sum; they
     // need no bit-exact agreement, only the forward recompute above does)

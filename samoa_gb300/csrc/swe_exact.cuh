@@ -8,13 +8,19 @@
 // reciprocal), an IEEE square root about 8. Here both take none: the
 // significands are integers, an approximation to about 62 bits comes from the
 // FP32 reciprocal (or reciprocal square root) and one or two Newton steps whose
-// residuals are formed exactly modulo 2^64, and it is rounded to 53 bits. Where
-// it lies so near the midpoint of two doubles that its error could matter, the
-// sign of the exact remainder decides (the usual remainder test of a rounding,
-// as in Muller et al., Handbook of Floating-Point Arithmetic, on "division" and
+// residuals are formed exactly modulo 2^64. Its top 53 bits or their successor
+// are the result, and the sign of the exact remainder against the midpoint
+// between the two says which (the usual remainder test of a rounding, as in
+// Muller et al., Handbook of Floating-Point Arithmetic, on "division" and
 // "square root"; neither a quotient nor a square root of 53-bit significands is
 // ever a midpoint itself). So every result is RN(a / b) or RN(sqrt(x)), bit for
 // bit; operands outside the handled range take the IEEE operation.
+//
+// The cores have no branches: a branch ends a basic block, and with one in every
+// quotient and root the compiler could not overlap their chains (a chain of about
+// 100 to 150 cycles each) with each other or with the FP64 instructions, of
+// which a warp can start one per 64 cycles. FastOps therefore only notes that an
+// operand was out of range, and the caller redoes such an edge with SafeOps.
 //
 // Plain C++ apart from the few shims below, so that the CPU can check it with
 // worst-case errors of the two FP32 approximations.
@@ -24,8 +30,10 @@
 
 #ifdef __CUDACC__
 #define SWE_EXACT_FN __device__ __forceinline__
+#define SWE_EXACT_FN_M __device__ __forceinline__
 #else
 #define SWE_EXACT_FN static inline
+#define SWE_EXACT_FN_M inline
 #endif
 
 namespace swe_exact {
@@ -46,7 +54,6 @@ SWE_EXACT_FN double double_of(u64 v) {
     asm("mov.b64 %0, %1;" : "=d"(r) : "l"(v));
     return r;
 }
-SWE_EXACT_FN u64 mulhi(u64 a, u64 b) { return __umul64hi(a, b); }
 SWE_EXACT_FN float float_of(unsigned v) { return __uint_as_float(v); }
 SWE_EXACT_FN unsigned fbits_of(float x) { return __float_as_uint(x); }
 SWE_EXACT_FN float ffma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
@@ -97,6 +104,24 @@ SWE_EXACT_FN u64 recip_fix(double b) {
     return e - 523u <= 1000u ? y : 0ull;
 }
 
+// RN(a / b) for normal a and b of exponents within [-500, 500], y = recip_fix(b).
+SWE_EXACT_FN double quot_core(u64 ua, u64 ub, u64 y) {
+    // the quotient of the significands times 2^63, low by less than 5 or high by less
+    // than 1 (the lowest partial product is left out), then normalised to [2^63, 2^64)
+    const unsigned ah = (unsigned)(ua >> 21) | 0x80000000u, al = (unsigned)ua << 11;
+    const unsigned yh = (unsigned)(y >> 32), yl = (unsigned)y;
+    u64 q = (u64)ah * yh + (((u64)ah * yl >> 32) + ((u64)al * yh >> 32));
+    const unsigned s = (unsigned)(q >> 63);
+    q <<= 1u - s;
+    // r or r + 1, r = q >> 11: by the sign of a 2^(54 - s) - b (2 r + 1), below 2^54 in
+    // magnitude, from its bits modulo 2^64
+    const u64 mb = (ub & 0x000fffffffffffffull) | 0x0010000000000000ull;
+    const u64 p = mb * ((q >> 10) | 1u);
+    const unsigned up = ((unsigned)(p >> 32) - ((unsigned)ua << (22u - s))) >> 31;
+    const unsigned e = ((unsigned)(ua >> 52) & 0x7ffu) - ((unsigned)(ub >> 52) & 0x7ffu) + 1021u + s;
+    return double_of((((u64)e << 52) + ((q >> 11) + up)) | ((ua ^ ub) & 0x8000000000000000ull));
+}
+
 // RN(a / b) from y = recip_fix(b).
 SWE_EXACT_FN double div_fix(double a, double b, u64 y) {
     const u64 ua = bits_of(a), ub = bits_of(b);
@@ -105,20 +130,7 @@ SWE_EXACT_FN double div_fix(double a, double b, u64 y) {
         if ((ua << 1) == 0 && eb - 1u < 2046u) return double_of((ua ^ ub) & 0x8000000000000000ull);  // +-0 / b
         return ieee_div(a, b);
     }
-    // the quotient of the significands times 2^63, error in (-3, 1); then normalised
-    // to [2^63, 2^64), error in (-6, 2)
-    u64 q = mulhi((ua << 11) | 0x8000000000000000ull, y);
-    const unsigned s = (unsigned)(q >> 63);
-    q <<= 1u - s;
-    u64 r = (q >> 11) + (((unsigned)q >> 10) & 1u);  // equal significands: q may be 2^64 - 2
-    if (((unsigned)q & 0x7ffu) - 0x3fau <= 8u) {  // q + (-2, 6) may hold a midpoint: the remainder's sign
-        const u64 ma = (ua & 0x000fffffffffffffull) | 0x0010000000000000ull;
-        const u64 mb = (ub & 0x000fffffffffffffull) | 0x0010000000000000ull;
-        r = q >> 11;
-        r += (s64)((ma << (54u - s)) - mb * (2u * r + 1u)) > 0 ? 1u : 0u;
-    }
-    const u64 e = (u64)(ea - eb + 1021u + s) << 52;
-    return double_of((e + r) | ((ua ^ ub) & 0x8000000000000000ull));
+    return quot_core(ua, ub, y);
 }
 
 // RN(a / b) for a divisor of its own.
@@ -134,12 +146,10 @@ SWE_EXACT_FN double recip_near(double b, u64 y) {
     return double_of((((u64)(2044u - eb) << 52) + r) | (ub & 0x8000000000000000ull));
 }
 
-// RN(sqrt(x)).
-SWE_EXACT_FN double sqrt_fix(double x) {
-    const u64 ux = bits_of(x);
+// RN(sqrt(x)) for a positive normal x.
+SWE_EXACT_FN double root_core(u64 ux) {
     const unsigned hi = (unsigned)(ux >> 32), lo = (unsigned)ux;
-    const unsigned e = hi >> 20;  // with the sign bit: negative x fails the range test
-    if (e - 1u >= 2046u) return (ux << 1) == 0 ? x : ieee_sqrt(x);
+    const unsigned e = hi >> 20;
     // x = M 4^k with M in [1, 4): M 2^52 is m
     const unsigned odd = (e & 1u) ^ 1u;
     const u64 m = ((ux & 0x000fffffffffffffull) | 0x0010000000000000ull) << odd;
@@ -157,13 +167,58 @@ SWE_EXACT_FN double sqrt_fix(double x) {
     const s64 d2 = (s64)((m << 32) - s2 * s2);
     const s64 c = (s64)(int)(d2 >> 14) * (s64)(int)(fbits_of(r0) - 0x3e800000u);
     const u64 s = (s2 << 21) + (u64)(c >> 32);  // error within 3
-    u64 r = (s >> 11) + (((unsigned)s >> 10) & 1u);
-    if (((unsigned)s & 0x7ffu) - 0x3fcu <= 8u) {  // s + [-4, 4] may hold a midpoint: the remainder's sign
-        r = s >> 11;
-        const u64 h = 2u * r + 1u;
-        r += (s64)((m << 54) - h * h) > 0 ? 1u : 0u;
-    }
-    return double_of(((u64)((e + 1021u - odd) >> 1) << 52) + r);
+    // r or r + 1, r = s >> 11: by the sign of M 2^106 - (2 r + 1)^2
+    const u64 h = (s >> 10) | 1u, p = h * h;
+    const unsigned up = ((unsigned)(p >> 32) - ((unsigned)m << 22)) >> 31;
+    return double_of(((u64)((e + 1021u - odd) >> 1) << 52) + ((s >> 11) + up));
 }
+
+// RN(sqrt(x)).
+SWE_EXACT_FN double sqrt_fix(double x) {
+    const u64 ux = bits_of(x);
+    // with the sign bit: negative x fails the range test
+    if ((unsigned)(ux >> 52) - 1u >= 2046u) return (ux << 1) == 0 ? x : ieee_sqrt(x);
+    return root_core(ux);
+}
+
+// A divisor with its reciprocal (recip_fix; 0 where it was left out or is out of range).
+struct Recip {
+    double b;
+    u64 y;
+};
+SWE_EXACT_FN Recip recip_of(double b) { return Recip{b, recip_fix(b)}; }
+
+// The quotients and roots of a formula, for every operand.
+struct SafeOps {
+    static constexpr bool kFast = false;
+    bool ok = true;
+    SWE_EXACT_FN_M double div(double a, const Recip& r) { return div_fix(a, r.b, r.y); }
+    SWE_EXACT_FN_M double div1(double a, double b) { return div_one(a, b); }
+    // a / b where `use`, b a depth above a tolerance >= 0; else any value
+    SWE_EXACT_FN_M double div_if(bool use, double a, const Recip& r) { return use ? div_fix(a, r.b, r.y) : 0.0; }
+    SWE_EXACT_FN_M double sqrt(double x) { return sqrt_fix(x); }
+};
+
+// The same without branches; ok is false after an operand that SafeOps has to take.
+struct FastOps {
+    static constexpr bool kFast = true;
+    bool ok = true;
+    SWE_EXACT_FN_M double quot(bool use, bool zero_free, double a, const Recip& r) {
+        const u64 ua = bits_of(a), ub = bits_of(r.b);
+        const bool zero = (ua << 1) == 0;
+        const bool in = ((unsigned)(ua >> 52) & 0x7ffu) - 523u <= 1000u;
+        ok = ok && (!use || (zero ? (zero_free || r.y != 0) : (in && r.y != 0)));
+        const double q = quot_core(ua, ub, r.y);
+        return zero ? double_of((ua ^ ub) & 0x8000000000000000ull) : q;
+    }
+    SWE_EXACT_FN_M double div(double a, const Recip& r) { return quot(true, false, a, r); }
+    SWE_EXACT_FN_M double div1(double a, double b) { return quot(true, false, a, recip_of(b)); }
+    SWE_EXACT_FN_M double div_if(bool use, double a, const Recip& r) { return quot(use, true, a, r); }
+    SWE_EXACT_FN_M double sqrt(double x) {
+        const u64 ux = bits_of(x);
+        ok = ok && (unsigned)(ux >> 52) - 1u < 2046u;
+        return root_core(ux);
+    }
+};
 
 }  // namespace swe_exact

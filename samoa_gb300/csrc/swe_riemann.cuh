@@ -124,16 +124,9 @@ __device__ __forceinline__ double scale_pow2(double x, int k, double p) {
     return mul_here(x, p);
 }
 
-// ---------------------------------------------------------------------------
 // Several quotients in the step share a divisor (a cell's depth divides its
 // edges' normal and tangential momenta; the two f-wave coefficients share
-// s2 - s1): the divisor with its reciprocal (recip_fix; 0 where it is left out or
-// out of range, and div_fix then takes the IEEE division).
-struct Recip {
-    double b;
-    u64 y;
-};
-__device__ __forceinline__ Recip recip_of(double b) { return Recip{b, recip_fix(b)}; }
+// s2 - s1): a Recip is the divisor with its reciprocal (swe_exact.cuh).
 __device__ __forceinline__ double div_rn(double a, const Recip& r) { return div_fix(a, r.b, r.y); }
 // 1 / b to about half an ulp, for cotangents, which need no correct rounding
 __device__ __forceinline__ double rcp_near(double b) { return recip_near(b, recip_fix(b)); }
@@ -142,10 +135,28 @@ __device__ __forceinline__ double rcp_near(double b) { return recip_near(b, reci
 __device__ __forceinline__ bool le(double a, double b) {  // a <= b
     return !is_nan(a) && !is_nan(b) && ord_key(a) <= ord_key(b);
 }
+// The predicates on numbers, for FastOps formulas: a NaN operand gives any answer
+// there, and the formula is then redone (FastOps::ok is false: every value
+// compared reaches a divisor, a dividend or a root, and none of those takes a NaN).
+__device__ __forceinline__ long long num_key(double x) {
+    const long long b = dbits(x), m = b & 0x7fffffffffffffffLL, t = b >> 63;
+    return (m ^ t) - t;
+}
+template <class Ops>
+__device__ __forceinline__ bool olt(double a, double b) { return Ops::kFast ? num_key(a) < num_key(b) : lt(a, b); }
+template <class Ops>
+__device__ __forceinline__ bool ole(double a, double b) { return Ops::kFast ? num_key(a) <= num_key(b) : le(a, b); }
+template <class Ops>
+__device__ __forceinline__ bool olt0(double x) {
+    return Ops::kFast ? dbits(x) < 0 && (dbits(x) << 1) != 0 : lt0(x);
+}
+template <class Ops>
+__device__ __forceinline__ bool ogt0(double x) { return Ops::kFast ? dbits(x) > 0 : gt0(x); }
+template <class Ops>
+__device__ __forceinline__ double omin(double a, double b) { return olt<Ops>(a, b) ? a : b; }
+template <class Ops>
+__device__ __forceinline__ double omax(double a, double b) { return olt<Ops>(b, a) ? a : b; }
 __device__ __forceinline__ double iabs(double x) { return bitsd(abs_bits(x)); }  // fabs
-
-// RN(1 / h) from y = recip_fix(h) (0: the IEEE division).
-__device__ __forceinline__ double inv_of(double h, u64 y) { return div_fix(1.0, h, y); }
 
 // The branch decisions of one augmented-solver evaluation, for its reverse
 // (the discrete adjoint re-evaluates the values; the decisions fix the branch).
@@ -165,21 +176,21 @@ struct AugRec {
 // sqL / sqR are sqrt(g * hL) and sqrt(g * hR) (the caller's, the same operands
 // and so the same bits as computing them here); yL / yR are recip_fix of hL / hR
 // (0: the IEEE division).
-template <bool REC>
+template <bool REC, class Ops>
 __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, double uL, double uR, double drytol,
                                                      double sqL, double sqR, u64 yL, u64 yR, double& hm, double& s1m, double& s2m,
-                                                     AugRec* rec) {
+                                                     AugRec* rec, Ops& o) {
     const double g = kG;
-    const bool r_lower = lt(hR, hL);  // h_min = dmn(hR, hL) is hR
+    const bool r_lower = olt<Ops>(hR, hL);  // h_min = dmn(hR, hL) is hR
     const double h_min = r_lower ? hR : hL, sq_min = r_lower ? sqR : sqL;
-    const bool r_higher = lt(hL, hR);  // h_max = dmx(hR, hL) is hR
+    const bool r_higher = olt<Ops>(hL, hR);  // h_max = dmx(hR, hL) is hR
     const double h_max = r_higher ? hR : hL, sq_max = r_higher ? sqR : sqL;
     if (REC) {
         rec->lowR = r_lower;
         rec->highR = r_higher;
     }
     double delu = uR - uL;
-    if (le(h_min, drytol)) {
+    if (ole<Ops>(h_min, drytol)) {
         if (REC) rec->rs = 0;
         hm = 0.0;
         double t = ((uR + uL) - scale_pow2(sqR, 1, 2.0)) + scale_pow2(sqL, 1, 2.0);
@@ -189,50 +200,50 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
     }
     double F_min = delu + scale_pow2(sq_min - sq_max, 1, 2.0);
     double F_max = 0.0;  // needed only when F_min <= 0
-    if (!gt0(F_min)) F_max = delu + (h_max - h_min) * sqrt_fix(div_one((0.5 * g) * (h_max + h_min), h_max * h_min));
-    if (gt0(F_min)) {  // two rarefactions
+    if (!ogt0<Ops>(F_min)) F_max = delu + (h_max - h_min) * o.sqrt(o.div1((0.5 * g) * (h_max + h_min), h_max * h_min));
+    if (ogt0<Ops>(F_min)) {  // two rarefactions
         const double t0 = -delu + scale_pow2(sqL + sqR, 1, 2.0);
-        double t = imax(0.0, t0);
+        double t = omax<Ops>(0.0, t0);
         if (REC) {
             rec->rs = 1;
-            rec->t_pos = !lt(t0, 0.0);
+            rec->t_pos = !olt<Ops>(t0, 0.0);
         }
         hm = (1.0 / (16.0 * g)) * (t * t);
-        const double sqm = sqrt_fix(g * hm);
+        const double sqm = o.sqrt(g * hm);
         s1m = (uL + scale_pow2(sqL, 1, 2.0)) - 3.0 * sqm;
         s2m = (uR - scale_pow2(sqR, 1, 2.0)) + 3.0 * sqm;
-    } else if (le(F_max, 0.0)) {  // two shocks: one Newton step on sqrt(h)
+    } else if (ole<Ops>(F_max, 0.0)) {  // two shocks: one Newton step on sqrt(h)
         if (REC) rec->rs = 2;
         double h0 = h_max;
-        const double i0 = r_higher ? inv_of(hR, yR) : inv_of(hL, yL);
-        const double iL = inv_of(hL, yL), iR = inv_of(hR, yR);
-        double gL = sqrt_fix((0.5 * g) * (i0 + iL));
-        double gR = sqrt_fix((0.5 * g) * (i0 + iR));
+        const double i0 = r_higher ? o.div(1.0, Recip{hR, yR}) : o.div(1.0, Recip{hL, yL});
+        const double iL = o.div(1.0, Recip{hL, yL}), iR = o.div(1.0, Recip{hR, yR});
+        double gL = o.sqrt((0.5 * g) * (i0 + iL));
+        double gR = o.sqrt((0.5 * g) * (i0 + iR));
         double F0 = (delu + (h0 - hL) * gL) + (h0 - hR) * gR;
-        double dfdh = ((gL - div_one(g * (h0 - hL), (4.0 * (h0 * h0)) * gL)) + gR) -
-                      div_one(g * (h0 - hR), (4.0 * (h0 * h0)) * gR);
-        const double sq0 = sqrt_fix(h0);
+        double dfdh = ((gL - o.div1(g * (h0 - hL), (4.0 * (h0 * h0)) * gL)) + gR) -
+                      o.div1(g * (h0 - hR), (4.0 * (h0 * h0)) * gR);
+        const double sq0 = o.sqrt(h0);
         double slope = scale_pow2(sq0, 1, 2.0) * dfdh;
-        double t = sq0 - div_one(F0, slope);
+        double t = sq0 - o.div1(F0, slope);
         hm = t * t;
-        const double im = div_one(1.0, hm);
-        double u1m = uL - (hm - hL) * sqrt_fix((0.5 * g) * (im + iL));
-        double u2m = uR + (hm - hR) * sqrt_fix((0.5 * g) * (im + iR));
-        const double sqm = sqrt_fix(g * hm);
+        const double im = o.div1(1.0, hm);
+        double u1m = uL - (hm - hL) * o.sqrt((0.5 * g) * (im + iL));
+        double u2m = uR + (hm - hR) * o.sqrt((0.5 * g) * (im + iR));
+        const double sqm = o.sqrt(g * hm);
         s1m = u1m - sqm;
         s2m = u2m + sqm;
     } else {  // one shock, one rarefaction
         if (REC) {
             rec->rs = 3;
-            rec->lhigh = lt(hR, hL);
+            rec->lhigh = olt<Ops>(hR, hL);
         }
         double h0 = h_min;
-        const double i0 = r_lower ? inv_of(hR, yR) : inv_of(hL, yL);
-        double F0 = (delu + scale_pow2(sq_min - sq_max, 1, 2.0)) + (h0 - h_min) * sqrt_fix((0.5 * g) * (i0 + i0));
-        double slope = div_one(F_max - F0, h_max - h_min);
-        hm = h0 - div_one(F0, slope);
-        const double sqm = sqrt_fix(g * hm);
-        if (lt(hR, hL)) {
+        const double i0 = r_lower ? o.div(1.0, Recip{hR, yR}) : o.div(1.0, Recip{hL, yL});
+        double F0 = (delu + scale_pow2(sq_min - sq_max, 1, 2.0)) + (h0 - h_min) * o.sqrt((0.5 * g) * (i0 + i0));
+        double slope = o.div1(F_max - F0, h_max - h_min);
+        hm = h0 - o.div1(F0, slope);
+        const double sqm = o.sqrt(g * hm);
+        if (olt<Ops>(hR, hL)) {
             s1m = (uL + scale_pow2(sqL, 1, 2.0)) - 3.0 * sqm;
             s2m = (uL + scale_pow2(sqL, 1, 2.0)) - sqm;
         } else {
@@ -240,11 +251,6 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
             s1m = (uR - scale_pow2(sqR, 1, 2.0)) + sqm;
         }
     }
-}
-
-__device__ __forceinline__ void riemann_structure_core(double hL, double hR, double uL, double uR, double drytol,
-                                                      double sqL, double sqR, u64 yL, u64 yR, double& hm, double& s1m, double& s2m) {
-    riemann_structure_rec<false>(hL, hR, uL, uR, drytol, sqL, sqR, yL, yR, hm, s1m, s2m, nullptr);
 }
 
 // The middle depth riemanntype gives for a wet side against its own mirror image
@@ -262,7 +268,8 @@ static __device__ __noinline__ double wall_depth(double h, double u, double sq, 
     if (y == 0) y = recip_fix(h);  // left out for a cell at rest
     if (y == 0) {
         double hm, s1m, s2m;
-        riemann_structure_core(h, h, u, -u, drytol, sq, sq, y, y, hm, s1m, s2m);
+        SafeOps o;
+        riemann_structure_rec<false>(h, h, u, -u, drytol, sq, sq, y, y, hm, s1m, s2m, nullptr, o);
         return hm;
     }
     const double delu = -u - u;
@@ -271,7 +278,7 @@ static __device__ __noinline__ double wall_depth(double h, double u, double sq, 
         t = imax(0.0, -delu + scale_pow2(sq + sq, 1, 2.0));
         return (1.0 / (16.0 * kG)) * (t * t);
     }
-    const double i = inv_of(h, y);
+    const double i = div_fix(1.0, h, y);
     const double gL = sqrt_fix((0.5 * kG) * (i + i));
     const double sq0 = sqrt_fix(h);
     t = sq0 - div_one(delu, scale_pow2(sq0, 1, 2.0) * (gL + gL));
@@ -309,23 +316,23 @@ __device__ __forceinline__ bool moderate(double x) { return abs_bits(x) < 0x52b0
 // f-waves, whose zeros the net-update accumulation turns into +0, except as a
 // divisor: a zero determinant, and operands that are not finite or so large
 // that a product could overflow, take the source's full expressions.
-template <bool REC>
+template <bool REC, class Ops>
 __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL, double huR, double bL, double bR,
                                                double uL, double uR, double vL, double vR, double delphi,
                                                double sE1, double sE2, double sqL, double sqR, u64 yL,
                                                u64 yR, double drytol, double sw[3],
-                                               double fw[3][3], AugRec* rec) {
+                                               double fw[3][3], AugRec* rec, Ops& o) {
     const double g = kG;
     double delh = hR - hL;
     double delhu = huR - huL;
     double delb = bR - bL;
     double hm, s1m, s2m;
-    riemann_structure_rec<REC>(hL, hR, uL, uR, drytol, sqL, sqR, yL, yR, hm, s1m, s2m, rec);
-    double l0 = imin(sE1, s2m);
-    double l2 = imax(sE2, s1m);
+    riemann_structure_rec<REC>(hL, hR, uL, uR, drytol, sqL, sqR, yL, yR, hm, s1m, s2m, rec, o);
+    double l0 = omin<Ops>(sE1, s2m);
+    double l2 = omax<Ops>(sE2, s1m);
     if (REC) {
-        rec->l0_sE1 = lt(sE1, s2m);
-        rec->l2_sE2 = lt(s1m, sE2);
+        rec->l0_sE1 = olt<Ops>(sE1, s2m);
+        rec->l2_sE2 = olt<Ops>(s1m, sE2);
         rec->s1m = s1m;
         rec->s2m = s2m;
     }
@@ -335,32 +342,32 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
     // reciprocal serves hstarHLL's divisor and the Cramer determinant
     const double dsp = sE2 - sE1;
     const Recip rsp = recip_of(dsp);
-    const double hq = div_rn(((huL - huR) + sE2 * hR) - sE1 * hL, rsp);
-    double hstarHLL = imax(hq, 0.0);
+    const double hq = o.div(((huL - huR) + sE2 * hR) - sE1 * hL, rsp);
+    double hstarHLL = omax<Ops>(hq, 0.0);
     double l1 = scale_pow2(l0 + l2, -1, 0.5);
-    if (lt(iabs(l1), 1e-20)) l1 = 0.0;
+    if (olt<Ops>(iabs(l1), 1e-20)) l1 = 0.0;
     const double r20 = l0 * l0, r22 = l2 * l2;
 
     const double ct = 1e-6;
     const double hhalf = scale_pow2(hL + hR, -1, 0.5);
-    double hbar = imax(hhalf, 0.0);
+    double hbar = omax<Ops>(hhalf, 0.0);
     double su = uL + uR;
     const double ghbar = g * hbar;
     double s1s2bar = scale_pow2(su * su, -2, 0.25) - ghbar;
     const double uLR = uL * uR;
-    double s1s2tilde = imax(0.0, uLR) - ghbar;
-    bool sonic = le(iabs(s1s2bar), ct);
-    sonic |= le(s1s2bar * s1s2tilde, ct);
-    sonic |= le((s1s2bar * sE1) * sE2, ct);
-    sonic |= lt(imin(iabs(sE1), iabs(sE2)), ct);
-    sonic |= lt0(sE1) && gt0(s1m);
-    sonic |= gt0(sE2) && lt0(s2m);
-    sonic |= lt0((uL + sqL) * (uR + sqR));  // sqrt(g * h) of the fixed-up depths
-    sonic |= lt0((uL - sqL) * (uR - sqR));
+    double s1s2tilde = omax<Ops>(0.0, uLR) - ghbar;
+    bool sonic = ole<Ops>(iabs(s1s2bar), ct);
+    sonic |= ole<Ops>(s1s2bar * s1s2tilde, ct);
+    sonic |= ole<Ops>((s1s2bar * sE1) * sE2, ct);
+    sonic |= olt<Ops>(omin<Ops>(iabs(sE1), iabs(sE2)), ct);
+    sonic |= olt0<Ops>(sE1) && ogt0<Ops>(s1m);
+    sonic |= ogt0<Ops>(sE2) && olt0<Ops>(s2m);
+    sonic |= olt0<Ops>((uL + sqL) * (uR + sqR));  // sqrt(g * h) of the fixed-up depths
+    sonic |= olt0<Ops>((uL - sqL) * (uR - sqR));
     if (REC) {
-        rec->hst_pos = lt(0.0, hq);
-        rec->hbar_pos = lt(0.0, hhalf);
-        rec->tilde_x = !lt(uLR, 0.0);
+        rec->hst_pos = olt<Ops>(0.0, hq);
+        rec->hbar_pos = olt<Ops>(0.0, hhalf);
+        rec->tilde_x = !olt<Ops>(uLR, 0.0);
         rec->sonic = sonic;
         rec->dcase = 0;
     }
@@ -372,44 +379,44 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
         deldelphi = flip(ghbar * delb, true);
     } else {
         const Recip rb = recip_of(s1s2bar);
-        deldelh = div_rn(dgh, rb);
-        deldelphi = flip(div_rn(dgh * s1s2tilde, rb), true);
+        deldelh = o.div(dgh, rb);
+        deldelphi = flip(o.div(dgh * s1s2tilde, rb), true);
     }
     const double hsd = hstarHLL * dsp;
     int dcase = 0;
     double lo = 0.0, hi = 0.0;  // the two bounds of the case
-    if (lt(sE1, -ct) && lt(ct, sE2)) {
+    if (olt<Ops>(sE1, -ct) && olt<Ops>(ct, sE2)) {
         dcase = 1;
-        hi = div_one(hsd, sE2);
-        lo = div_one(hsd, sE1);
-    } else if (le(ct, sE1)) {
+        hi = o.div1(hsd, sE2);
+        lo = o.div1(hsd, sE1);
+    } else if (ole<Ops>(ct, sE1)) {
         dcase = 2;
-        hi = div_one(hsd, sE1);
+        hi = o.div1(hsd, sE1);
         lo = flip(hL, true);
-    } else if (le(sE2, -ct)) {
+    } else if (ole<Ops>(sE2, -ct)) {
         dcase = 3;
         hi = hR;
-        lo = div_one(hsd, sE2);
+        lo = o.div1(hsd, sE2);
     }
     if (dcase) {
-        const double x1 = imin(deldelh, hi);
+        const double x1 = omin<Ops>(deldelh, hi);
         if (REC) {
             rec->dcase = (int8_t)dcase;
-            rec->dd_min_first = lt(deldelh, hi);
-            rec->dd_max_first = lt(lo, x1);
+            rec->dd_min_first = olt<Ops>(deldelh, hi);
+            rec->dd_max_first = olt<Ops>(lo, x1);
         }
-        deldelh = imax(x1, lo);
+        deldelh = omax<Ops>(x1, lo);
     }
     const double pl = flip(hL * delb, true), pr = flip(hR * delb, true);
-    const double gmx = g * imax(pl, pr), gmn = g * imin(pl, pr);
-    const double y1 = imin(deldelphi, gmx);
+    const double gmx = g * omax<Ops>(pl, pr), gmn = g * omin<Ops>(pl, pr);
+    const double y1 = omin<Ops>(deldelphi, gmx);
     if (REC) {
-        rec->ph_mx_pl = lt(pr, pl);
-        rec->ph_min_first = lt(deldelphi, gmx);
-        rec->ph_mn_pl = lt(pl, pr);
-        rec->ph_max_first = lt(gmn, y1);
+        rec->ph_mx_pl = olt<Ops>(pr, pl);
+        rec->ph_min_first = olt<Ops>(deldelphi, gmx);
+        rec->ph_mn_pl = olt<Ops>(pl, pr);
+        rec->ph_max_first = olt<Ops>(gmn, y1);
     }
-    deldelphi = imax(y1, gmn);
+    deldelphi = omax<Ops>(y1, gmn);
     double d0 = delh - deldelh, d1 = delhu, d2 = delphi - deldelphi;
 
     double beta0, beta1, beta2;
@@ -418,11 +425,12 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
                        (dbits(det) << 1) != 0;
     // beta1's numerator, the source's expression with the products by 1 dropped
     const double n1 = ((d1 * r22 - l2 * d2) - d0 * (l0 * r22 - l2 * r20)) + (l0 * d2 - d1 * r20);
-    if (quick) {
+    if (Ops::kFast || quick) {
+        o.ok = o.ok && quick;
         const Recip rd{det, rsp.y};  // det = -(sE2 - sE1): the same significand
-        beta0 = div_rn(d1 - d0 * l2, rd);
-        beta1 = div_rn(n1, rd);
-        beta2 = div_rn(d0 * l0 - d1, rd);
+        beta0 = o.div(d1 - d0 * l2, rd);
+        beta1 = o.div(n1, rd);
+        beta2 = o.div(d0 * l0 - d1, rd);
     } else {
         const double r00 = 1.0, r01 = 0.0, r02 = 1.0, r10 = l0, r11 = 0.0, r12 = l2, r21 = 1.0;
         const double dt = det3(r00, r01, r02, r10, r11, r12, r20, r21, r22);
@@ -439,15 +447,6 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
     fw[0][1] = mul0(beta1); fw[1][1] = beta1;
     fw[0][2] = beta2 * l2; fw[1][2] = beta2 * r22; fw[2][2] = (beta2 * l2) * vR;
     fw[2][1] = ((((hR * uR) * vR) - ((hL * uL) * vL)) - fw[2][0]) - fw[2][2];
-}
-
-static __device__ __noinline__ void riemann_aug(double hL, double hR, double huL, double huR, double bL, double bR,
-                                                double uL, double uR, double vL, double vR, double delphi,
-                                                double sE1, double sE2, double sqL, double sqR, u64 yL,
-                                                u64 yR, double drytol, double sw[3],
-                                                double fw[3][3]) {
-    riemann_aug_rec<false>(hL, hR, huL, huR, bL, bR, uL, uR, vL, vR, delphi, sE1, sE2, sqL, sqR, yL, yR,
-                           drytol, sw, fw, nullptr);
 }
 
 // Wet/dry handling, wave speeds and net updates of c_bind_geoclaw_solver_dp
@@ -472,11 +471,11 @@ __device__ __forceinline__ bool fzb(uint16_t* fz, int bit, bool v) {
     return v;
 }
 
-template <int SOLVER, int FZ = 0>
+template <int SOLVER, int FZ, class Ops>
 __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL, double huR, double hvL,
                                                double hvR, double bL, double bR, double sqL0, double sqR0,
                                                u64 yL0, u64 yR0, double drytol, double netL[3],
-                                               double netR[3], double& maxspeed, uint16_t* fz = nullptr) {
+                                               double netR[3], double& maxspeed, uint16_t* fz, Ops& o) {
     const double g = kG;
     netL[0] = netL[1] = netL[2] = 0.0;
     netR[0] = netR[1] = netR[2] = 0.0;
@@ -489,28 +488,22 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
         if (wetR0) sqR0 = sqrt_fix(g * hR);
     }
     double uL, uR, vL, vR;
-    if (wetR0) {
-        if (FZ == 2) {
-            uR = huR / hR;
-            vR = hvR / hR;
-        } else {
-            const Recip r{hR, yR0};
-            uR = div_rn(huR, r);
-            vR = div_rn(hvR, r);
-        }
+    if (FZ == 2) {
+        uR = wetR0 ? huR / hR : 0.0;
+        vR = wetR0 ? hvR / hR : 0.0;
+        uL = wetL0 ? huL / hL : 0.0;
+        vL = wetL0 ? hvL / hL : 0.0;
     } else {
+        const Recip rL{hL, yL0}, rR{hR, yR0};
+        uR = o.div_if(wetR0, huR, rR);
+        vR = o.div_if(wetR0, hvR, rR);
+        uL = o.div_if(wetL0, huL, rL);
+        vL = o.div_if(wetL0, hvL, rL);
+    }
+    if (!wetR0) {
         hR = 0.0; huR = 0.0; hvR = 0.0; uR = 0.0; vR = 0.0;
     }
-    if (wetL0) {
-        if (FZ == 2) {
-            uL = huL / hL;
-            vL = hvL / hL;
-        } else {
-            const Recip r{hL, yL0};
-            uL = div_rn(huL, r);
-            vL = div_rn(hvL, r);
-        }
-    } else {
+    if (!wetL0) {
         hL = 0.0; huL = 0.0; hvL = 0.0; uL = 0.0; vL = 0.0;
     }
     bool wall_l = false, wall_r = false;  // wall(1) = 0 resp. wall(3) = 0 (wall(2) = 0 with either)
@@ -546,25 +539,26 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     double sqR = wetR ? (wall_r ? sqL0 : sqR0) : 0.0;
     double sL = uL - sqL;
     double sR = uR + sqR;
-    double uhat = div_one(prod(sqL, uL) + prod(sqR, uR), sqR + sqL);
-    double chat = sqrt_fix(ghalf_h);
+    double uhat = o.div1(prod(sqL, uL) + prod(sqR, uR), sqR + sqL);
+    double chat = o.sqrt(ghalf_h);
     const double r1 = uhat - chat, r2 = uhat + chat;
-    double sE1 = fzb<FZ>(fz, 7, lt(sL, r1)) ? sL : r1;  // imin(sL, r1)
-    double sE2 = fzb<FZ>(fz, 8, lt(r2, sR)) ? sR : r2;  // imax(sR, r2)
+    double sE1 = fzb<FZ>(fz, 7, olt<Ops>(sL, r1)) ? sL : r1;  // imin(sL, r1)
+    double sE2 = fzb<FZ>(fz, 8, olt<Ops>(r2, sR)) ? sR : r2;  // imax(sR, r2)
 
     double sw[3], fw[3][3];
     if (SOLVER == AUG_RIEMANN) {
         // the reciprocals of the fixed-up depths: a wet side's own, a wall's mirrored one
         const u64 yLf = wall_l ? yR0 : yL0, yRf = wall_r ? yL0 : yR0;
-        riemann_aug(hL, hR, huL, huR, bL, bR, uL, uR, vL, vR, delphi, sE1, sE2, sqL, sqR, yLf, yRf, drytol, sw, fw);
+        riemann_aug_rec<false>(hL, hR, huL, huR, bL, bR, uL, uR, vL, vR, delphi, sE1, sE2, sqL, sqR, yLf, yRf, drytol, sw,
+                               fw, nullptr, o);
     } else {
         double delhu = huR - huL;
         double delb = bR - bL;
         double deldelphi = -prod(ghalf_h, delb);
         double dpd = delphi - deldelphi;
         const Recip rD = recip_of(sE2 - sE1);
-        double beta1 = div_rn(prod(sE2, delhu) - dpd, rD);
-        double beta2 = div_rn(dpd - prod(sE1, delhu), rD);
+        double beta1 = o.div(prod(sE2, delhu) - dpd, rD);
+        double beta2 = o.div(dpd - prod(sE1, delhu), rD);
         sw[0] = sE1; sw[1] = scale_pow2(sE1 + sE2, -1, 0.5); sw[2] = sE2;
         fw[0][0] = beta1; fw[1][0] = prod(beta1, sE1); fw[2][0] = prod(beta1, vL);
         fw[0][2] = beta2; fw[1][2] = prod(beta2, sE2); fw[2][2] = prod(beta2, vR);
@@ -595,7 +589,7 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     };
 #pragma unroll
     for (int w = 0; w < 3; ++w) {
-        const bool neg = fzb<FZ>(fz, 9 + 2 * w, lt0(sw[w])), pos = fzb<FZ>(fz, 10 + 2 * w, gt0(sw[w]));
+        const bool neg = fzb<FZ>(fz, 9 + 2 * w, olt0<Ops>(sw[w])), pos = fzb<FZ>(fz, 10 + 2 * w, ogt0<Ops>(sw[w]));
 #pragma unroll
         for (int e = 0; e < 3; ++e) {
             if (SOLVER != AUG_RIEMANN && w == 1 && e < 2) continue;
@@ -629,6 +623,89 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
 // (|n1| = |n2| = c) the four products of each rotation are +-RN(c p1) and
 // +-RN(c p2), since RN(-x) = -RN(x): two products per side, the signs set on
 // the bit patterns. Otherwise the general form runs.
+template <int SOLVER, int FZ, class Ops>
+__device__ __forceinline__ void geoclaw_rotated(double n1, double n2, const State& QL, const State& QR, double dL,
+                                                double dR, double sqL, double sqR, u64 yL, u64 yR, double drytol,
+                                                Update& fL, Update& fR, int axis, uint16_t* fz, Ops& o) {
+    const bool fin = is_finite(QL.p1) && is_finite(QL.p2) && is_finite(QR.p1) && is_finite(QR.p2);
+    const bool fast = axis != 0 && fin;
+    const bool diag = axis == 0 && fin && abs_bits(n1) == abs_bits(n2);
+    const bool sn = axis == 1 ? lt0(n1) : lt0(n2);  // sign of the nonzero component
+    const bool g1 = dbits(n1) < 0, g2 = dbits(n2) < 0;  // sign bits of the normal
+    const double c = bitsd(abs_bits(n1));
+    double pL1, pL2, pR1, pR2;
+    if (diag) {
+        // RN(n1 p1) = +-a1, RN(n2 p2) = +-a2, RN(-n2 p1) = -+a1, RN(n1 p2) = +-a2
+        const double aL1 = prod_rot(c, QL.p1), aL2 = prod_rot(c, QL.p2);
+        const double aR1 = prod_rot(c, QR.p1), aR2 = prod_rot(c, QR.p2);
+        pL1 = z0(flip(aL1, g1)) + flip(aL2, g2);
+        pL2 = z0(flip(aL1, !g2)) + flip(aL2, g1);
+        pR1 = z0(flip(aR1, g1)) + flip(aR2, g2);
+        pR2 = z0(flip(aR1, !g2)) + flip(aR2, g1);
+    } else if (fast) {
+        if (axis == 1) {
+            pL1 = z0(flip(QL.p1, sn)); pL2 = z0(flip(QL.p2, sn));
+            pR1 = z0(flip(QR.p1, sn)); pR2 = z0(flip(QR.p2, sn));
+        } else {
+            pL1 = z0(flip(QL.p2, sn)); pL2 = z0(flip(QL.p1, !sn));
+            pR1 = z0(flip(QR.p2, sn)); pR2 = z0(flip(QR.p1, !sn));
+        }
+    } else {
+        // T = [[n1, n2], [-n2, n1]]; p_edge = T p
+        pL1 = z0(prod_rot(n1, QL.p1)) + prod_rot(n2, QL.p2);
+        pL2 = z0(prod_rot(-n2, QL.p1)) + prod_rot(n1, QL.p2);
+        pR1 = z0(prod_rot(n1, QR.p1)) + prod_rot(n2, QR.p2);
+        pR2 = z0(prod_rot(-n2, QR.p1)) + prod_rot(n1, QR.p2);
+    }
+    double netL[3], netR[3], ms;
+    geoclaw_solver<SOLVER, FZ>(dL, dR, pL1, pR1, pL2, pR2, QL.b, QR.b, sqL, sqR, yL, yR, drytol, netL, netR, ms, fz,
+                               o);
+    fL.h = netL[0];
+    fL.s = ms;
+    fR.h = netR[0];
+    fR.s = ms;
+    const bool nfin = is_finite(netL[1]) && is_finite(netL[2]) && is_finite(netR[1]) && is_finite(netR[2]);
+    if (diag && nfin) {
+        // RN(m1 n1) = +-b1, RN(m2 (-n2)) = -+b2, RN(m1 n2) = +-b1, RN(m2 n1) = +-b2
+        const double bL1 = prod_rot(netL[1], c), bL2 = prod_rot(netL[2], c);
+        const double bR1 = prod_rot(netR[1], c), bR2 = prod_rot(netR[2], c);
+        fL.p1 = z0(flip(bL1, g1)) + flip(bL2, !g2);
+        fL.p2 = z0(flip(bL1, g2)) + flip(bL2, g1);
+        fR.p1 = z0(flip(bR1, g1)) + flip(bR2, !g2);
+        fR.p2 = z0(flip(bR1, g2)) + flip(bR2, g1);
+    } else if (fast && nfin) {
+        if (axis == 1) {
+            fL.p1 = z0(flip(netL[1], sn)); fL.p2 = z0(flip(netL[2], sn));
+            fR.p1 = z0(flip(netR[1], sn)); fR.p2 = z0(flip(netR[2], sn));
+        } else {
+            fL.p1 = z0(flip(netL[2], !sn)); fL.p2 = z0(flip(netL[1], sn));
+            fR.p1 = z0(flip(netR[2], !sn)); fR.p2 = z0(flip(netR[1], sn));
+        }
+    } else {
+        // p = net(2:3) T
+        fL.p1 = z0(prod_rot(netL[1], n1)) + prod_rot(netL[2], -n2);
+        fL.p2 = z0(prod_rot(netL[1], n2)) + prod_rot(netL[2], n1);
+        fR.p1 = z0(prod_rot(netR[1], n1)) + prod_rot(netR[2], -n2);
+        fR.p2 = z0(prod_rot(netR[1], n2)) + prod_rot(netR[2], n1);
+    }
+}
+
+// The flux of an edge whose operands FastOps does not take (a call, so that the
+// callers keep their registers).
+struct SafeEdge {
+    double n1, n2, dL, dR, sqL, sqR, drytol;
+    u64 yL, yR;
+    State QL, QR;
+    int axis;
+    Update fL, fR;
+};
+template <int SOLVER>
+static __device__ __noinline__ void geoclaw_safe(SafeEdge& e) {
+    SafeOps o;
+    geoclaw_rotated<SOLVER, 0>(e.n1, e.n2, e.QL, e.QR, e.dL, e.dR, e.sqL, e.sqR, e.yL, e.yR, e.drytol, e.fL, e.fR,
+                               e.axis, nullptr, o);
+}
+
 template <int SOLVER, int FZ = 0>
 __device__ __forceinline__ void geoclaw_flux(double n1, double n2, const State& QL, const State& QR, double dL,
                                              double dR, double sqL, double sqR, u64 yL, u64 yR,
@@ -681,66 +758,18 @@ __device__ __forceinline__ void geoclaw_flux(double n1, double n2, const State& 
             }
         }
     }
-    const bool fin = is_finite(QL.p1) && is_finite(QL.p2) && is_finite(QR.p1) && is_finite(QR.p2);
-    const bool fast = axis != 0 && fin;
-    const bool diag = axis == 0 && fin && abs_bits(n1) == abs_bits(n2);
-    const bool sn = axis == 1 ? lt0(n1) : lt0(n2);  // sign of the nonzero component
-    const bool g1 = dbits(n1) < 0, g2 = dbits(n2) < 0;  // sign bits of the normal
-    const double c = bitsd(abs_bits(n1));
-    double pL1, pL2, pR1, pR2;
-    if (diag) {
-        // RN(n1 p1) = +-a1, RN(n2 p2) = +-a2, RN(-n2 p1) = -+a1, RN(n1 p2) = +-a2
-        const double aL1 = prod_rot(c, QL.p1), aL2 = prod_rot(c, QL.p2);
-        const double aR1 = prod_rot(c, QR.p1), aR2 = prod_rot(c, QR.p2);
-        pL1 = z0(flip(aL1, g1)) + flip(aL2, g2);
-        pL2 = z0(flip(aL1, !g2)) + flip(aL2, g1);
-        pR1 = z0(flip(aR1, g1)) + flip(aR2, g2);
-        pR2 = z0(flip(aR1, !g2)) + flip(aR2, g1);
-    } else if (fast) {
-        if (axis == 1) {
-            pL1 = z0(flip(QL.p1, sn)); pL2 = z0(flip(QL.p2, sn));
-            pR1 = z0(flip(QR.p1, sn)); pR2 = z0(flip(QR.p2, sn));
-        } else {
-            pL1 = z0(flip(QL.p2, sn)); pL2 = z0(flip(QL.p1, !sn));
-            pR1 = z0(flip(QR.p2, sn)); pR2 = z0(flip(QR.p1, !sn));
+    if (FZ == 0) {
+        FastOps o;
+        geoclaw_rotated<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, nullptr, o);
+        if (!o.ok) {
+            SafeEdge e{n1, n2, dL, dR, sqL, sqR, drytol, yL, yR, QL, QR, axis, {}, {}};
+            geoclaw_safe<SOLVER>(e);
+            fL = e.fL;
+            fR = e.fR;
         }
     } else {
-        // T = [[n1, n2], [-n2, n1]]; p_edge = T p
-        pL1 = z0(prod_rot(n1, QL.p1)) + prod_rot(n2, QL.p2);
-        pL2 = z0(prod_rot(-n2, QL.p1)) + prod_rot(n1, QL.p2);
-        pR1 = z0(prod_rot(n1, QR.p1)) + prod_rot(n2, QR.p2);
-        pR2 = z0(prod_rot(-n2, QR.p1)) + prod_rot(n1, QR.p2);
-    }
-    double netL[3], netR[3], ms;
-    geoclaw_solver<SOLVER, FZ>(dL, dR, pL1, pR1, pL2, pR2, QL.b, QR.b, sqL, sqR, yL, yR, drytol, netL, netR, ms,
-                               fz);
-    fL.h = netL[0];
-    fL.s = ms;
-    fR.h = netR[0];
-    fR.s = ms;
-    const bool nfin = is_finite(netL[1]) && is_finite(netL[2]) && is_finite(netR[1]) && is_finite(netR[2]);
-    if (diag && nfin) {
-        // RN(m1 n1) = +-b1, RN(m2 (-n2)) = -+b2, RN(m1 n2) = +-b1, RN(m2 n1) = +-b2
-        const double bL1 = prod_rot(netL[1], c), bL2 = prod_rot(netL[2], c);
-        const double bR1 = prod_rot(netR[1], c), bR2 = prod_rot(netR[2], c);
-        fL.p1 = z0(flip(bL1, g1)) + flip(bL2, !g2);
-        fL.p2 = z0(flip(bL1, g2)) + flip(bL2, g1);
-        fR.p1 = z0(flip(bR1, g1)) + flip(bR2, !g2);
-        fR.p2 = z0(flip(bR1, g2)) + flip(bR2, g1);
-    } else if (fast && nfin) {
-        if (axis == 1) {
-            fL.p1 = z0(flip(netL[1], sn)); fL.p2 = z0(flip(netL[2], sn));
-            fR.p1 = z0(flip(netR[1], sn)); fR.p2 = z0(flip(netR[2], sn));
-        } else {
-            fL.p1 = z0(flip(netL[2], !sn)); fL.p2 = z0(flip(netL[1], sn));
-            fR.p1 = z0(flip(netR[2], !sn)); fR.p2 = z0(flip(netR[1], sn));
-        }
-    } else {
-        // p = net(2:3) T
-        fL.p1 = z0(prod_rot(netL[1], n1)) + prod_rot(netL[2], -n2);
-        fL.p2 = z0(prod_rot(netL[1], n2)) + prod_rot(netL[2], n1);
-        fR.p1 = z0(prod_rot(netR[1], n1)) + prod_rot(netR[2], -n2);
-        fR.p2 = z0(prod_rot(netR[1], n2)) + prod_rot(netR[2], n1);
+        SafeOps o;
+        geoclaw_rotated<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, fz, o);
     }
 }
 

@@ -22,7 +22,6 @@ typedef long long s64;
 static int off = 0;  // error added to the approximations, in units of 2^-24
 static inline u64 bits_of(double x) { u64 r; memcpy(&r, &x, 8); return r; }
 static inline double double_of(u64 v) { double r; memcpy(&r, &v, 8); return r; }
-static inline u64 mulhi(u64 a, u64 b) { return (u64)((unsigned __int128)a * b >> 64); }
 static inline float float_of(unsigned v) { float r; memcpy(&r, &v, 4); return r; }
 static inline unsigned fbits_of(float x) { unsigned r; memcpy(&r, &x, 4); return r; }
 static inline float ffma(float a, float b, float c) { return fmaf(a, b, c); }
@@ -54,7 +53,7 @@ static double top53(unsigned __int128 p, int e) {
     while (p >> 53) p >>= 1;
     return ldexp((double)(u64)p, e);
 }
-static long bad = 0;
+static long bad = 0, fast = 0;
 static void same(double got, double want) {
     if (bits_of(got) != bits_of(want) && !(std::isnan(got) && std::isnan(want)) && bad++ < 5) printf("%a want %a\n", got, want);
 }
@@ -73,10 +72,13 @@ int main(int argc, char** argv) {
         same(div_fix(a, b, y), a / b);
         same(sqrt_fix(x), sqrt(x));
         same(sqrt_fix(a), sqrt(a));
+        FastOps f;
+        const double fq = f.div(a, recip_of(b)), f1 = f.div1(b, x), fr = f.sqrt(x);
+        if (f.ok) same(fq, a / b), same(f1, b / x), same(fr, sqrt(x)), ++fast;
         if (y && llabs((long long)(bits_of(recip_near(b, y)) - bits_of(1.0 / b))) > 1) ++bad;
     }
-    printf("%ld differ\n", bad);
-    return bad != 0;
+    printf("%ld differ, %ld fast\n", bad, fast);
+    return bad != 0 || fast < atol(argv[2]) / 2;
 }
 """
 
