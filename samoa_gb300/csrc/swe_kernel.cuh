@@ -231,7 +231,7 @@ __device__ __forceinline__ void flush_instance(const StepArgs& A, int inst, bool
 template <int SOLVER>
 __device__ __forceinline__ void cross_depth_terms(const StepArgs& A, int c, const State& Q, double drytol, double& d,
                                                   double& sq, u64& y) {
-    d = Q.h - Q.b;
+    d = depth_of(Q.h, Q.b);
     const bool wet = lt(drytol, d);
     sq = 0.0;
     y = 0;
@@ -402,7 +402,7 @@ __device__ __forceinline__ unsigned int edge_task(const StepArgs& A, const SegMe
     };
     auto near = [&](int i, State& Q, double& d, double& sq, u64& y) {
         Q = State{M.h[i], M.hu()[i], M.hv()[i], M.b()[i]};
-        d = Q.h - Q.b;
+        d = depth_of(Q.h, Q.b);
         sq = M.sq[i];
         y = M.rh[i];
     };
@@ -519,28 +519,37 @@ __device__ __forceinline__ CellOut update_cell(const SegMem& M, const DepthTab& 
     double h = M.h[i], p1 = M.hu()[i], p2 = M.hv()[i];
     const double b = M.b()[i];
     uint8_t br = 0;
-    const double bdry = b + P.drytol;
-    // flooded land starts at the dry tolerance, at rest
-    if (FZ == 2 ? (rb & 1u) != 0 : (lt(h, bdry) && gt0(dh))) {
-        h = bdry;
-        p1 = 0.0;
-        p2 = 0.0;
-        br = 1;
-    }
-    if (quiet) {
+    // A wet cell (sq > 0: RN(h - b) > drytol, so h > b + drytol and h >= bdry) cannot
+    // be below bdry now, and not after a quiet update either: it needs no bdry.
+    const bool deep = FZ == 0 && dbits(M.sq[i]) != 0;
+    if (quiet && deep) {
         h = add_zero(h, dh);
         p1 = add_zero(p1, dp1);
         p2 = add_zero(p2, dp2);
     } else {
-        h = h + dh;
-        p1 = p1 + dp1;
-        p2 = p2 + dp2;
-    }
-    if (FZ == 2 ? (rb & 2u) != 0 : lt(h, bdry)) {  // dried out: surface to min(b, 0), at rest
-        h = lt0(b) ? b : 0.0;
-        p1 = 0.0;
-        p2 = 0.0;
-        br |= 2;
+        const double bdry = add_here(b, P.drytol);
+        // flooded land starts at the dry tolerance, at rest
+        if (FZ == 2 ? (rb & 1u) != 0 : (!deep && lt(h, bdry) && gt0(dh))) {
+            h = bdry;
+            p1 = 0.0;
+            p2 = 0.0;
+            br = 1;
+        }
+        if (quiet) {
+            h = add_zero(h, dh);
+            p1 = add_zero(p1, dp1);
+            p2 = add_zero(p2, dp2);
+        } else {
+            h = h + dh;
+            p1 = p1 + dp1;
+            p2 = p2 + dp2;
+        }
+        if (FZ == 2 ? (rb & 2u) != 0 : lt(h, bdry)) {  // dried out: surface to min(b, 0), at rest
+            h = lt0(b) ? b : 0.0;
+            p1 = 0.0;
+            p2 = 0.0;
+            br |= 2;
+        }
     }
     o.h = h;
     o.p1 = p1;
@@ -715,7 +724,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
             // to step); the memo holds only pairs (d, sqrt(g d)), written by the CTA
             // that owns the cell, so a hit is the value the square root would give
             M.dep[i] = A.depth[c0 + i];
-            const double d = M.h[i] - M.b()[i];
+            const double d = depth_of(M.h[i], M.b()[i]);
             const bool wet = lt(drytol, d);
             const bool need_y = wet && (SOLVER != FWAVE || ((dbits(M.hu()[i]) | dbits(M.hv()[i])) << 1) != 0);
             double sq = 0.0;
@@ -922,7 +931,7 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const StepArgs A, const
     // cell whose depth kept its bits keeps them (a reciprocal left out while the
     // cell was at rest is taken when it moves)
     auto terms = [&](int i, double drytol, bool same_depth) {
-        const double d = M.h[i] - M.b()[i];
+        const double d = depth_of(M.h[i], M.b()[i]);
         const bool wet = lt(drytol, d);
         const bool need_y = wet && (SOLVER != FWAVE || ((dbits(M.hu()[i]) | dbits(M.hv()[i])) << 1) != 0);
         if (!same_depth) M.sq[i] = wet ? sqrt_fix(kG * d) : 0.0;

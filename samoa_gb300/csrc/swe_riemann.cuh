@@ -100,6 +100,23 @@ __device__ __forceinline__ double mul_here(double a, double b) {
     asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
     return r;
 }
+__device__ __forceinline__ double sub_here(double a, double b) {
+    double r;
+    asm volatile("sub.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    return r;
+}
+__device__ __forceinline__ double add_here(double a, double b) {
+    double r;
+    asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    return r;
+}
+// The depth RN(h - b); -b, without an FP64 instruction, where the surface is at
+// +-0 (a zero -b as +0: a dry cell either way).
+__device__ __forceinline__ double depth_of(double h, double b) {
+    double d = z0(flip(b, true));
+    if ((dbits(h) << 1) != 0) d = sub_here(h, b);
+    return d;
+}
 // x + z for z = +-0, as IEEE addition gives it: x itself, except that a zero x
 // takes +0 unless both are -0; a NaN x takes the FP64 add.
 __device__ __forceinline__ double add_zero(double x, double z) {
@@ -582,6 +599,26 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     // net updates: each accumulator starts at +0 and takes its waves in wave order;
     // +0 + x is z0(x), and the f-wave's wave 2 carries exact +0 in h and hu,
     // which leaves an accumulator unchanged (it is never -0)
+    const bool neg1 = olt0<Ops>(sw[1]);
+    if (FZ == 0 && !wall_l && !wall_r && olt0<Ops>(sw[0]) && ogt0<Ops>(sw[2]) && (neg1 || ogt0<Ops>(sw[1]))) {
+        // subcritical flow, as almost everywhere: wave 0 goes left, wave 2 right, the
+        // middle one to one side, in one sum and without branches
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const double f0 = z0(fw[e][0]), f2 = fw[e][2];
+            if (SOLVER != AUG_RIEMANN && e < 2) {
+                netL[e] = f0;
+                netR[e] = z0(f2);
+            } else {
+                const double sum = (neg1 ? f0 : z0(fw[e][1])) + (neg1 ? fw[e][1] : f2);
+                netL[e] = neg1 ? sum : f0;
+                netR[e] = neg1 ? z0(f2) : sum;
+            }
+        }
+        const long long m = max(abs_bits(sw[0]), max(abs_bits(sw[1]), abs_bits(sw[2])));
+        maxspeed = bitsd(m);
+        return;
+    }
     bool tL[3] = {false, false, false}, tR[3] = {false, false, false};
     auto acc = [](double& a, bool& t, double c) {
         a = t ? a + c : z0(c);
@@ -747,9 +784,12 @@ __device__ __forceinline__ void geoclaw_flux(double n1, double n2, const State& 
         // inf - inf is NaN). hL > drytol >= 0 is positive, so equal values have
         // equal bit patterns: one FP64 addition fewer per edge.
         const bool still = ((dbits(QL.p1) | dbits(QL.p2) | dbits(QR.p1) | dbits(QR.p2)) << 1) == 0;
-        if (still && lt(drytol, dL) && lt(drytol, dR)) {
-            const double x = (QR.b + dR) - QL.b;
-            if (dbits(x) == dbits(dL) && is_finite(dL)) {
+        // Where both surfaces are at +-0 (the sea level), dL = -bL and dR = -bR
+        // exactly, so x = 0 - bL = dL for finite depths: no FP64 arithmetic at all.
+        if (still && lt(drytol, dL) && lt(drytol, dR) && is_finite(dL) && is_finite(dR)) {
+            bool level = ((dbits(QL.h) | dbits(QR.h)) << 1) == 0;
+            if (!level) level = dbits(sub_here(QR.b + dR, QL.b)) == dbits(dL);
+            if (level) {
                 const long long m = dbits(sqL) > dbits(sqR) ? dbits(sqL) : dbits(sqR);
                 const double ms = bitsd(m);
                 fL = Update{0.0, 0.0, 0.0, ms};
@@ -863,7 +903,7 @@ __device__ __forceinline__ void edge_flux(double n1, double n2, const State& QL,
 
 // depth, sqrt(g * depth) and recip_fix(depth) of a state, as the edge code needs them
 __device__ __forceinline__ void depth_terms(const State& Q, double drytol, double& d, double& sq, u64& y) {
-    d = Q.h - Q.b;
+    d = depth_of(Q.h, Q.b);
     const bool wet = lt(drytol, d);
     sq = wet ? sqrt_fix(kG * d) : 0.0;
     y = wet ? recip_fix(d) : 0;
