@@ -768,6 +768,7 @@ template <int SOLVER>
 __device__ __forceinline__ void lf_vjp(double n1, double n2, const State& QL, const State& QR, double dL0,
                                        double dR0, double drytol, const double gL[3], const double gR[3],
                                        Grad4& outL, Grad4& outR) {
+    SafeOps so;
     const double g = kG;
     if (SOLVER == LF_BATH || SOLVER == LLF_BATH) {
         const double dL = dL0, dR = dR0;
@@ -781,7 +782,7 @@ __device__ __forceinline__ void lf_vjp(double n1, double n2, const State& QL, co
             const double* gg = right ? gR : gL;
             const double sgw = right ? -1.0 : 1.0;  // fR: -(0.5 v p) - pr n; fL: +(0.5 v p) + pr n
             const double hw = dmx(d, 0.0);
-            const double v = normal_velocity(n1, n2, Q.p1, Q.p2, recip_of(d));
+            const double v = normal_velocity(n1, n2, Q.p1, Q.p2, recip_of(d), so);
             const double sp = sqrt_fix(g * hw) + fabs(v);
             double b_v = sgw * 0.5 * fma(gg[1], Q.p1, gg[2] * Q.p2);
             const double b_pr = sgw * fma(gg[1], n1, gg[2] * n2);
@@ -800,8 +801,8 @@ __device__ __forceinline__ void lf_vjp(double n1, double n2, const State& QL, co
             return;
         }
         const double hL = dmx(dL, 0.0), hR = dmx(dR, 0.0);
-        const double vL = normal_velocity(n1, n2, QL.p1, QL.p2, recip_of(dL));
-        const double vR = normal_velocity(n1, n2, QR.p1, QR.p2, recip_of(dR));
+        const double vL = normal_velocity(n1, n2, QL.p1, QL.p2, recip_of(dL), so);
+        const double vR = normal_velocity(n1, n2, QR.p1, QR.p2, recip_of(dR), so);
         const double sL = sqrt_fix(g * hL) + fabs(vL), sR = sqrt_fix(g * hR) + fabs(vR);
         const bool left_max = sL > sR;
         const double alpha = (SOLVER == LLF_BATH) ? (left_max ? sL : sR) : 100.0;
@@ -846,8 +847,8 @@ __device__ __forceinline__ void lf_vjp(double n1, double n2, const State& QL, co
         // no bathymetry: depth = surface
         const double dL = QL.h - 0.0, dR = QR.h - 0.0;
         const double hL = dmx(dL, 0.0), hR = dmx(dR, 0.0);
-        const double vL = normal_velocity(n1, n2, QL.p1, QL.p2, recip_of(dL));
-        const double vR = normal_velocity(n1, n2, QR.p1, QR.p2, recip_of(dR));
+        const double vL = normal_velocity(n1, n2, QL.p1, QL.p2, recip_of(dL), so);
+        const double vR = normal_velocity(n1, n2, QR.p1, QR.p2, recip_of(dR), so);
         const double sL = sqrt_fix(g * dL) + fabs(vL), sR = sqrt_fix(g * dR) + fabs(vR);
         const bool left_max = sL > sR;
         const double alpha = (SOLVER == LLF) ? (left_max ? sL : sR) : 100.0;

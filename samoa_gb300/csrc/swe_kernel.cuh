@@ -231,7 +231,7 @@ __device__ __forceinline__ void flush_instance(const StepArgs& A, int inst, bool
 template <int SOLVER>
 __device__ __forceinline__ void cross_depth_terms(const StepArgs& A, int c, const State& Q, double drytol, double& d,
                                                   double& sq, u64& y) {
-    d = depth_of(Q.h, Q.b);
+    d = Q.h - Q.b;
     const bool wet = lt(drytol, d);
     sq = 0.0;
     y = 0;
@@ -244,15 +244,16 @@ __device__ __forceinline__ void cross_depth_terms(const StepArgs& A, int c, cons
             hit = true;
         }
     }
-    if (!hit) sq = sqrt_fix(kG * d);
+    SWE_IF(!hit) sq = sqrt_fix(kG * d);
     const bool still = ((dbits(Q.p1) | dbits(Q.p2)) << 1) == 0;
     y = (SOLVER == FWAVE && still) ? 0 : recip_fix(d);
 }
 
-template <int SOLVER, int FZ = 0>
-__global__ void __launch_bounds__(256) cross_edges_kernel(const StepArgs A) {
-    const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= A.n_xtasks) return;
+template <int SOLVER>
+static __device__ __noinline__ void cross_edge_redo(const StepArgs& A, long long j);
+
+template <int SOLVER, int FZ, class Ops>
+__device__ __forceinline__ void cross_edge(const StepArgs& A, long long j) {
     const long long step = A.gs->step;
     const int odd = (int)(step & 1);
     const int ib = A.fixed_io ? 0 : odd;
@@ -283,8 +284,13 @@ __global__ void __launch_bounds__(256) cross_edges_kernel(const StepArgs A) {
     cross_depth_terms<SOLVER>(A, L, QL, drytol, dL, sqL, yL);
     cross_depth_terms<SOLVER>(A, R, QR, drytol, dR, sqR, yR);
     Update fL, fR;
+    Ops o;
     edge_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, (int)((meta >> 15) & 3u),
-                          FZ ? &A.xrec[j] : nullptr);
+                          FZ ? &A.xrec[j] : nullptr, o);
+    if (!o.ok) {
+        cross_edge_redo<SOLVER>(A, j);
+        return;
+    }
     const Update& ua = odd ? fR : fL;
     const Update& ub = odd ? fL : fR;
     double2* out = reinterpret_cast<double2*>(A.xflux + 8 * j);
@@ -292,6 +298,19 @@ __global__ void __launch_bounds__(256) cross_edges_kernel(const StepArgs A) {
     out[1] = make_double2(ua.p2, ua.s);
     out[2] = make_double2(ub.h, ub.p1);
     out[3] = make_double2(ub.p2, ub.s);
+}
+
+template <int SOLVER>
+static __device__ __noinline__ void cross_edge_redo(const StepArgs& A, long long j) {
+    cross_edge<SOLVER, 0, SafeOps>(A, j);
+}
+
+template <int SOLVER, int FZ = 0>
+__global__ void __launch_bounds__(256) cross_edges_kernel(const __grid_constant__ StepArgs A) {
+    const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= A.n_xtasks) return;
+    if (FZ) cross_edge<SOLVER, FZ, SafeOps>(A, j);
+    else cross_edge<SOLVER, 0, FastOps>(A, j);
 }
 
 // Round-up float of |x| for x = +-0 or 2^-100 <= |x| < 2^101, from the bit
@@ -368,12 +387,14 @@ struct SegMem {
 // One edge task (skeleton_scalar_op / bnd_skeleton_scalar_op,
 // src/SWE/SWE_euler_timestep.f90:196-255): the updates of both sides into the
 // slots of the cells in the segment. With SHARED_STATE other CTAs write the
-// neighbours' state in this launch, so it is read past the L1 cache. Returns
-// nonzero on a bad index.
-template <int SOLVER, int FZ, bool SHARED_STATE>
-__device__ __forceinline__ unsigned int edge_task(const StepArgs& A, const SegMem& M, const int4 tk, uint16_t* erec,
+// neighbours' state in this launch, so it is read past the L1 cache. Returns 0,
+// kBadIndex, or kRedo where FastOps does not take the edge's operands (nothing is
+// written then).
+constexpr unsigned int kBadIndex = 1u, kRedo = 8u;
+template <int SOLVER, int FZ, bool SHARED_STATE, class Ops>
+__device__ __forceinline__ unsigned int edge_task_with(const StepArgs& A, const SegMem& M, const int4 tk, uint16_t* erec,
                                                   int c0, int cn, int odd, double drytol, int bc, const double* hin,
-                                                  const double* huin, const double* hvin) {
+                                                       const double* huin, const double* hvin) {
     const int T = M.T;
     const uint32_t meta = (uint32_t)tk.z;
     const bool bnd = (meta >> 14) & 1u;
@@ -387,7 +408,7 @@ __device__ __forceinline__ unsigned int edge_task(const StepArgs& A, const SegMe
     }
     if ((unsigned)L >= (unsigned)A.n_cells_total || (!bnd && (unsigned)R >= (unsigned)A.n_cells_total) || iL > 2 ||
         iR > 2 || pL > 16)
-        return 1u;
+        return kBadIndex;
     const double n1 = c_normal[pL][iL][0], n2 = c_normal[pL][iL][1];
     const int sl = L - c0, sr = R - c0;
     const bool lin = (unsigned)sl < (unsigned)cn;
@@ -402,7 +423,7 @@ __device__ __forceinline__ unsigned int edge_task(const StepArgs& A, const SegMe
     };
     auto near = [&](int i, State& Q, double& d, double& sq, u64& y) {
         Q = State{M.h[i], M.hu()[i], M.hv()[i], M.b()[i]};
-        d = depth_of(Q.h, Q.b);
+        d = Q.h - Q.b;
         sq = M.sq[i];
         y = M.rh[i];
     };
@@ -421,7 +442,9 @@ __device__ __forceinline__ unsigned int edge_task(const StepArgs& A, const SegMe
         far(R, QR, dR, sqR, yR);
     }
     Update fL, fR;
-    edge_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, (int)((meta >> 15) & 3u), erec);
+    Ops o;
+    edge_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, (int)((meta >> 15) & 3u), erec, o);
+    if (!o.ok) return kRedo;
     if (lin) {
         M.upd[(0 * 3 + iL) * T + sl] = fL.h;
         M.upd[(1 * 3 + iL) * T + sl] = fL.p1;
@@ -435,6 +458,26 @@ __device__ __forceinline__ unsigned int edge_task(const StepArgs& A, const SegMe
         M.upd[(3 * 3 + iR) * T + sr] = fR.s;
     }
     return 0u;
+}
+
+// The task again with SafeOps (a call, so that the callers keep their registers;
+// it reads the operands again, so that they need not hold them either).
+template <int SOLVER, bool SHARED_STATE>
+static __device__ __noinline__ unsigned int edge_task_redo(const StepArgs& A, const SegMem M, const int4 tk, int c0,
+                                                           int cn, int odd, double drytol, int bc, int ib) {
+    return edge_task_with<SOLVER, 0, SHARED_STATE, SafeOps>(A, M, tk, nullptr, c0, cn, odd, drytol, bc, A.h[ib],
+                                                            A.hu[ib], A.hv[ib]);
+}
+template <int SOLVER, int FZ, bool SHARED_STATE>
+__device__ __forceinline__ unsigned int edge_task(const StepArgs& A, const SegMem& M, const int4 tk, uint16_t* erec,
+                                                  int c0, int cn, int odd, double drytol, int bc, int ib) {
+    if (FZ)
+        return edge_task_with<SOLVER, FZ, SHARED_STATE, SafeOps>(A, M, tk, erec, c0, cn, odd, drytol, bc, A.h[ib],
+                                                                 A.hu[ib], A.hv[ib]);
+    unsigned int rc = edge_task_with<SOLVER, 0, SHARED_STATE, FastOps>(A, M, tk, nullptr, c0, cn, odd, drytol, bc,
+                                                                       A.h[ib], A.hu[ib], A.hv[ib]);
+    if (rc == kRedo) rc = edge_task_redo<SOLVER, SHARED_STATE>(A, M, tk, c0, cn, odd, drytol, bc, ib);
+    return rc;
 }
 
 // A cell's new state, its flag and its branch bits (cell_update_op + volume_op,
@@ -467,67 +510,68 @@ __device__ __forceinline__ CellOut update_cell(const SegMem& M, const DepthTab& 
     // each sum below is +0 (positive edge lengths), RN(ndv * +0) is a zero with
     // ndv's sign, and adding it leaves the state as add_zero says: the same
     // bits, without the FP64 arithmetic. Water at rest still has wave speeds,
-    // so the speed sum ds has its own test below.
+    // so the speed sum ds has its own test.
     const bool quiet = nz == 0 && is_finite(ndv);
-    double dh = 0.0, dp1 = 0.0, dp2 = 0.0, ds = 0.0;
-    if (__any_sync(__activemask(), !quiet)) {
-        if (!quiet) {
-            dh = z0(prod_cell(leg, u[0][0])) + prod_cell(hyp, u[0][1]);
-            dh = dh + prod_cell(leg, u[0][2]);
-            dp1 = z0(prod_cell(leg, u[1][0])) + prod_cell(hyp, u[1][1]);
-            dp1 = dp1 + prod_cell(leg, u[1][2]);
-            dp2 = z0(prod_cell(leg, u[2][0])) + prod_cell(hyp, u[2][1]);
-            dp2 = dp2 + prod_cell(leg, u[2][2]);
-        }
-    }
     // ds is +0 when every speed is +-0 (dry land) or when the cell's key stays
     // below wkey (key_below), else it is summed
+    double ds = 0.0;
     bool need_ds = sz != 0;
     if (need_ds && wkey != 0ull) need_ds = !key_below(tab.up[di], u[3][0], u[3][1], u[3][2], d + 1, wkey);
-    if (__any_sync(__activemask(), need_ds)) {
-        if (need_ds) {
-            ds = z0(prod_cell(leg, u[3][0])) + prod_cell(hyp, u[3][1]);
-            ds = ds + prod_cell(leg, u[3][2]);
+    SWE_IF(need_ds) {
+        ds = z0(prod_cell(leg, u[3][0])) + prod_cell(hyp, u[3][1]);
+        ds = ds + prod_cell(leg, u[3][2]);
+    }
+    // ds >= 0, so its bits order like its value; RN(ds * 2^(d+1))
+    unsigned long long key = (unsigned long long)dbits(scaled(dbits(ds), d + 1));
+    SWE_IF(!P.dt_by_max || !scales(dbits(ds), d + 1)) {
+        if (P.dt_by_max) {
+            key = (unsigned long long)dbits(ds * tab.pow[di]);
+        } else {  // r_dt_new = min(huge, volume / ds): a NaN quotient never wins
+            const double q = div_one(tab.vol[di], ds);
+            key = q < DBL_MAX ? ~(unsigned long long)dbits(q) : 0ull;
         }
     }
-    CellOut o;
-    o.flag = 0;
-    // |dh| > thr and |dh| < thr / 8 on the bit patterns (thresholds are positive;
-    // a NaN |dh| passes neither test, as in IEEE)
-    const long long nrm = abs_bits(dh);
-    if (d < P.max_depth && not_nan(nrm) && nrm > __double_as_longlong(P.thr_refine)) {
-        o.flag = 1;
-        ++r.nref;
-    } else if (d > P.min_depth && nrm < __double_as_longlong(P.thr_coarsen)) {
-        o.flag = -1;
-    }
-    unsigned long long key;
-    if (P.dt_by_max) {  // ds >= 0, so its bits order like its value; RN(ds * 2^(d+1))
-        key = (unsigned long long)dbits(scale_pow2(ds, d + 1, tab.pow[di]));
-    } else {  // r_dt_new = min(huge, volume / ds): a NaN quotient never wins
-        const double q = tab.vol[di] / ds;
-        key = q < DBL_MAX ? ~(unsigned long long)dbits(q) : 0ull;
-    }
     r.key = key > r.key ? key : r.key;
-    if (quiet) {
-        dh = dp1 = dp2 = bitsd(dbits(ndv) & (long long)0x8000000000000000ULL);  // RN(ndv * +0)
-    } else {
-        dh = prod_cell(ndv, dh);
-        dp1 = prod_cell(ndv, dp1);
-        dp2 = prod_cell(ndv, dp2);
-    }
     double h = M.h[i], p1 = M.hu()[i], p2 = M.hv()[i];
     const double b = M.b()[i];
     uint8_t br = 0;
+    long long nrm = 0;  // bits of |sum of the lengths times the updates of h|
     // A wet cell (sq > 0: RN(h - b) > drytol, so h > b + drytol and h >= bdry) cannot
     // be below bdry now, and not after a quiet update either: it needs no bdry.
     const bool deep = FZ == 0 && dbits(M.sq[i]) != 0;
-    if (quiet && deep) {
-        h = add_zero(h, dh);
-        p1 = add_zero(p1, dp1);
-        p2 = add_zero(p2, dp2);
-    } else {
-        const double bdry = add_here(b, P.drytol);
+    if (quiet) {
+        const double z = bitsd(dbits(ndv) & (long long)0x8000000000000000ULL);  // RN(ndv * +0)
+        double h1 = add_zero(h, z), q1 = add_zero(p1, z), q2 = add_zero(p2, z);
+        SWE_IF(!deep) {
+            const double bdry = b + P.drytol;
+            // (no flooding: the update is not positive) a branch-frozen run takes the recorded fixes
+            if (FZ == 2 && (rb & 1u) != 0) {
+                h1 = bdry + z;
+                q1 = q2 = 0.0 + z;
+                br = 1;
+            }
+            if (FZ == 2 ? (rb & 2u) != 0 : lt(h1, bdry)) {  // dried out: surface to min(b, 0), at rest
+                h1 = lt0(b) ? b : 0.0;
+                q1 = q2 = 0.0;
+                br |= 2;
+            }
+        }
+        h = h1;
+        p1 = q1;
+        p2 = q2;
+    }
+    SWE_IF(!quiet) {
+        double dh = z0(prod_cell(leg, u[0][0])) + prod_cell(hyp, u[0][1]);
+        dh = dh + prod_cell(leg, u[0][2]);
+        double dp1 = z0(prod_cell(leg, u[1][0])) + prod_cell(hyp, u[1][1]);
+        dp1 = dp1 + prod_cell(leg, u[1][2]);
+        double dp2 = z0(prod_cell(leg, u[2][0])) + prod_cell(hyp, u[2][1]);
+        dp2 = dp2 + prod_cell(leg, u[2][2]);
+        nrm = abs_bits(dh);
+        dh = prod_cell(ndv, dh);
+        dp1 = prod_cell(ndv, dp1);
+        dp2 = prod_cell(ndv, dp2);
+        const double bdry = b + P.drytol;
         // flooded land starts at the dry tolerance, at rest
         if (FZ == 2 ? (rb & 1u) != 0 : (!deep && lt(h, bdry) && gt0(dh))) {
             h = bdry;
@@ -535,21 +579,25 @@ __device__ __forceinline__ CellOut update_cell(const SegMem& M, const DepthTab& 
             p2 = 0.0;
             br = 1;
         }
-        if (quiet) {
-            h = add_zero(h, dh);
-            p1 = add_zero(p1, dp1);
-            p2 = add_zero(p2, dp2);
-        } else {
-            h = h + dh;
-            p1 = p1 + dp1;
-            p2 = p2 + dp2;
-        }
+        h = h + dh;
+        p1 = p1 + dp1;
+        p2 = p2 + dp2;
         if (FZ == 2 ? (rb & 2u) != 0 : lt(h, bdry)) {  // dried out: surface to min(b, 0), at rest
             h = lt0(b) ? b : 0.0;
             p1 = 0.0;
             p2 = 0.0;
             br |= 2;
         }
+    }
+    CellOut o;
+    o.flag = 0;
+    // |dh| > thr and |dh| < thr / 8 on the bit patterns (thresholds are positive;
+    // a NaN |dh| passes neither test, as in IEEE)
+    if (d < P.max_depth && not_nan(nrm) && nrm > __double_as_longlong(P.thr_refine)) {
+        o.flag = 1;
+        ++r.nref;
+    } else if (d > P.min_depth && nrm < __double_as_longlong(P.thr_coarsen)) {
+        o.flag = -1;
     }
     o.h = h;
     o.p1 = p1;
@@ -564,7 +612,7 @@ __device__ __forceinline__ unsigned long long warp_key_bound(unsigned long long 
 }
 
 template <int SOLVER, int FZ = 0>
-__global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
+__global__ void SWE_STEP_BOUNDS step_kernel(const __grid_constant__ StepArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int T = A.seg_cells;
     // staging buffers [stage_depth][h, hu, hv, b][T]: with depth 2 the next
@@ -724,7 +772,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
             // to step); the memo holds only pairs (d, sqrt(g d)), written by the CTA
             // that owns the cell, so a hit is the value the square root would give
             M.dep[i] = A.depth[c0 + i];
-            const double d = depth_of(M.h[i], M.b()[i]);
+            const double d = M.h[i] - M.b()[i];
             const bool wet = lt(drytol, d);
             const bool need_y = wet && (SOLVER != FWAVE || ((dbits(M.hu()[i]) | dbits(M.hv()[i])) << 1) != 0);
             double sq = 0.0;
@@ -737,13 +785,11 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
                     miss = false;
                 }
             }
-            if (__any_sync(__activemask(), miss)) {
-                if (miss) {
-                    sq = sqrt_fix(kG * d);
-                    if (A.memo) A.memo[c0 + i] = make_double2(d, sq);
-                }
+            SWE_IF(miss) {
+                sq = sqrt_fix(kG * d);
+                if (A.memo) A.memo[c0 + i] = make_double2(d, sq);
             }
-            if (__any_sync(__activemask(), need_y)) y = need_y ? recip_fix(d) : y;
+            if (need_y) y = recip_fix(d);
             M.rh[i] = y;
             M.sq[i] = sq;
         }
@@ -782,7 +828,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const StepArgs A) {
                 const int4 tk = next;
                 if (t + (int)blockDim.x < nm) next = __ldg(&tasks[t + blockDim.x]);
                 if (edge_task<SOLVER, FZ, false>(A, M, tk, FZ ? A.erec + t0 + t : nullptr, c0, cn, odd, drytol, P.bc,
-                                                 hin, huin, hvin))
+                                                 ib))
                     atomicOr(&s_error, 1u);
             }
         }
@@ -887,7 +933,7 @@ __device__ __forceinline__ bool wait_count(const unsigned int* count, unsigned i
 // in step k + 2, past another meeting).
 // For instances with dt_by_max and a dt from the CFL condition.
 template <int SOLVER>
-__global__ void __launch_bounds__(256) multi_step_kernel(const StepArgs A, const int n_steps) {
+__global__ void __launch_bounds__(256) multi_step_kernel(const __grid_constant__ StepArgs A, const int n_steps) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int T = A.seg_cells, tid = threadIdx.x, bd = blockDim.x;
     SegMem M;
@@ -931,10 +977,14 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const StepArgs A, const
     // cell whose depth kept its bits keeps them (a reciprocal left out while the
     // cell was at rest is taken when it moves)
     auto terms = [&](int i, double drytol, bool same_depth) {
-        const double d = depth_of(M.h[i], M.b()[i]);
+        const double d = M.h[i] - M.b()[i];
         const bool wet = lt(drytol, d);
         const bool need_y = wet && (SOLVER != FWAVE || ((dbits(M.hu()[i]) | dbits(M.hv()[i])) << 1) != 0);
-        if (!same_depth) M.sq[i] = wet ? sqrt_fix(kG * d) : 0.0;
+        if (!same_depth) {
+            double sq = 0.0;
+            SWE_IF(wet) sq = sqrt_fix(kG * d);
+            M.sq[i] = sq;
+        }
         if (!same_depth || (need_y && M.rh[i] == 0)) M.rh[i] = need_y ? recip_fix(d) : 0;
     };
     __syncthreads();
@@ -951,7 +1001,6 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const StepArgs A, const
         const int odd = (int)((step0 + k) & 1);
         // ---- edges: tid, tid + bd, ... of those inside the segment, then the halo tasks
         // from the last warp down; dt before a warp's edges if it has none inside
-        const double *hin = A.h[odd], *huin = A.hu[odd], *hvin = A.hv[odd];
         unsigned int bad = 0;
         bool met = k == 0;
         auto meet = [&]() {
@@ -980,7 +1029,7 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const StepArgs A, const
             const int4 tk = next;
             t = t < nm ? after(t) : t + bd;
             if (t < nt) next = __ldg(&tasks[t]);
-            bad = edge_task<SOLVER, 0, true>(A, M, tk, nullptr, c0, cn, odd, drytol, P.bc, hin, huin, hvin);
+            bad = edge_task<SOLVER, 0, true>(A, M, tk, nullptr, c0, cn, odd, drytol, P.bc, odd);
         }
         if (dt_warp && bd - 32 < nm) prepare_dt();
         if (bad) atomicOr(&s_error, bad);

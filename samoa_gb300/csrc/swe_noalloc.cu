@@ -131,7 +131,12 @@ __global__ void edges_kernel(Args A, unsigned char* scratch) {
         depth_terms(QL, A.drytol, dL, sqL, yL);
         depth_terms(QR, A.drytol, dR, sqR, yR);
         Update fL, fR;
-        edge_flux<SOLVER>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, A.drytol, fL, fR);
+        FastOps f;
+        edge_flux<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, A.drytol, fL, fR, 0, nullptr, f);
+        if (!f.ok) {
+            SafeOps o;
+            edge_flux<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, A.drytol, fL, fR, 0, nullptr, o);
+        }
         slots[(0 * 3 + iL) * M + L] = fL.h;
         slots[(1 * 3 + iL) * M + L] = fL.p1;
         slots[(2 * 3 + iL) * M + L] = fL.p2;

@@ -94,51 +94,41 @@ __device__ __forceinline__ double imax(double a, double b) { return lt(b, a) ? a
 __device__ __forceinline__ double flip(double x, bool neg) {
     return bitsd(dbits(x) ^ (neg ? (long long)0x8000000000000000ULL : 0LL));
 }
-// An FP64 multiply the compiler keeps inside the branch it is written in.
-__device__ __forceinline__ double mul_here(double a, double b) {
-    double r;
-    asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
-    return r;
+// `SWE_IF(c) { ... }` is `if (c) { ... }` that stays a branch: a loop whose end the
+// compiler cannot see. Conditional FP64 code needs it. The compiler turns short
+// conditional blocks into predicated instructions, and a predicated FP64
+// instruction holds the FP64 pipe for its 16 to 19 cycles per warp and SM even
+// when no lane executes it (measured: one or six multiplies behind an `if`, a warp
+// vote or a bra.uni that is never taken cost as much as multiplies always done).
+__device__ __forceinline__ unsigned int opaque_zero() {
+    unsigned int v;
+    asm volatile("mov.u32 %0, 0;" : "=r"(v));
+    return v;
 }
-__device__ __forceinline__ double sub_here(double a, double b) {
-    double r;
-    asm volatile("sub.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
-    return r;
-}
-__device__ __forceinline__ double add_here(double a, double b) {
-    double r;
-    asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
-    return r;
-}
-// The depth RN(h - b); -b, without an FP64 instruction, where the surface is at
-// +-0 (a zero -b as +0: a dry cell either way).
-__device__ __forceinline__ double depth_of(double h, double b) {
-    double d = z0(flip(b, true));
-    if ((dbits(h) << 1) != 0) d = sub_here(h, b);
-    return d;
-}
+#define SWE_IF(c) for (unsigned int swe_if_ = (c) ? 1u : 0u; swe_if_; swe_if_ = opaque_zero())
+
 // x + z for z = +-0, as IEEE addition gives it: x itself, except that a zero x
-// takes +0 unless both are -0; a NaN x takes the FP64 add.
+// takes +0 unless both are -0, and a NaN x comes back quiet.
 __device__ __forceinline__ double add_zero(double x, double z) {
     const long long b = dbits(x);
     if ((b << 1) == 0) return bitsd(b & dbits(z));  // -0 only when both are -0
-    if (abs_bits(x) > 0x7ff0000000000000LL) {
-        double r;
-        asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(x), "d"(z));
-        return r;
-    }
-    return x;
+    return abs_bits(x) > 0x7ff0000000000000LL ? bitsd(b | 0x0008000000000000LL) : x;
 }
 // RN(x * p) for p = 2^k: while x and the result are normal numbers the product
 // is exact and only the exponent field moves (an integer add on the bit
 // pattern); +-0 stays itself; a subnormal, infinite or NaN operand and an
 // under- or overflowing result take the FP64 multiply.
-__device__ __forceinline__ double scale_pow2(double x, int k, double p) {
-    const long long b = dbits(x);
+__device__ __forceinline__ bool scales(long long b, int k) {  // a zero, or normal before and after
     const int e = (int)((b >> 52) & 0x7ff);
-    if ((unsigned)(e - 1) <= 2045u && (unsigned)(e + k - 1) <= 2045u) return bitsd(b + ((long long)k << 52));
-    if ((b << 1) == 0) return x;
-    return mul_here(x, p);
+    return (b << 1) == 0 || ((unsigned)(e - 1) <= 2045u && (unsigned)(e + k - 1) <= 2045u);
+}
+__device__ __forceinline__ double scaled(long long b, int k) {
+    return bitsd((b << 1) == 0 ? b : b + ((long long)k << 52));
+}
+__device__ __forceinline__ double scale_pow2(double x, int k, double p) {
+    double r = scaled(dbits(x), k);
+    SWE_IF(!scales(dbits(x), k)) r = x * p;
+    return r;
 }
 
 // Several quotients in the step share a divisor (a cell's depth divides its
@@ -169,6 +159,13 @@ __device__ __forceinline__ bool olt0(double x) {
 }
 template <class Ops>
 __device__ __forceinline__ bool ogt0(double x) { return Ops::kFast ? dbits(x) > 0 : gt0(x); }
+// RN(x 2^k), p = 2^k
+template <class Ops>
+__device__ __forceinline__ double oscale(double x, int k, double p, Ops& o) {
+    if (!Ops::kFast) return scale_pow2(x, k, p);
+    o.ok = o.ok && scales(dbits(x), k);
+    return scaled(dbits(x), k);
+}
 template <class Ops>
 __device__ __forceinline__ double omin(double a, double b) { return olt<Ops>(a, b) ? a : b; }
 template <class Ops>
@@ -210,16 +207,16 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
     if (ole<Ops>(h_min, drytol)) {
         if (REC) rec->rs = 0;
         hm = 0.0;
-        double t = ((uR + uL) - scale_pow2(sqR, 1, 2.0)) + scale_pow2(sqL, 1, 2.0);
+        double t = ((uR + uL) - oscale(sqR, 1, 2.0, o)) + oscale(sqL, 1, 2.0, o);
         s1m = t;
         s2m = t;
         return;
     }
-    double F_min = delu + scale_pow2(sq_min - sq_max, 1, 2.0);
+    double F_min = delu + oscale(sq_min - sq_max, 1, 2.0, o);
     double F_max = 0.0;  // needed only when F_min <= 0
     if (!ogt0<Ops>(F_min)) F_max = delu + (h_max - h_min) * o.sqrt(o.div1((0.5 * g) * (h_max + h_min), h_max * h_min));
     if (ogt0<Ops>(F_min)) {  // two rarefactions
-        const double t0 = -delu + scale_pow2(sqL + sqR, 1, 2.0);
+        const double t0 = -delu + oscale(sqL + sqR, 1, 2.0, o);
         double t = omax<Ops>(0.0, t0);
         if (REC) {
             rec->rs = 1;
@@ -227,8 +224,8 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
         }
         hm = (1.0 / (16.0 * g)) * (t * t);
         const double sqm = o.sqrt(g * hm);
-        s1m = (uL + scale_pow2(sqL, 1, 2.0)) - 3.0 * sqm;
-        s2m = (uR - scale_pow2(sqR, 1, 2.0)) + 3.0 * sqm;
+        s1m = (uL + oscale(sqL, 1, 2.0, o)) - 3.0 * sqm;
+        s2m = (uR - oscale(sqR, 1, 2.0, o)) + 3.0 * sqm;
     } else if (ole<Ops>(F_max, 0.0)) {  // two shocks: one Newton step on sqrt(h)
         if (REC) rec->rs = 2;
         double h0 = h_max;
@@ -240,7 +237,7 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
         double dfdh = ((gL - o.div1(g * (h0 - hL), (4.0 * (h0 * h0)) * gL)) + gR) -
                       o.div1(g * (h0 - hR), (4.0 * (h0 * h0)) * gR);
         const double sq0 = o.sqrt(h0);
-        double slope = scale_pow2(sq0, 1, 2.0) * dfdh;
+        double slope = oscale(sq0, 1, 2.0, o) * dfdh;
         double t = sq0 - o.div1(F0, slope);
         hm = t * t;
         const double im = o.div1(1.0, hm);
@@ -256,16 +253,16 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
         }
         double h0 = h_min;
         const double i0 = r_lower ? o.div(1.0, Recip{hR, yR}) : o.div(1.0, Recip{hL, yL});
-        double F0 = (delu + scale_pow2(sq_min - sq_max, 1, 2.0)) + (h0 - h_min) * o.sqrt((0.5 * g) * (i0 + i0));
+        double F0 = (delu + oscale(sq_min - sq_max, 1, 2.0, o)) + (h0 - h_min) * o.sqrt((0.5 * g) * (i0 + i0));
         double slope = o.div1(F_max - F0, h_max - h_min);
         hm = h0 - o.div1(F0, slope);
         const double sqm = o.sqrt(g * hm);
         if (olt<Ops>(hR, hL)) {
-            s1m = (uL + scale_pow2(sqL, 1, 2.0)) - 3.0 * sqm;
-            s2m = (uL + scale_pow2(sqL, 1, 2.0)) - sqm;
+            s1m = (uL + oscale(sqL, 1, 2.0, o)) - 3.0 * sqm;
+            s2m = (uL + oscale(sqL, 1, 2.0, o)) - sqm;
         } else {
-            s2m = (uR - scale_pow2(sqR, 1, 2.0)) + 3.0 * sqm;
-            s1m = (uR - scale_pow2(sqR, 1, 2.0)) + sqm;
+            s2m = (uR - oscale(sqR, 1, 2.0, o)) + 3.0 * sqm;
+            s1m = (uR - oscale(sqR, 1, 2.0, o)) + sqm;
         }
     }
 }
@@ -361,16 +358,16 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
     const Recip rsp = recip_of(dsp);
     const double hq = o.div(((huL - huR) + sE2 * hR) - sE1 * hL, rsp);
     double hstarHLL = omax<Ops>(hq, 0.0);
-    double l1 = scale_pow2(l0 + l2, -1, 0.5);
+    double l1 = oscale(l0 + l2, -1, 0.5, o);
     if (olt<Ops>(iabs(l1), 1e-20)) l1 = 0.0;
     const double r20 = l0 * l0, r22 = l2 * l2;
 
     const double ct = 1e-6;
-    const double hhalf = scale_pow2(hL + hR, -1, 0.5);
+    const double hhalf = oscale(hL + hR, -1, 0.5, o);
     double hbar = omax<Ops>(hhalf, 0.0);
     double su = uL + uR;
     const double ghbar = g * hbar;
-    double s1s2bar = scale_pow2(su * su, -2, 0.25) - ghbar;
+    double s1s2bar = oscale(su * su, -2, 0.25, o) - ghbar;
     const double uLR = uL * uR;
     double s1s2tilde = omax<Ops>(0.0, uLR) - ghbar;
     bool sonic = ole<Ops>(iabs(s1s2bar), ct);
@@ -436,7 +433,7 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
     deldelphi = omax<Ops>(y1, gmn);
     double d0 = delh - deldelh, d1 = delhu, d2 = delphi - deldelphi;
 
-    double beta0, beta1, beta2;
+    double beta0 = 0.0, beta1 = 0.0, beta2 = 0.0;
     const double det = l0 - l2;
     const bool quick = moderate(l0) && moderate(l2) && moderate(d0) && moderate(d1) && moderate(d2) &&
                        (dbits(det) << 1) != 0;
@@ -448,7 +445,7 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
         beta0 = o.div(d1 - d0 * l2, rd);
         beta1 = o.div(n1, rd);
         beta2 = o.div(d0 * l0 - d1, rd);
-    } else {
+    } else if (!Ops::kFast) {
         const double r00 = 1.0, r01 = 0.0, r02 = 1.0, r10 = l0, r11 = 0.0, r12 = l2, r21 = 1.0;
         const double dt = det3(r00, r01, r02, r10, r11, r12, r20, r21, r22);
         beta0 = det3(d0, r01, r02, d1, r11, r12, d2, r21, r22) / dt;
@@ -461,7 +458,7 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
     sw[2] = l2;
     // f-waves: beta times rows 2 and 3 of R (r11 = 0, r21 = 1)
     fw[0][0] = beta0 * l0; fw[1][0] = beta0 * r20; fw[2][0] = (beta0 * l0) * vL;
-    fw[0][1] = mul0(beta1); fw[1][1] = beta1;
+    fw[0][1] = Ops::kFast ? bitsd(dbits(beta1) & (long long)0x8000000000000000ULL) : mul0(beta1); fw[1][1] = beta1;
     fw[0][2] = beta2 * l2; fw[1][2] = beta2 * r22; fw[2][2] = (beta2 * l2) * vR;
     fw[2][1] = ((((hR * uR) * vR) - ((hL * uL) * vL)) - fw[2][0]) - fw[2][2];
 }
@@ -523,25 +520,28 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     if (!wetL0) {
         hL = 0.0; huL = 0.0; hvL = 0.0; uL = 0.0; vL = 0.0;
     }
-    bool wall_l = false, wall_r = false;  // wall(1) = 0 resp. wall(3) = 0 (wall(2) = 0 with either)
-    if (!wetR0) {  // hR is now 0.0, and 0.0 <= drytol
-        const double hstar = FZ != 2 ? wall_depth(hL, uL, sqL0, yL0, drytol) : 0.0;
-        double hstartest = dmx(hL, hstar);
-        if (fzb<FZ>(fz, 3, hstartest + bL < bR)) {
-            wall_r = true;
+    // A dry side is a wall where the wet side's water cannot reach its bottom (wall(1)
+    // = 0 resp. wall(3) = 0, wall(2) = 0 with either), else its bottom is lowered to
+    // the wet side's surface. Both orientations in one block: each of its parts is a
+    // chain of its own for the warp.
+    bool wall_l = false, wall_r = false;
+    if (!wetL0 || !wetR0) {
+        const bool rdry = !wetR0;  // hR is now 0.0, and 0.0 <= drytol
+        const double h = rdry ? hL : hR, u = rdry ? uL : -uR, b = rdry ? bL : bR, bd = rdry ? bR : bL;
+        const double hstar = FZ != 2 ? wall_depth(h, u, rdry ? sqL0 : sqR0, rdry ? yL0 : yR0, drytol) : 0.0;
+        const double low = h + b;
+        const bool wall = fzb<FZ>(fz, rdry ? 3 : 5, lt(imax(h, hstar) + b, bd));
+        const bool lower = wall ? false : fzb<FZ>(fz, rdry ? 4 : 6, lt(low, bd));
+        wall_r = wall && rdry;
+        wall_l = wall && !rdry;
+        if (wall_r) {
             hR = hL; huR = -huL; bR = bL; uR = -uL; vR = vL;
-        } else if (fzb<FZ>(fz, 4, hL + bL < bR)) {
-            bR = hL + bL;
         }
-    } else if (!wetL0) {
-        const double hstar = FZ != 2 ? wall_depth(hR, -uR, sqR0, yR0, drytol) : 0.0;
-        double hstartest = dmx(hR, hstar);
-        if (fzb<FZ>(fz, 5, hstartest + bR < bL)) {
-            wall_l = true;
+        if (wall_l) {
             hL = hR; huL = -huR; bL = bR; uL = -uR; vL = vR;
-        } else if (fzb<FZ>(fz, 6, hR + bR < bL)) {
-            bL = hR + bR;
         }
+        bR = lower && rdry ? low : bR;
+        bL = lower && !rdry ? low : bL;
     }
     const double hsum = hR + hL;
     const double ghalf_h = prod(g * 0.5, hsum);  // (0.5 * g) * (hR + hL): delphi, chat, the f-wave's deldelphi
@@ -576,69 +576,74 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
         const Recip rD = recip_of(sE2 - sE1);
         double beta1 = o.div(prod(sE2, delhu) - dpd, rD);
         double beta2 = o.div(dpd - prod(sE1, delhu), rD);
-        sw[0] = sE1; sw[1] = scale_pow2(sE1 + sE2, -1, 0.5); sw[2] = sE2;
+        sw[0] = sE1; sw[1] = oscale(sE1 + sE2, -1, 0.5, o); sw[2] = sE2;
         fw[0][0] = beta1; fw[1][0] = prod(beta1, sE1); fw[2][0] = prod(beta1, vL);
         fw[0][2] = beta2; fw[1][2] = prod(beta2, sE2); fw[2][2] = prod(beta2, vR);
         fw[0][1] = 0.0; fw[1][1] = 0.0;
         fw[2][1] = ((prod(huR, vR) - prod(huL, vL)) - fw[2][0]) - fw[2][2];
     }
-    // eliminate ghost fluxes of a wall (multiplication by 0 keeps the sign of zero)
-    auto zero_wave = [&](const int w) {
-        sw[w] = sw[w] * 0.0;
-        fw[0][w] = fw[0][w] * 0.0;
-        fw[1][w] = fw[1][w] * 0.0;
-        fw[2][w] = fw[2][w] * 0.0;
-    };
-    if (wall_l) {
-        zero_wave(0);
-        zero_wave(1);
-    } else if (wall_r) {
-        zero_wave(1);
-        zero_wave(2);
+    // eliminate ghost fluxes of a wall: multiplication by 0, i.e. zeros whose signs the
+    // net updates drop, except for values that are not finite
+#pragma unroll
+    for (int w = 0; w < 3; ++w) {
+        const bool gone = (wall_l && w < 2) || (wall_r && w > 0);
+        if (Ops::kFast) {
+            o.ok = o.ok && (!gone || (is_finite(sw[w]) && is_finite(fw[0][w]) && is_finite(fw[1][w]) && is_finite(fw[2][w])));
+            sw[w] = gone ? 0.0 : sw[w];
+            fw[0][w] = gone ? 0.0 : fw[0][w];
+            fw[1][w] = gone ? 0.0 : fw[1][w];
+            fw[2][w] = gone ? 0.0 : fw[2][w];
+        } else if (gone) {
+            sw[w] = sw[w] * 0.0;
+            fw[0][w] = fw[0][w] * 0.0;
+            fw[1][w] = fw[1][w] * 0.0;
+            fw[2][w] = fw[2][w] * 0.0;
+        }
     }
     // net updates: each accumulator starts at +0 and takes its waves in wave order;
     // +0 + x is z0(x), and the f-wave's wave 2 carries exact +0 in h and hu,
     // which leaves an accumulator unchanged (it is never -0)
     const bool neg1 = olt0<Ops>(sw[1]);
-    if (FZ == 0 && !wall_l && !wall_r && olt0<Ops>(sw[0]) && ogt0<Ops>(sw[2]) && (neg1 || ogt0<Ops>(sw[1]))) {
-        // subcritical flow, as almost everywhere: wave 0 goes left, wave 2 right, the
-        // middle one to one side, in one sum and without branches
+    const bool sub = FZ == 0 && olt0<Ops>(sw[0]) && ogt0<Ops>(sw[2]) && (neg1 || ogt0<Ops>(sw[1]));
+    // subcritical flow, as almost everywhere: wave 0 goes left, wave 2 right, the
+    // middle one to one side, in one sum and without branches
 #pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            const double f0 = z0(fw[e][0]), f2 = fw[e][2];
-            if (SOLVER != AUG_RIEMANN && e < 2) {
-                netL[e] = f0;
-                netR[e] = z0(f2);
-            } else {
-                const double sum = (neg1 ? f0 : z0(fw[e][1])) + (neg1 ? fw[e][1] : f2);
-                netL[e] = neg1 ? sum : f0;
-                netR[e] = neg1 ? z0(f2) : sum;
-            }
+    for (int e = 0; e < 3; ++e) {
+        const double f0 = z0(fw[e][0]), f2 = fw[e][2];
+        if (FZ != 0) continue;
+        if (SOLVER != AUG_RIEMANN && e < 2) {
+            netL[e] = f0;
+            netR[e] = z0(f2);
+        } else {
+            const double sum = (neg1 ? f0 : z0(fw[e][1])) + (neg1 ? fw[e][1] : f2);
+            netL[e] = neg1 ? sum : f0;
+            netR[e] = neg1 ? z0(f2) : sum;
         }
-        const long long m = max(abs_bits(sw[0]), max(abs_bits(sw[1]), abs_bits(sw[2])));
-        maxspeed = bitsd(m);
-        return;
     }
-    bool tL[3] = {false, false, false}, tR[3] = {false, false, false};
-    auto acc = [](double& a, bool& t, double c) {
-        a = t ? a + c : z0(c);
-        t = true;
-    };
+    SWE_IF(!sub) {
+        bool tL[3] = {false, false, false}, tR[3] = {false, false, false};
+        auto acc = [](double& a, bool& t, double c) {
+            a = t ? a + c : z0(c);
+            t = true;
+        };
 #pragma unroll
-    for (int w = 0; w < 3; ++w) {
-        const bool neg = fzb<FZ>(fz, 9 + 2 * w, olt0<Ops>(sw[w])), pos = fzb<FZ>(fz, 10 + 2 * w, ogt0<Ops>(sw[w]));
+        for (int e = 0; e < 3; ++e) netL[e] = netR[e] = 0.0;
 #pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            if (SOLVER != AUG_RIEMANN && w == 1 && e < 2) continue;
-            const double f = fw[e][w];
-            if (neg) {
-                acc(netL[e], tL[e], f);
-            } else if (pos) {
-                acc(netR[e], tR[e], f);
-            } else {
-                const double hf = 0.5 * f;
-                acc(netL[e], tL[e], hf);
-                acc(netR[e], tR[e], hf);
+        for (int w = 0; w < 3; ++w) {
+            const bool neg = fzb<FZ>(fz, 9 + 2 * w, olt0<Ops>(sw[w])), pos = fzb<FZ>(fz, 10 + 2 * w, ogt0<Ops>(sw[w]));
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                if (SOLVER != AUG_RIEMANN && w == 1 && e < 2) continue;
+                const double f = fw[e][w];
+                if (neg) {
+                    acc(netL[e], tL[e], f);
+                } else if (pos) {
+                    acc(netR[e], tR[e], f);
+                } else {
+                    const double hf = 0.5 * f;
+                    acc(netL[e], tL[e], hf);
+                    acc(netR[e], tR[e], hf);
+                }
             }
         }
     }
@@ -646,8 +651,8 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     // patterns (non-negative values order like them; a NaN candidate never wins)
     long long m = abs_bits(sw[0]);
     const long long a1 = abs_bits(sw[1]), a2 = abs_bits(sw[2]);
-    if (a1 > m && not_nan(a1)) m = a1;
-    if (a2 > m && not_nan(a2)) m = a2;
+    if (a1 > m && (Ops::kFast || not_nan(a1))) m = a1;
+    if (a2 > m && (Ops::kFast || not_nan(a2))) m = a2;
     maxspeed = bitsd(m);
 }
 
@@ -670,8 +675,13 @@ __device__ __forceinline__ void geoclaw_rotated(double n1, double n2, const Stat
     const bool sn = axis == 1 ? lt0(n1) : lt0(n2);  // sign of the nonzero component
     const bool g1 = dbits(n1) < 0, g2 = dbits(n2) < 0;  // sign bits of the normal
     const double c = bitsd(abs_bits(n1));
-    double pL1, pL2, pR1, pR2;
-    if (diag) {
+    // FastOps takes the mesh's normals and finite momenta
+    o.ok = o.ok && (!Ops::kFast || diag || fast);
+    // axis-aligned; for a diagonal or a general normal overwritten below
+    const bool ax1 = axis == 1;
+    double pL1 = z0(flip(ax1 ? QL.p1 : QL.p2, sn)), pL2 = z0(flip(ax1 ? QL.p2 : QL.p1, ax1 ? sn : !sn));
+    double pR1 = z0(flip(ax1 ? QR.p1 : QR.p2, sn)), pR2 = z0(flip(ax1 ? QR.p2 : QR.p1, ax1 ? sn : !sn));
+    SWE_IF(diag) {
         // RN(n1 p1) = +-a1, RN(n2 p2) = +-a2, RN(-n2 p1) = -+a1, RN(n1 p2) = +-a2
         const double aL1 = prod_rot(c, QL.p1), aL2 = prod_rot(c, QL.p2);
         const double aR1 = prod_rot(c, QR.p1), aR2 = prod_rot(c, QR.p2);
@@ -679,15 +689,8 @@ __device__ __forceinline__ void geoclaw_rotated(double n1, double n2, const Stat
         pL2 = z0(flip(aL1, !g2)) + flip(aL2, g1);
         pR1 = z0(flip(aR1, g1)) + flip(aR2, g2);
         pR2 = z0(flip(aR1, !g2)) + flip(aR2, g1);
-    } else if (fast) {
-        if (axis == 1) {
-            pL1 = z0(flip(QL.p1, sn)); pL2 = z0(flip(QL.p2, sn));
-            pR1 = z0(flip(QR.p1, sn)); pR2 = z0(flip(QR.p2, sn));
-        } else {
-            pL1 = z0(flip(QL.p2, sn)); pL2 = z0(flip(QL.p1, !sn));
-            pR1 = z0(flip(QR.p2, sn)); pR2 = z0(flip(QR.p1, !sn));
-        }
-    } else {
+    }
+    if (!Ops::kFast && !diag && !fast) {
         // T = [[n1, n2], [-n2, n1]]; p_edge = T p
         pL1 = z0(prod_rot(n1, QL.p1)) + prod_rot(n2, QL.p2);
         pL2 = z0(prod_rot(-n2, QL.p1)) + prod_rot(n1, QL.p2);
@@ -702,7 +705,10 @@ __device__ __forceinline__ void geoclaw_rotated(double n1, double n2, const Stat
     fR.h = netR[0];
     fR.s = ms;
     const bool nfin = is_finite(netL[1]) && is_finite(netL[2]) && is_finite(netR[1]) && is_finite(netR[2]);
-    if (diag && nfin) {
+    o.ok = o.ok && (!Ops::kFast || nfin);
+    fL.p1 = z0(flip(ax1 ? netL[1] : netL[2], ax1 ? sn : !sn)); fL.p2 = z0(flip(ax1 ? netL[2] : netL[1], sn));
+    fR.p1 = z0(flip(ax1 ? netR[1] : netR[2], ax1 ? sn : !sn)); fR.p2 = z0(flip(ax1 ? netR[2] : netR[1], sn));
+    SWE_IF(diag && (Ops::kFast || nfin)) {
         // RN(m1 n1) = +-b1, RN(m2 (-n2)) = -+b2, RN(m1 n2) = +-b1, RN(m2 n1) = +-b2
         const double bL1 = prod_rot(netL[1], c), bL2 = prod_rot(netL[2], c);
         const double bR1 = prod_rot(netR[1], c), bR2 = prod_rot(netR[2], c);
@@ -710,15 +716,8 @@ __device__ __forceinline__ void geoclaw_rotated(double n1, double n2, const Stat
         fL.p2 = z0(flip(bL1, g2)) + flip(bL2, g1);
         fR.p1 = z0(flip(bR1, g1)) + flip(bR2, !g2);
         fR.p2 = z0(flip(bR1, g2)) + flip(bR2, g1);
-    } else if (fast && nfin) {
-        if (axis == 1) {
-            fL.p1 = z0(flip(netL[1], sn)); fL.p2 = z0(flip(netL[2], sn));
-            fR.p1 = z0(flip(netR[1], sn)); fR.p2 = z0(flip(netR[2], sn));
-        } else {
-            fL.p1 = z0(flip(netL[2], !sn)); fL.p2 = z0(flip(netL[1], sn));
-            fR.p1 = z0(flip(netR[2], !sn)); fR.p2 = z0(flip(netR[1], sn));
-        }
-    } else {
+    }
+    if (!Ops::kFast && (!nfin || (!diag && !fast))) {
         // p = net(2:3) T
         fL.p1 = z0(prod_rot(netL[1], n1)) + prod_rot(netL[2], -n2);
         fL.p2 = z0(prod_rot(netL[1], n2)) + prod_rot(netL[2], n1);
@@ -727,37 +726,18 @@ __device__ __forceinline__ void geoclaw_rotated(double n1, double n2, const Stat
     }
 }
 
-// The flux of an edge whose operands FastOps does not take (a call, so that the
-// callers keep their registers).
-struct SafeEdge {
-    double n1, n2, dL, dR, sqL, sqR, drytol;
-    u64 yL, yR;
-    State QL, QR;
-    int axis;
-    Update fL, fR;
-};
-template <int SOLVER>
-static __device__ __noinline__ void geoclaw_safe(SafeEdge& e) {
-    SafeOps o;
-    geoclaw_rotated<SOLVER, 0>(e.n1, e.n2, e.QL, e.QR, e.dL, e.dR, e.sqL, e.sqR, e.yL, e.yR, e.drytol, e.fL, e.fR,
-                               e.axis, nullptr, o);
-}
-
-template <int SOLVER, int FZ = 0>
+template <int SOLVER, int FZ, class Ops>
 __device__ __forceinline__ void geoclaw_flux(double n1, double n2, const State& QL, const State& QR, double dL,
                                              double dR, double sqL, double sqR, u64 yL, u64 yR,
-                                             double drytol, Update& fL, Update& fR, int axis = 0,
-                                             uint16_t* fz = nullptr) {
+                                             double drytol, Update& fL, Update& fR, int axis, uint16_t* fz, Ops& o) {
     // both sides dry: the solver returns zero net updates and speed, and their
     // rotation back is +0 in every component, so neither rotation is needed
     const bool dry2 = FZ == 2 ? ((*fz & 1u) != 0)
                               : (!lt(drytol, dL) && !lt(drytol, dR) && !is_nan(dL) && !is_nan(dR) && !is_nan(drytol));
-    if (dry2) {
-        if (FZ == 1) *fz = 1;
-        fL = Update{0.0, 0.0, 0.0, 0.0};
-        fR = Update{0.0, 0.0, 0.0, 0.0};
-        return;
-    }
+    // (one branch decides between the trivial edges and the solver: a return from
+    // inside a nested test would keep the lanes that pass it apart for the whole
+    // solver, which the warp then runs twice)
+    bool rest = false;
     if (SOLVER == FWAVE && FZ == 0) {
         // Water at rest on both sides under one surface (lake at rest): every
         // momentum is +-0, both sides are wet and the c-binding's surface
@@ -786,76 +766,71 @@ __device__ __forceinline__ void geoclaw_flux(double n1, double n2, const State& 
         const bool still = ((dbits(QL.p1) | dbits(QL.p2) | dbits(QR.p1) | dbits(QR.p2)) << 1) == 0;
         // Where both surfaces are at +-0 (the sea level), dL = -bL and dR = -bR
         // exactly, so x = 0 - bL = dL for finite depths: no FP64 arithmetic at all.
-        if (still && lt(drytol, dL) && lt(drytol, dR) && is_finite(dL) && is_finite(dR)) {
-            bool level = ((dbits(QL.h) | dbits(QR.h)) << 1) == 0;
-            if (!level) level = dbits(sub_here(QR.b + dR, QL.b)) == dbits(dL);
-            if (level) {
-                const long long m = dbits(sqL) > dbits(sqR) ? dbits(sqL) : dbits(sqR);
-                const double ms = bitsd(m);
-                fL = Update{0.0, 0.0, 0.0, ms};
-                fR = Update{0.0, 0.0, 0.0, ms};
-                return;
-            }
-        }
+        const bool can = still && lt(drytol, dL) && lt(drytol, dR) && is_finite(dL) && is_finite(dR);
+        const bool level = ((dbits(QL.h) | dbits(QR.h)) << 1) == 0;
+        rest = can && level;
+        SWE_IF(can && !level) rest = dbits((QR.b + dR) - QL.b) == dbits(dL);
     }
-    if (FZ == 0) {
-        FastOps o;
-        geoclaw_rotated<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, nullptr, o);
-        if (!o.ok) {
-            SafeEdge e{n1, n2, dL, dR, sqL, sqR, drytol, yL, yR, QL, QR, axis, {}, {}};
-            geoclaw_safe<SOLVER>(e);
-            fL = e.fL;
-            fR = e.fR;
-        }
+    if (dry2 || rest) {
+        if (FZ == 1) *fz = 1;
+        const double ms = rest ? bitsd(dbits(sqL) > dbits(sqR) ? dbits(sqL) : dbits(sqR)) : 0.0;
+        fL = Update{0.0, 0.0, 0.0, ms};
+        fR = Update{0.0, 0.0, 0.0, ms};
     } else {
-        SafeOps o;
         geoclaw_rotated<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, fz, o);
     }
 }
 
 // z0(n1 (p1 / d)) + n2 (p2 / d), r = {d, recip_fix(d)}
-__device__ __forceinline__ double normal_velocity(double n1, double n2, double p1, double p2, const Recip& r) {
-    return z0(n1 * div_rn(p1, r)) + n2 * div_rn(p2, r);
+template <class Ops>
+__device__ __forceinline__ double normal_velocity(double n1, double n2, double p1, double p2, const Recip& r, Ops& o) {
+    return z0(n1 * o.div(p1, r)) + n2 * o.div(p2, r);
 }
 
 // compute_lf_flux, src/SWE/SWE_euler_timestep.f90:359-446
 // sqL / sqR, yL / yR: sqrt(g * depth) and recip_fix of the two depths where they are
 // above the dry tolerance (else not read).
-template <int SOLVER>
+template <int SOLVER, class Ops>
 __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, const State& QR, double dL,
                                         double dR, double drytol, Update& fL, Update& fR, double sqL,
-                                        double sqR, u64 yL, u64 yR) {
+                                        double sqR, u64 yL, u64 yR, Ops& o) {
     const double g = kG;
     if (SOLVER == LF_BATH || SOLVER == LLF_BATH) {
         const bool aL = lt(drytol, dL), aR = lt(drytol, dR);
         const Recip rL{dL, aL ? yL : recip_fix(dL)}, rR{dR, aR ? yR : recip_fix(dR)};
-        if (dL < drytol || dR < drytol) {
+        const bool dryL = lt(dL, drytol), dryR = lt(dR, drytol);
+        if (dryL || dryR) {
             fL = Update{0.0, 0.0, 0.0, 0.0};
             fR = Update{0.0, 0.0, 0.0, 0.0};
-            if (dL < drytol && dR < drytol) {
-            } else if (dL < drytol) {
-                double hR = dmx(dR, 0.0);
-                double vR = normal_velocity(n1, n2, QR.p1, QR.p2, rR);
-                fR.s = (aR ? sqR : sqrt_fix(g * hR)) + fabs(vR);
+            SWE_IF(dryL && !dryR) {
+                double hR = imax(dR, 0.0);
+                double vR = normal_velocity(n1, n2, QR.p1, QR.p2, rR, o);
+                fR.s = (aR ? sqR : o.sqrt(g * hR)) + iabs(vR);
                 double pr = ((0.5 * g) * hR) * hR;
                 fR.p1 = (-((0.5 * vR) * QR.p1) - pr * n1) + (0.5 * fR.s) * QR.p1;
                 fR.p2 = (-((0.5 * vR) * QR.p2) - pr * n2) + (0.5 * fR.s) * QR.p2;
-            } else {
-                double hL = dmx(dL, 0.0);
-                double vL = normal_velocity(n1, n2, QL.p1, QL.p2, rL);
-                fL.s = (aL ? sqL : sqrt_fix(g * hL)) + fabs(vL);
+            }
+            SWE_IF(dryR && !dryL) {
+                double hL = imax(dL, 0.0);
+                double vL = normal_velocity(n1, n2, QL.p1, QL.p2, rL, o);
+                fL.s = (aL ? sqL : o.sqrt(g * hL)) + iabs(vL);
                 double pr = ((0.5 * g) * hL) * hL;
                 fL.p1 = ((0.5 * vL) * QL.p1 + pr * n1) + (0.5 * fL.s) * QL.p1;
                 fL.p2 = ((0.5 * vL) * QL.p2 + pr * n2) + (0.5 * fL.s) * QL.p2;
             }
             return;
         }
-        double hL = dmx(dL, 0.0), hR = dmx(dR, 0.0);
-        double vL = normal_velocity(n1, n2, QL.p1, QL.p2, rL);
-        double vR = normal_velocity(n1, n2, QR.p1, QR.p2, rR);
-        fL.s = (aL ? sqL : sqrt_fix(g * hL)) + fabs(vL);
-        fR.s = (aR ? sqR : sqrt_fix(g * hR)) + fabs(vR);
-        double alpha = (SOLVER == LLF_BATH) ? dmx(fL.s, fR.s) : 100.0;
+        double hL = imax(dL, 0.0), hR = imax(dR, 0.0);
+        double vL = normal_velocity(n1, n2, QL.p1, QL.p2, rL, o);
+        double vR = normal_velocity(n1, n2, QR.p1, QR.p2, rR, o);
+        double cL = sqL, cR = sqR;
+        SWE_IF(!aL || !aR) {  // a depth at the tolerance
+            cL = aL ? sqL : sqrt_fix(g * hL);
+            cR = aR ? sqR : sqrt_fix(g * hR);
+        }
+        fL.s = cL + iabs(vL);
+        fR.s = cR + iabs(vR);
+        double alpha = (SOLVER == LLF_BATH) ? imax(fL.s, fR.s) : 100.0;
         fL.h = 0.5 * ((hL * vL + hR * vR) + alpha * (QL.h - QR.h));
         fR.h = -fL.h;
         double pr = (0.5 * g) * (hL * hL + hR * hR);
@@ -871,12 +846,12 @@ __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, c
     } else {
         dL = QL.h - 0.0;
         dR = QR.h - 0.0;
-        double hL = dmx(dL, 0.0), hR = dmx(dR, 0.0);
-        double vL = normal_velocity(n1, n2, QL.p1, QL.p2, recip_of(dL));
-        double vR = normal_velocity(n1, n2, QR.p1, QR.p2, recip_of(dR));
-        fL.s = sqrt_fix(g * dL) + fabs(vL);
-        fR.s = sqrt_fix(g * dR) + fabs(vR);
-        double alpha = (SOLVER == LLF) ? dmx(fL.s, fR.s) : 100.0;
+        double hL = imax(dL, 0.0), hR = imax(dR, 0.0);
+        double vL = normal_velocity(n1, n2, QL.p1, QL.p2, recip_of(dL), o);
+        double vR = normal_velocity(n1, n2, QR.p1, QR.p2, recip_of(dR), o);
+        fL.s = o.sqrt(g * dL) + iabs(vL);
+        fR.s = o.sqrt(g * dR) + iabs(vR);
+        double alpha = (SOLVER == LLF) ? imax(fL.s, fR.s) : 100.0;
         fL.h = 0.5 * ((vL * hL + vR * hR) + alpha * (QL.h - QR.h));
         fR.h = -fL.h;
         double sc = (vL * vL) * hL + (vR * vR) * hR;
@@ -891,19 +866,20 @@ __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, c
 // One edge: dL/dR are the depths h - b of the two states, sqL/sqR their
 // sqrt(g * depth) and yL/yR recip_fix(depth) (only read for depths above the dry
 // tolerance).
-template <int SOLVER, int FZ = 0>
+// With FastOps the updates count only where o.ok is true afterwards.
+template <int SOLVER, int FZ, class Ops>
 __device__ __forceinline__ void edge_flux(double n1, double n2, const State& QL, const State& QR, double dL,
                                           double dR, double sqL, double sqR, u64 yL, u64 yR, double drytol,
-                                          Update& fL, Update& fR, int axis = 0, uint16_t* fz = nullptr) {
+                                          Update& fL, Update& fR, int axis, uint16_t* fz, Ops& o) {
     if (SOLVER == FWAVE || SOLVER == AUG_RIEMANN)
-        geoclaw_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, fz);
+        geoclaw_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, fz, o);
     else
-        lf_flux<SOLVER>(n1, n2, QL, QR, dL, dR, drytol, fL, fR, sqL, sqR, yL, yR);
+        lf_flux<SOLVER>(n1, n2, QL, QR, dL, dR, drytol, fL, fR, sqL, sqR, yL, yR, o);
 }
 
 // depth, sqrt(g * depth) and recip_fix(depth) of a state, as the edge code needs them
 __device__ __forceinline__ void depth_terms(const State& Q, double drytol, double& d, double& sq, u64& y) {
-    d = depth_of(Q.h, Q.b);
+    d = Q.h - Q.b;
     const bool wet = lt(drytol, d);
     sq = wet ? sqrt_fix(kG * d) : 0.0;
     y = wet ? recip_fix(d) : 0;
