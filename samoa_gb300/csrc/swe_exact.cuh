@@ -194,8 +194,9 @@ struct SafeOps {
     bool ok = true;
     SWE_EXACT_FN_M double div(double a, const Recip& r) { return div_fix(a, r.b, r.y); }
     SWE_EXACT_FN_M double div1(double a, double b) { return div_one(a, b); }
-    // a / b where `use`, b a depth above a tolerance >= 0; else any value
+    // a / b where `use`, else any value; div_if: b a depth above a tolerance >= 0
     SWE_EXACT_FN_M double div_if(bool use, double a, const Recip& r) { return use ? div_fix(a, r.b, r.y) : 0.0; }
+    SWE_EXACT_FN_M double div1_if(bool use, double a, double b) { return use ? div_one(a, b) : 0.0; }
     SWE_EXACT_FN_M double sqrt(double x) { return sqrt_fix(x); }
 };
 
@@ -214,6 +215,7 @@ struct FastOps {
     SWE_EXACT_FN_M double div(double a, const Recip& r) { return quot(true, false, a, r); }
     SWE_EXACT_FN_M double div1(double a, double b) { return quot(true, false, a, recip_of(b)); }
     SWE_EXACT_FN_M double div_if(bool use, double a, const Recip& r) { return quot(use, true, a, r); }
+    SWE_EXACT_FN_M double div1_if(bool use, double a, double b) { return quot(use, false, a, recip_of(b)); }
     SWE_EXACT_FN_M double sqrt(double x) {
         const u64 ux = bits_of(x);
         ok = ok && (unsigned)(ux >> 52) - 1u < 2046u;

@@ -490,6 +490,7 @@ struct CellOut {
     int8_t flag;
     uint8_t branch;
 };
+static __device__ __noinline__ double quotient(double a, double b) { return div_one(a, b); }
 template <int FZ>
 __device__ __forceinline__ CellOut update_cell(const SegMem& M, const DepthTab& tab, const InstParams& P, int i,
                                                int odd, unsigned long long wkey, uint8_t rb, Reduced& r) {
@@ -527,7 +528,7 @@ __device__ __forceinline__ CellOut update_cell(const SegMem& M, const DepthTab& 
         if (P.dt_by_max) {
             key = (unsigned long long)dbits(ds * tab.pow[di]);
         } else {  // r_dt_new = min(huge, volume / ds): a NaN quotient never wins
-            const double q = div_one(tab.vol[di], ds);
+            const double q = quotient(tab.vol[di], ds);
             key = q < DBL_MAX ? ~(unsigned long long)dbits(q) : 0ull;
         }
     }

@@ -228,14 +228,33 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
         s2m = (uR - oscale(sqR, 1, 2.0, o)) + 3.0 * sqm;
     } else if (ole<Ops>(F_max, 0.0)) {  // two shocks: one Newton step on sqrt(h)
         if (REC) rec->rs = 2;
-        double h0 = h_max;
-        const double i0 = r_higher ? o.div(1.0, Recip{hR, yR}) : o.div(1.0, Recip{hL, yL});
-        const double iL = o.div(1.0, Recip{hL, yL}), iR = o.div(1.0, Recip{hR, yR});
-        double gL = o.sqrt((0.5 * g) * (i0 + iL));
-        double gR = o.sqrt((0.5 * g) * (i0 + iR));
-        double F0 = (delu + (h0 - hL) * gL) + (h0 - hR) * gR;
-        double dfdh = ((gL - o.div1(g * (h0 - hL), (4.0 * (h0 * h0)) * gL)) + gR) -
-                      o.div1(g * (h0 - hR), (4.0 * (h0 * h0)) * gR);
+        const double h0 = h_max;
+        double iL, iR, F0, dfdh;
+        if (Ops::kFast) {
+            // h0 is one side's depth, whose terms in F0 and dfdh are products of a zero
+            // with a finite value: the other ("low") side's remain, in the order of
+            // F0 = (delu + (h0 - hL) gL) + (h0 - hR) gR and
+            // dfdh = ((gL - XL) + gR) - XR, X = g (h0 - h) / ((4 h0^2) g_side)
+            const bool l_low = r_higher;
+            const double hl = l_low ? hL : hR;
+            const double i0 = o.div(1.0, l_low ? Recip{hR, yR} : Recip{hL, yL});
+            const double il = o.div(1.0, l_low ? Recip{hL, yL} : Recip{hR, yR});
+            const double g0 = o.sqrt((0.5 * g) * (i0 + i0)), gl = o.sqrt((0.5 * g) * (i0 + il));
+            const double dl = h0 - hl;
+            F0 = delu + dl * gl;
+            const double xl = flip(o.div1(g * dl, (4.0 * (h0 * h0)) * gl), true);
+            dfdh = ((l_low ? gl : g0) + (l_low ? xl : gl)) + (l_low ? g0 : xl);
+            iL = l_low ? il : i0;
+            iR = l_low ? i0 : il;
+        } else {
+            const double i0 = r_higher ? o.div(1.0, Recip{hR, yR}) : o.div(1.0, Recip{hL, yL});
+            iL = o.div(1.0, Recip{hL, yL});
+            iR = o.div(1.0, Recip{hR, yR});
+            const double gL = o.sqrt((0.5 * g) * (i0 + iL)), gR = o.sqrt((0.5 * g) * (i0 + iR));
+            F0 = (delu + (h0 - hL) * gL) + (h0 - hR) * gR;
+            dfdh = ((gL - o.div1(g * (h0 - hL), (4.0 * (h0 * h0)) * gL)) + gR) -
+                   o.div1(g * (h0 - hR), (4.0 * (h0 * h0)) * gR);
+        }
         const double sq0 = o.sqrt(h0);
         double slope = oscale(sq0, 1, 2.0, o) * dfdh;
         double t = sq0 - o.div1(F0, slope);
@@ -251,9 +270,12 @@ __device__ __forceinline__ void riemann_structure_rec(double hL, double hR, doub
             rec->rs = 3;
             rec->lhigh = olt<Ops>(hR, hL);
         }
-        double h0 = h_min;
-        const double i0 = r_lower ? o.div(1.0, Recip{hR, yR}) : o.div(1.0, Recip{hL, yL});
-        double F0 = (delu + oscale(sq_min - sq_max, 1, 2.0, o)) + (h0 - h_min) * o.sqrt((0.5 * g) * (i0 + i0));
+        const double h0 = h_min;
+        double F0 = F_min;  // + (h0 - h_min) sqrt(...), a zero while the root is finite
+        if (!Ops::kFast) {
+            const double i0 = r_lower ? o.div(1.0, Recip{hR, yR}) : o.div(1.0, Recip{hL, yL});
+            F0 = F_min + (h0 - h_min) * o.sqrt((0.5 * g) * (i0 + i0));
+        }
         double slope = o.div1(F_max - F0, h_max - h_min);
         hm = h0 - o.div1(F0, slope);
         const double sqm = o.sqrt(g * hm);
@@ -386,32 +408,20 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
         rec->dcase = 0;
     }
 
-    double deldelh, deldelphi;
     const double dgh = (delb * g) * hbar;
-    if (sonic) {
-        deldelh = flip(delb, true);
-        deldelphi = flip(ghbar * delb, true);
-    } else {
-        const Recip rb = recip_of(s1s2bar);
-        deldelh = o.div(dgh, rb);
-        deldelphi = flip(o.div(dgh * s1s2tilde, rb), true);
-    }
+    const double qh = o.div1_if(!sonic, dgh, s1s2bar);
+    const double qphi = flip(o.div1_if(!sonic, dgh * s1s2tilde, s1s2bar), true);
+    double deldelh = sonic ? flip(delb, true) : qh;
+    double deldelphi = sonic ? flip(ghbar * delb, true) : qphi;
     const double hsd = hstarHLL * dsp;
     int dcase = 0;
-    double lo = 0.0, hi = 0.0;  // the two bounds of the case
-    if (olt<Ops>(sE1, -ct) && olt<Ops>(ct, sE2)) {
-        dcase = 1;
-        hi = o.div1(hsd, sE2);
-        lo = o.div1(hsd, sE1);
-    } else if (ole<Ops>(ct, sE1)) {
-        dcase = 2;
-        hi = o.div1(hsd, sE1);
-        lo = flip(hL, true);
-    } else if (ole<Ops>(sE2, -ct)) {
-        dcase = 3;
-        hi = hR;
-        lo = o.div1(hsd, sE2);
-    }
+    if (olt<Ops>(sE1, -ct) && olt<Ops>(ct, sE2)) dcase = 1;
+    else if (ole<Ops>(ct, sE1)) dcase = 2;
+    else if (ole<Ops>(sE2, -ct)) dcase = 3;
+    // the two bounds of the case, without a branch per case
+    const double q1 = o.div1_if(dcase == 1 || dcase == 2, hsd, sE1), q2 = o.div1_if(dcase == 1 || dcase == 3, hsd, sE2);
+    const double hi = dcase == 1 ? q2 : (dcase == 2 ? q1 : hR);
+    const double lo = dcase == 1 ? q1 : (dcase == 2 ? flip(hL, true) : q2);
     if (dcase) {
         const double x1 = omin<Ops>(deldelh, hi);
         if (REC) {
