@@ -200,7 +200,8 @@ struct SafeOps {
     SWE_EXACT_FN_M double sqrt(double x) { return sqrt_fix(x); }
 };
 
-// The same without branches; ok is false after an operand that SafeOps has to take.
+// The same without branches (and without the short-circuit tests that may become some);
+// ok is false after an operand that SafeOps has to take.
 struct FastOps {
     static constexpr bool kFast = true;
     bool ok = true;
@@ -208,7 +209,8 @@ struct FastOps {
         const u64 ua = bits_of(a), ub = bits_of(r.b);
         const bool zero = (ua << 1) == 0;
         const bool in = ((unsigned)(ua >> 52) & 0x7ffu) - 523u <= 1000u;
-        ok = ok && (!use || (zero ? (zero_free || r.y != 0) : (in && r.y != 0)));
+        const bool y = r.y != 0;
+        ok = ok & (!use | (zero ? (zero_free | y) : (in & y)));
         const double q = quot_core(ua, ub, r.y);
         return zero ? double_of((ua ^ ub) & 0x8000000000000000ull) : q;
     }
@@ -218,7 +220,7 @@ struct FastOps {
     SWE_EXACT_FN_M double div1_if(bool use, double a, double b) { return quot(use, false, a, recip_of(b)); }
     SWE_EXACT_FN_M double sqrt(double x) {
         const u64 ux = bits_of(x);
-        ok = ok && (unsigned)(ux >> 52) - 1u < 2046u;
+        ok = ok & ((unsigned)(ux >> 52) - 1u < 2046u);
         return root_core(ux);
     }
 };

@@ -72,11 +72,11 @@ __device__ __forceinline__ bool is_finite(double x) { return abs_bits(x) < 0x7ff
 __device__ __forceinline__ bool lt0(double x) {  // x < 0.0
     const long long b = dbits(x);
     const long long a = b & 0x7fffffffffffffffLL;
-    return b < 0 && a != 0 && not_nan(a);
+    return (b < 0) & (a != 0) & not_nan(a);
 }
 __device__ __forceinline__ bool gt0(double x) {  // x > 0.0
     const long long b = dbits(x);
-    return b > 0 && b <= 0x7ff0000000000000LL;
+    return (b > 0) & (b <= 0x7ff0000000000000LL);
 }
 __device__ __forceinline__ bool is_nan(double x) { return abs_bits(x) > 0x7ff0000000000000LL; }
 // A key that orders like the value for non-NaN doubles, with -0 equal to +0.
@@ -86,7 +86,7 @@ __device__ __forceinline__ long long ord_key(double x) {
     return b >= 0 ? b : (b ^ 0x7fffffffffffffffLL);
 }
 __device__ __forceinline__ bool lt(double a, double b) {  // a < b
-    return !is_nan(a) && !is_nan(b) && ord_key(a) < ord_key(b);
+    return !is_nan(a) & !is_nan(b) & (ord_key(a) < ord_key(b));
 }
 __device__ __forceinline__ double imin(double a, double b) { return lt(a, b) ? a : b; }  // dmn on the integer pipe
 __device__ __forceinline__ double imax(double a, double b) { return lt(b, a) ? a : b; }  // dmx on the integer pipe
@@ -120,7 +120,7 @@ __device__ __forceinline__ double add_zero(double x, double z) {
 // under- or overflowing result take the FP64 multiply.
 __device__ __forceinline__ bool scales(long long b, int k) {  // a zero, or normal before and after
     const int e = (int)((b >> 52) & 0x7ff);
-    return (b << 1) == 0 || ((unsigned)(e - 1) <= 2045u && (unsigned)(e + k - 1) <= 2045u);
+    return ((b << 1) == 0) | (((unsigned)(e - 1) <= 2045u) & ((unsigned)(e + k - 1) <= 2045u));
 }
 __device__ __forceinline__ double scaled(long long b, int k) {
     return bitsd((b << 1) == 0 ? b : b + ((long long)k << 52));
@@ -140,7 +140,7 @@ __device__ __forceinline__ double rcp_near(double b) { return recip_near(b, reci
 
 // Non-strict comparisons on the integer pipe with IEEE semantics (false if either is NaN).
 __device__ __forceinline__ bool le(double a, double b) {  // a <= b
-    return !is_nan(a) && !is_nan(b) && ord_key(a) <= ord_key(b);
+    return !is_nan(a) & !is_nan(b) & (ord_key(a) <= ord_key(b));
 }
 // The predicates on numbers, for FastOps formulas: a NaN operand gives any answer
 // there, and the formula is then redone (FastOps::ok is false: every value
@@ -155,7 +155,7 @@ template <class Ops>
 __device__ __forceinline__ bool ole(double a, double b) { return Ops::kFast ? num_key(a) <= num_key(b) : le(a, b); }
 template <class Ops>
 __device__ __forceinline__ bool olt0(double x) {
-    return Ops::kFast ? dbits(x) < 0 && (dbits(x) << 1) != 0 : lt0(x);
+    return Ops::kFast ? (dbits(x) < 0) & ((dbits(x) << 1) != 0) : lt0(x);
 }
 template <class Ops>
 __device__ __forceinline__ bool ogt0(double x) { return Ops::kFast ? dbits(x) > 0 : gt0(x); }
@@ -163,7 +163,7 @@ __device__ __forceinline__ bool ogt0(double x) { return Ops::kFast ? dbits(x) > 
 template <class Ops>
 __device__ __forceinline__ double oscale(double x, int k, double p, Ops& o) {
     if (!Ops::kFast) return scale_pow2(x, k, p);
-    o.ok = o.ok && scales(dbits(x), k);
+    o.ok = o.ok & scales(dbits(x), k);
     return scaled(dbits(x), k);
 }
 template <class Ops>
@@ -396,8 +396,8 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
     sonic |= ole<Ops>(s1s2bar * s1s2tilde, ct);
     sonic |= ole<Ops>((s1s2bar * sE1) * sE2, ct);
     sonic |= olt<Ops>(omin<Ops>(iabs(sE1), iabs(sE2)), ct);
-    sonic |= olt0<Ops>(sE1) && ogt0<Ops>(s1m);
-    sonic |= ogt0<Ops>(sE2) && olt0<Ops>(s2m);
+    sonic |= olt0<Ops>(sE1) & ogt0<Ops>(s1m);
+    sonic |= ogt0<Ops>(sE2) & olt0<Ops>(s2m);
     sonic |= olt0<Ops>((uL + sqL) * (uR + sqR));  // sqrt(g * h) of the fixed-up depths
     sonic |= olt0<Ops>((uL - sqL) * (uR - sqR));
     if (REC) {
@@ -414,23 +414,19 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
     double deldelh = sonic ? flip(delb, true) : qh;
     double deldelphi = sonic ? flip(ghbar * delb, true) : qphi;
     const double hsd = hstarHLL * dsp;
-    int dcase = 0;
-    if (olt<Ops>(sE1, -ct) && olt<Ops>(ct, sE2)) dcase = 1;
-    else if (ole<Ops>(ct, sE1)) dcase = 2;
-    else if (ole<Ops>(sE2, -ct)) dcase = 3;
+    const bool apart = olt<Ops>(sE1, -ct) & olt<Ops>(ct, sE2);
+    const int dcase = apart ? 1 : (ole<Ops>(ct, sE1) ? 2 : (ole<Ops>(sE2, -ct) ? 3 : 0));
     // the two bounds of the case, without a branch per case
-    const double q1 = o.div1_if(dcase == 1 || dcase == 2, hsd, sE1), q2 = o.div1_if(dcase == 1 || dcase == 3, hsd, sE2);
+    const double q1 = o.div1_if((dcase == 1) | (dcase == 2), hsd, sE1), q2 = o.div1_if((dcase == 1) | (dcase == 3), hsd, sE2);
     const double hi = dcase == 1 ? q2 : (dcase == 2 ? q1 : hR);
     const double lo = dcase == 1 ? q1 : (dcase == 2 ? flip(hL, true) : q2);
-    if (dcase) {
-        const double x1 = omin<Ops>(deldelh, hi);
-        if (REC) {
-            rec->dcase = (int8_t)dcase;
-            rec->dd_min_first = olt<Ops>(deldelh, hi);
-            rec->dd_max_first = olt<Ops>(lo, x1);
-        }
-        deldelh = omax<Ops>(x1, lo);
+    const double x1 = omin<Ops>(deldelh, hi);
+    if (REC && dcase) {
+        rec->dcase = (int8_t)dcase;
+        rec->dd_min_first = olt<Ops>(deldelh, hi);
+        rec->dd_max_first = olt<Ops>(lo, x1);
     }
+    deldelh = dcase ? omax<Ops>(x1, lo) : deldelh;
     const double pl = flip(hL * delb, true), pr = flip(hR * delb, true);
     const double gmx = g * omax<Ops>(pl, pr), gmn = g * omin<Ops>(pl, pr);
     const double y1 = omin<Ops>(deldelphi, gmx);
@@ -445,12 +441,12 @@ __device__ __forceinline__ void riemann_aug_rec(double hL, double hR, double huL
 
     double beta0 = 0.0, beta1 = 0.0, beta2 = 0.0;
     const double det = l0 - l2;
-    const bool quick = moderate(l0) && moderate(l2) && moderate(d0) && moderate(d1) && moderate(d2) &&
-                       (dbits(det) << 1) != 0;
+    const bool quick = moderate(l0) & moderate(l2) & moderate(d0) & moderate(d1) & moderate(d2) &
+                       ((dbits(det) << 1) != 0);
     // beta1's numerator, the source's expression with the products by 1 dropped
     const double n1 = ((d1 * r22 - l2 * d2) - d0 * (l0 * r22 - l2 * r20)) + (l0 * d2 - d1 * r20);
     if (Ops::kFast || quick) {
-        o.ok = o.ok && quick;
+        o.ok = o.ok & quick;
         const Recip rd{det, rsp.y};  // det = -(sE2 - sE1): the same significand
         beta0 = o.div(d1 - d0 * l2, rd);
         beta1 = o.div(n1, rd);
@@ -535,7 +531,7 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     // the wet side's surface. Both orientations in one block: each of its parts is a
     // chain of its own for the warp.
     bool wall_l = false, wall_r = false;
-    if (!wetL0 || !wetR0) {
+    if (!(wetL0 & wetR0)) {
         const bool rdry = !wetR0;  // hR is now 0.0, and 0.0 <= drytol
         const double h = rdry ? hL : hR, u = rdry ? uL : -uR, b = rdry ? bL : bR, bd = rdry ? bR : bL;
         const double hstar = FZ != 2 ? wall_depth(h, u, rdry ? sqL0 : sqR0, rdry ? yL0 : yR0, drytol) : 0.0;
@@ -596,9 +592,9 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     // net updates drop, except for values that are not finite
 #pragma unroll
     for (int w = 0; w < 3; ++w) {
-        const bool gone = (wall_l && w < 2) || (wall_r && w > 0);
+        const bool gone = (wall_l & (w < 2)) | (wall_r & (w > 0));
         if (Ops::kFast) {
-            o.ok = o.ok && (!gone || (is_finite(sw[w]) && is_finite(fw[0][w]) && is_finite(fw[1][w]) && is_finite(fw[2][w])));
+            o.ok = o.ok & (!gone | (is_finite(sw[w]) & is_finite(fw[0][w]) & is_finite(fw[1][w]) & is_finite(fw[2][w])));
             sw[w] = gone ? 0.0 : sw[w];
             fw[0][w] = gone ? 0.0 : fw[0][w];
             fw[1][w] = gone ? 0.0 : fw[1][w];
@@ -614,7 +610,7 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     // +0 + x is z0(x), and the f-wave's wave 2 carries exact +0 in h and hu,
     // which leaves an accumulator unchanged (it is never -0)
     const bool neg1 = olt0<Ops>(sw[1]);
-    const bool sub = FZ == 0 && olt0<Ops>(sw[0]) && ogt0<Ops>(sw[2]) && (neg1 || ogt0<Ops>(sw[1]));
+    const bool sub = (FZ == 0) & olt0<Ops>(sw[0]) & ogt0<Ops>(sw[2]) & (neg1 | ogt0<Ops>(sw[1]));
     // subcritical flow, as almost everywhere: wave 0 goes left, wave 2 right, the
     // middle one to one side, in one sum and without branches
 #pragma unroll
@@ -679,14 +675,14 @@ template <int SOLVER, int FZ, class Ops>
 __device__ __forceinline__ void geoclaw_rotated(double n1, double n2, const State& QL, const State& QR, double dL,
                                                 double dR, double sqL, double sqR, u64 yL, u64 yR, double drytol,
                                                 Update& fL, Update& fR, int axis, uint16_t* fz, Ops& o) {
-    const bool fin = is_finite(QL.p1) && is_finite(QL.p2) && is_finite(QR.p1) && is_finite(QR.p2);
-    const bool fast = axis != 0 && fin;
-    const bool diag = axis == 0 && fin && abs_bits(n1) == abs_bits(n2);
+    const bool fin = is_finite(QL.p1) & is_finite(QL.p2) & is_finite(QR.p1) & is_finite(QR.p2);
+    const bool fast = (axis != 0) & fin;
+    const bool diag = (axis == 0) & fin & (abs_bits(n1) == abs_bits(n2));
     const bool sn = axis == 1 ? lt0(n1) : lt0(n2);  // sign of the nonzero component
     const bool g1 = dbits(n1) < 0, g2 = dbits(n2) < 0;  // sign bits of the normal
     const double c = bitsd(abs_bits(n1));
     // FastOps takes the mesh's normals and finite momenta
-    o.ok = o.ok && (!Ops::kFast || diag || fast);
+    o.ok = o.ok & (!Ops::kFast | diag | fast);
     // axis-aligned; for a diagonal or a general normal overwritten below
     const bool ax1 = axis == 1;
     double pL1 = z0(flip(ax1 ? QL.p1 : QL.p2, sn)), pL2 = z0(flip(ax1 ? QL.p2 : QL.p1, ax1 ? sn : !sn));
@@ -714,8 +710,8 @@ __device__ __forceinline__ void geoclaw_rotated(double n1, double n2, const Stat
     fL.s = ms;
     fR.h = netR[0];
     fR.s = ms;
-    const bool nfin = is_finite(netL[1]) && is_finite(netL[2]) && is_finite(netR[1]) && is_finite(netR[2]);
-    o.ok = o.ok && (!Ops::kFast || nfin);
+    const bool nfin = is_finite(netL[1]) & is_finite(netL[2]) & is_finite(netR[1]) & is_finite(netR[2]);
+    o.ok = o.ok & (!Ops::kFast | nfin);
     fL.p1 = z0(flip(ax1 ? netL[1] : netL[2], ax1 ? sn : !sn)); fL.p2 = z0(flip(ax1 ? netL[2] : netL[1], sn));
     fR.p1 = z0(flip(ax1 ? netR[1] : netR[2], ax1 ? sn : !sn)); fR.p2 = z0(flip(ax1 ? netR[2] : netR[1], sn));
     SWE_IF(diag && (Ops::kFast || nfin)) {
@@ -742,11 +738,11 @@ __device__ __forceinline__ void geoclaw_flux(double n1, double n2, const State& 
                                              double drytol, Update& fL, Update& fR, int axis, uint16_t* fz, Ops& o) {
     // both sides dry: the solver returns zero net updates and speed, and their
     // rotation back is +0 in every component, so neither rotation is needed
+    // (the tests of these branches are joined with & and |: a short-circuit test is a
+    // chain of branches, and lanes that leave it at different tests stay apart for
+    // the whole solver, which the warp then runs twice)
     const bool dry2 = FZ == 2 ? ((*fz & 1u) != 0)
-                              : (!lt(drytol, dL) && !lt(drytol, dR) && !is_nan(dL) && !is_nan(dR) && !is_nan(drytol));
-    // (one branch decides between the trivial edges and the solver: a return from
-    // inside a nested test would keep the lanes that pass it apart for the whole
-    // solver, which the warp then runs twice)
+                              : !(lt(drytol, dL) | lt(drytol, dR) | is_nan(dL) | is_nan(dR) | is_nan(drytol));
     bool rest = false;
     if (SOLVER == FWAVE && FZ == 0) {
         // Water at rest on both sides under one surface (lake at rest): every
@@ -776,12 +772,12 @@ __device__ __forceinline__ void geoclaw_flux(double n1, double n2, const State& 
         const bool still = ((dbits(QL.p1) | dbits(QL.p2) | dbits(QR.p1) | dbits(QR.p2)) << 1) == 0;
         // Where both surfaces are at +-0 (the sea level), dL = -bL and dR = -bR
         // exactly, so x = 0 - bL = dL for finite depths: no FP64 arithmetic at all.
-        const bool can = still && lt(drytol, dL) && lt(drytol, dR) && is_finite(dL) && is_finite(dR);
+        const bool can = still & lt(drytol, dL) & lt(drytol, dR) & is_finite(dL) & is_finite(dR);
         const bool level = ((dbits(QL.h) | dbits(QR.h)) << 1) == 0;
-        rest = can && level;
-        SWE_IF(can && !level) rest = dbits((QR.b + dR) - QL.b) == dbits(dL);
+        rest = can & level;
+        SWE_IF(can & !level) rest = dbits((QR.b + dR) - QL.b) == dbits(dL);
     }
-    if (dry2 || rest) {
+    if (dry2 | rest) {
         if (FZ == 1) *fz = 1;
         const double ms = rest ? bitsd(dbits(sqL) > dbits(sqR) ? dbits(sqL) : dbits(sqR)) : 0.0;
         fL = Update{0.0, 0.0, 0.0, ms};
