@@ -378,20 +378,33 @@ struct SegMem {
     u64* rh;      // recip_fix(depth) where the cell is wet
     double* sq;   // sqrt(g * depth) where the cell is wet
     double* upd;  // [4 quantities][3 local edges][T]
-    int8_t* dep;  // the cells' depths
+    double* d;    // depth h - b, in an array of its own or in the staged surface's place (h)
+    double* tab;  // DepthTab's
+    int8_t* dep;  // the cells' refinement depths
+    // The arrays after the staging buffers.
+    __device__ __forceinline__ void lay_out(double* after, bool own_d, int max_ndepth) {
+        rh = reinterpret_cast<u64*>(after);
+        sq = after + T;
+        upd = after + 2 * T;
+        d = own_d ? after + 14 * T : nullptr;
+        tab = after + (own_d ? 15 : 14) * T;
+        dep = reinterpret_cast<int8_t*>(tab + 6 * max_ndepth);
+    }
     __device__ __forceinline__ double* hu() const { return h + T; }
     __device__ __forceinline__ double* hv() const { return h + 2 * T; }
     __device__ __forceinline__ double* b() const { return h + 3 * T; }
 };
 
+__host__ __device__ constexpr bool geoclaw(int solver) { return solver == FWAVE || solver == AUG_RIEMANN; }
+
 // One edge task (skeleton_scalar_op / bnd_skeleton_scalar_op,
 // src/SWE/SWE_euler_timestep.f90:196-255): the updates of both sides into the
 // slots of the cells in the segment. With SHARED_STATE other CTAs write the
-// neighbours' state in this launch, so it is read past the L1 cache. Returns 0,
-// kBadIndex, or kRedo where FastOps does not take the edge's operands (nothing is
-// written then).
+// neighbours' state in this launch, so it is read past the L1 cache. DEPTHS: M.d holds
+// the depths. Returns 0, kBadIndex, or kRedo where FastOps does not take the edge's
+// operands (nothing is written then).
 constexpr unsigned int kBadIndex = 1u, kRedo = 8u;
-template <int SOLVER, int FZ, bool SHARED_STATE, class Ops>
+template <int SOLVER, int FZ, bool SHARED_STATE, bool DEPTHS, class Ops>
 __device__ __forceinline__ unsigned int edge_task_with(const StepArgs& A, const SegMem& M, const int4 tk, uint16_t* erec,
                                                   int c0, int cn, int odd, double drytol, int bc, const double* hin,
                                                        const double* huin, const double* hvin) {
@@ -422,8 +435,8 @@ __device__ __forceinline__ unsigned int edge_task_with(const StepArgs& A, const 
         depth_terms(Q, drytol, d, sq, y);
     };
     auto near = [&](int i, State& Q, double& d, double& sq, u64& y) {
-        Q = State{M.h[i], M.hu()[i], M.hv()[i], M.b()[i]};
-        d = Q.h - Q.b;
+        Q = State{M.h[i], M.hu()[i], M.hv()[i], M.b()[i]};  // (h is d where d took its place)
+        d = DEPTHS ? M.d[i] : Q.h - Q.b;
         sq = M.sq[i];
         y = M.rh[i];
     };
@@ -462,21 +475,21 @@ __device__ __forceinline__ unsigned int edge_task_with(const StepArgs& A, const 
 
 // The task again with SafeOps (a call, so that the callers keep their registers;
 // it reads the operands again, so that they need not hold them either).
-template <int SOLVER, bool SHARED_STATE>
+template <int SOLVER, bool SHARED_STATE, bool DEPTHS>
 static __device__ __noinline__ unsigned int edge_task_redo(const StepArgs& A, const SegMem M, const int4 tk, int c0,
                                                            int cn, int odd, double drytol, int bc, int ib) {
-    return edge_task_with<SOLVER, 0, SHARED_STATE, SafeOps>(A, M, tk, nullptr, c0, cn, odd, drytol, bc, A.h[ib],
+    return edge_task_with<SOLVER, 0, SHARED_STATE, DEPTHS, SafeOps>(A, M, tk, nullptr, c0, cn, odd, drytol, bc, A.h[ib],
                                                             A.hu[ib], A.hv[ib]);
 }
-template <int SOLVER, int FZ, bool SHARED_STATE>
+template <int SOLVER, int FZ, bool SHARED_STATE, bool DEPTHS>
 __device__ __forceinline__ unsigned int edge_task(const StepArgs& A, const SegMem& M, const int4 tk, uint16_t* erec,
                                                   int c0, int cn, int odd, double drytol, int bc, int ib) {
     if (FZ)
-        return edge_task_with<SOLVER, FZ, SHARED_STATE, SafeOps>(A, M, tk, erec, c0, cn, odd, drytol, bc, A.h[ib],
+        return edge_task_with<SOLVER, FZ, SHARED_STATE, DEPTHS, SafeOps>(A, M, tk, erec, c0, cn, odd, drytol, bc, A.h[ib],
                                                                  A.hu[ib], A.hv[ib]);
-    unsigned int rc = edge_task_with<SOLVER, 0, SHARED_STATE, FastOps>(A, M, tk, nullptr, c0, cn, odd, drytol, bc,
+    unsigned int rc = edge_task_with<SOLVER, 0, SHARED_STATE, DEPTHS, FastOps>(A, M, tk, nullptr, c0, cn, odd, drytol, bc,
                                                                        A.h[ib], A.hu[ib], A.hv[ib]);
-    if (rc == kRedo) rc = edge_task_redo<SOLVER, SHARED_STATE>(A, M, tk, c0, cn, odd, drytol, bc, ib);
+    if (rc == kRedo) rc = edge_task_redo<SOLVER, SHARED_STATE, DEPTHS>(A, M, tk, c0, cn, odd, drytol, bc, ib);
     return rc;
 }
 
@@ -490,10 +503,11 @@ struct CellOut {
     int8_t flag;
     uint8_t branch;
 };
+__device__ __forceinline__ int high_word(double x) { return (int)(dbits(x) >> 32); }
 static __device__ __noinline__ double quotient(double a, double b) { return div_one(a, b); }
 template <int FZ>
 __device__ __forceinline__ CellOut update_cell(const SegMem& M, const DepthTab& tab, const InstParams& P, int i,
-                                               int odd, unsigned long long wkey, uint8_t rb, Reduced& r) {
+                                               double h, double depth, int odd, unsigned long long wkey, uint8_t rb, Reduced& r) {
     const int T = M.T, k0 = odd ? 2 : 0, k2 = odd ? 0 : 2;
     const int d = M.dep[i];
     const int di = d - P.dmin;
@@ -533,7 +547,7 @@ __device__ __forceinline__ CellOut update_cell(const SegMem& M, const DepthTab& 
         }
     }
     r.key = key > r.key ? key : r.key;
-    double h = M.h[i], p1 = M.hu()[i], p2 = M.hv()[i];
+    double p1 = M.hu()[i], p2 = M.hv()[i];
     const double b = M.b()[i];
     uint8_t br = 0;
     long long nrm = 0;  // bits of |sum of the lengths times the updates of h|
@@ -572,18 +586,29 @@ __device__ __forceinline__ CellOut update_cell(const SegMem& M, const DepthTab& 
         dh = prod_cell(ndv, dh);
         dp1 = prod_cell(ndv, dp1);
         dp2 = prod_cell(ndv, dp2);
-        const double bdry = b + P.drytol;
-        // flooded land starts at the dry tolerance, at rest
-        if (FZ == 2 ? (rb & 1u) != 0 : (!deep && lt(h, bdry) && gt0(dh))) {
-            h = bdry;
-            p1 = 0.0;
-            p2 = 0.0;
-            br = 1;
+        // A wet cell that certainly stays wet, from the high words, without b + drytol: with
+        // depth = RN(h - b) in [2^e, 2^(e + 1)), |dh| and drytol at most depth / 8 (and 2^(e - 23)),
+        // the sums h + dh and b + drytol are at least depth / 2 apart, and with |h| and |b| below
+        // 2^(e + 47) their roundings move them by less than 2^(e - 5). The words of
+        // infinities and NaN are above every bound.
+        const int room = high_word(depth);
+        const bool stays = deep & (max(high_word(iabs(dh)), high_word(P.drytol)) <= room - (3 << 20)) &
+                           (max(high_word(iabs(h)), high_word(iabs(b))) - (45 << 20) <= room) & (room < (1900 << 20));
+        double bdry = 0.0;
+        SWE_IF(!stays) {
+            bdry = b + P.drytol;
+            // flooded land starts at the dry tolerance, at rest
+            if (FZ == 2 ? (rb & 1u) != 0 : (!deep && lt(h, bdry) && gt0(dh))) {
+                h = bdry;
+                p1 = 0.0;
+                p2 = 0.0;
+                br = 1;
+            }
         }
         h = h + dh;
         p1 = p1 + dp1;
         p2 = p2 + dp2;
-        if (FZ == 2 ? (rb & 2u) != 0 : lt(h, bdry)) {  // dried out: surface to min(b, 0), at rest
+        if (!stays && (FZ == 2 ? (rb & 2u) != 0 : lt(h, bdry))) {  // dried out: surface to min(b, 0), at rest
             h = lt0(b) ? b : 0.0;
             p1 = 0.0;
             p2 = 0.0;
@@ -612,9 +637,18 @@ __device__ __forceinline__ unsigned long long warp_key_bound(unsigned long long 
     return (unsigned long long)__reduce_max_sync(0xffffffffu, (unsigned)(key >> 32)) << 32;
 }
 
-template <int SOLVER, int FZ = 0>
+// The GeoClaw edges read a cell's depth instead of subtracting twice per edge (3 FP64
+// instructions per cell): it takes the staged surface's place, and the cell update reads
+// the surface from memory again (from the L2 cache). An array of its own would take the
+// place of 32 of a segment's 384 cells; a segment of 352 with it measured 2495 us for 4
+// steps of a 2^22-cell bowl and 2276 of a 2^23-cell basin against 2489 and 2245. Where
+// the state is in host memory (HOST) the second read would cross the link again (2^20
+// cells: 294 us against 275), so there the edges subtract; the Lax-Friedrichs edges need
+// the surface.
+template <int SOLVER, int FZ = 0, bool HOST = false>
 __global__ void SWE_STEP_BOUNDS step_kernel(const __grid_constant__ StepArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr bool kDepths = geoclaw(SOLVER) && !HOST;
     const int T = A.seg_cells;
     // staging buffers [stage_depth][h, hu, hv, b][T]: with depth 2 the next
     // segment's bulk copies land in one buffer while the CTA works on the other
@@ -622,11 +656,8 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const __grid_constant__ StepArgs A) 
     double* stage = reinterpret_cast<double*>(smem_raw);
     SegMem M;
     M.T = T;
-    M.rh = reinterpret_cast<u64*>(stage + (depth2 ? 8 : 4) * T);
-    M.sq = reinterpret_cast<double*>(M.rh + T);
-    M.upd = M.sq + T;
-    const DepthTab tab(M.upd + 12 * T, A.max_ndepth);
-    M.dep = reinterpret_cast<int8_t*>(tab.up + A.max_ndepth);
+    M.lay_out(stage + (depth2 ? 8 : 4) * T, false, A.max_ndepth);
+    const DepthTab tab(M.tab, A.max_ndepth);
     __shared__ uint64_t bar[2];
     __shared__ RedSlots red;
     __shared__ InstParams P;  // the running instance's
@@ -762,6 +793,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const __grid_constant__ StepArgs A) 
         __syncthreads();
         if (s_error) break;
         M.h = stage + (size_t)kbuf * 4 * T;
+        M.d = M.h;
         const double drytol = P.drytol;
         for (int i = tid; i < cn; i += blockDim.x) {
             // depth_terms, with the square root and reciprocal skipped by warps of dry cells.
@@ -793,6 +825,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const __grid_constant__ StepArgs A) 
             if (need_y) y = recip_fix(d);
             M.rh[i] = y;
             M.sq[i] = sq;
+            if (kDepths) M.h[i] = d;
         }
         // halo tasks: the cross-edge pass computed these edges' updates; copy
         // this segment's side into its slot
@@ -828,7 +861,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const __grid_constant__ StepArgs A) 
             for (int t = tid; t < nm; t += blockDim.x) {
                 const int4 tk = next;
                 if (t + (int)blockDim.x < nm) next = __ldg(&tasks[t + blockDim.x]);
-                if (edge_task<SOLVER, FZ, false>(A, M, tk, FZ ? A.erec + t0 + t : nullptr, c0, cn, odd, drytol, P.bc,
+                if (edge_task<SOLVER, FZ, false, kDepths>(A, M, tk, FZ ? A.erec + t0 + t : nullptr, c0, cn, odd, drytol, P.bc,
                                                  ib))
                     atomicOr(&s_error, 1u);
             }
@@ -846,7 +879,8 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const __grid_constant__ StepArgs A) 
         double* hvout = A.hv[ib ^ 1];
         for (int i = tid; i < cn; i += blockDim.x) {
             const int c = c0 + i;
-            const CellOut o = update_cell<FZ>(M, tab, P, i, odd, wkey, FZ == 2 ? A.branch[c] : (uint8_t)0, r);
+            const double h = kDepths ? hin[c] : M.h[i], depth = kDepths ? M.d[i] : 0.0;
+            const CellOut o = update_cell<FZ>(M, tab, P, i, h, depth, odd, wkey, FZ == 2 ? A.branch[c] : (uint8_t)0, r);
             if (FZ != 2 && A.branch) A.branch[c] = o.branch;
             hout[c] = o.h;
             huout[c] = o.p1;
@@ -940,11 +974,8 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const __grid_constant__
     SegMem M;
     M.T = T;
     M.h = reinterpret_cast<double*>(smem_raw);
-    M.rh = reinterpret_cast<u64*>(M.h + 4 * T);
-    M.sq = reinterpret_cast<double*>(M.rh + T);
-    M.upd = M.sq + T;
-    const DepthTab tab(M.upd + 12 * T, A.max_ndepth);
-    M.dep = reinterpret_cast<int8_t*>(tab.up + A.max_ndepth);
+    M.lay_out(M.h + 4 * T, true, A.max_ndepth);
+    const DepthTab tab(M.tab, A.max_ndepth);
     __shared__ RedSlots red;
     __shared__ InstParams P;
     __shared__ unsigned int s_error;
@@ -987,6 +1018,7 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const __grid_constant__
             M.sq[i] = sq;
         }
         if (!same_depth || (need_y && M.rh[i] == 0)) M.rh[i] = need_y ? recip_fix(d) : 0;
+        M.d[i] = d;
     };
     __syncthreads();
     const double drytol = P.drytol;
@@ -1030,7 +1062,7 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const __grid_constant__
             const int4 tk = next;
             t = t < nm ? after(t) : t + bd;
             if (t < nt) next = __ldg(&tasks[t]);
-            bad = edge_task<SOLVER, 0, true>(A, M, tk, nullptr, c0, cn, odd, drytol, P.bc, odd);
+            bad = edge_task<SOLVER, 0, true, geoclaw(SOLVER)>(A, M, tk, nullptr, c0, cn, odd, drytol, P.bc, odd);
         }
         if (dt_warp && bd - 32 < nm) prepare_dt();
         if (bad) atomicOr(&s_error, bad);
@@ -1042,7 +1074,7 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const __grid_constant__
         const bool last = k == n_steps - 1;
         double *hout = A.h[odd ^ 1], *huout = A.hu[odd ^ 1], *hvout = A.hv[odd ^ 1];
         for (int i = tid; i < cn; i += bd) {
-            const CellOut o = update_cell<0>(M, tab, P, i, odd, 0ull, 0, r);
+            const CellOut o = update_cell<0>(M, tab, P, i, M.h[i], M.d[i], odd, 0ull, 0, r);
             const bool same = dbits(o.h) == dbits(M.h[i]);
             M.h[i] = o.h;
             M.hu()[i] = o.p1;

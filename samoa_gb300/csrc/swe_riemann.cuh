@@ -582,7 +582,13 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
         const Recip rD = recip_of(sE2 - sE1);
         double beta1 = o.div(prod(sE2, delhu) - dpd, rD);
         double beta2 = o.div(dpd - prod(sE1, delhu), rD);
-        sw[0] = sE1; sw[1] = oscale(sE1 + sE2, -1, 0.5, o); sw[2] = sE2;
+        // Of the middle speed (sE1 + sE2) / 2 the net updates read the sign, which is the
+        // exact sum's (a sum of doubles rounds to zero only where it is zero, and with sE2 -
+        // sE1 in the reciprocal's range halving it does not underflow), and the maximum
+        // never takes it: half a rounded sum is at most the larger of the two magnitudes.
+        const long long k1 = num_key(sE1), k2 = num_key(flip(sE2, true));
+        const double sign = k1 < k2 ? -1.0 : (k1 > k2 ? 1.0 : 0.0);
+        sw[0] = sE1; sw[1] = Ops::kFast ? sign : scale_pow2(sE1 + sE2, -1, 0.5); sw[2] = sE2;
         fw[0][0] = beta1; fw[1][0] = prod(beta1, sE1); fw[2][0] = prod(beta1, vL);
         fw[0][2] = beta2; fw[1][2] = prod(beta2, sE2); fw[2][2] = prod(beta2, vR);
         fw[0][1] = 0.0; fw[1][1] = 0.0;
@@ -657,7 +663,7 @@ __device__ __forceinline__ void geoclaw_solver(double hL, double hR, double huL,
     // patterns (non-negative values order like them; a NaN candidate never wins)
     long long m = abs_bits(sw[0]);
     const long long a1 = abs_bits(sw[1]), a2 = abs_bits(sw[2]);
-    if (a1 > m && (Ops::kFast || not_nan(a1))) m = a1;
+    if (Ops::kFast ? SOLVER == AUG_RIEMANN && a1 > m : a1 > m && not_nan(a1)) m = a1;
     if (a2 > m && (Ops::kFast || not_nan(a2))) m = a2;
     maxspeed = bitsd(m);
 }

@@ -203,10 +203,11 @@ __global__ void misfit_kernel(const double* value, const double* obs, int64_t n,
 
 typedef void (*StepKernel)(StepArgs);
 
-static StepKernel kernel_for(int solver) {
+// host: for a state in the caller's (host) memory
+static StepKernel kernel_for(int solver, bool host = false) {
     switch (solver) {
-        case FWAVE: return step_kernel<FWAVE>;
-        case AUG_RIEMANN: return step_kernel<AUG_RIEMANN>;
+        case FWAVE: return host ? step_kernel<FWAVE, 0, true> : step_kernel<FWAVE>;
+        case AUG_RIEMANN: return host ? step_kernel<AUG_RIEMANN, 0, true> : step_kernel<AUG_RIEMANN>;
         case LF: return step_kernel<LF>;
         case LF_BATH: return step_kernel<LF_BATH>;
         case LLF: return step_kernel<LLF>;
@@ -239,7 +240,7 @@ static void* multi_kernel_for(int solver) {
     }
 }
 
-void* fma_step_kernel(int solver);
+void* fma_step_kernel(int solver, bool host);
 void* fma_cross_kernel(int solver);
 void* fma_multi_kernel(int solver);
 cudaError_t fma_upload_tables();
@@ -284,6 +285,7 @@ struct swe_ctx {
     int grid = 0, max_ndepth = 1;
     size_t smem = 0;
     std::vector<int32_t> first_seg; // of each instance, and n_seg
+    size_t multi_smem = 0;          // of the multi-step kernel, whose segments hold their depths too
     bool multi_fits = false;        // every segment has a CTA of the multi-step kernel on the GPU at once
     // device memory
     double* h[2] = {nullptr, nullptr};
@@ -377,16 +379,18 @@ int device_alloc(void** p, size_t bytes) {
     return SWE_OK;
 }
 
-size_t smem_bytes_for(int64_t seg_cells, int stage_depth, int max_ndepth) {
-    // staging [depth][4][T], recip_fix(depth) and sqrt(g depth) [2][T], edge slots [12][T], depth tables [6][nd],
-    // the cells' depths [T] bytes
-    return (size_t)(14 + 4 * stage_depth) * (size_t)seg_cells * sizeof(double) + (size_t)6 * max_ndepth * sizeof(double) +
-           (((size_t)seg_cells + 15) & ~(size_t)15);
+size_t smem_bytes_for(int64_t seg_cells, int stage_depth, int max_ndepth, bool own_d = false) {
+    // staging [depth][4][T], recip_fix(depth) and sqrt(g depth) [2][T], edge slots [12][T], with own_d the depths
+    // h - b [T], depth tables [6][nd], the cells' refinement depths [T] bytes
+    return (size_t)(14 + 4 * stage_depth + (own_d ? 1 : 0)) * (size_t)seg_cells * sizeof(double) +
+           (size_t)6 * max_ndepth * sizeof(double) + (((size_t)seg_cells + 15) & ~(size_t)15);
 }
 
-size_t smem_bytes(const swe_ctx* c) { return smem_bytes_for(c->seg_cells, c->stage_depth, c->max_ndepth); }
+size_t smem_bytes(const swe_ctx* c, bool own_d) {
+    return smem_bytes_for(c->seg_cells, c->stage_depth, c->max_ndepth, own_d);
+}
 
-constexpr size_t kMaxSmem = 227 * 1024;
+constexpr size_t kMaxSmem = 227 * 1024, kStaticSmem = 1024;  // of a CTA; more than the kernels' static part
 
 int check_params(const swe_params* p) {
     if (!kernel_for(p->solver)) return set_error(SWE_E_INVALID, "unknown solver %d", p->solver);
@@ -472,14 +476,15 @@ int raise_smem_limit(const void* k, size_t bytes) {
 }
 
 int configure_launch(swe_ctx* c) {
-    c->smem = smem_bytes(c);
     StepKernel k = kernel_for(c->params.empty() ? FWAVE : c->params[0].solver);
     if (!k) return set_error(SWE_E_INVALID, "unknown solver");
     int rc;
+    c->smem = smem_bytes(c, false);
     for (int s : {FWAVE, AUG_RIEMANN, LF, LF_BATH, LLF, LLF_BATH}) {
-        if ((rc = raise_smem_limit((const void*)kernel_for(s), c->smem)) ||
-            (rc = raise_smem_limit((const void*)fma_step_kernel(s), c->smem)))
-            return rc;
+        for (bool host : {false, true})
+            if ((rc = raise_smem_limit((const void*)kernel_for(s, host), c->smem)) ||
+                (rc = raise_smem_limit((const void*)fma_step_kernel(s, host), c->smem)))
+                return rc;
     }
     if ((rc = raise_smem_limit((const void*)step_kernel<FWAVE, 1>, c->smem)) ||
         (rc = raise_smem_limit((const void*)step_kernel<FWAVE, 2>, c->smem)))
@@ -491,10 +496,12 @@ int configure_launch(swe_ctx* c) {
                          c->block_threads);
     int64_t g = (int64_t)per_sm * c->num_sms;
     c->grid = (int)std::max<int64_t>(1, std::min<int64_t>(g, c->n_seg));
-    c->multi_fits = true;
+    c->multi_smem = smem_bytes(c, true);
+    c->multi_fits = c->multi_smem + kStaticSmem <= kMaxSmem;
     for (void* m : {multi_kernel_for(c->params[0].solver), fma_multi_kernel(c->params[0].solver)}) {
-        if ((rc = raise_smem_limit(m, c->smem))) return rc;
-        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, m, c->block_threads, c->smem));
+        if (!c->multi_fits) break;
+        if ((rc = raise_smem_limit(m, c->multi_smem))) return rc;
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, m, c->block_threads, c->multi_smem));
         c->multi_fits = c->multi_fits && c->n_seg <= (int64_t)per_sm * c->num_sms;
     }
     drop_graphs(c);
@@ -819,7 +826,8 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     // the adjoint's forward step (branch output) always runs the strict kernel,
     // so its branches are the ones the reverse sweep re-evaluates
     const bool fma = c->arith == SWE_ARITH_FMA && !branch;
-    void* k = fma ? fma_step_kernel(c->params[0].solver) : (void*)kernel_for(c->params[0].solver);
+    void* k = fma ? fma_step_kernel(c->params[0].solver, io != nullptr)
+                  : (void*)kernel_for(c->params[0].solver, io != nullptr);
     void* kx = fma ? fma_cross_kernel(c->params[0].solver) : cross_kernel_for(c->params[0].solver);
     A.erec = erec;
     A.xrec = erec ? erec + c->n_tasks : nullptr;
@@ -846,7 +854,7 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)c->n_seg);
         cfg.blockDim = dim3((unsigned)c->block_threads);
-        cfg.dynamicSmemBytes = c->smem;
+        cfg.dynamicSmemBytes = c->multi_smem;
         cfg.stream = c->stream;
         cfg.attrs = &at;
         cfg.numAttrs = 1;

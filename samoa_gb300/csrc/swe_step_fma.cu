@@ -9,10 +9,14 @@
 
 namespace swe {
 
-void* fma_step_kernel(int solver) {
+void* fma_step_kernel(int solver, bool host) {
     switch (solver) {
-        case swe_fma::FWAVE: return (void*)swe_fma::step_kernel<swe_fma::FWAVE>;
-        case swe_fma::AUG_RIEMANN: return (void*)swe_fma::step_kernel<swe_fma::AUG_RIEMANN>;
+        case swe_fma::FWAVE:
+            return host ? (void*)swe_fma::step_kernel<swe_fma::FWAVE, 0, true>
+                        : (void*)swe_fma::step_kernel<swe_fma::FWAVE>;
+        case swe_fma::AUG_RIEMANN:
+            return host ? (void*)swe_fma::step_kernel<swe_fma::AUG_RIEMANN, 0, true>
+                        : (void*)swe_fma::step_kernel<swe_fma::AUG_RIEMANN>;
         case swe_fma::LF: return (void*)swe_fma::step_kernel<swe_fma::LF>;
         case swe_fma::LF_BATH: return (void*)swe_fma::step_kernel<swe_fma::LF_BATH>;
         case swe_fma::LLF: return (void*)swe_fma::step_kernel<swe_fma::LLF>;
