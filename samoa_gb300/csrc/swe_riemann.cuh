@@ -799,13 +799,73 @@ __device__ __forceinline__ double normal_velocity(double n1, double n2, double p
     return z0(n1 * o.div(p1, r)) + n2 * o.div(p2, r);
 }
 
+// lf_flux of two sides at or above the dry tolerance (the fluxes with bathymetry) for
+// the mesh's normals, in 33 (axis-aligned) or 44 (diagonal) FP64 instructions instead
+// of 49: a product with a component +-1 is a sign, one with +-0 a signed zero, whose
+// addition only decides the sign of a zero sum (add_zero); the products of one value
+// with the two components of a diagonal normal differ in sign; halves are exponents.
+// `on` is the component along an axis-aligned normal, `off` the other one. For FastOps:
+// other normals and values that are not finite leave o.ok false.
+template <int SOLVER, class Ops>
+__device__ __forceinline__ void lf_bath_wet(double n1, double n2, const State& QL, const State& QR, double hL,
+                                            double hR, double cL, double cR, const Recip& rL, const Recip& rR,
+                                            Update& fL, Update& fR, int axis, Ops& o) {
+    const double g = kG;
+    const bool second = axis == 2, diag = axis == 0;
+    const double non = second ? n2 : n1, noff = second ? n1 : n2;
+    const bool gon = dbits(non) < 0, goff = dbits(noff) < 0;
+    const double pLon = second ? QL.p2 : QL.p1, pLoff = second ? QL.p1 : QL.p2;
+    const double pRon = second ? QR.p2 : QR.p1, pRoff = second ? QR.p1 : QR.p2;
+    const double pr = (0.5 * g) * (hL * hL + hR * hR);
+    const double src = ((0.25 * g) * (hL + hR)) * (QR.b - QL.b);
+    const double qL = o.div(pLon, rL), qR = o.div(pRon, rR);
+    // (the off-axis quotients are finite, so their products with +-0 are zeros)
+    auto bounded = [](double x) { return abs_bits(x) < 1524ll << 52; };
+    o.ok = o.ok & is_finite(pr) & is_finite(src) & bounded(pLoff) & bounded(pRoff) &
+           (!diag | (abs_bits(n1) == abs_bits(n2)));
+    const u64 sign = 0x8000000000000000ull;
+    double vL = z0(flip(qL, gon)), vR = z0(flip(qR, gon));
+    double pon = flip(pr, gon), poff = bitsd((dbits(pr) ^ dbits(noff)) & (long long)sign);
+    double son = flip(src, gon), soff = bitsd((dbits(src) ^ dbits(noff)) & (long long)sign);
+    SWE_IF(diag) {
+        const double c = iabs(n1);
+        vL = z0(flip(c * qL, gon)) + flip(c * o.div(pLoff, rL), goff);
+        vR = z0(flip(c * qR, gon)) + flip(c * o.div(pRoff, rR), goff);
+        const double cp = c * pr, cs = c * src;
+        pon = flip(cp, gon);
+        poff = flip(cp, goff);
+        son = flip(cs, gon);
+        soff = flip(cs, goff);
+    }
+    fL.s = cL + iabs(vL);
+    fR.s = cR + iabs(vR);
+    const double alpha = (SOLVER == LLF_BATH) ? omax<Ops>(fL.s, fR.s) : 100.0;
+    fL.h = oscale((hL * vL + hR * vR) + alpha * (QL.h - QR.h), -1, 0.5, o);
+    fR.h = flip(fL.h, true);
+    const double aon = pLon * vL + pRon * vR, aoff = pLoff * vL + pRoff * vR;
+    double boff = add_zero(aoff, poff);
+    SWE_IF(diag) boff = aoff + poff;
+    const double fon = oscale((aon + pon) + alpha * (pLon - pRon), -1, 0.5, o);
+    const double foff = oscale(boff + alpha * (pLoff - pRoff), -1, 0.5, o);
+    const double lon = fon + son, ron = flip(fon, true) + son;
+    double loff = add_zero(foff, soff), roff = add_zero(flip(foff, true), soff);
+    SWE_IF(diag) {
+        loff = foff + soff;
+        roff = flip(foff, true) + soff;
+    }
+    fL.p1 = second ? loff : lon;
+    fL.p2 = second ? lon : loff;
+    fR.p1 = second ? roff : ron;
+    fR.p2 = second ? ron : roff;
+}
+
 // compute_lf_flux, src/SWE/SWE_euler_timestep.f90:359-446
 // sqL / sqR, yL / yR: sqrt(g * depth) and recip_fix of the two depths where they are
 // above the dry tolerance (else not read).
 template <int SOLVER, class Ops>
 __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, const State& QR, double dL,
                                         double dR, double drytol, Update& fL, Update& fR, double sqL,
-                                        double sqR, u64 yL, u64 yR, Ops& o) {
+                                        double sqR, u64 yL, u64 yR, int axis, Ops& o) {
     const double g = kG;
     if (SOLVER == LF_BATH || SOLVER == LLF_BATH) {
         const bool aL = lt(drytol, dL), aR = lt(drytol, dR);
@@ -833,13 +893,17 @@ __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, c
             return;
         }
         double hL = imax(dL, 0.0), hR = imax(dR, 0.0);
-        double vL = normal_velocity(n1, n2, QL.p1, QL.p2, rL, o);
-        double vR = normal_velocity(n1, n2, QR.p1, QR.p2, rR, o);
         double cL = sqL, cR = sqR;
         SWE_IF(!aL || !aR) {  // a depth at the tolerance
             cL = aL ? sqL : sqrt_fix(g * hL);
             cR = aR ? sqR : sqrt_fix(g * hR);
         }
+        if (Ops::kFast) {
+            lf_bath_wet<SOLVER>(n1, n2, QL, QR, hL, hR, cL, cR, rL, rR, fL, fR, axis, o);
+            return;
+        }
+        double vL = normal_velocity(n1, n2, QL.p1, QL.p2, rL, o);
+        double vR = normal_velocity(n1, n2, QR.p1, QR.p2, rR, o);
         fL.s = cL + iabs(vL);
         fR.s = cR + iabs(vR);
         double alpha = (SOLVER == LLF_BATH) ? imax(fL.s, fR.s) : 100.0;
@@ -875,6 +939,12 @@ __device__ __forceinline__ void lf_flux(double n1, double n2, const State& QL, c
     }
 }
 
+// The direction of a normal, as the fluxes take it: 1 = (+-1, +-0), 2 = (+-0, +-1), 0 = any other.
+__device__ __forceinline__ int axis_of(double n1, double n2) {
+    const long long one = 0x3ff0000000000000ll, a = abs_bits(n1), b = abs_bits(n2);
+    return (a == one) & (b == 0) ? 1 : ((a == 0) & (b == one) ? 2 : 0);
+}
+
 // One edge: dL/dR are the depths h - b of the two states, sqL/sqR their
 // sqrt(g * depth) and yL/yR recip_fix(depth) (only read for depths above the dry
 // tolerance).
@@ -886,7 +956,7 @@ __device__ __forceinline__ void edge_flux(double n1, double n2, const State& QL,
     if (SOLVER == FWAVE || SOLVER == AUG_RIEMANN)
         geoclaw_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, fz, o);
     else
-        lf_flux<SOLVER>(n1, n2, QL, QR, dL, dR, drytol, fL, fR, sqL, sqR, yL, yR, o);
+        lf_flux<SOLVER>(n1, n2, QL, QR, dL, dR, drytol, fL, fR, sqL, sqR, yL, yR, axis, o);
 }
 
 // depth, sqrt(g * depth) and recip_fix(depth) of a state, as the edge code needs them

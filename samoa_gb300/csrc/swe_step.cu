@@ -56,7 +56,8 @@ __global__ void riemann_batch_kernel(int64_t n, const double* nrm, const double*
         edge_flux<SOLVER, 0>(nrm[2 * i], nrm[2 * i + 1], L, R, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, 0, nullptr, o);
         FastOps f;
         Update gL, gR;
-        edge_flux<SOLVER, 0>(nrm[2 * i], nrm[2 * i + 1], L, R, dL, dR, sqL, sqR, yL, yR, drytol, gL, gR, 0, nullptr, f);
+        edge_flux<SOLVER, 0>(nrm[2 * i], nrm[2 * i + 1], L, R, dL, dR, sqL, sqR, yL, yR, drytol, gL, gR,
+                             axis_of(nrm[2 * i], nrm[2 * i + 1]), nullptr, f);
         if (f.ok) {
             fL = gL;
             fR = gR;
