@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <memory>
+#include <system_error>
 #include <thread>
 #include <type_traits>
 #include <utility>
@@ -121,14 +122,18 @@ int set_error(int code, const char* fmt, ...);
 
 // Host passes over large meshes run on several threads: [0, n) is split into
 // `parts` contiguous ranges, fn(begin, end, part) runs each (part 0 on the
-// calling thread). Meshes below 2^20 items stay on one thread.
+// calling thread). A thread takes about 15 us to start and 2^SWE_PART_LOG2 items 100 us,
+// so lists below twice that stay on one thread.
 #ifndef SWE_HOST_THREADS
 #define SWE_HOST_THREADS 16
 #endif
+#ifndef SWE_PART_LOG2
+#define SWE_PART_LOG2 15
+#endif
 inline int host_parts(int64_t n) {
-    if (n < ((int64_t)1 << 20)) return 1;
+    if (n < ((int64_t)2 << SWE_PART_LOG2)) return 1;
     const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-    return (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)std::min(hw, SWE_HOST_THREADS), n >> 16}));
+    return (int)std::min<int64_t>(std::min(hw, SWE_HOST_THREADS), n >> SWE_PART_LOG2);
 }
 template <class F>
 void parallel_parts(int64_t n, int parts, F&& fn) {
@@ -137,10 +142,15 @@ void parallel_parts(int64_t n, int parts, F&& fn) {
         e = n * (p + 1) / parts;
     };
     std::vector<std::thread> th;
+    th.reserve((size_t)parts);
     for (int p = 1; p < parts; ++p) {
         int64_t b, e;
         range(p, b, e);
-        th.emplace_back([&fn, b, e, p] { fn(b, e, p); });
+        try {
+            th.emplace_back([&fn, b, e, p] { fn(b, e, p); });
+        } catch (const std::system_error&) {  // no thread to be had: this one does the part
+            fn(b, e, p);
+        }
     }
     int64_t b, e;
     range(0, b, e);

@@ -263,26 +263,40 @@ int export_mesh(const BuiltMesh& m, int8_t* depth_out, int8_t* plotter_out, int6
 // a task in both (each keeps its own side, so no segment waits for another). A
 // boundary edge is a task in its cell's segment. Boundary tasks come first in a
 // segment, then inner edges in stream (first-touch) order.
-// Direction of the outward normal of local edge k (0..2) of a cell with plotter
-// type p: 1 = along x, 2 = along y, 0 = diagonal.
-// Direction of the outward normal of local edge k of a cell of plotter type p:
-// 0 diagonal, 1 along x, 2 along y (a table built once, thread-safe).
-static int normal_axis(int p, int k) {
-    struct AxisTable {
-        int8_t axis[17][3];
-        AxisTable() {
-            double normal[17][3][2], leg[kMaxDepth + 2], vol[kMaxDepth + 1];
-            geometry_tables(leg, vol, normal);
-            for (int q = 0; q < 17; ++q)
-                for (int e = 0; e < 3; ++e) {
-                    const double* nv = normal[q][e];
-                    axis[q][e] = (nv[1] == 0.0 && nv[0] != 0.0) ? 1 : (nv[0] == 0.0 && nv[1] != 0.0) ? 2 : 0;
-                }
-        }
-    };
+// Direction of the outward normal of local edge k of a cell of plotter type p, at
+// [p + 8][k]: 0 diagonal, 1 along x, 2 along y (a table built once, thread-safe).
+struct AxisTable {
+    int8_t axis[17][3];
+    AxisTable() {
+        double normal[17][3][2], leg[kMaxDepth + 2], vol[kMaxDepth + 1];
+        geometry_tables(leg, vol, normal);
+        for (int q = 0; q < 17; ++q)
+            for (int e = 0; e < 3; ++e) {
+                const double* nv = normal[q][e];
+                axis[q][e] = (nv[1] == 0.0 && nv[0] != 0.0) ? 1 : (nv[0] == 0.0 && nv[1] != 0.0) ? 2 : 0;
+            }
+    }
+    int operator()(int p, int k) const { return axis[p + 8][k]; }
+};
+static const AxisTable& axis_table() {
     static const AxisTable table;
-    return table.axis[p + 8][k];
+    return table;
 }
+
+// The segment of a cell; consecutive edges mostly ask for the same one (a division
+// per edge and side was a third of the time of the lists).
+struct SegmentOf {
+    uint32_t T, lo = 0, seg = 0;
+    explicit SegmentOf(int32_t t) : T((uint32_t)t) {}
+    uint32_t operator()(int64_t cell) {
+        const uint32_t c = (uint32_t)cell;
+        if (c - lo >= T) {
+            seg = c / T;
+            lo = seg * T;
+        }
+        return seg;
+    }
+};
 
 // The segment lists: per segment the edges to compute, diagonal ones first, then
 // the axis-aligned ones (so a warp's tasks mostly take the same branch of the
@@ -299,31 +313,34 @@ int build_tasks(const HostMesh& m, int64_t offset, int32_t inst, int32_t T, std:
     // placed in list order (boundary edges first, then inner edges; cross edges
     // numbered in edge order), so the lists do not depend on the number of parts.
     const int PB = host_parts(m.n_bnd), PE = host_parts(m.n_edges);
+    const AxisTable& normal_axis = axis_table();
     const size_t ns = (size_t)(3 * nseg);
     std::vector<std::vector<int64_t>> cb((size_t)PB), ce((size_t)PE);
     std::vector<int64_t> xc((size_t)PE, 0);
     parallel_parts(m.n_bnd, PB, [&](int64_t j0, int64_t j1, int p) {
         std::vector<int64_t>& c = cb[(size_t)p];
         c.assign(ns, 0);
+        SegmentOf seg(T);
         for (int64_t j = j0; j < j1; ++j) {
             const int64_t cell = m.bc[(size_t)j];
             const int ax = normal_axis(m.plotter[(size_t)cell], m.bl[(size_t)j] - 1);
-            c[(size_t)(3 * (cell / T) + (ax ? 1 : 0))]++;
+            c[(size_t)(3 * seg(cell) + (ax ? 1 : 0))]++;
         }
     });
     parallel_parts(m.n_edges, PE, [&](int64_t e0, int64_t e1, int p) {
         std::vector<int64_t>& c = ce[(size_t)p];
         c.assign(ns, 0);
         int64_t x = 0;
+        SegmentOf seg(T), seg_b(T);
         for (int64_t e = e0; e < e1; ++e) {
             const int64_t a = m.ea[(size_t)e], b = m.eb[(size_t)e];
-            const int64_t sa = a / T, sb = b / T;
-            if (sa == sb) {
+            const uint32_t sa = seg(a);
+            if ((uint32_t)b - seg.lo < seg.T) {
                 const int ax = normal_axis(m.plotter[(size_t)a], m.la[(size_t)e] - 1);
                 c[(size_t)(3 * sa + (ax ? 1 : 0))]++;
             } else {
                 c[(size_t)(3 * sa + 2)]++;
-                c[(size_t)(3 * sb + 2)]++;
+                c[(size_t)(3 * seg_b(b) + 2)]++;
                 ++x;
             }
         }
@@ -377,6 +394,7 @@ int build_tasks(const HostMesh& m, int64_t offset, int32_t inst, int32_t T, std:
     xtasks.resize((size_t)nx);
     parallel_parts(m.n_bnd, PB, [&](int64_t j0, int64_t j1, int p) {
         std::vector<int64_t>& at = cb[(size_t)p];
+        SegmentOf seg(T);
         for (int64_t j = j0; j < j1; ++j) {
             const int64_t c = m.bc[(size_t)j];
             const int ax = normal_axis(m.plotter[(size_t)c], m.bl[(size_t)j] - 1);
@@ -385,12 +403,13 @@ int build_tasks(const HostMesh& m, int64_t offset, int32_t inst, int32_t T, std:
             t.b = -1;
             t.meta = pack_meta(m.bl[(size_t)j] - 1, 0, m.plotter[(size_t)c], 1, true, ax);
             t.pad = 0;
-            tasks[(size_t)at[(size_t)(3 * (c / T) + (ax ? 1 : 0))]++] = t;
+            tasks[(size_t)at[(size_t)(3 * seg(c) + (ax ? 1 : 0))]++] = t;
         }
     });
     parallel_parts(m.n_edges, PE, [&](int64_t e0, int64_t e1, int p) {
         std::vector<int64_t>& at = ce[(size_t)p];
         int64_t xi = xc[(size_t)p];
+        SegmentOf seg(T), seg_b(T);
         for (int64_t e = e0; e < e1; ++e) {
             const int64_t a = m.ea[(size_t)e], b = m.eb[(size_t)e];
             const int ax = normal_axis(m.plotter[(size_t)a], m.la[(size_t)e] - 1);
@@ -400,8 +419,8 @@ int build_tasks(const HostMesh& m, int64_t offset, int32_t inst, int32_t T, std:
             t.meta = pack_meta(m.la[(size_t)e] - 1, m.lb[(size_t)e] - 1, m.plotter[(size_t)a], m.plotter[(size_t)b],
                                false, ax);
             t.pad = 0;
-            const int64_t sa = a / T, sb = b / T;
-            if (sb == sa) {
+            const uint32_t sa = seg(a);
+            if ((uint32_t)b - seg.lo < seg.T) {
                 tasks[(size_t)at[(size_t)(3 * sa + (ax ? 1 : 0))]++] = t;
                 continue;
             }
@@ -413,7 +432,7 @@ int build_tasks(const HostMesh& m, int64_t offset, int32_t inst, int32_t T, std:
             t.pad = (uint32_t)inst;
             xtasks[(size_t)xi++] = t;
             tasks[(size_t)at[(size_t)(3 * sa + 2)]++] = h;
-            tasks[(size_t)at[(size_t)(3 * sb + 2)]++] = h;
+            tasks[(size_t)at[(size_t)(3 * seg_b(b) + 2)]++] = h;
         }
     });
     return SWE_OK;

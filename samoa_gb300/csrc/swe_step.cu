@@ -267,7 +267,8 @@ struct swe_ctx {
     cudaStream_t own_stream = nullptr;
     int num_sms = 0;
     // instances
-    std::vector<HostMesh> mesh;
+    std::vector<HostMesh> mesh, spare_mesh;  // spare: an earlier mesh's storage, for the next upload
+    hvec<Task> host_tasks, host_xtasks;      // likewise the task lists'
     std::vector<swe_params> params;
     std::vector<int64_t> offset;   // device cell offset of each instance (even)
     int64_t cells_total = 0;       // padded length of the device arrays
@@ -308,7 +309,10 @@ struct swe_ctx {
     InstScalars* is = nullptr;
     GlobalScalars* gs = nullptr;
     double* dt_seq = nullptr;
-    int64_t dt_seq_len = 0;
+    int64_t dt_seq_len = 0;         // 0: no sequence
+    size_t cap_dt_seq = 0;          // bytes of dt_seq, kept for the next sequence
+    void* sweep = nullptr;          // swe_gauge_gradient's buffers, up to kKeptSweep bytes, for the next call
+    size_t cap_sweep = 0;
     std::vector<double> dt_seq_host;
     uint8_t* branch = nullptr;      // wet/dry branch flags of the last forward step (adjoint)
     // per cell (d, sqrt(g d)) of the last depth the step kernel took a square root of: a
@@ -346,9 +350,8 @@ void drop_graphs(swe_ctx* c) {
 // `release` (else kept for a re-upload that fits them).
 void free_mesh_buffers(swe_ctx* c, bool release = true) {
     drop_graphs(c);
-    cudaFree(c->dt_seq); cudaFree(c->branch);
+    cudaFree(c->branch);
     c->branch = nullptr;
-    c->dt_seq = nullptr;
     c->dt_seq_len = 0;
     c->dt_seq_host.clear();
     c->has_mesh = c->has_state = false;
@@ -360,6 +363,10 @@ void free_mesh_buffers(swe_ctx* c, bool release = true) {
     cudaFree(c->b); cudaFree(c->depth); cudaFree(c->flags); cudaFree(c->tasks); cudaFree(c->seg_ptr);
     cudaFree(c->seg_info); cudaFree(c->seg_order); cudaFree(c->ip); cudaFree(c->is); cudaFree(c->xtasks); cudaFree(c->xflux);
     cudaFree(c->memo);
+    cudaFree(c->dt_seq); cudaFree(c->sweep);
+    c->dt_seq = nullptr;
+    c->sweep = nullptr;
+    c->cap_dt_seq = c->cap_sweep = 0;
     cudaFree(c->rows);
     c->rows = nullptr;
     c->cap_rows = 0;
@@ -536,10 +543,20 @@ static std::vector<int32_t> spread_order(const std::vector<SegInfo>& seg_info) {
     return order;
 }
 
+// Bytes of a sweep's buffers that stay with the context between calls.
+constexpr size_t kKeptSweep = (size_t)512 << 20;
+
+// Host lists of up to this many cells or tasks (up to 32 MB) stay with the context from
+// one mesh upload to the next: a fresh list of a small mesh costs more in page faults
+// than in filling it.
+constexpr size_t kKeptItems = (size_t)1 << 21;
+
 int rebuild_tasks(swe_ctx* c) {
     std::vector<int64_t> seg_ptr;
     std::vector<SegInfo> seg_info;
-    hvec<Task> tasks, xtasks;
+    hvec<Task>&tasks = c->host_tasks, &xtasks = c->host_xtasks;
+    tasks.clear();
+    xtasks.clear();
     c->first_seg.assign(1, 0);
     for (int i = 0; i < n_inst(c); ++i) {
         int rc = build_tasks(c->mesh[(size_t)i], c->offset[(size_t)i], i, c->seg_cells, seg_ptr, seg_info, tasks,
@@ -598,7 +615,11 @@ int rebuild_tasks(swe_ctx* c) {
     if (order.size() != seg_info.size()) return set_error(SWE_E_INVALID, "segment order is not a permutation");
     CUDA_TRY(cudaMemcpyAsync(c->seg_order, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice,
                              c->stream));
-    if ((rc = upload_inst_params(c))) return rc;  // they carry the instances' segments
+    if ((rc = upload_inst_params(c))) return rc;  // they carry the instances' segments (and it waits for the copies)
+    if (tasks.size() > kKeptItems) {
+        hvec<Task>().swap(tasks);
+        hvec<Task>().swap(xtasks);
+    }
     return configure_launch(c);
 }
 
@@ -667,7 +688,9 @@ int upload_meshes(swe_ctx* c, int64_t ni, const int64_t* n_cells, const int64_t*
     cudaSetDevice(c->device);
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     free_mesh_buffers(c, false);
-    std::vector<HostMesh> meshes((size_t)ni);
+    std::vector<HostMesh> meshes = std::move(c->spare_mesh);
+    c->spare_mesh.clear();
+    meshes.resize((size_t)ni);
     std::vector<int64_t> offset((size_t)ni);
     int64_t pc = 0, pe = 0, pb = 0, off = 0;
     int dmin = kMaxDepth, dmax = 0, max_nd = 1;
@@ -691,6 +714,7 @@ int upload_meshes(swe_ctx* c, int64_t ni, const int64_t* n_cells, const int64_t*
     }
     if (off >= ((int64_t)1 << 31) - 1) return set_error(SWE_E_INVALID, "total cells %lld >= 2^31", (long long)off);
     c->mesh.swap(meshes);
+    if ((size_t)c->cells_packed <= kKeptItems) c->spare_mesh = std::move(meshes);  // (of the mesh until now)
     c->offset.swap(offset);
     c->cells_total = off;
     c->cells_packed = pc;
@@ -1294,14 +1318,17 @@ int swe_set_dt_sequence(swe_ctx* c, int64_t n_steps, const double* dts) {
     if (n_steps < 0 || (n_steps > 0 && !dts)) return set_error(SWE_E_INVALID, "bad dt sequence");
     cudaSetDevice(c->device);
     CUDA_TRY(cudaStreamSynchronize(c->stream));
-    cudaFree(c->dt_seq);
-    c->dt_seq = nullptr;
     c->dt_seq_len = 0;
     drop_graphs(c);
     if (n_steps == 0) return SWE_OK;
     const size_t bytes = sizeof(double) * (size_t)n_steps * (size_t)n_inst(c);
-    int rc = device_alloc((void**)&c->dt_seq, bytes);
-    if (rc) return rc;
+    if (bytes > c->cap_dt_seq) {
+        cudaFree(c->dt_seq);
+        c->dt_seq = nullptr;
+        c->cap_dt_seq = 0;
+        if (int rc = device_alloc((void**)&c->dt_seq, bytes)) return rc;
+        c->cap_dt_seq = bytes;
+    }
     CUDA_TRY(cudaMemcpyAsync(c->dt_seq, dts, bytes, cudaMemcpyHostToDevice, c->stream));
     c->dt_seq_host.assign(dts, dts + (size_t)n_steps * (size_t)n_inst(c));
     mark_seq_base_kernel<<<1, 1, 0, c->stream>>>(c->gs);
@@ -1826,18 +1853,26 @@ int swe_gauge_gradient(swe_ctx* c, int64_t n_steps, const double* dts, int32_t s
     if ((rc = swe_set_dt_sequence(c, n_steps, dts))) return rc;
     S.s0 = c->step_mirror;
     const size_t nb = (size_t)S.N * 8;
-    double* work = nullptr;  // lam[2][3], out gauge values if not given
+    // lam[2][3], J, gauge values if not given, the snapshots, the branches: one buffer,
+    // kept with the context up to kKeptSweep bytes (three allocations and their
+    // releases, which wait for the GPU, took a good part of a small mesh's sweep)
     const size_t n_work = 6 * (size_t)S.N + (gauge_values ? 0 : (size_t)n_steps * (size_t)n_gauges) + 1;
-    if ((rc = device_alloc((void**)&work, n_work * 8))) return rc;
-    if ((rc = device_alloc((void**)&S.slots, (size_t)snapshots * 3 * nb))) {
-        cudaFree(work);
-        return rc;
+    const size_t n_slots = (size_t)snapshots * 3 * (size_t)S.N;
+    const size_t bytes = (n_work + n_slots) * 8 + (size_t)n_steps * (size_t)S.stride;
+    double* work = (double*)c->sweep;
+    double* own = nullptr;  // a buffer of this call
+    if (bytes > c->cap_sweep) {
+        if ((rc = device_alloc((void**)&work, bytes))) return rc;
+        if (bytes <= kKeptSweep) {
+            cudaFree(c->sweep);
+            c->sweep = work;
+            c->cap_sweep = bytes;
+        } else {
+            own = work;
+        }
     }
-    if ((rc = device_alloc((void**)&S.branches, (size_t)n_steps * (size_t)S.stride))) {
-        cudaFree(work);
-        cudaFree(S.slots);
-        return rc;
-    }
+    S.slots = work + n_work;
+    S.branches = (uint8_t*)(S.slots + n_slots);
     for (int i = 0; i < 2; ++i)
         for (int q = 0; q < 3; ++q) S.lam[i][q] = work + (size_t)(3 * i + q) * (size_t)S.N;
     double* dJ = work + 6 * (size_t)S.N;
@@ -1864,9 +1899,7 @@ int swe_gauge_gradient(swe_ctx* c, int64_t n_steps, const double* dts, int32_t s
         if (e != cudaSuccess) rc = set_error(SWE_E_CUDA, "gauge gradient: %s", cudaGetErrorString(e));
     }
     cudaStreamSynchronize(c->stream);
-    cudaFree(work);
-    cudaFree(S.slots);
-    cudaFree(S.branches);
+    cudaFree(own);
     if (forward_steps) *forward_steps = S.forward_steps;
     if (!rc) rc = check_device_error(c);
     return rc;
