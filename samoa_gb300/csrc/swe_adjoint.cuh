@@ -392,8 +392,8 @@ __device__ __forceinline__ void aug_rev(const AugRec& r, const double F[3][3], d
 }
 
 // VJP of the f-wave edge flux: given the cotangents gL / gR of the left/right
-// net updates (h, hu, hv, world frame), add the cotangents of the inputs to
-// outL / outR. QL / QR are the states (h = surface), dL / dR their depths,
+// net updates (h, hu, hv, world frame), the cotangents of the inputs in outL / outR
+// (zeros when passed). QL / QR are the states (h = surface), dL / dR their depths,
 // sqL0 / sqR0 their sqrt(g * depth) as in the forward step.
 // axis: the normal's direction as in geoclaw_flux (0 diagonal, 1 along x, 2 along y).
 // SOLVER: FWAVE or AUG_RIEMANN (the solver core between the shared wet/dry
@@ -439,22 +439,22 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
             const double gb2 = fma(sE2, nR, gR[0]);
             const double g_du = fma(sE2, gb1, -(sE1 * gb2)) * rD;  // cotangent of delhu
             const double g_dh = ghalf * ((gb2 - gb1) * rD);          // of hR' (minus it for hL')
-            outL.h -= g_dh;
-            outR.h += g_dh;
+            outL.h = flip(g_dh, true);
+            outR.h = g_dh;
             if (ax) {
                 const double t = flip(g_du, sg);
                 if (k == 1) {
-                    outL.hu -= t;
-                    outR.hu += t;
+                    outL.hu = flip(t, true);
+                    outR.hu = t;
                 } else {
-                    outL.hv -= t;
-                    outR.hv += t;
+                    outL.hv = flip(t, true);
+                    outR.hv = t;
                 }
             } else {
-                outL.hu = fma(-g_du, n1, outL.hu);
-                outL.hv = fma(-g_du, n2, outL.hv);
-                outR.hu = fma(g_du, n1, outR.hu);
-                outR.hv = fma(g_du, n2, outR.hv);
+                outR.hu = g_du * n1;
+                outR.hv = g_du * n2;
+                outL.hu = flip(outR.hu, true);
+                outL.hv = flip(outR.hv, true);
             }
             return;
         }
@@ -463,8 +463,11 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
     const bool fin = is_finite(QL.p1) && is_finite(QL.p2) && is_finite(QR.p1) && is_finite(QR.p2);
     const bool fast = axis != 0 && fin;
     const bool sn = axis == 1 ? lt0(n1) : lt0(n2);
-    double pL1, pL2, pR1, pR2;
-    if (axis == 0 && fin && abs_bits(n1) == abs_bits(n2)) {  // diagonal: two products per side
+    // (FP64 work that only some edges need stays behind real branches, as in the forward step)
+    const bool diag = axis == 0 && fin && abs_bits(n1) == abs_bits(n2), ax1 = axis == 1;
+    double pL1 = z0(flip(ax1 ? QL.p1 : QL.p2, sn)), pL2 = z0(flip(ax1 ? QL.p2 : QL.p1, ax1 ? sn : !sn));
+    double pR1 = z0(flip(ax1 ? QR.p1 : QR.p2, sn)), pR2 = z0(flip(ax1 ? QR.p2 : QR.p1, ax1 ? sn : !sn));
+    SWE_IF(diag) {  // two products per side
         const bool g1 = dbits(n1) < 0, g2 = dbits(n2) < 0;
         const double cn = bitsd(abs_bits(n1));
         const double aL1 = cn * QL.p1, aL2 = cn * QL.p2, aR1 = cn * QR.p1, aR2 = cn * QR.p2;
@@ -472,15 +475,8 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
         pL2 = z0(flip(aL1, !g2)) + flip(aL2, g1);
         pR1 = z0(flip(aR1, g1)) + flip(aR2, g2);
         pR2 = z0(flip(aR1, !g2)) + flip(aR2, g1);
-    } else if (fast) {
-        if (axis == 1) {
-            pL1 = z0(flip(QL.p1, sn)); pL2 = z0(flip(QL.p2, sn));
-            pR1 = z0(flip(QR.p1, sn)); pR2 = z0(flip(QR.p2, sn));
-        } else {
-            pL1 = z0(flip(QL.p2, sn)); pL2 = z0(flip(QL.p1, !sn));
-            pR1 = z0(flip(QR.p2, sn)); pR2 = z0(flip(QR.p1, !sn));
-        }
-    } else {
+    }
+    SWE_IF(!diag && !fast) {
         pL1 = z0(n1 * QL.p1) + n2 * QL.p2;
         pL2 = z0(-n2 * QL.p1) + n1 * QL.p2;
         pR1 = z0(n1 * QR.p1) + n2 * QR.p2;
@@ -553,7 +549,8 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
         beta1 = div_rn(sE2 * delhu - dpd, rD);
         beta2 = div_rn(dpd - sE1 * delhu, rD);
         sw[0] = sE1;
-        sw[1] = 0.5 * (sE1 + sE2);
+        sw[1] = flip(sE2, true);  // only the sign of (sE1 + sE2) / 2 is needed: that of sE1 against -sE2
+        sw[1] = lt(sE1, sw[1]) ? -1.0 : (lt(sw[1], sE1) ? 1.0 : 0.0);
         sw[2] = sE2;
     } else {  // the same call as geoclaw_solver's, recording the branch decisions
         const u64 yLf = wall_l ? yR0 : yL0, yRf = wall_r ? yL0 : yR0;
@@ -568,26 +565,29 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
     double nL[3], nR[3];
     nL[0] = gL[0];
     nR[0] = gR[0];
-    if (axis == 1) {
-        nL[1] = flip(gL[1], sn); nL[2] = flip(gL[2], sn);
-        nR[1] = flip(gR[1], sn); nR[2] = flip(gR[2], sn);
-    } else if (axis == 2) {
-        nL[1] = flip(gL[2], sn); nL[2] = flip(gL[1], !sn);
-        nR[1] = flip(gR[2], sn); nR[2] = flip(gR[1], !sn);
-    } else {
+    nL[1] = flip(ax1 ? gL[1] : gL[2], sn); nL[2] = flip(ax1 ? gL[2] : gL[1], ax1 ? sn : !sn);
+    nR[1] = flip(ax1 ? gR[1] : gR[2], sn); nR[2] = flip(ax1 ? gR[2] : gR[1], ax1 ? sn : !sn);
+    SWE_IF(axis == 0) {
         nL[1] = fma(gL[1], n1, gL[2] * n2); nL[2] = fma(-gL[1], n2, gL[2] * n1);
         nR[1] = fma(gR[1], n1, gR[2] * n2); nR[2] = fma(-gR[1], n2, gR[2] * n1);
     }
     // net-update split by wave-speed sign; walls remove waves
     double F[3][3];
+    bool still_wave = false;  // a wave that goes neither way
 #pragma unroll
     for (int w = 0; w < 3; ++w) {
         const bool zeroed = (wall_l && w < 2) || (wall_r && w > 0);
         const bool neg = lt0(sw[w]), pos = gt0(sw[w]);
+        still_wave = still_wave | !(zeroed | neg | pos);
 #pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            double f = neg ? nL[e] : (pos ? nR[e] : 0.5 * (nL[e] + nR[e]));
-            F[e][w] = zeroed ? 0.0 : f;
+        for (int e = 0; e < 3; ++e) F[e][w] = zeroed ? 0.0 : (neg ? nL[e] : nR[e]);
+    }
+    SWE_IF(still_wave) {
+#pragma unroll
+        for (int w = 0; w < 3; ++w) {
+            const bool zeroed = (wall_l && w < 2) || (wall_r && w > 0);
+            if (!zeroed && !lt0(sw[w]) && !gt0(sw[w]))
+                for (int e = 0; e < 3; ++e) F[e][w] = 0.5 * (nL[e] + nR[e]);
         }
     }
     double b_huR, b_vR, b_huL, b_vL, b_sE1, b_sE2, b_delphi, b_dB, b_Hs;
@@ -649,9 +649,10 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
     double b_sR = e2_is_sR ? b_sE2 : 0.0, b_r2 = e2_is_sR ? 0.0 : b_sE2;
     const double b_uhat = b_r1 + b_r2;
     const double b_chat = b_r2 - b_r1;
-    if (chat > 0.0) b_Hs = fma(b_chat * (0.5 * rcp_near(chat)), g * 0.5, b_Hs);
-    double b_uL = b_sL + k_uL, b_uR = b_sR + k_uR;
-    double b_sqL = k_sqL - b_sL, b_sqR = b_sR + k_sqR;
+    if (gt0(chat)) b_Hs = fma(b_chat * (0.5 * rcp_near(chat)), g * 0.5, b_Hs);
+    constexpr bool fw = SOLVER == FWAVE;  // (whose core adds no cotangents of its own)
+    double b_uL = fw ? b_sL : b_sL + k_uL, b_uR = fw ? b_sR : b_sR + k_uR;
+    double b_sqL = fw ? flip(b_sL, true) : k_sqL - b_sL, b_sqR = fw ? b_sR : b_sR + k_sqR;
     const double b_A = b_uhat * yB, b_B = -b_uhat * uhat * yB;
     b_sqL += fma(b_A, uL, b_B);
     b_sqR += fma(b_A, uR, b_B);
@@ -666,12 +667,12 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
         b_huL -= dsu;
         b_uL += fma(d, dhu, -(d * uR * dh));
         b_uR += fma(d, dhu, -(d * uL * dh));
-        double b_hR = fma(-d, uu, k_hR), b_hL = fma(d, uu, k_hL);
+        double b_hR = fw ? -d * uu : fma(-d, uu, k_hR), b_hL = fw ? d * uu : fma(d, uu, k_hL);
         const double b_X = d * c * Hs;
         b_Hs += fma(d, c * X, -(d * c * dB));
         b_dB = fma(-d, c * Hs, b_dB);
         // X = ((bR + hR) - bL) - hL
-        double b_bR = b_X + k_bR, b_bL = k_bL - b_X;
+        double b_bR = fw ? b_X : b_X + k_bR, b_bL = fw ? flip(b_X, true) : k_bL - b_X;
         b_hR += b_X;
         b_hL -= b_X;
         // Hs = hR + hL, dB = bR - bL
@@ -680,8 +681,8 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
         b_bR += b_dB;
         b_bL -= b_dB;
         // sqrt(g h) of the fixed-up depths
-        if (sqL > 0.0) b_hL = fma(b_sqL, 0.5 * g * rcp_near(sqL), b_hL);
-        if (sqR > 0.0) b_hR = fma(b_sqR, 0.5 * g * rcp_near(sqR), b_hR);
+        if (gt0(sqL)) b_hL = fma(b_sqL, 0.5 * g * rcp_near(sqL), b_hL);
+        if (gt0(sqR)) b_hR = fma(b_sqR, 0.5 * g * rcp_near(sqR), b_hR);
         // undo the wall / lowering fix-ups: map the cotangents back to the original sides
         double b_hL0 = 0.0, b_hR0 = 0.0, b_bL0 = 0.0, b_bR0 = 0.0;
         if (wall_r) {  // hR = hL, huR = -huL, bR = bL, uR = -uL, vR = vL
@@ -712,32 +713,28 @@ __device__ __forceinline__ void geoclaw_vjp(double n1, double n2, const State& Q
         double b_pL1 = 0.0, b_pL2 = 0.0, b_pR1 = 0.0, b_pR2 = 0.0;
         if (wetR) {
             const double iR = recip_near(hR, yR0);
-            b_pR1 += fma(b_uR, iR, b_huR);
-            b_pR2 = fma(b_vR, iR, b_pR2);
+            b_pR1 = fma(b_uR, iR, b_huR);
+            b_pR2 = b_vR * iR;
             b_hR0 = fma(-fma(b_uR, uR, b_vR * vR), iR, b_hR);
         }
         if (wetL) {
             const double iL = recip_near(hL, yL0);
-            b_pL1 += fma(b_uL, iL, b_huL);
-            b_pL2 = fma(b_vL, iL, b_pL2);
+            b_pL1 = fma(b_uL, iL, b_huL);
+            b_pL2 = b_vL * iL;
             b_hL0 = fma(-fma(b_uL, uL, b_vL * vL), iL, b_hL);
         }
         // depths h - b, rotations p_edge = T p
-        outL.h += b_hL0;
-        outL.b += b_bL0 - b_hL0;
-        outR.h += b_hR0;
-        outR.b += b_bR0 - b_hR0;
-        if (axis == 1) {
-            outL.hu += flip(b_pL1, sn); outL.hv += flip(b_pL2, sn);
-            outR.hu += flip(b_pR1, sn); outR.hv += flip(b_pR2, sn);
-        } else if (axis == 2) {
-            outL.hu += flip(b_pL2, !sn); outL.hv += flip(b_pL1, sn);
-            outR.hu += flip(b_pR2, !sn); outR.hv += flip(b_pR1, sn);
-        } else {
-            outL.hu += fma(b_pL1, n1, -(b_pL2 * n2));
-            outL.hv += fma(b_pL1, n2, b_pL2 * n1);
-            outR.hu += fma(b_pR1, n1, -(b_pR2 * n2));
-            outR.hv += fma(b_pR1, n2, b_pR2 * n1);
+        outL.h = b_hL0;
+        outL.b = b_bL0 - b_hL0;
+        outR.h = b_hR0;
+        outR.b = b_bR0 - b_hR0;
+        outL.hu = flip(ax1 ? b_pL1 : b_pL2, ax1 ? sn : !sn); outL.hv = flip(ax1 ? b_pL2 : b_pL1, sn);
+        outR.hu = flip(ax1 ? b_pR1 : b_pR2, ax1 ? sn : !sn); outR.hv = flip(ax1 ? b_pR2 : b_pR1, sn);
+        SWE_IF(axis == 0) {
+            outL.hu = fma(b_pL1, n1, -(b_pL2 * n2));
+            outL.hv = fma(b_pL1, n2, b_pL2 * n1);
+            outR.hu = fma(b_pR1, n1, -(b_pR2 * n2));
+            outR.hv = fma(b_pR1, n2, b_pR2 * n1);
         }
     }
 }
@@ -1005,7 +1002,6 @@ __global__ void SWE_ADJ_BOUNDS adjoint_kernel(const AdjointArgs A) {
         for (int i = tid; i < cn; i += blockDim.x) {
             const int cc = c0 + i;
             const double h = A.h[cc], b = A.b[cc];
-            sh_h[i] = h;
             sh_hu[i] = A.hu[cc];
             sh_hv[i] = A.hv[cc];
             sh_b[i] = b;
@@ -1015,7 +1011,9 @@ __global__ void SWE_ADJ_BOUNDS adjoint_kernel(const AdjointArgs A) {
             // reciprocal is left to the VJP of an edge that takes the general path
             // (0 here) when the cell's momenta are +-0, since its edges may all be
             // at rest; a cell with momentum has general edges and gets it here.
+            // The GeoClaw edges read the depth, the Lax-Friedrichs ones the surface.
             const double d = h - b;
+            sh_h[i] = geoclaw(SOLVER) ? d : h;
             const bool wet = lt(P.drytol, d);
             double sq = 0.0;
             bool miss = wet;
@@ -1071,7 +1069,7 @@ __global__ void SWE_ADJ_BOUNDS adjoint_kernel(const AdjointArgs A) {
             int depL, depR = 0;
             if (lin) {
                 QL = State{sh_h[sl], sh_hu[sl], sh_hv[sl], sh_b[sl]};
-                dL = QL.h - QL.b;
+                dL = geoclaw(SOLVER) ? QL.h : QL.h - QL.b;
                 sqL = sh_sq[sl];
                 yL = sh_rh[sl];
                 mL[0] = sh_mu[sl]; mL[1] = sh_mu[T + sl]; mL[2] = sh_mu[2 * T + sl];
@@ -1092,7 +1090,7 @@ __global__ void SWE_ADJ_BOUNDS adjoint_kernel(const AdjointArgs A) {
             } else {
                 if (rin) {
                     QR = State{sh_h[sr], sh_hu[sr], sh_hv[sr], sh_b[sr]};
-                    dR = QR.h - QR.b;
+                    dR = geoclaw(SOLVER) ? QR.h : QR.h - QR.b;
                     sqR = sh_sq[sr];
                     yR = sh_rh[sr];
                     mR[0] = sh_mu[sr]; mR[1] = sh_mu[T + sr]; mR[2] = sh_mu[2 * T + sr];
@@ -1147,16 +1145,10 @@ __global__ void SWE_ADJ_BOUNDS adjoint_kernel(const AdjointArgs A) {
             const int cc = c0 + i;
             const uint8_t br = A.branch[cc];
             const double lh = A.lam_h[cc], lu = A.lam_hu[cc], lv = A.lam_hv[cc];
-            double gh = 0.0, gu = 0.0, gv = 0.0, gb = 0.0;
-            if (br & 2u) {  // drying clamp: h' = min(b, 0), p' = 0
-                if (sh_b[i] < 0.0) gb += lh;
-            } else if (br & 1u) {  // wetting fix: h~ = b + drytol, p~ = 0
-                gb += lh;
-            } else {
-                gh = lh;
-                gu = lu;
-                gv = lv;
-            }
+            // drying clamp (h' = min(b, 0), p' = 0) or wetting fix (h~ = b + drytol, p~ = 0)
+            const bool dried = (br & 2u) != 0, fixed = (br & 3u) != 0;
+            double gh = fixed ? 0.0 : lh, gu = fixed ? 0.0 : lu, gv = fixed ? 0.0 : lv;
+            double gb = fixed && (!dried || lt0(sh_b[i])) ? lh : 0.0;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 gh += slot[(0 * 3 + k) * T + i];
