@@ -652,18 +652,31 @@ int current_index(swe_ctx* c, int* idx) {
 // 216 x 256 27.0, 108 x 128 31.2, 256 x 256 29.7; 2^17: 432 x 256 41, 216 x 128
 // 49), but not below 64 cells, whose edges give one warp to each of an SM's four
 // schedulers (2^12 cells: 64 x 128 12.2, 32 x 64 14.5). Larger meshes take the
-// step kernel: 256 x 256 below 2^19 cells (2^18: 97 against 102 at 128 threads),
-// then 384 x 128 (an ensemble of 5e5 cells: 159 against 169 at 256 x 256; 2^22: 346 against 443 at 256 threads where the water rests, 768
-// against 830 where it moves).
+// step kernel (us per step, 128 threads unless said):
+// - an ensemble beyond that 384 x 128 (5.2e5 cells in 36 bowls: 128, 256 x 256 139; 2.6e5:
+//   80 against 83);
+// - GeoClaw fluxes below 2^19 cells 256 x 256 (3.2e5 refined cells, augmented: 191, 256 x 128
+//   213, 216 x 128 194), up to 1.5 * 2^20 256 x 128 (2^19: bowl 105, basin 61, all moving
+//   149; 384 x 128 108, 68 and 152; 2^20: 189, 105, 279 against 196, 108, 286, augmented 341
+//   against 360), then 384 x 128 (2^21: 324 and 503 against 325 and 508; 2^23 basin 561 against
+//   615);
+// - the cheaper Lax-Friedrichs fluxes below 2^19 cells 216 x 128 (2^18: 52.1, 256 x 256 57.5;
+//   3.2e5 refined: 58.2 against 65.5), then 384 x 128 (2^19: 78, 256 x 128 83).
+// The solver is the one set when the mesh comes.
 void auto_tiling(swe_ctx* c) {
     const int64_t n = c->cells_total, resident = (int64_t)2 * c->num_sms;
     int32_t seg = 384, threads = 128;
     if (n <= resident * 750) {
         seg = (int32_t)std::max<int64_t>(64, ((n + resident - 1) / resident + 1) & ~(int64_t)1);
         threads = seg > 64 ? 256 : 128;
-    } else if (n < ((int64_t)1 << 19)) {
-        seg = 256;
-        threads = 256;
+    } else if (n_inst(c) == 1) {
+        const bool geo = c->params.empty() || geoclaw(c->params[0].solver);
+        if (n < ((int64_t)1 << 19)) {
+            seg = geo ? 256 : 216;
+            threads = geo ? 256 : 128;
+        } else if (geo && n <= (int64_t)3 << 19) {
+            seg = 256;
+        }
     }
     if (!c->tiling_set) c->seg_cells = seg;
     if (!c->threads_set && !c->tiling_set) c->block_threads = threads;
