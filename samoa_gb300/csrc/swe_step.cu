@@ -164,7 +164,7 @@ __global__ void gauge_kernel(const GlobalScalars* G, const double* h0, const dou
 // a cell's first listing adds all of its listings in list order (the same sums
 // in the same order as one thread walking the list, without its chain of
 // dependent loads); beyond that, one thread walks the list.
-constexpr int64_t kResidualParallel = 4096;
+constexpr int64_t kResidualParallel = 4096;  // 48 KB of shared memory
 __global__ void gauge_residual_kernel(double* lam_h, const int64_t* cells, int64_t n, const double* value,
                                       const double* obs) {
     if (n > kResidualParallel) {
@@ -172,14 +172,22 @@ __global__ void gauge_residual_kernel(double* lam_h, const int64_t* cells, int64
             for (int64_t i = 0; i < n; ++i) lam_h[cells[i]] += 2.0 * (value[i] - obs[i]);
         return;
     }
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const int64_t c = cells[i];
-        bool first = true;
-        for (int64_t j = 0; j < i && first; ++j) first = cells[j] != c;
-        if (!first) continue;
+    extern __shared__ __align__(16) unsigned char gauge_smem[];
+    double* r = reinterpret_cast<double*>(gauge_smem);  // 2 (value - obs)
+    int* cell = reinterpret_cast<int*>(r + n);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        cell[i] = (int)cells[i];
+        r[i] = 2.0 * (value[i] - obs[i]);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int c = cell[i];
         double acc = lam_h[c];
-        for (int64_t j = i; j < n; ++j)
-            if (cells[j] == c) acc += 2.0 * (value[j] - obs[j]);
+        bool first = true;
+        for (int j = 0; j < i; ++j) first = first & (cell[j] != c);
+        if (!first) continue;
+        for (int j = i; j < n; ++j)
+            if (cell[j] == c) acc += r[j];
         lam_h[c] = acc;
     }
 }
@@ -1743,7 +1751,8 @@ struct Sweep {
     double* lam[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
     int li = 0;
     double* bbar = nullptr;
-    int64_t cur = 0;
+    int64_t cur = 0;           // the step of the context's current state
+    bool behind = false;       // the other state buffer still holds the state of step cur - 1
     int64_t forward_steps = 0, adjoint_steps = 0;
     int rc = SWE_OK;
 
@@ -1761,17 +1770,30 @@ struct Sweep {
         *out = k;
         return SWE_OK;
     }
+    // The state of step t: the current one (a state just stored, or just reversed), the one
+    // a step was just taken from (in the other buffer), or slot k's. Of the 41 of a sweep
+    // of 24 steps with 6 slots the first two are 24.
     int restore(int k, int64_t t) {
+        if (cur == t) return SWE_OK;
+        if (behind && cur == t + 1) return step_back();
+        behind = false;
         const int b = (int)((s0 + t) & 1);
         const size_t bytes = (size_t)N * 8;
         CUDA_TRY(cudaMemcpyAsync(c->h[b], slot(k, 0), bytes, cudaMemcpyDeviceToDevice, c->stream));
         CUDA_TRY(cudaMemcpyAsync(c->hu[b], slot(k, 1), bytes, cudaMemcpyDeviceToDevice, c->stream));
         CUDA_TRY(cudaMemcpyAsync(c->hv[b], slot(k, 2), bytes, cudaMemcpyDeviceToDevice, c->stream));
+        return set_step(t);
+    }
+    int set_step(int64_t t) {
         set_step_kernel<<<1, 1, 0, c->stream>>>(c->gs, s0 + t);
         CUDA_TRY(cudaGetLastError());
         c->step_mirror = s0 + t;
         cur = t;
         return SWE_OK;
+    }
+    int step_back() {
+        behind = false;
+        return set_step(cur - 1);
     }
     int advance(int64_t k) {
         for (int64_t i = 0; i < k; ++i) {
@@ -1785,6 +1807,7 @@ struct Sweep {
                 done[(size_t)t] = 1;
             }
             cur = t + 1;
+            behind = true;
             ++forward_steps;
         }
         return SWE_OK;
@@ -1794,15 +1817,12 @@ struct Sweep {
                                        (long long)t);
         if (!done[(size_t)t]) {  // run step t once (branches, gauges), then x_t is still in its buffer
             int r = advance(1);
-            if (r) return r;
-            set_step_kernel<<<1, 1, 0, c->stream>>>(c->gs, s0 + t);
-            CUDA_TRY(cudaGetLastError());
-            c->step_mirror = s0 + t;
-            cur = t;
+            if (r || (r = step_back())) return r;
         }
         double** in = lam[li];
         double** out = lam[li ^ 1];
-        gauge_residual_kernel<<<1, (unsigned)std::min<int64_t>(std::max<int64_t>(G, 32), 256), 0, c->stream>>>(
+        gauge_residual_kernel<<<1, (unsigned)std::min<int64_t>(std::max<int64_t>(G, 32), 256),
+                                G <= kResidualParallel ? (size_t)G * 12 : 0, c->stream>>>(
             in[0], gauges, G, gv + (size_t)t * (size_t)G, obs + (size_t)t * (size_t)G);
         CUDA_TRY(cudaGetLastError());
         int r = launch_adjoint(c, s0 + t, branches + (size_t)t * (size_t)stride, in[0], in[1], in[2], out[0],
