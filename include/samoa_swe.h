@@ -143,8 +143,8 @@ int swe_last_error(char* buf, size_t n);
  * the current value. A mesh upload or
  * this call rebuilds the segment task lists. Until a segment length is set
  * here, each mesh upload picks it by size: 384 cells on large meshes and for
- * ensembles, 256 (or 216, for a Lax-Friedrichs flux set before the upload) on
- * middling ones, and on meshes that fit the GPU at once two segments per SM (at
+ * ensembles, 256 on middling ones (where the flux set before the upload and the
+ * size decide), and on meshes that fit the GPU at once two segments per SM (at
  * least 64 cells); it then picks the threads too, unless they were set. */
 int swe_set_tiling(swe_ctx* ctx, int32_t segment_cells, int32_t block_threads);
 

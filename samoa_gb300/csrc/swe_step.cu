@@ -337,6 +337,7 @@ struct swe_ctx {
     bool capturing = false;
     std::vector<InstParams> ip_host;
     int adj_grid = 0;               // adjoint launch shape for the current tiling (0 = not configured)
+    int adj_threads = 256;
     int32_t adj_seg_cells = 0;
     int adj_solver = 0;
     // CUDA graphs of n steps
@@ -668,8 +669,9 @@ int current_index(swe_ctx* c, int* idx) {
 //   149; 384 x 128 108, 68 and 152; 2^20: 189, 105, 279 against 196, 108, 286, augmented 341
 //   against 360), then 384 x 128 (2^21: 324 and 503 against 325 and 508; 2^23 basin 561 against
 //   615);
-// - the cheaper Lax-Friedrichs fluxes below 2^19 cells 216 x 128 (2^18: 52.1, 256 x 256 57.5;
-//   3.2e5 refined: 58.2 against 65.5), then 384 x 128 (2^19: 78, 256 x 128 83).
+// - the cheaper Lax-Friedrichs fluxes below 2^19 cells 256 x 128 (2^18: 53.9, 256 x 256 57.5;
+//   3.2e5 refined: 60.3 against 65.5; 216 x 128 takes 52.1 and 58.2 but their reverse step
+//   125 against 111), then 384 x 128 (2^19: 78, 256 x 128 83).
 // The solver is the one set when the mesh comes.
 void auto_tiling(swe_ctx* c) {
     const int64_t n = c->cells_total, resident = (int64_t)2 * c->num_sms;
@@ -680,7 +682,7 @@ void auto_tiling(swe_ctx* c) {
     } else if (n_inst(c) == 1) {
         const bool geo = c->params.empty() || geoclaw(c->params[0].solver);
         if (n < ((int64_t)1 << 19)) {
-            seg = geo ? 256 : 216;
+            seg = 256;
             threads = geo ? 256 : 128;
         } else if (geo && n <= (int64_t)3 << 19) {
             seg = 256;
@@ -1526,23 +1528,31 @@ int launch_adjoint(swe_ctx* c, long long t, const uint8_t* branch, const double*
         for (int d = 0; d <= kMaxDepth; ++d) A.ndv_tab[d] = -A.dt / (s2 * c->vol[d]);
         for (int d = 0; d <= kMaxDepth + 1; ++d) A.len_tab[d] = A.P.scaling * c->leg[d];
     }
-    // the reverse kernel holds more registers per thread than the step: it runs
-    // 256 threads per CTA so an SM still has two CTAs' worth of warps
-    const int threads = 256;
     const size_t smem = (size_t)21 * c->seg_cells * sizeof(double);
     const int solver = c->params[0].solver;
     const AdjKernel kern = adjoint_kernel_for(solver);
     if (!kern) return set_error(SWE_E_INVALID, "the adjoint differentiates the f-wave, augmented and Lax-Friedrichs fluxes");
     if (c->adj_seg_cells != c->seg_cells || c->adj_solver != solver) {
         if (int rc = raise_smem_limit((const void*)kern, smem)) return rc;
+        // 256 threads, or 192 where those hold more warps on an SM: the augmented solver's
+        // reverse (146 registers) has one CTA of 256 but two of 192 (2^18 cells: 571 us
+        // against 533), the fluxes with bathymetry three of 192 (113.6 against 111.1)
         int per_sm = 0;
-        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+        c->adj_threads = 0;
+        for (int threads : {256, 192}) {
+            int fit = 0;
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, threads, smem));
+            if (fit * threads > per_sm * c->adj_threads) {
+                per_sm = fit;
+                c->adj_threads = threads;
+            }
+        }
         if (per_sm < 1) return set_error(SWE_E_INVALID, "adjoint tiling does not fit an SM");
         c->adj_grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * c->num_sms, c->n_seg));
         c->adj_seg_cells = c->seg_cells;
         c->adj_solver = solver;
     }
-    kern<<<c->adj_grid, threads, smem, c->stream>>>(A);
+    kern<<<c->adj_grid, c->adj_threads, smem, c->stream>>>(A);
     CUDA_TRY(cudaGetLastError());
     return SWE_OK;
 }
