@@ -669,9 +669,8 @@ int current_index(swe_ctx* c, int* idx) {
 //   149; 384 x 128 108, 68 and 152; 2^20: 189, 105, 279 against 196, 108, 286, augmented 341
 //   against 360), then 384 x 128 (2^21: 324 and 503 against 325 and 508; 2^23 basin 561 against
 //   615);
-// - the cheaper Lax-Friedrichs fluxes below 2^19 cells 256 x 128 (2^18: 53.9, 256 x 256 57.5;
-//   3.2e5 refined: 60.3 against 65.5; 216 x 128 takes 52.1 and 58.2 but their reverse step
-//   125 against 111), then 384 x 128 (2^19: 78, 256 x 128 83).
+// - the cheaper Lax-Friedrichs fluxes below 2^19 cells 216 x 128 (2^18: 52.1, 256 x 256 57.5;
+//   3.2e5 refined: 58.2 against 65.5), then 384 x 128 (2^19: 78, 256 x 128 83).
 // The solver is the one set when the mesh comes.
 void auto_tiling(swe_ctx* c) {
     const int64_t n = c->cells_total, resident = (int64_t)2 * c->num_sms;
@@ -682,7 +681,7 @@ void auto_tiling(swe_ctx* c) {
     } else if (n_inst(c) == 1) {
         const bool geo = c->params.empty() || geoclaw(c->params[0].solver);
         if (n < ((int64_t)1 << 19)) {
-            seg = 256;
+            seg = geo ? 256 : 216;
             threads = geo ? 256 : 128;
         } else if (geo && n <= (int64_t)3 << 19) {
             seg = 256;
@@ -1534,18 +1533,15 @@ int launch_adjoint(swe_ctx* c, long long t, const uint8_t* branch, const double*
     if (!kern) return set_error(SWE_E_INVALID, "the adjoint differentiates the f-wave, augmented and Lax-Friedrichs fluxes");
     if (c->adj_seg_cells != c->seg_cells || c->adj_solver != solver) {
         if (int rc = raise_smem_limit((const void*)kern, smem)) return rc;
-        // 256 threads, or 192 where those hold more warps on an SM: the augmented solver's
-        // reverse (146 registers) has one CTA of 256 but two of 192 (2^18 cells: 571 us
-        // against 533), the fluxes with bathymetry three of 192 (113.6 against 111.1)
+        // 256 threads (us at 2^18 cells: f-wave 157, with 192, 160 and 128 threads 183, 160 and
+        // 173; LLF with bathymetry 114 against 124, 111 and 123), but 128 where an SM holds
+        // only one CTA of 256: the augmented solver's reverse (146 registers) 571 with 256,
+        // 541, 533 and 530 with fewer
         int per_sm = 0;
-        c->adj_threads = 0;
-        for (int threads : {256, 192}) {
-            int fit = 0;
-            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, threads, smem));
-            if (fit * threads > per_sm * c->adj_threads) {
-                per_sm = fit;
-                c->adj_threads = threads;
-            }
+        for (int threads : {256, 128}) {
+            c->adj_threads = threads;
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+            if (per_sm > 1) break;
         }
         if (per_sm < 1) return set_error(SWE_E_INVALID, "adjoint tiling does not fit an SM");
         c->adj_grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * c->num_sms, c->n_seg));
