@@ -827,6 +827,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const __grid_constant__ StepArgs A) 
             M.sq[i] = sq;
             if (kDepths) M.h[i] = d;
         }
+        if (kDepths) fence_proxy_async();  // before a later bulk copy into this buffer (barriers follow)
         // halo tasks: the cross-edge pass computed these edges' updates; copy
         // this segment's side into its slot
         const long long t0 = __ldg(&A.seg_ptr[seg]);
