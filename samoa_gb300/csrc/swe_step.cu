@@ -425,6 +425,11 @@ float float_not_below(double x) {
     return (double)f < x ? std::nextafterf(f, INFINITY) : f;
 }
 
+// Every instance's dt is a quotient by the largest speed sum (the multi-step kernel takes no other).
+bool all_by_max(const std::vector<InstParams>& v) {
+    return std::all_of(v.begin(), v.end(), [](const InstParams& q) { return q.dt_by_max != 0; });
+}
+
 int upload_inst_params(swe_ctx* c) {
     const int n = n_inst(c);
     std::vector<InstParams> v((size_t)n);
@@ -473,6 +478,7 @@ int upload_inst_params(swe_ctx* c) {
     }
     CUDA_TRY(cudaMemcpyAsync(c->rows, rows.data(), sizeof(DepthRow) * rows.size(), cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(cudaMemcpyAsync(c->ip, v.data(), sizeof(InstParams) * v.size(), cudaMemcpyHostToDevice, c->stream));
+    if (all_by_max(v) != all_by_max(c->ip_host)) drop_graphs(c);  // which kernel a graph holds depends on it
     c->ip_host = v;
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     return SWE_OK;
@@ -889,9 +895,8 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     // (90 registers) fit 5 per SM, 20 warps, against 2 CTAs of 256 threads
     constexpr int kCrossThreads = 128;
     // many plain steps of a mesh that fits the GPU at once: the multi-step kernel
-    bool multi = n_steps > 1 && c->multi_fits && !io && !branch && !fz && c->dt_seq_len == 0 && c->stage_depth == 1 &&
-                 c->cross_mode == SWE_CROSS_AUTO && c->inject == SWE_INJECT_NONE;
-    for (const InstParams& q : c->ip_host) multi = multi && q.dt_by_max;
+    const bool multi = n_steps > 1 && c->multi_fits && !io && !branch && !fz && c->dt_seq_len == 0 && c->stage_depth == 1 &&
+                 c->cross_mode == SWE_CROSS_AUTO && c->inject == SWE_INJECT_NONE && all_by_max(c->ip_host);
     if (multi) {
         constexpr int64_t kMaxSteps = 4096;  // of one launch
         void* km = fma ? fma_multi_kernel(c->params[0].solver) : multi_kernel_for(c->params[0].solver);
