@@ -199,6 +199,10 @@ int swe_set_segment_order(swe_ctx* ctx, int32_t mode);
 int swe_get_task_counts(swe_ctx* ctx, int64_t* n_segments, int64_t* n_tasks, int64_t* n_cross_edges,
                         int32_t* launches_per_step);
 
+/* Kernel launches that swe_traverse(ctx, n_steps) would make now: one per 4096
+ * steps where they run in one kernel, else those of swe_get_task_counts for each step. */
+int swe_get_launch_count(swe_ctx* ctx, int64_t n_steps, int64_t* launches);
+
 /* Vertices of the cells of swe_mesh_uniform(depth) in the unit square, in the
  * same cell order: vertices[6 k + 2 v + {0, 1}] = (x, y) of vertex v of cell k
  * (exact dyadic values). The node coordinates samoa_get_grid hands out

@@ -25,7 +25,7 @@ EXPORTS = [
     "swe_division_check", "swe_step_host", "swe_gauge_gradient",
     "swe_traverse_gauges", "swe_mesh_uniform_vertices", "swe_mesh_build", "swe_mesh_adapt",
     "swe_set_staging", "swe_get_task_counts", "swe_set_cross_pass", "swe_traverse_frozen",
-    "swe_set_segment_order", "swe_set_fault_injection",
+    "swe_set_segment_order", "swe_set_fault_injection", "swe_get_launch_count",
 ]
 
 
@@ -73,6 +73,7 @@ def load():
         "swe_set_tiling": [P, i32, i32],
         "swe_get_tiling": [P, P, P],
         "swe_get_task_counts": [P, P, P, P, P],
+        "swe_get_launch_count": [P, i64, P],
         "swe_set_cross_pass": [P, i32],
         "swe_set_segment_order": [P, i32],
         "swe_traverse_frozen": [P, i64, i32, P, i64, P, i64, i64, P, P],

@@ -707,6 +707,13 @@ bool cross_pass(const swe_ctx* c, bool host_io) {
     return c->cross_mode == SWE_CROSS_PASS || (!host_io && c->cells_total >= ((int64_t)1 << 20));
 }
 
+// Whether n_steps plain steps of a device-resident state run in the multi-step kernel.
+constexpr int64_t kMultiSteps = 4096;  // of one launch
+bool multi_steps(const swe_ctx* c, int64_t n_steps) {
+    return n_steps > 1 && c->multi_fits && c->dt_seq_len == 0 && c->stage_depth == 1 &&
+           c->cross_mode == SWE_CROSS_AUTO && c->inject == SWE_INJECT_NONE && all_by_max(c->ip_host);
+}
+
 // Ingest and upload the instances' meshes (arrays concatenated, indices local to each instance).
 int upload_meshes(swe_ctx* c, int64_t ni, const int64_t* n_cells, const int64_t* n_edges, const int64_t* n_bnd,
                   const int8_t* depth, const int8_t* plotter, const int64_t* edge_cells, const int8_t* edge_local,
@@ -895,10 +902,7 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     // (90 registers) fit 5 per SM, 20 warps, against 2 CTAs of 256 threads
     constexpr int kCrossThreads = 128;
     // many plain steps of a mesh that fits the GPU at once: the multi-step kernel
-    const bool multi = n_steps > 1 && c->multi_fits && !io && !branch && !fz && c->dt_seq_len == 0 && c->stage_depth == 1 &&
-                 c->cross_mode == SWE_CROSS_AUTO && c->inject == SWE_INJECT_NONE && all_by_max(c->ip_host);
-    if (multi) {
-        constexpr int64_t kMaxSteps = 4096;  // of one launch
+    if (!io && !branch && !fz && multi_steps(c, n_steps)) {
         void* km = fma ? fma_multi_kernel(c->params[0].solver) : multi_kernel_for(c->params[0].solver);
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeCooperative;
@@ -910,8 +914,8 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
         cfg.stream = c->stream;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        for (int64_t s = 0; s < n_steps; s += kMaxSteps) {
-            int ns = (int)std::min<int64_t>(kMaxSteps, n_steps - s);
+        for (int64_t s = 0; s < n_steps; s += kMultiSteps) {
+            int ns = (int)std::min<int64_t>(kMultiSteps, n_steps - s);
             void* margs[] = {&A, &ns};
             CUDA_TRY(cudaLaunchKernelExC(&cfg, km, margs));
             if (!c->capturing) c->step_mirror += ns;
@@ -1119,6 +1123,14 @@ int swe_get_task_counts(swe_ctx* c, int64_t* n_segments, int64_t* n_tasks, int64
     if (n_cross_edges) *n_cross_edges = c->n_xtasks;
     if (launches_per_step)
         *launches_per_step = cross_pass(c, false) ? 2 : 1;
+    return SWE_OK;
+}
+
+int swe_get_launch_count(swe_ctx* c, int64_t n_steps, int64_t* launches) {
+    if (!c || !launches || n_steps < 0) return set_error(SWE_E_INVALID, "bad arguments");
+    if (!c->has_mesh) return set_error(SWE_E_NOMESH, "upload a mesh first");
+    *launches = multi_steps(c, n_steps) ? (n_steps + kMultiSteps - 1) / kMultiSteps
+                                        : n_steps * (cross_pass(c, false) ? 2 : 1);
     return SWE_OK;
 }
 

@@ -212,6 +212,12 @@ class SweContext:
         _lib.check(self.L.swe_get_task_counts(self.ptr, C.byref(s), C.byref(t), C.byref(x), C.byref(k)))
         return {"segments": s.value, "tasks": t.value, "cross_edges": x.value, "launches_per_step": k.value}
 
+    def launch_count(self, n_steps):
+        """Kernel launches that traverse(n_steps) would make now."""
+        k = C.c_int64()
+        _lib.check(self.L.swe_get_launch_count(self.ptr, int(n_steps), C.byref(k)))
+        return k.value
+
     def upload_mesh(self, mesh):
         ec = np.ascontiguousarray(mesh.edge_cells, np.int64)
         el = np.ascontiguousarray(mesh.edge_local, np.int8)

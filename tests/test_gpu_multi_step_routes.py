@@ -40,3 +40,27 @@ def test_graph_replayed_after_parameters_the_multi_step_kernel_does_not_take(swe
             _compare(ctx, S, "scaling %g" % scaling)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("solver", ["fwave", "aug_riemann", "llfbath"])
+@pytest.mark.parametrize("log2,discs", [(1, 0), (9, 1), (13, 1), (16, 1), (17, 1)])
+def test_many_steps_of_a_small_mesh_are_one_launch(swe_lib, log2, discs, solver):
+    g, cfg = _grid(log2, discs, solver, "slip")
+    ctx = _context(g, cfg)
+    try:
+        assert [ctx.launch_count(n) for n in (0, 1, 2, 4096, 4097)] == [0, 1, 1, 1, 2]
+        ctx.set_cross_pass("inkernel")
+        assert ctx.launch_count(8) == 8
+        ctx.set_cross_pass("pass")
+        assert ctx.launch_count(8) == 8 * ctx.task_counts()["launches_per_step"]
+    finally:
+        ctx.close()
+
+
+def test_many_steps_of_a_large_mesh_are_a_launch_each(swe_lib):
+    g, cfg = _grid(19, 0, "fwave", "slip")
+    ctx = _context(g, cfg)
+    try:
+        assert ctx.launch_count(8) == 8
+    finally:
+        ctx.close()
