@@ -396,9 +396,14 @@ int swe_division_check(int64_t n, uint64_t seed, int32_t exponent_span, int64_t*
  * segment and the step reports SWE_E_DEVICE at the next swe_synchronize. The
  * report clears the device flag; the failed step's state is undefined, so
  * upload a state (or a mesh) before stepping on. Applies to device-resident
- * steps (swe_traverse); stays set until SWE_INJECT_NONE. */
+ * steps (swe_traverse); stays set until SWE_INJECT_NONE. SWE_INJECT_MEETING:
+ * where many steps run in one kernel, its CTAs' waits for one another between
+ * two steps count one CTA too many and give up the same way;
+ * SWE_INJECT_LAST_MEETING: the wait for the last step's CTAs does. */
 #define SWE_INJECT_NONE 0
 #define SWE_INJECT_STAGING_TX 1
+#define SWE_INJECT_MEETING 2
+#define SWE_INJECT_LAST_MEETING 3
 int swe_set_fault_injection(swe_ctx* ctx, int32_t kind);
 
 /* One time step on caller-owned device memory, allocating nothing. No

@@ -711,7 +711,7 @@ bool cross_pass(const swe_ctx* c, bool host_io) {
 constexpr int64_t kMultiSteps = 4096;  // of one launch
 bool multi_steps(const swe_ctx* c, int64_t n_steps) {
     return n_steps > 1 && c->multi_fits && c->dt_seq_len == 0 && c->stage_depth == 1 &&
-           c->cross_mode == SWE_CROSS_AUTO && c->inject == SWE_INJECT_NONE && all_by_max(c->ip_host);
+           c->cross_mode == SWE_CROSS_AUTO && c->inject != SWE_INJECT_STAGING_TX && all_by_max(c->ip_host);
 }
 
 // Ingest and upload the instances' meshes (arrays concatenated, indices local to each instance).
@@ -870,10 +870,13 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     A.fixed_io = 0;
     // fault injection (tests): the staging barrier expects 16 bytes that no copy
     // delivers, so its phase never completes and the bounded wait, shortened to
-    // 20 ms, gives up; every issued copy still lands before the CTA leaves
+    // 20 ms, gives up; every issued copy still lands before the CTA leaves. Likewise the
+    // multi-step kernel's meetings, or its wait for the last step, count one CTA too many
     A.memo = c->memo;
     A.extra_tx = c->inject == SWE_INJECT_STAGING_TX ? 16u : 0u;
-    A.wait_ns = c->inject == SWE_INJECT_STAGING_TX ? 20000000ull : kWaitNs;
+    A.extra_meet = c->inject == SWE_INJECT_MEETING ? 1u : 0u;
+    A.extra_end = c->inject == SWE_INJECT_LAST_MEETING ? 1u : 0u;
+    A.wait_ns = c->inject != SWE_INJECT_NONE ? 20000000ull : kWaitNs;
     const bool pass = cross_pass(c, io != nullptr);
     A.halo_solve = pass ? 0 : 1;
     if (io) {
@@ -1637,7 +1640,7 @@ int swe_get_step_count(swe_ctx* c, int64_t* steps) {
 
 int swe_set_fault_injection(swe_ctx* c, int32_t kind) {
     if (!c) return set_error(SWE_E_INVALID, "null context");
-    if (kind != SWE_INJECT_NONE && kind != SWE_INJECT_STAGING_TX)
+    if (kind < SWE_INJECT_NONE || kind > SWE_INJECT_LAST_MEETING)
         return set_error(SWE_E_INVALID, "unknown fault injection %d", kind);
     c->inject = kind;
     return SWE_OK;

@@ -1,0 +1,41 @@
+"""The multi-step kernel's waits between its CTAs run out (the injections make them count one CTA too many, with a
+limit of 20 ms): the call reports it, and the context then steps like the oracle, refinement count included."""
+import pytest
+
+from samoa_gb300 import _lib
+from tests.helpers import omp_state, oracle_params
+from tests.test_gpu_multi_step import _compare, _grid
+from tests.test_gpu_multi_step_routes import _context
+
+pytestmark = pytest.mark.gpu
+
+SWE_E_DEVICE = -6
+NONE, MEETING, LAST_MEETING = 0, 2, 3
+
+
+@pytest.mark.parametrize("kind", [MEETING, LAST_MEETING])
+@pytest.mark.parametrize("log2,discs", [(5, 0), (12, 1), (16, 0)])
+def test_meeting_runs_out_and_context_recovers(swe_lib, oracle_lib, log2, discs, kind):
+    g, cfg = _grid(log2, discs, "fwave", "slip")
+    cfg.i_max_depth = log2 + 12  # so that cells do ask for refinement
+    L = _lib.load()
+    ctx = _context(g, cfg)
+    try:
+        _lib.check(L.swe_set_fault_injection(ctx.ptr, kind))
+        assert ctx.launch_count(4) == 1
+        ctx.traverse(4)
+        with pytest.raises(_lib.SweError) as err:
+            ctx.synchronize()
+        assert err.value.code == SWE_E_DEVICE and "ran out" in str(err.value)
+        ctx.synchronize()  # reported once
+        _lib.check(L.swe_set_fault_injection(ctx.ptr, NONE))
+        ctx.upload_state(g.h, g.hu, g.hv, g.b)  # the time is still that of the state before the failed steps
+        S, P = omp_state(g.mesh, g), oracle_params(cfg)
+        for n in (2, 3):
+            S.steps(P, n)
+            ctx.traverse(n)
+            ctx.synchronize()
+            _compare(ctx, S, "%d steps" % n)
+            assert S.n_refine > 0
+    finally:
+        ctx.close()
