@@ -52,15 +52,13 @@ __global__ void riemann_batch_kernel(int64_t n, const double* nrm, const double*
         depth_terms(L, drytol, dL, sqL, yL);
         depth_terms(R, drytol, dR, sqR, yR);
         Update fL, fR;
-        SafeOps o;
-        edge_flux<SOLVER, 0>(nrm[2 * i], nrm[2 * i + 1], L, R, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, 0, nullptr, o);
         FastOps f;
-        Update gL, gR;
-        edge_flux<SOLVER, 0>(nrm[2 * i], nrm[2 * i + 1], L, R, dL, dR, sqL, sqR, yL, yR, drytol, gL, gR,
+        edge_flux<SOLVER, 0>(nrm[2 * i], nrm[2 * i + 1], L, R, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR,
                              axis_of(nrm[2 * i], nrm[2 * i + 1]), nullptr, f);
-        if (f.ok) {
-            fL = gL;
-            fR = gR;
+        if (!f.ok) {
+            SafeOps o;
+            edge_flux<SOLVER, 0>(nrm[2 * i], nrm[2 * i + 1], L, R, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, 0, nullptr,
+                                 o);
         }
         ol[4 * i] = fL.h; ol[4 * i + 1] = fL.p1; ol[4 * i + 2] = fL.p2; ol[4 * i + 3] = fL.s;
         orr[4 * i] = fR.h; orr[4 * i + 1] = fR.p1; orr[4 * i + 2] = fR.p2; orr[4 * i + 3] = fR.s;
