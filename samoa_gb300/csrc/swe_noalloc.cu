@@ -126,18 +126,8 @@ __global__ void edges_kernel(Args A, unsigned char* scratch) {
         } else {
             QR = load(A, R);
         }
-        double dL, dR, sqL, sqR;
-        u64 yL, yR;
-        depth_terms(QL, A.drytol, dL, sqL, yL);
-        depth_terms(QR, A.drytol, dR, sqR, yR);
         Update fL, fR;
-        const int axis = axis_of(n1, n2);
-        FastOps f;
-        edge_flux<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, A.drytol, fL, fR, axis, nullptr, f);
-        if (!f.ok) {
-            SafeOps o;
-            edge_flux<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, A.drytol, fL, fR, axis, nullptr, o);
-        }
+        flux_of_states<SOLVER>(n1, n2, QL, QR, A.drytol, fL, fR);
         slots[(0 * 3 + iL) * M + L] = fL.h;
         slots[(1 * 3 + iL) * M + L] = fL.p1;
         slots[(2 * 3 + iL) * M + L] = fL.p2;

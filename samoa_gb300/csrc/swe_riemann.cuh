@@ -967,6 +967,31 @@ __device__ __forceinline__ void depth_terms(const State& Q, double drytol, doubl
     y = wet ? recip_fix(d) : 0;
 }
 
+// One edge between two states, for the entry points without a context, whose tolerance
+// may be negative: a depth at or below zero is then wet. FastOps' quotients of zeros by
+// a wet depth take that depth for positive, and the Lax-Friedrichs fluxes the root of a
+// negative one for 0 (their sqrt(g max(d, 0))), the GeoClaw ones for NaN.
+template <int SOLVER>
+__device__ __forceinline__ void flux_of_states(double n1, double n2, const State& QL, const State& QR, double drytol,
+                                               Update& fL, Update& fR) {
+    double dL, dR, sqL, sqR;
+    u64 yL, yR;
+    depth_terms(QL, drytol, dL, sqL, yL);
+    depth_terms(QR, drytol, dR, sqR, yR);
+    if (SOLVER != FWAVE && SOLVER != AUG_RIEMANN) {
+        if (lt0(dL)) sqL = 0.0;
+        if (lt0(dR)) sqR = 0.0;
+    }
+    const int axis = axis_of(n1, n2);
+    if (!lt0(drytol)) {
+        FastOps f;
+        edge_flux<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, nullptr, f);
+        if (f.ok) return;
+    }
+    SafeOps o;
+    edge_flux<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, nullptr, o);
+}
+
 // Ghost state of bnd_skeleton_scalar_op, src/SWE/SWE_euler_timestep.f90:231-255.
 template <int BC>
 __device__ __forceinline__ State boundary_ghost(double n1, double n2, const State& Q) {

@@ -47,19 +47,8 @@ __global__ void riemann_batch_kernel(int64_t n, const double* nrm, const double*
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         State L{ql[4 * i], ql[4 * i + 1], ql[4 * i + 2], ql[4 * i + 3]};
         State R{qr[4 * i], qr[4 * i + 1], qr[4 * i + 2], qr[4 * i + 3]};
-        double dL, dR, sqL, sqR;
-        u64 yL, yR;
-        depth_terms(L, drytol, dL, sqL, yL);
-        depth_terms(R, drytol, dR, sqR, yR);
         Update fL, fR;
-        FastOps f;
-        edge_flux<SOLVER, 0>(nrm[2 * i], nrm[2 * i + 1], L, R, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR,
-                             axis_of(nrm[2 * i], nrm[2 * i + 1]), nullptr, f);
-        if (!f.ok) {
-            SafeOps o;
-            edge_flux<SOLVER, 0>(nrm[2 * i], nrm[2 * i + 1], L, R, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, 0, nullptr,
-                                 o);
-        }
+        flux_of_states<SOLVER>(nrm[2 * i], nrm[2 * i + 1], L, R, drytol, fL, fR);
         ol[4 * i] = fL.h; ol[4 * i + 1] = fL.p1; ol[4 * i + 2] = fL.p2; ol[4 * i + 3] = fL.s;
         orr[4 * i] = fR.h; orr[4 * i + 1] = fR.p1; orr[4 * i + 2] = fR.p2; orr[4 * i + 3] = fR.s;
     }
