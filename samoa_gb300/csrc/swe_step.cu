@@ -260,6 +260,7 @@ struct swe_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
+    bool stream_changed = false;    // since the last look at it by settle_streams
     int num_sms = 0;
     // instances
     std::vector<HostMesh> mesh, spare_mesh;  // spare: an earlier mesh's storage, for the next upload
@@ -701,6 +702,14 @@ bool multi_steps(const swe_ctx* c, int64_t n_steps) {
            c->cross_mode == SWE_CROSS_AUTO && c->inject != SWE_INJECT_STAGING_TX && all_by_max(c->ip_host);
 }
 
+// Steps on a stream that the context worked on before may still read the dt sequence:
+// wait for them before its buffer is written again (as its release would).
+int settle_streams(swe_ctx* c) {
+    if (c->stream_changed && c->dt_seq) CUDA_TRY(cudaDeviceSynchronize());
+    c->stream_changed = false;
+    return SWE_OK;
+}
+
 // Ingest and upload the instances' meshes (arrays concatenated, indices local to each instance).
 int upload_meshes(swe_ctx* c, int64_t ni, const int64_t* n_cells, const int64_t* n_edges, const int64_t* n_bnd,
                   const int8_t* depth, const int8_t* plotter, const int64_t* edge_cells, const int8_t* edge_local,
@@ -709,6 +718,7 @@ int upload_meshes(swe_ctx* c, int64_t ni, const int64_t* n_cells, const int64_t*
     if (!n_cells || !n_edges || !n_bnd) return set_error(SWE_E_INVALID, "null size arrays");
     cudaSetDevice(c->device);
     CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if (int rc = settle_streams(c)) return rc;
     free_mesh_buffers(c, false);
     std::vector<HostMesh> meshes = std::move(c->spare_mesh);
     c->spare_mesh.clear();
@@ -997,7 +1007,9 @@ int swe_destroy(swe_ctx* c) {
 
 int swe_set_stream(swe_ctx* c, void* stream) {
     if (!c) return set_error(SWE_E_INVALID, "null context");
-    c->stream = stream ? (cudaStream_t)stream : c->own_stream;
+    const cudaStream_t s = stream ? (cudaStream_t)stream : c->own_stream;
+    c->stream_changed = c->stream_changed || s != c->stream;
+    c->stream = s;
     drop_graphs(c);
     return SWE_OK;
 }
@@ -1347,6 +1359,7 @@ int swe_set_dt_sequence(swe_ctx* c, int64_t n_steps, const double* dts) {
     if (n_steps < 0 || (n_steps > 0 && !dts)) return set_error(SWE_E_INVALID, "bad dt sequence");
     cudaSetDevice(c->device);
     CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if (int rc = settle_streams(c)) return rc;
     c->dt_seq_len = 0;
     drop_graphs(c);
     if (n_steps == 0) return SWE_OK;
