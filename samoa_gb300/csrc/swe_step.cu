@@ -6,10 +6,13 @@
 // instances. The plain C-ABI calls work on a one-instance context; the
 // swe_ensemble_* calls set up many instances that step together in one
 // launch per time step, each with its own dt.
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -284,7 +287,8 @@ struct swe_ctx {
     size_t smem = 0;
     std::vector<int32_t> first_seg; // of each instance, and n_seg
     size_t multi_smem = 0;          // of the multi-step kernel, whose segments hold their depths too
-    bool multi_fits = false;        // every segment has a CTA of the multi-step kernel on the GPU at once
+    int multi_per_sm = 0;           // the multi-step kernel's CTAs per SM; 0: its segments do not fit one
+    int stream_sms = 0;             // SMs that work on the stream runs on
     // device memory
     double* h[2] = {nullptr, nullptr};
     double* hu[2] = {nullptr, nullptr};
@@ -490,6 +494,7 @@ int configure_launch(swe_ctx* c) {
     StepKernel k = kernel_for(c->params.empty() ? FWAVE : c->params[0].solver);
     if (!k) return set_error(SWE_E_INVALID, "unknown solver");
     int rc;
+    c->multi_per_sm = 0;  // until it is known
     c->smem = smem_bytes(c, false);
     for (int s : {FWAVE, AUG_RIEMANN, LF, LF_BATH, LLF, LLF_BATH}) {
         for (bool host : {false, true})
@@ -508,12 +513,14 @@ int configure_launch(swe_ctx* c) {
     int64_t g = (int64_t)per_sm * c->num_sms;
     c->grid = (int)std::max<int64_t>(1, std::min<int64_t>(g, c->n_seg));
     c->multi_smem = smem_bytes(c, true);
-    c->multi_fits = c->multi_smem + kStaticSmem <= kMaxSmem;
-    for (void* m : {multi_kernel_for(c->params[0].solver), fma_multi_kernel(c->params[0].solver)}) {
-        if (!c->multi_fits) break;
-        if ((rc = raise_smem_limit(m, c->multi_smem))) return rc;
-        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, m, c->block_threads, c->multi_smem));
-        c->multi_fits = c->multi_fits && c->n_seg <= (int64_t)per_sm * c->num_sms;
+    if (c->multi_smem + kStaticSmem <= kMaxSmem) {
+        int fit = INT_MAX;
+        for (void* m : {multi_kernel_for(c->params[0].solver), fma_multi_kernel(c->params[0].solver)}) {
+            if ((rc = raise_smem_limit(m, c->multi_smem))) return rc;
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, m, c->block_threads, c->multi_smem));
+            fit = std::min(fit, per_sm);
+        }
+        c->multi_per_sm = fit;
     }
     drop_graphs(c);
     return SWE_OK;
@@ -695,10 +702,31 @@ bool cross_pass(const swe_ctx* c, bool host_io) {
     return c->cross_mode == SWE_CROSS_PASS || (!host_io && c->cells_total >= ((int64_t)1 << 20));
 }
 
+// The SMs that work on a stream may run on: its green context's, else the device's.
+int sms_of_stream(cudaStream_t s, int device_sms) {
+    void *get_ctx = nullptr, *get_resource = nullptr;
+    cudaDriverEntryPointQueryResult q1, q2;
+    if (cudaGetDriverEntryPointByVersion("cuStreamGetCtx", &get_ctx, 12050, cudaEnableDefault, &q1) != cudaSuccess ||
+        cudaGetDriverEntryPointByVersion("cuGreenCtxGetDevResource", &get_resource, 12040, cudaEnableDefault, &q2) !=
+            cudaSuccess ||
+        q1 != cudaDriverEntryPointSuccess || q2 != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        return device_sms;  // a driver without green contexts
+    }
+    CUcontext ctx = nullptr;
+    CUgreenCtx green = nullptr;
+    CUdevResource r;
+    if (((PFN_cuStreamGetCtx_v12050)get_ctx)(s, &ctx, &green) != CUDA_SUCCESS || !green ||
+        ((PFN_cuGreenCtxGetDevResource_v12040)get_resource)(green, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+        return device_sms;
+    return std::min(device_sms, (int)r.sm.smCount);
+}
+
 // Whether n_steps plain steps of a device-resident state run in the multi-step kernel.
 constexpr int64_t kMultiSteps = 4096;  // of one launch
 bool multi_steps(const swe_ctx* c, int64_t n_steps) {
-    return n_steps > 1 && c->multi_fits && c->dt_seq_len == 0 && c->stage_depth == 1 &&
+    // every segment needs a CTA on the GPU at once
+    return n_steps > 1 && c->n_seg <= (int64_t)c->multi_per_sm * c->stream_sms && c->dt_seq_len == 0 && c->stage_depth == 1 &&
            c->cross_mode == SWE_CROSS_AUTO && c->inject != SWE_INJECT_STAGING_TX && all_by_max(c->ip_host);
 }
 
@@ -967,6 +995,7 @@ int swe_create(swe_ctx** out, int device) {
     }
     c->stream = c->own_stream;
     cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
+    c->stream_sms = c->num_sms;
     if ((rc = device_alloc((void**)&c->gs, sizeof(GlobalScalars)))) {
         cudaStreamDestroy(c->own_stream);
         delete c;
@@ -1010,6 +1039,8 @@ int swe_set_stream(swe_ctx* c, void* stream) {
     const cudaStream_t s = stream ? (cudaStream_t)stream : c->own_stream;
     c->stream_changed = c->stream_changed || s != c->stream;
     c->stream = s;
+    cudaSetDevice(c->device);
+    c->stream_sms = s == c->own_stream ? c->num_sms : sms_of_stream(s, c->num_sms);
     drop_graphs(c);
     return SWE_OK;
 }
