@@ -289,6 +289,7 @@ struct swe_ctx {
     size_t multi_smem = 0;          // of the multi-step kernel, whose segments hold their depths too
     int multi_per_sm = 0;           // the multi-step kernel's CTAs per SM; 0: its segments do not fit one
     int stream_sms = 0;             // SMs that work on the stream runs on
+    bool multi_refused = false;     // a launch of it on this stream, with this configuration, was refused
     // device memory
     double* h[2] = {nullptr, nullptr};
     double* hu[2] = {nullptr, nullptr};
@@ -495,6 +496,7 @@ int configure_launch(swe_ctx* c) {
     if (!k) return set_error(SWE_E_INVALID, "unknown solver");
     int rc;
     c->multi_per_sm = 0;  // until it is known
+    c->multi_refused = false;
     c->smem = smem_bytes(c, false);
     for (int s : {FWAVE, AUG_RIEMANN, LF, LF_BATH, LLF, LLF_BATH}) {
         for (bool host : {false, true})
@@ -726,8 +728,9 @@ int sms_of_stream(cudaStream_t s, int device_sms) {
 constexpr int64_t kMultiSteps = 4096;  // of one launch
 bool multi_steps(const swe_ctx* c, int64_t n_steps) {
     // every segment needs a CTA on the GPU at once
-    return n_steps > 1 && c->n_seg <= (int64_t)c->multi_per_sm * c->stream_sms && c->dt_seq_len == 0 && c->stage_depth == 1 &&
-           c->cross_mode == SWE_CROSS_AUTO && c->inject != SWE_INJECT_STAGING_TX && all_by_max(c->ip_host);
+    const bool fits = !c->multi_refused && c->n_seg <= (int64_t)c->multi_per_sm * c->stream_sms;
+    return n_steps > 1 && fits && c->dt_seq_len == 0 && c->stage_depth == 1 && c->cross_mode == SWE_CROSS_AUTO &&
+           c->inject != SWE_INJECT_STAGING_TX && all_by_max(c->ip_host);
 }
 
 // Steps on a stream that the context worked on before may still read the dt sequence:
@@ -901,7 +904,7 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     A.extra_tx = c->inject == SWE_INJECT_STAGING_TX ? 16u : 0u;
     A.extra_meet = c->inject == SWE_INJECT_MEETING ? 1u : 0u;
     A.extra_end = c->inject == SWE_INJECT_LAST_MEETING ? 1u : 0u;
-    A.wait_ns = c->inject != SWE_INJECT_NONE ? 20000000ull : kWaitNs;
+    A.wait_ns = A.extra_tx | A.extra_meet | A.extra_end ? 20000000ull : kWaitNs;
     const bool pass = cross_pass(c, io != nullptr);
     A.halo_solve = pass ? 0 : 1;
     if (io) {
@@ -930,6 +933,7 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     // (90 registers) fit 5 per SM, 20 warps, against 2 CTAs of 256 threads
     constexpr int kCrossThreads = 128;
     // many plain steps of a mesh that fits the GPU at once: the multi-step kernel
+    int64_t s = 0;
     if (!io && !branch && !fz && multi_steps(c, n_steps)) {
         void* km = fma ? fma_multi_kernel(c->params[0].solver) : multi_kernel_for(c->params[0].solver);
         cudaLaunchAttribute at;
@@ -942,17 +946,23 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
         cfg.stream = c->stream;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        for (int64_t s = 0; s < n_steps; s += kMultiSteps) {
+        for (; s < n_steps; s += kMultiSteps) {
             int ns = (int)std::min<int64_t>(kMultiSteps, n_steps - s);
             void* margs[] = {&A, &ns};
-            CUDA_TRY(cudaLaunchKernelExC(&cfg, km, margs));
+            const cudaError_t e = c->inject == SWE_INJECT_REFUSED_LAUNCH ? cudaErrorCooperativeLaunchTooLarge
+                                                                         : cudaLaunchKernelExC(&cfg, km, margs);
+            if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+                cudaGetLastError();
+                c->multi_refused = true;  // a launch per step from here on
+                break;
+            }
+            CUDA_TRY(e);
             if (!c->capturing) c->step_mirror += ns;
         }
-        return SWE_OK;
     }
     const unsigned xblocks = pass ? (unsigned)((c->n_xtasks + kCrossThreads - 1) / kCrossThreads) : 0u;
     void* args[] = {&A};
-    for (int64_t s = 0; s < n_steps; ++s) {
+    for (; s < n_steps; ++s) {
         if (xblocks) CUDA_TRY(cudaLaunchKernel(kx, dim3(xblocks), dim3(kCrossThreads), args, 0, c->stream));
         CUDA_TRY(cudaLaunchKernel(k, dim3(c->grid), dim3(c->block_threads), args, c->smem, c->stream));
         if (!c->capturing) ++c->step_mirror;
@@ -1040,6 +1050,7 @@ int swe_set_stream(swe_ctx* c, void* stream) {
     c->stream_changed = c->stream_changed || s != c->stream;
     c->stream = s;
     cudaSetDevice(c->device);
+    c->multi_refused = false;
     c->stream_sms = s == c->own_stream ? c->num_sms : sms_of_stream(s, c->num_sms);
     drop_graphs(c);
     return SWE_OK;
@@ -1671,7 +1682,7 @@ int swe_get_step_count(swe_ctx* c, int64_t* steps) {
 
 int swe_set_fault_injection(swe_ctx* c, int32_t kind) {
     if (!c) return set_error(SWE_E_INVALID, "null context");
-    if (kind < SWE_INJECT_NONE || kind > SWE_INJECT_LAST_MEETING)
+    if (kind < SWE_INJECT_NONE || kind > SWE_INJECT_REFUSED_LAUNCH)
         return set_error(SWE_E_INVALID, "unknown fault injection %d", kind);
     c->inject = kind;
     return SWE_OK;

@@ -39,3 +39,24 @@ def test_meeting_runs_out_and_context_recovers(swe_lib, oracle_lib, log2, discs,
             assert S.n_refine > 0
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_a_refused_launch_is_made_step_by_step(swe_lib, oracle_lib, graph):
+    g, cfg = _grid(12, 1, "fwave", "slip")
+    L = _lib.load()
+    ctx = _context(g, cfg)
+    try:
+        _lib.check(L.swe_set_fault_injection(ctx.ptr, 4))
+        S, P = omp_state(g.mesh, g), oracle_params(cfg)
+        for n in (5, 4):
+            S.steps(P, n)
+            (ctx.traverse_graph if graph else ctx.traverse)(n)
+            ctx.synchronize()
+            _compare(ctx, S, "%d steps" % n)
+        assert ctx.launch_count(4) == 4 and ctx.step_count() == 9
+        _lib.check(L.swe_set_fault_injection(ctx.ptr, NONE))
+        ctx.upload_mesh(g.mesh)
+        assert ctx.launch_count(4) == 1
+    finally:
+        ctx.close()
