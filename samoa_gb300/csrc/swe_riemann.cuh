@@ -969,8 +969,9 @@ __device__ __forceinline__ void depth_terms(const State& Q, double drytol, doubl
 
 // One edge between two states, for the entry points without a context, whose tolerance
 // may be negative: a depth at or below zero is then wet. FastOps' quotients of zeros by
-// a wet depth take that depth for positive, and the Lax-Friedrichs fluxes the root of a
-// negative one for 0 (their sqrt(g max(d, 0))), the GeoClaw ones for NaN.
+// a wet depth and the f-wave's shortcut for water at rest take that depth for positive,
+// and the Lax-Friedrichs fluxes the root of a negative one for 0 (their
+// sqrt(g max(d, 0))), the GeoClaw ones for NaN.
 template <int SOLVER>
 __device__ __forceinline__ void flux_of_states(double n1, double n2, const State& QL, const State& QR, double drytol,
                                                Update& fL, Update& fR) {
@@ -989,7 +990,10 @@ __device__ __forceinline__ void flux_of_states(double n1, double n2, const State
         if (f.ok) return;
     }
     SafeOps o;
-    edge_flux<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, nullptr, o);
+    if ((SOLVER == FWAVE || SOLVER == AUG_RIEMANN) && lt0(drytol))
+        geoclaw_rotated<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, nullptr, o);
+    else
+        edge_flux<SOLVER, 0>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, axis, nullptr, o);
 }
 
 // Ghost state of bnd_skeleton_scalar_op, src/SWE/SWE_euler_timestep.f90:231-255.
