@@ -285,6 +285,7 @@ struct swe_ctx {
     int64_t n_seg = 0, n_tasks = 0;
     int grid = 0, max_ndepth = 1;
     size_t smem = 0;
+    bool stage_dep = true;          // the cells' refinement depths fit into it too
     std::vector<int32_t> first_seg; // of each instance, and n_seg
     size_t multi_smem = 0;          // of the multi-step kernel, whose segments hold their depths too
     int multi_per_sm = 0;           // the multi-step kernel's CTAs per SM; 0: its segments do not fit one
@@ -389,16 +390,16 @@ int device_alloc(void** p, size_t bytes) {
     return SWE_OK;
 }
 
+// Shared memory of the step kernel's arrays without the cells' refinement depths.
 size_t smem_bytes_for(int64_t seg_cells, int stage_depth, int max_ndepth, bool own_d = false) {
     // staging [depth][4][T], recip_fix(depth) and sqrt(g depth) [2][T], edge slots [12][T], with own_d the depths
-    // h - b [T], depth tables [6][nd], the cells' refinement depths [T] bytes
+    // h - b [T], depth tables [6][nd]
     return (size_t)(14 + 4 * stage_depth + (own_d ? 1 : 0)) * (size_t)seg_cells * sizeof(double) +
-           (size_t)6 * max_ndepth * sizeof(double) + (((size_t)seg_cells + 15) & ~(size_t)15);
+           (size_t)6 * max_ndepth * sizeof(double);
 }
 
-size_t smem_bytes(const swe_ctx* c, bool own_d) {
-    return smem_bytes_for(c->seg_cells, c->stage_depth, c->max_ndepth, own_d);
-}
+// Of the refinement depths [T] bytes.
+size_t dep_bytes(const swe_ctx* c) { return ((size_t)c->seg_cells + 15) & ~(size_t)15; }
 
 constexpr size_t kMaxSmem = 227 * 1024, kStaticSmem = 1024;  // of a CTA; more than the kernels' static part
 
@@ -497,7 +498,9 @@ int configure_launch(swe_ctx* c) {
     int rc;
     c->multi_per_sm = 0;  // until it is known
     c->multi_refused = false;
-    c->smem = smem_bytes(c, false);
+    c->smem = smem_bytes_for(c->seg_cells, c->stage_depth, c->max_ndepth);
+    c->stage_dep = c->smem + dep_bytes(c) + kStaticSmem <= kMaxSmem;
+    if (c->stage_dep) c->smem += dep_bytes(c);
     for (int s : {FWAVE, AUG_RIEMANN, LF, LF_BATH, LLF, LLF_BATH}) {
         for (bool host : {false, true})
             if ((rc = raise_smem_limit((const void*)kernel_for(s, host), c->smem)) ||
@@ -514,7 +517,7 @@ int configure_launch(swe_ctx* c) {
                          c->block_threads);
     int64_t g = (int64_t)per_sm * c->num_sms;
     c->grid = (int)std::max<int64_t>(1, std::min<int64_t>(g, c->n_seg));
-    c->multi_smem = smem_bytes(c, true);
+    c->multi_smem = smem_bytes_for(c->seg_cells, c->stage_depth, c->max_ndepth, true) + dep_bytes(c);
     if (c->multi_smem + kStaticSmem <= kMaxSmem) {
         int fit = INT_MAX;
         for (void* m : {multi_kernel_for(c->params[0].solver), fma_multi_kernel(c->params[0].solver)}) {
@@ -895,6 +898,7 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     A.n_cells_total = (int32_t)c->cells_total;
     A.use_tma = use_tma;
     A.stage_depth = c->stage_depth;
+    A.stage_dep = c->stage_dep ? 1 : 0;
     A.fixed_io = 0;
     // fault injection (tests): the staging barrier expects 16 bytes that no copy
     // delivers, so its phase never completes and the bounded wait, shortened to
