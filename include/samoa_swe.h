@@ -397,16 +397,14 @@ int swe_division_check(int64_t n, uint64_t seed, int32_t exponent_span, int64_t*
  * report clears the device flag; the failed step's state is undefined, so
  * upload a state (or a mesh) before stepping on. Applies to device-resident
  * steps (swe_traverse); stays set until SWE_INJECT_NONE. SWE_INJECT_MEETING:
- * where many steps run in one kernel, its CTAs' waits for one another between
- * two steps count one CTA too many and give up the same way;
- * SWE_INJECT_LAST_MEETING: the wait for the last step's CTAs does.
+ * where many steps run in one kernel (with this injection one step too), its
+ * CTAs' waits for one another count one CTA too few and give up the same way.
  * SWE_INJECT_REFUSED_LAUNCH: the launch of that kernel is not made and counts as
  * refused by the driver, upon which each step is launched by itself. */
 #define SWE_INJECT_NONE 0
 #define SWE_INJECT_STAGING_TX 1
 #define SWE_INJECT_MEETING 2
-#define SWE_INJECT_LAST_MEETING 3
-#define SWE_INJECT_REFUSED_LAUNCH 4
+#define SWE_INJECT_REFUSED_LAUNCH 3
 int swe_set_fault_injection(swe_ctx* ctx, int32_t kind);
 
 /* One time step on caller-owned device memory, allocating nothing. No

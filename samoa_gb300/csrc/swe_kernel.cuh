@@ -76,7 +76,6 @@ struct StepArgs {
     int32_t halo_solve;        // 1: solve the halo tasks here (no cross-edge pass); 0: copy the pass's updates
     double2* memo;             // per cell (d, sqrt(g d)) of an earlier step, or null: see the staging loop
     uint32_t extra_tx;         // fault injection only: bytes the staging barrier expects beyond the copies (0)
-    uint32_t extra_meet, extra_end;  // fault injection only: arrivals the multi-step kernel's waits expect beyond its CTAs' (0)
     unsigned long long wait_ns;  // limit of one mbarrier wait, in ns of the global timer
 };
 
@@ -1040,7 +1039,7 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const __grid_constant__
         unsigned int bad = 0;
         bool met = k == 0;
         auto meet = [&]() {
-            if (!met && !wait_count(&S->arrived, (unsigned int)k * n_cta + A.extra_meet, A.wait_ns)) bad = 4u;
+            if (!met && !wait_count(&S->arrived, (unsigned int)k * n_cta, A.wait_ns)) bad = 4u;
             met = true;
         };
         auto prepare_dt = [&]() {
@@ -1101,7 +1100,7 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const __grid_constant__
     }
     // ---- the instance's scalars, and the counters for the next launch
     if (keeper && k == n_steps) {
-        if (wait_count(&S->arrived, (unsigned int)n_steps * n_cta + A.extra_end, A.wait_ns)) {
+        if (wait_count(&S->arrived, (unsigned int)n_steps * n_cta, A.wait_ns)) {
             advance_time(S, P, time, DBL_MAX, __ldcg(&S->ds_ring[(n_steps - 1) % 3]), __ldcg(&S->refine_acc));
         } else {
             atomicOr(&s_error, 4u);

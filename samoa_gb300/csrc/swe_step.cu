@@ -732,7 +732,7 @@ constexpr int64_t kMultiSteps = 4096;  // of one launch
 bool multi_steps(const swe_ctx* c, int64_t n_steps) {
     // every segment needs a CTA on the GPU at once
     const bool fits = !c->multi_refused && c->n_seg <= (int64_t)c->multi_per_sm * c->stream_sms;
-    return n_steps > 1 && fits && c->dt_seq_len == 0 && c->stage_depth == 1 && c->cross_mode == SWE_CROSS_AUTO &&
+    return n_steps > (c->inject == SWE_INJECT_MEETING ? 0 : 1) && fits && c->dt_seq_len == 0 && c->stage_depth == 1 && c->cross_mode == SWE_CROSS_AUTO &&
            c->inject != SWE_INJECT_STAGING_TX && all_by_max(c->ip_host);
 }
 
@@ -902,13 +902,11 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     A.fixed_io = 0;
     // fault injection (tests): the staging barrier expects 16 bytes that no copy
     // delivers, so its phase never completes and the bounded wait, shortened to
-    // 20 ms, gives up; every issued copy still lands before the CTA leaves. Likewise the
-    // multi-step kernel's meetings, or its wait for the last step, count one CTA too many
+    // 20 ms, gives up; every issued copy still lands before the CTA leaves
     A.memo = c->memo;
     A.extra_tx = c->inject == SWE_INJECT_STAGING_TX ? 16u : 0u;
-    A.extra_meet = c->inject == SWE_INJECT_MEETING ? 1u : 0u;
-    A.extra_end = c->inject == SWE_INJECT_LAST_MEETING ? 1u : 0u;
-    A.wait_ns = A.extra_tx | A.extra_meet | A.extra_end ? 20000000ull : kWaitNs;
+    const bool short_waits = c->inject == SWE_INJECT_STAGING_TX || c->inject == SWE_INJECT_MEETING;
+    A.wait_ns = short_waits ? 20000000ull : kWaitNs;
     const bool pass = cross_pass(c, io != nullptr);
     A.halo_solve = pass ? 0 : 1;
     if (io) {
@@ -953,6 +951,9 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
         for (; s < n_steps; s += kMultiSteps) {
             int ns = (int)std::min<int64_t>(kMultiSteps, n_steps - s);
             void* margs[] = {&A, &ns};
+            // fault injection (tests): the instances' counts of arrived CTAs start at -1
+            for (int i = 0; c->inject == SWE_INJECT_MEETING && i < A.n_inst; ++i)
+                CUDA_TRY(cudaMemsetAsync(&c->is[i].arrived, 0xff, sizeof(c->is[i].arrived), c->stream));
             const cudaError_t e = c->inject == SWE_INJECT_REFUSED_LAUNCH ? cudaErrorCooperativeLaunchTooLarge
                                                                          : cudaLaunchKernelExC(&cfg, km, margs);
             if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {

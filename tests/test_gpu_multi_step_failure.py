@@ -1,5 +1,6 @@
-"""The multi-step kernel's waits between its CTAs run out (the injections make them count one CTA too many, with a
-limit of 20 ms): the call reports it, and the context then steps like the oracle, refinement count included."""
+"""The multi-step kernel's waits between its CTAs run out (an injection makes them count one CTA too few, with a limit
+of 20 ms), the wait between two steps or, in a run of one, that for the last: the call reports it, and the context
+then steps like the oracle, refinement count included."""
 import pytest
 
 from samoa_gb300 import _lib
@@ -10,27 +11,27 @@ from tests.test_gpu_multi_step_routes import _context
 pytestmark = pytest.mark.gpu
 
 SWE_E_DEVICE = -6
-NONE, MEETING, LAST_MEETING = 0, 2, 3
+NONE, MEETING, REFUSED_LAUNCH = 0, 2, 3
 
 
-@pytest.mark.parametrize("kind", [MEETING, LAST_MEETING])
+@pytest.mark.parametrize("steps", [2, 4, 1])
 @pytest.mark.parametrize("log2,discs", [(5, 0), (12, 1), (16, 0)])
-def test_meeting_runs_out_and_context_recovers(swe_lib, oracle_lib, log2, discs, kind):
+def test_meeting_runs_out_and_context_recovers(swe_lib, oracle_lib, log2, discs, steps):
     g, cfg = _grid(log2, discs, "fwave", "slip")
     cfg.i_max_depth = log2 + 12  # so that cells do ask for refinement
     L = _lib.load()
     ctx = _context(g, cfg)
     try:
-        _lib.check(L.swe_set_fault_injection(ctx.ptr, kind))
-        assert ctx.launch_count(4) == 1
-        ctx.traverse(4)
+        _lib.check(L.swe_set_fault_injection(ctx.ptr, MEETING))
+        assert ctx.launch_count(steps) == 1
+        ctx.traverse(steps)
         with pytest.raises(_lib.SweError) as err:
             ctx.synchronize()
         assert err.value.code == SWE_E_DEVICE and "ran out" in str(err.value)
         ctx.synchronize()  # reported once
         _lib.check(L.swe_set_fault_injection(ctx.ptr, NONE))
         ctx.upload_state(g.h, g.hu, g.hv, g.b)  # the time is still that of the state before the failed steps
-        S, P = omp_state(g.mesh, g), oracle_params(cfg)
+        S, P = omp_state(g.mesh, g, parity=steps & 1), oracle_params(cfg)
         for n in (2, 3):
             S.steps(P, n)
             ctx.traverse(n)
@@ -47,7 +48,7 @@ def test_a_refused_launch_is_made_step_by_step(swe_lib, oracle_lib, graph):
     L = _lib.load()
     ctx = _context(g, cfg)
     try:
-        _lib.check(L.swe_set_fault_injection(ctx.ptr, 4))
+        _lib.check(L.swe_set_fault_injection(ctx.ptr, REFUSED_LAUNCH))
         S, P = omp_state(g.mesh, g), oracle_params(cfg)
         for n in (5, 4):
             S.steps(P, n)
