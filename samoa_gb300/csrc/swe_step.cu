@@ -1602,13 +1602,20 @@ int launch_adjoint(swe_ctx* c, long long t, const uint8_t* branch, const double*
         if (int rc = raise_smem_limit((const void*)kern, smem)) return rc;
         // 256 threads (us at 2^18 cells: f-wave 157, with 192, 160 and 128 threads 183, 160 and
         // 173; LLF with bathymetry 114 against 124, 111 and 123), but 128 where an SM holds
-        // only one CTA of 256: the augmented solver's reverse (146 registers) 571 with 256,
-        // 541, 533 and 530 with fewer
-        int per_sm = 0;
-        for (int threads : {256, 128}) {
-            c->adj_threads = threads;
-            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
-            if (per_sm > 1) break;
+        // only one CTA of 256 and two or more of 128, that is where the registers are the limit:
+        // the augmented solver's reverse (146 registers) 571 with 256, 541, 533 and 530 with
+        // fewer, in segments of 660 cells of a mesh of 2e5 418 against 385. From 690 cells on it
+        // is the shared memory (168 bytes per cell), and 128 threads are just fewer (704 cells,
+        // 2^20 in all: f-wave 935 with 128, 678 with 256, augmented 3105 and 2131)
+        int per_sm = 0, small = 0;
+        c->adj_threads = 256;
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
+        if (per_sm < 2) {
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&small, kern, 128, smem));
+            if (small > per_sm) {
+                c->adj_threads = 128;
+                per_sm = small;
+            }
         }
         if (per_sm < 1) return set_error(SWE_E_INVALID, "adjoint tiling does not fit an SM");
         c->adj_grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * c->num_sms, c->n_seg));
