@@ -660,14 +660,38 @@ int current_index(swe_ctx* c, int* idx) {
     return SWE_OK;
 }
 
+// The shortest segments, of 64 cells or more, that are at most `most`: segments never
+// span instances, so each instance's last one is rounded up. 0 if that takes more than
+// 750 cells. With more instances than that the length that divides their cells, but not
+// above the largest instance.
+int32_t resident_segment(const swe_ctx* c, int64_t most) {
+    const int64_t even = ((c->cells_total + most - 1) / most + 1) & ~(int64_t)1;
+    if (even > 750) return 0;
+    int64_t largest = 0;
+    for (const HostMesh& m : c->mesh) largest = std::max(largest, m.n_cells);
+    if ((int64_t)c->mesh.size() > most)
+        return (int32_t)std::max<int64_t>(64, std::min(even, (largest + 1) & ~(int64_t)1));
+    for (int64_t seg = std::max<int64_t>(64, even); seg <= 750; seg += 2) {
+        int64_t segs = 0;
+        for (const HostMesh& m : c->mesh) segs += (m.n_cells + seg - 1) / seg;
+        if (segs <= most) return (int32_t)seg;
+    }
+    return 0;
+}
+
 // Segment length and block size until the caller sets them, by the cells of all
 // instances (measured on wet/dry bowls and water moving everywhere).
 // Up to 1500 cells per SM a mesh is resident (multi_step_kernel): two CTAs of
 // 256 threads per SM, in segments that give every SM two (2^16 cells, us per step:
 // 216 x 256 27.0, 108 x 128 31.2, 256 x 256 29.7; 2^17: 432 x 256 41, 216 x 128
-// 49), but not below 64 cells, whose edges give one warp to each of an SM's four
-// schedulers (2^12 cells: 64 x 128 12.2, 32 x 64 14.5). Larger meshes take the
-// step kernel (us per step, 128 threads unless said):
+// 49; 2.27e5: 748 x 256 57.7, 256 x 256 74.3, 384 x 128 68.9; ensembles in segments
+// that divide the cells evenly, and so a few more than two per SM: four each of 2^5 to
+// 2^13 cells 33.4, now 24.7, of 2^6 to 2^14 50.2 and 40.9), but not below 64 cells,
+// whose edges give one warp to each of an SM's four schedulers (2^12 cells: 64 x 128
+// 12.2, 32 x 64 14.5). More instances than two per SM take the step kernel in
+// segments of their size (1000 of 64 cells: 64 x 128 51.5, 212 x 256 62.6; 400 of
+// 512: 512 x 256 88, 384 x 128 112). Larger meshes take it too
+// (us per step, 128 threads unless said):
 // - an ensemble beyond that 384 x 128 (5.2e5 cells in 36 bowls: 128, 256 x 256 139; 2.6e5:
 //   80 against 83);
 // - GeoClaw fluxes below 2^19 cells 256 x 256 (3.2e5 refined cells, augmented: 191, 256 x 128
@@ -679,10 +703,10 @@ int current_index(swe_ctx* c, int* idx) {
 //   3.2e5 refined: 58.2 against 65.5), then 384 x 128 (2^19: 78, 256 x 128 83).
 // The solver is the one set when the mesh comes.
 void auto_tiling(swe_ctx* c) {
-    const int64_t n = c->cells_total, resident = (int64_t)2 * c->num_sms;
+    const int64_t n = c->cells_total;
     int32_t seg = 384, threads = 128;
-    if (n <= resident * 750) {
-        seg = (int32_t)std::max<int64_t>(64, ((n + resident - 1) / resident + 1) & ~(int64_t)1);
+    if (const int32_t fit = resident_segment(c, (int64_t)2 * c->num_sms)) {
+        seg = fit;
         threads = seg > 64 ? 256 : 128;
     } else if (n_inst(c) == 1) {
         const bool geo = c->params.empty() || geoclaw(c->params[0].solver);
