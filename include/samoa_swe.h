@@ -140,8 +140,8 @@ int swe_last_error(char* buf, size_t n);
 /* Kernel tuning: cells per segment (even, 64..1536; 18 doubles of shared
  * memory per cell, 22 with staging depth 2, at most 227 KB in all) and threads
  * per block (multiple of 32, 64..256); 0 keeps
- * the current value. A mesh upload or
- * this call rebuilds the segment task lists. Until a segment length is set
+ * the current value, but threads that were never set are 128 with a segment
+ * length set here. A mesh upload or this call rebuilds the segment task lists. Until a segment length is set
  * here, each mesh upload picks it by size: 384 cells on large meshes and for
  * ensembles, 256 on middling ones (where the flux set before the upload and the
  * size decide), and on meshes that fit the GPU at once two segments per SM (at

@@ -688,8 +688,8 @@ int32_t resident_segment(const swe_ctx* c, int64_t most) {
 // that divide the cells evenly, and so a few more than two per SM: four each of 2^5 to
 // 2^13 cells 33.4, now 24.7, of 2^6 to 2^14 50.2 and 40.9), but not below 64 cells,
 // whose edges give one warp to each of an SM's four schedulers (2^12 cells: 64 x 128
-// 12.2, 32 x 64 14.5). More instances than two per SM take the step kernel in
-// segments of their size (1000 of 64 cells: 64 x 128 51.5, 212 x 256 62.6; 400 of
+// 12.2, 32 x 64 14.5). More instances than two per SM get segments of their size
+// and mostly the step kernel (1000 of 64 cells: 64 x 128 51.5, 212 x 256 62.6; 400 of
 // 512: 512 x 256 88, 384 x 128 112). Larger meshes take it too
 // (us per step, 128 threads unless said):
 // - an ensemble beyond that 384 x 128 (5.2e5 cells in 36 bowls: 128, 256 x 256 139; 2.6e5:
@@ -718,7 +718,7 @@ void auto_tiling(swe_ctx* c) {
         }
     }
     if (!c->tiling_set) c->seg_cells = seg;
-    if (!c->threads_set && !c->tiling_set) c->block_threads = threads;
+    if (!c->threads_set) c->block_threads = c->tiling_set ? 128 : threads;
 }
 
 // Whether the edges between two segments get a pass of their own before the
@@ -1133,6 +1133,7 @@ int swe_set_tiling(swe_ctx* c, int32_t seg_cells, int32_t block_threads) {
     if (seg_cells) {
         c->seg_cells = seg_cells;
         c->tiling_set = true;
+        if (!c->threads_set) c->block_threads = 128;  // not what an earlier mesh's own tiling had
     }
     if (block_threads) {
         c->block_threads = block_threads;

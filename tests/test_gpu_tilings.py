@@ -57,3 +57,20 @@ def test_ensembles_that_fit_the_gpu_at_once(swe_lib, oracle_lib, kind):
             assert_state_equal("instance %d" % i, x, y, z, S.h, S.hu, S.hv)
     finally:
         ens.close()
+
+
+def test_threads_with_a_segment_length_of_the_callers(swe_lib):
+    """128 threads unless they were set, whatever an earlier mesh's own tiling had picked."""
+    g, cfg = _grid(16, 0, "fwave", "slip")
+    ctx = _context(g, cfg)
+    try:
+        assert ctx.get_tiling()[1] == 256
+        ctx.set_tiling(512)
+        assert ctx.get_tiling() == (512, 128)
+        ctx.upload_mesh(g.mesh)
+        assert ctx.get_tiling() == (512, 128)
+        ctx.set_tiling(0, 192)
+        ctx.set_tiling(256)
+        assert ctx.get_tiling() == (256, 192)
+    finally:
+        ctx.close()
