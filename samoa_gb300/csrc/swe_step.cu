@@ -751,13 +751,24 @@ int sms_of_stream(cudaStream_t s, int device_sms) {
     return std::min(device_sms, (int)r.sm.smCount);
 }
 
-// Whether n_steps plain steps of a device-resident state run in the multi-step kernel.
+// Of the next n_steps, the first that may take their dt from the sequence. In a capture
+// all: its replays can start at any step.
+int64_t frozen_steps(const swe_ctx* c, int64_t n_steps) {
+    if (c->dt_seq_len == 0) return 0;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess) cudaGetLastError();
+    if (capture != cudaStreamCaptureStatusNone) return n_steps;
+    return std::max<int64_t>(0, std::min<int64_t>(n_steps, c->dt_seq_len - (c->step_mirror - c->seq_base_mirror)));
+}
+
+// Whether n_steps plain steps of a device-resident state, their dt from the CFL
+// condition, run in the multi-step kernel.
 constexpr int64_t kMultiSteps = 4096;  // of one launch
 bool multi_steps(const swe_ctx* c, int64_t n_steps) {
     // every segment needs a CTA on the GPU at once
     const bool fits = !c->multi_refused && c->n_seg <= (int64_t)c->multi_per_sm * c->stream_sms;
-    return n_steps > (c->inject == SWE_INJECT_MEETING ? 0 : 1) && fits && c->dt_seq_len == 0 && c->stage_depth == 1 && c->cross_mode == SWE_CROSS_AUTO &&
-           c->inject != SWE_INJECT_STAGING_TX && all_by_max(c->ip_host);
+    return n_steps > (c->inject == SWE_INJECT_MEETING ? 0 : 1) && fits && c->stage_depth == 1 &&
+           c->cross_mode == SWE_CROSS_AUTO && c->inject != SWE_INJECT_STAGING_TX && all_by_max(c->ip_host);
 }
 
 // Steps on a stream that the context worked on before may still read the dt sequence:
@@ -888,6 +899,12 @@ int copy_state(swe_ctx* c, int to_device, double* h, double* hu, double* hv, dou
 int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double* const* io = nullptr,
                  const double* b = nullptr, int8_t* flags = nullptr, int use_tma = 1, int fz = 0,
                  uint16_t* erec = nullptr) {
+    const bool plain = !io && !branch && !fz;
+    const int64_t frozen = plain ? frozen_steps(c, n_steps) : n_steps;
+    if (frozen > 0 && frozen < n_steps) {
+        if (int rc = launch_steps(c, frozen)) return rc;
+        return launch_steps(c, n_steps - frozen);
+    }
     StepArgs A;
     A.branch = branch;
     for (int k = 0; k < 2; ++k) {
@@ -960,7 +977,7 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     constexpr int kCrossThreads = 128;
     // many plain steps of a mesh that fits the GPU at once: the multi-step kernel
     int64_t s = 0;
-    if (!io && !branch && !fz && multi_steps(c, n_steps)) {
+    if (frozen == 0 && multi_steps(c, n_steps)) {
         void* km = fma ? fma_multi_kernel(c->params[0].solver) : multi_kernel_for(c->params[0].solver);
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeCooperative;
@@ -1203,8 +1220,11 @@ int swe_get_task_counts(swe_ctx* c, int64_t* n_segments, int64_t* n_tasks, int64
 int swe_get_launch_count(swe_ctx* c, int64_t n_steps, int64_t* launches) {
     if (!c || !launches || n_steps < 0) return set_error(SWE_E_INVALID, "bad arguments");
     if (!c->has_mesh) return set_error(SWE_E_NOMESH, "upload a mesh first");
-    *launches = multi_steps(c, n_steps) ? (n_steps + kMultiSteps - 1) / kMultiSteps
-                                        : n_steps * (cross_pass(c, false) ? 2 : 1);
+    int64_t single = frozen_steps(c, n_steps);
+    const int64_t rest = n_steps - single;
+    const bool multi = multi_steps(c, rest);
+    if (!multi) single += rest;
+    *launches = single * (cross_pass(c, false) ? 2 : 1) + (multi ? (rest + kMultiSteps - 1) / kMultiSteps : 0);
     return SWE_OK;
 }
 
