@@ -275,7 +275,8 @@ int swe_traverse_graph(swe_ctx* ctx, int64_t n_steps);
 /* Freeze the time-step sequence: the k-th step after this call uses
  * dts[k * n_instances + i] for instance i instead of the CFL dt (for adjoint
  * and finite-difference runs, where dt must not depend on the state);
- * n_steps = 0 clears it. No reference counterpart. */
+ * n_steps = 0 clears it and gives back the device buffers that the context
+ * keeps for sequences and for swe_gauge_gradient. No reference counterpart. */
 int swe_set_dt_sequence(swe_ctx* ctx, int64_t n_steps, const double* dts);
 
 /* ---- discrete adjoint (single-instance contexts; the f-wave and augmented
@@ -343,7 +344,9 @@ int swe_traverse_gauges(swe_ctx* ctx, int64_t n_steps, int64_t n_gauges, const i
  * grad_hu, grad_hv (may be NULL), grad_b (dJ/db); J and forward_steps (may be
  * NULL) on the host. The context is left at x_0 and its step count; the dt
  * sequence stays set. Synchronises before returning. Allocates
- * snapshots * 24 * n_cells + n_steps * n_cells bytes for the sweep.
+ * snapshots * 24 * n_cells + n_steps * n_cells bytes for the sweep, and up to
+ * 512 MB of them stay with the context for the next gradient, until a larger mesh
+ * comes or swe_set_dt_sequence(ctx, 0, NULL) gives them back.
  * No counterpart in the reference. */
 int swe_gauge_gradient(swe_ctx* ctx, int64_t n_steps, const double* dts, int32_t snapshots, int64_t n_gauges,
                        const int64_t* gauges, const double* obs, double* gauge_values, double* grad_h,

@@ -348,6 +348,13 @@ void drop_graphs(swe_ctx* c) {
     c->graphs.clear();
 }
 
+// Give back the buffers kept for swe_gauge_gradient.
+void free_sweep(swe_ctx* c) {
+    cudaFree(c->sweep);
+    c->sweep = nullptr;
+    c->cap_sweep = 0;
+}
+
 // Forget the mesh: graphs, the frozen dt sequence and the adjoint's branch
 // buffer always go; the cell, instance and task buffers are released only with
 // `release` (else kept for a re-upload that fits them).
@@ -366,10 +373,10 @@ void free_mesh_buffers(swe_ctx* c, bool release = true) {
     cudaFree(c->b); cudaFree(c->depth); cudaFree(c->flags); cudaFree(c->tasks); cudaFree(c->seg_ptr);
     cudaFree(c->seg_info); cudaFree(c->seg_order); cudaFree(c->ip); cudaFree(c->is); cudaFree(c->xtasks); cudaFree(c->xflux);
     cudaFree(c->memo);
-    cudaFree(c->dt_seq); cudaFree(c->sweep);
+    free_sweep(c);
+    cudaFree(c->dt_seq);
     c->dt_seq = nullptr;
-    c->sweep = nullptr;
-    c->cap_dt_seq = c->cap_sweep = 0;
+    c->cap_dt_seq = 0;
     cudaFree(c->rows);
     c->rows = nullptr;
     c->cap_rows = 0;
@@ -561,8 +568,8 @@ static std::vector<int32_t> spread_order(const std::vector<SegInfo>& seg_info) {
 // Bytes of a sweep's buffers that stay with the context between calls.
 constexpr size_t kKeptSweep = (size_t)512 << 20;
 
-// Host lists of up to this many cells or tasks (up to 32 MB) stay with the context from
-// one mesh upload to the next: a fresh list of a small mesh costs more in page faults
+// Host lists of up to this many cells or tasks (32 MB of tasks, 60 MB of a mesh of that
+// size) stay with the context from one mesh upload to the next: a fresh list of a small mesh costs more in page faults
 // than in filling it.
 constexpr size_t kKeptItems = (size_t)1 << 21;
 
@@ -1454,7 +1461,13 @@ int swe_set_dt_sequence(swe_ctx* c, int64_t n_steps, const double* dts) {
     if (int rc = settle_streams(c)) return rc;
     c->dt_seq_len = 0;
     drop_graphs(c);
-    if (n_steps == 0) return SWE_OK;
+    if (n_steps == 0) {
+        free_sweep(c);
+        cudaFree(c->dt_seq);
+        c->dt_seq = nullptr;
+        c->cap_dt_seq = 0;
+        return SWE_OK;
+    }
     const size_t bytes = sizeof(double) * (size_t)n_steps * (size_t)n_inst(c);
     if (bytes > c->cap_dt_seq) {
         cudaFree(c->dt_seq);
@@ -2020,9 +2033,9 @@ int swe_gauge_gradient(swe_ctx* c, int64_t n_steps, const double* dts, int32_t s
     double* work = (double*)c->sweep;
     double* own = nullptr;  // a buffer of this call
     if (bytes > c->cap_sweep) {
+        free_sweep(c);  // never two at once
         if ((rc = device_alloc((void**)&work, bytes))) return rc;
         if (bytes <= kKeptSweep) {
-            cudaFree(c->sweep);
             c->sweep = work;
             c->cap_sweep = bytes;
         } else {
