@@ -152,7 +152,9 @@ int swe_set_tiling(swe_ctx* ctx, int32_t segment_cells, int32_t block_threads);
  * shared memory, then works on it; 2 = it stages the next segment (bulk copies
  * in flight) while it works on the current one, at 4 * segment_cells doubles
  * more shared memory. Default 1; SWE_E_INVALID if the tiling then exceeds
- * shared memory. No counterpart in the reference. */
+ * shared memory. The longest segments of a mesh with many depths may leave room
+ * for one only, and are then staged as with 1 (the results are the same). No
+ * counterpart in the reference. */
 int swe_set_staging(swe_ctx* ctx, int32_t depth);
 
 /* Arithmetic of the step kernel. STRICT (the default): every FP64 operation

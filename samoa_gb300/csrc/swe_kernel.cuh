@@ -71,7 +71,6 @@ struct StepArgs {
     int32_t n_seg, n_inst, seg_cells, max_ndepth, n_cells_total;
     int32_t use_tma;
     int32_t fixed_io;          // 1: read h[0], hu[0], hv[0] and write h[1].. on every step (caller's buffers)
-    int32_t stage_dep;         // 1: the cells' refinement depths have a place in shared memory
     int32_t stage_depth;       // 1: stage a segment, then work on it; 2: stage the next one meanwhile
     int32_t halo_solve;        // 1: solve the halo tasks here (no cross-edge pass); 0: copy the pass's updates
     double2* memo;             // per cell (d, sqrt(g d)) of an earlier step, or null: see the staging loop
@@ -381,7 +380,7 @@ struct SegMem {
     double* upd;  // [4 quantities][3 local edges][T]
     double* d;    // depth h - b, in an array of its own or in the staged surface's place (h)
     double* tab;  // DepthTab's
-    int8_t* dep;  // the cells' refinement depths (the step kernel's longest segments leave no room for them)
+    int8_t* dep;  // the cells' refinement depths
     // The arrays after the staging buffers.
     __device__ __forceinline__ void lay_out(double* after, bool own_d, int max_ndepth) {
         rh = reinterpret_cast<u64*>(after);
@@ -508,8 +507,9 @@ __device__ __forceinline__ int high_word(double x) { return (int)(dbits(x) >> 32
 static __device__ __noinline__ double quotient(double a, double b) { return div_one(a, b); }
 template <int FZ>
 __device__ __forceinline__ CellOut update_cell(const SegMem& M, const DepthTab& tab, const InstParams& P, int i,
-                                               int d, double h, double depth, int odd, unsigned long long wkey, uint8_t rb, Reduced& r) {
+                                               double h, double depth, int odd, unsigned long long wkey, uint8_t rb, Reduced& r) {
     const int T = M.T, k0 = odd ? 2 : 0, k2 = odd ? 0 : 2;
+    const int d = M.dep[i];
     const int di = d - P.dmin;
     const double leg = tab.leg[di], hyp = tab.hyp[di], ndv = tab.ndv[di];
     double u[4][3];
@@ -804,7 +804,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const __grid_constant__ StepArgs A) 
             // the depth it was last taken for (water at rest keeps its depth from step
             // to step); the memo holds only pairs (d, sqrt(g d)), written by the CTA
             // that owns the cell, so a hit is the value the square root would give
-            if (A.stage_dep) M.dep[i] = A.depth[c0 + i];
+            M.dep[i] = A.depth[c0 + i];
             const double d = M.h[i] - M.b()[i];
             const bool wet = lt(drytol, d);
             const bool need_y = wet && (SOLVER != FWAVE || ((dbits(M.hu()[i]) | dbits(M.hv()[i])) << 1) != 0);
@@ -881,8 +881,7 @@ __global__ void SWE_STEP_BOUNDS step_kernel(const __grid_constant__ StepArgs A) 
         for (int i = tid; i < cn; i += blockDim.x) {
             const int c = c0 + i;
             const double h = kDepths ? hin[c] : M.h[i], depth = kDepths ? M.d[i] : 0.0;
-            const int dep = A.stage_dep ? M.dep[i] : A.depth[c];
-            const CellOut o = update_cell<FZ>(M, tab, P, i, dep, h, depth, odd, wkey, FZ == 2 ? A.branch[c] : (uint8_t)0, r);
+            const CellOut o = update_cell<FZ>(M, tab, P, i, h, depth, odd, wkey, FZ == 2 ? A.branch[c] : (uint8_t)0, r);
             if (FZ != 2 && A.branch) A.branch[c] = o.branch;
             hout[c] = o.h;
             huout[c] = o.p1;
@@ -1076,7 +1075,7 @@ __global__ void __launch_bounds__(256) multi_step_kernel(const __grid_constant__
         const bool last = k == n_steps - 1;
         double *hout = A.h[odd ^ 1], *huout = A.hu[odd ^ 1], *hvout = A.hv[odd ^ 1];
         for (int i = tid; i < cn; i += bd) {
-            const CellOut o = update_cell<0>(M, tab, P, i, M.dep[i], M.h[i], M.d[i], odd, 0ull, 0, r);
+            const CellOut o = update_cell<0>(M, tab, P, i, M.h[i], M.d[i], odd, 0ull, 0, r);
             const bool same = dbits(o.h) == dbits(M.h[i]);
             M.h[i] = o.h;
             M.hu()[i] = o.p1;

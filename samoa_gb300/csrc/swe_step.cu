@@ -277,7 +277,8 @@ struct swe_ctx {
     // until the caller sets a tiling, auto_tiling picks both
     int32_t seg_cells = 384, block_threads = 128;
     bool tiling_set = false, threads_set = false;
-    int32_t stage_depth = 1;                        // segments staged ahead per CTA (1 or 2)
+    int32_t stage_depth = 1;                        // segments staged ahead per CTA (1 or 2): as set,
+    int32_t stage_used = 1;                         // and as the segments leave room for
     int32_t arith = SWE_ARITH_STRICT;
     int32_t cross_mode = SWE_CROSS_AUTO;
     int32_t seg_order_mode = SWE_ORDER_AUTO;
@@ -285,7 +286,6 @@ struct swe_ctx {
     int64_t n_seg = 0, n_tasks = 0;
     int grid = 0, max_ndepth = 1;
     size_t smem = 0;
-    bool stage_dep = true;          // the cells' refinement depths fit into it too
     std::vector<int32_t> first_seg; // of each instance, and n_seg
     size_t multi_smem = 0;          // of the multi-step kernel, whose segments hold their depths too
     int multi_per_sm = 0;           // the multi-step kernel's CTAs per SM; 0: its segments do not fit one
@@ -505,9 +505,13 @@ int configure_launch(swe_ctx* c) {
     int rc;
     c->multi_per_sm = 0;  // until it is known
     c->multi_refused = false;
-    c->smem = smem_bytes_for(c->seg_cells, c->stage_depth, c->max_ndepth);
-    c->stage_dep = c->smem + dep_bytes(c) + kStaticSmem <= kMaxSmem;
-    if (c->stage_dep) c->smem += dep_bytes(c);
+    // the longest segments leave no room for two staging buffers beside the refinement depths
+    c->stage_used = c->stage_depth;
+    c->smem = smem_bytes_for(c->seg_cells, c->stage_used, c->max_ndepth) + dep_bytes(c);
+    if (c->stage_used == 2 && c->smem + kStaticSmem > kMaxSmem) {
+        c->stage_used = 1;
+        c->smem = smem_bytes_for(c->seg_cells, c->stage_used, c->max_ndepth) + dep_bytes(c);
+    }
     for (int s : {FWAVE, AUG_RIEMANN, LF, LF_BATH, LLF, LLF_BATH}) {
         for (bool host : {false, true})
             if ((rc = raise_smem_limit((const void*)kernel_for(s, host), c->smem)) ||
@@ -945,8 +949,7 @@ int launch_steps(swe_ctx* c, int64_t n_steps, uint8_t* branch = nullptr, double*
     A.max_ndepth = c->max_ndepth;
     A.n_cells_total = (int32_t)c->cells_total;
     A.use_tma = use_tma;
-    A.stage_depth = c->stage_depth;
-    A.stage_dep = c->stage_dep ? 1 : 0;
+    A.stage_depth = c->stage_used;
     A.fixed_io = 0;
     // fault injection (tests): the staging barrier expects 16 bytes that no copy
     // delivers, so its phase never completes and the bounded wait, shortened to
