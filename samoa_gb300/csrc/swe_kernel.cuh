@@ -456,7 +456,9 @@ __device__ __forceinline__ unsigned int edge_task_with(const StepArgs& A, const 
     }
     Update fL, fR;
     Ops o;
-    edge_flux<SOLVER, FZ>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, (int)((meta >> 15) & 3u), erec, o);
+    constexpr bool kSurface = SHARED_STATE || !DEPTHS;  // the multi-step kernel has the depths in an array of their own
+    edge_flux<SOLVER, FZ, kSurface>(n1, n2, QL, QR, dL, dR, sqL, sqR, yL, yR, drytol, fL, fR, (int)((meta >> 15) & 3u),
+                                    erec, o);
     if (!o.ok) return kRedo;
     if (lin) {
         M.upd[(0 * 3 + iL) * T + sl] = fL.h;
