@@ -1758,6 +1758,7 @@ int swe_set_fault_injection(swe_ctx* c, int32_t kind) {
     if (kind < SWE_INJECT_NONE || kind > SWE_INJECT_REFUSED_LAUNCH)
         return set_error(SWE_E_INVALID, "unknown fault injection %d", kind);
     c->inject = kind;
+    drop_graphs(c);  // what they were captured with stays in them
     return SWE_OK;
 }
 

@@ -61,3 +61,24 @@ def test_a_refused_launch_is_made_step_by_step(swe_lib, oracle_lib, graph):
         assert ctx.launch_count(4) == 1
     finally:
         ctx.close()
+
+
+def test_graphs_do_not_outlive_an_injection(swe_lib, oracle_lib):
+    g, cfg = _grid(9, 0, "fwave", "slip")
+    L = _lib.load()
+    ctx = _context(g, cfg)
+    try:
+        _lib.check(L.swe_set_fault_injection(ctx.ptr, MEETING))
+        ctx.traverse_graph(2)
+        with pytest.raises(_lib.SweError):
+            ctx.synchronize()
+        ctx.upload_state(g.h, g.hu, g.hv, g.b)
+        ctx.set_time(0.0, g.r_dt)
+        _lib.check(L.swe_set_fault_injection(ctx.ptr, NONE))
+        S, P = omp_state(g.mesh, g), oracle_params(cfg)
+        S.steps(P, 2)
+        ctx.traverse_graph(2)
+        ctx.synchronize()
+        _compare(ctx, S, "after the injection")
+    finally:
+        ctx.close()
