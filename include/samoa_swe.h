@@ -141,11 +141,12 @@ int swe_last_error(char* buf, size_t n);
  * memory per cell, 22 with staging depth 2, at most 227 KB in all) and threads
  * per block (multiple of 32, 64..256); 0 keeps
  * the current value, but threads that were never set are 128 with a segment
- * length set here. A mesh upload or this call rebuilds the segment task lists. Until a segment length is set
- * here, each mesh upload picks it by size: 384 cells on large meshes and for
- * ensembles, 256 on middling ones (where the flux set before the upload and the
- * size decide), and on meshes that fit the GPU at once two segments per SM (at
- * least 64 cells); it then picks the threads too, unless they were set. */
+ * length set here. A mesh upload or this call rebuilds the segment task lists.
+ * Until a segment length is set here, each mesh upload picks it by size: 384
+ * cells on large meshes and ensembles, 256 on middling ones (where the flux set
+ * before the upload and the size decide), and where all instances fit the GPU at
+ * once at most two segments per SM (of at least 64 cells); it then picks the
+ * threads too, unless they were set. */
 int swe_set_tiling(swe_ctx* ctx, int32_t segment_cells, int32_t block_threads);
 
 /* Staging depth of the step kernel: 1 = a CTA stages a segment's state into
@@ -161,8 +162,10 @@ int swe_set_staging(swe_ctx* ctx, int32_t depth);
  * rounded separately, in the reference's evaluation order, so results are bit
  * identical to a strict-IEEE CPU evaluation of the reference step. FMA: the
  * same kernel with multiply-adds fused by the compiler; faster on GB300's FP64
- * pipe, results within a few ulps per step of STRICT (not bit identical). No
- * reference counterpart (the reference's precision is a compile-time choice,
+ * pipe, results within a few ulps per step of STRICT (not bit identical; nor are
+ * the routes of a step to one another, each of which the compiler fuses by
+ * itself: one step or many per call, the modes of swe_set_cross_pass,
+ * swe_step_host). No reference counterpart (the reference's precision is a compile-time choice,
  * SConstruct:272-278). Adjoint steps always use STRICT. */
 #define SWE_ARITH_STRICT 0
 #define SWE_ARITH_FMA 1
@@ -175,8 +178,9 @@ int swe_get_tiling(swe_ctx* ctx, int32_t* segment_cells, int32_t* block_threads)
  * PASS for steps on device-resident state of 2^20 cells and more, INKERNEL for
  * smaller meshes and for swe_step_host, whose state is in host memory; and many
  * steps of one call on a mesh whose segments all fit the GPU at once run in one
- * launch that keeps each segment's state on its SM. The results are bit
- * identical. No reference counterpart. */
+ * launch that keeps each segment's state on its SM (the SMs of the context's
+ * stream, where that is a green context's). With SWE_ARITH_STRICT the results are
+ * bit identical. No reference counterpart. */
 #define SWE_CROSS_AUTO 0
 #define SWE_CROSS_PASS 1
 #define SWE_CROSS_INKERNEL 2

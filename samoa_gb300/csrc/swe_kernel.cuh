@@ -1,19 +1,21 @@
 // The fused SWE time-step kernel (sm_103a).
 //
-// One launch = one explicit Euler time step of every instance of the context
-// (one instance for the plain step, many for an ensemble) of
-// t_swe_euler_timestep_traversal (src/SWE/SWE_euler_timestep.f90). Cells are
-// cut into segments of consecutive cells of the space-filling curve; a
-// segment never spans two instances. A persistent grid of CTAs walks the
-// segments; per segment:
+// One launch of step_kernel = one explicit Euler time step of every instance of
+// the context (one instance for the plain step, many for an ensemble) of
+// t_swe_euler_timestep_traversal (src/SWE/SWE_euler_timestep.f90); on meshes
+// that fit the GPU at once a launch of multi_step_kernel (at the end of this
+// file) runs many. Cells are cut into segments of consecutive cells of the
+// space-filling curve; a segment never spans two instances. A persistent grid
+// of CTAs walks the segments; per segment:
 //   1. stage h, hu, hv, b into shared memory with 1-D TMA bulk copies
 //      (cp.async.bulk, completion on an mbarrier with a bounded wait), then
 //      the depth h - b and sqrt(g * depth) once per cell;
 //   2. evaluate each edge task once: the Riemann solver with the first-touched
 //      cell as the left side writes left/right updates into per-(cell, local
 //      edge) slots in shared memory, each slot written by one task, no atomics;
-//      an edge between two segments is evaluated by both CTAs, each keeping
-//      its own side, so no CTA waits for another;
+//      an edge between two segments is evaluated once by cross_edges_kernel
+//      before, or by both CTAs, each keeping its own side, so that no CTA waits
+//      for another;
 //   3. update each cell from its three slots in local edge index order, clamp
 //      wet/dry, write the other state buffer, set the refinement flag, fold
 //      volume / sum(len * speed) into a running minimum;
